@@ -86,7 +86,7 @@ class Context:
         check(self.handle, self._L.dg_ctx_profile(self.handle, 1 if enable else 0), "dg_ctx_profile")
 
     def set_matvec_form(self, form: str):
-        """FP32 element loop form: "runs" (default) or "pairs"."""
+        """Element loop form, "runs" or "pairs": one loop now serves both."""
         check(self.handle, self._L.dg_ctx_set_matvec_form(self.handle, {"runs": 0, "pairs": 1}[form]),
               "set_matvec_form")
 
@@ -669,7 +669,7 @@ class MultiGrid:
 
     def matvec(self, level: int, x, precision: int = 64):
         """DirichletJacobianMatMult on a level: FP64 (64), FP32 (32), or FP64
-        vectors in double-single arithmetic (48)."""
+        vectors in 64-bit fixed point (48)."""
         n = self.sizes[level][1]
         return self._op(self.ctx._L.dg_mg_matvec, level, x, n, n, precision)
 
@@ -687,8 +687,8 @@ class MultiGrid:
         check(self.ctx.handle, self.ctx._L.dg_mg_set_smoother(self.handle, omega, nu_pre, nu_post), "set_smoother")
 
     def set_cg_operator(self, precision: int = 48, reliable_delta: float = 1e-3):
-        """The CG's operator q = A p with an FP32 V-cycle: double-single
-        arithmetic on FP64 vectors (48, the default), FP64 (64), or FP32
+        """The CG's operator q = A p with an FP32 V-cycle: 64-bit fixed
+        point on FP64 vectors (48, the default), FP64 (64), or FP32
         with FP64 residual replacement (32)."""
         check(self.ctx.handle, self.ctx._L.dg_mg_set_cg_operator(self.handle, precision, reliable_delta),
               "set_cg_operator")

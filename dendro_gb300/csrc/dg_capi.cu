@@ -172,13 +172,8 @@ int dg_ctx_destroy(dg_ctx ctx) {
   if (ctx->c.h_scratch) cudaFreeHost(ctx->c.h_scratch);
   if (ctx->c.d_sten64) cudaFree(ctx->c.d_sten64);
   if (ctx->c.d_sten32) cudaFree(ctx->c.d_sten32);
-  if (ctx->c.d_comb64) cudaFree(ctx->c.d_comb64);
-  if (ctx->c.d_comb32) cudaFree(ctx->c.d_comb32);
-  if (ctx->c.d_comb_ds) cudaFree(ctx->c.d_comb_ds);
-  if (ctx->c.d_comb_rowabs) cudaFree(ctx->c.d_comb_rowabs);
-  if (ctx->c.d_csten64) cudaFree(ctx->c.d_csten64);
-  if (ctx->c.d_csten32) cudaFree(ctx->c.d_csten32);
-  if (ctx->c.d_cperm) cudaFree(ctx->c.d_cperm);
+  for (dg::Context::DiagTable *t : {&ctx->c.dtab64, &ctx->c.dtab32})
+    if (t->p) cudaFree(t->p);
   if (ctx->c.d_etype_of) cudaFree(ctx->c.d_etype_of);
   if (ctx->c.d_etype_mask) cudaFree(ctx->c.d_etype_mask);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
@@ -246,8 +241,7 @@ int dg_ctx_profile_entry(dg_ctx ctx, int index, char *name, size_t name_len, dou
 
 int dg_ctx_set_matvec_form(dg_ctx ctx, int form) {
   if (!ctx || (form != 0 && form != 1)) return DG_ERR_INVALID_ARG;
-  ctx->c.matvec_form = form;
-  return DG_OK;
+  return DG_OK;  // one loop serves both (dg_elem.cuh)
 }
 
 int dg_dense_spd_inverse(dg_ctx ctx, float *X, size_t n) {
@@ -720,7 +714,7 @@ int dg_mg_level_octree(dg_ctx ctx, dg_mg mg, size_t level, uint32_t *xyzl, int d
 int dg_mg_matvec(dg_ctx ctx, dg_mg mg, size_t level, const void *in, void *out, int precision, int on_device) {
   if (!mg || level >= mg->mg.lv.size()) return DG_ERR_INVALID_ARG;
   const dg::MGLevel &L = mg->mg.lv[level];
-  const bool ds = precision == 48;  // FP64 vectors, double-single arithmetic
+  const bool ds = precision == 48;  // FP64 vectors, fixed-point arithmetic
   return level_op(ctx, mg, L.mesh.n_node, L.mesh.n_node, in, out, ds ? 64 : precision, on_device,
                   [&](dg::Context &c, const void *x, void *y) {
                     if (ds) dg::dirichlet_matvec_ds(c, L, (const double *)x, (double *)y);

@@ -24,7 +24,6 @@
 // and the TF32 truncation of lo are below 2^-21 of each product, so the
 // inverse keeps close to FP32 accuracy.
 #include "dg_mg.cuh"
-#include "dg_elem.cuh"
 
 #include <algorithm>
 
@@ -34,6 +33,17 @@ namespace {
 
 constexpr int GJB = 64;      // pivots per block
 constexpr int GJT = 64 + 4;  // shared tile row stride (floats)
+
+// two FP32 fused multiply-adds in one instruction (Blackwell f32x2)
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
 
 // ---- k_gj_diag: P = inv(X_KK) for one diagonal block (one CTA of 256
 // threads): thread t holds 16 entries of row t / 4 in registers.  Per pivot

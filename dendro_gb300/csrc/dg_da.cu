@@ -140,58 +140,6 @@ void ensure_stencils(Context &ctx) {
   ctx.d_sten32 = d32;
   ctx.d_etype_of = det;
   ctx.d_etype_mask = dem;
-  // canonical stencils: S(c,t) = S(0,t) relabelled by a cube symmetry
-  std::vector<double> c64(fsten_entries<double>(), 0.0);
-  std::vector<float> c32(fsten_entries<float>(), 0.0f);
-  std::vector<uint32_t> cperm(8 * 18);
-  for (int t = 0; t < 18; t++)
-    for (int q = 0; q < 64; q++) {
-      c64[t * fsten_stride<double>() + q] = lap[t * 64 + q];
-      c64[t * fsten_stride<double>() + 64 + q] = mass[t * 64 + q];
-      c32[t * fsten_stride<float>() + q] = (float)lap[t * 64 + q];
-      c32[t * fsten_stride<float>() + 64 + q] = (float)mass[t * 64 + q];
-    }
-  static const int axes[6][3] = {{0, 1, 2}, {0, 2, 1}, {1, 0, 2}, {1, 2, 0}, {2, 0, 1}, {2, 1, 0}};
-  for (int c = 0; c < 8; c++)
-    for (int t = 0; t < 18; t++) {
-      double best = 1e300;
-      uint32_t best_sig = 0;
-      for (int a = 0; a < 6; a++)
-        for (int fl = 0; fl < 8; fl++) {
-          int pk[8];
-          for (int k = 0; k < 8; k++) {
-            int nb = 0;
-            for (int i = 0; i < 3; i++) nb |= (((k >> axes[a][i]) & 1) ^ ((fl >> i) & 1)) << i;
-            pk[k] = nb;
-          }
-          double err = 0;
-          const int ct = c * 18 + t;
-          for (int k = 0; k < 8; k++)
-            for (int j = 0; j < 8; j++) {
-              err = std::max(err, std::fabs(lap[t * 64 + 8 * pk[k] + pk[j]] - lap[ct * 64 + 8 * k + j]));
-              err = std::max(err, std::fabs(mass[t * 64 + 8 * pk[k] + pk[j]] - mass[ct * 64 + 8 * k + j]));
-            }
-          if (err < best) {
-            best = err;
-            best_sig = 0;
-            for (int k = 0; k < 8; k++) best_sig |= (uint32_t)k << (3 * pk[k]);  // slot of relabelled vertex pk[k]
-          }
-        }
-      if (!(best <= 1e-12)) fail(DG_ERR_INTERNAL, "stencil tables: a (child, type) stencil has no canonical form");
-      cperm[c * 18 + t] = best_sig;
-    }
-  double *dc64 = nullptr;
-  float *dc32 = nullptr;
-  uint32_t *dcp = nullptr;
-  DG_CUDA(cudaMalloc((void **)&dc64, c64.size() * sizeof(double)));
-  DG_CUDA(cudaMalloc((void **)&dc32, c32.size() * sizeof(float)));
-  DG_CUDA(cudaMalloc((void **)&dcp, cperm.size() * sizeof(uint32_t)));
-  DG_CUDA(cudaMemcpy(dc64, c64.data(), c64.size() * sizeof(double), cudaMemcpyHostToDevice));
-  DG_CUDA(cudaMemcpy(dc32, c32.data(), c32.size() * sizeof(float), cudaMemcpyHostToDevice));
-  DG_CUDA(cudaMemcpy(dcp, cperm.data(), cperm.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-  ctx.d_csten64 = dc64;
-  ctx.d_csten32 = dc32;
-  ctx.d_cperm = dcp;
 }
 
 // ------------------------------------------------------------------------
@@ -391,439 +339,329 @@ __global__ void k_mesh_conn(const Key128 *__restrict__ keys, size_t n, const uin
 }
 
 // ------------------------------------------------------------------------
-// element loop tables: per patch, the (element, vertex) pairs grouped by node
+// element loop tables: families of siblings, their lattices, and the nodes
+// of each patch of families (layout: dg_elem.cuh)
 // ------------------------------------------------------------------------
-__global__ void k_node_incidence(const uint32_t *__restrict__ conn, size_t n8, uint32_t *__restrict__ cnt) {
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += stride) atomicAdd(&cnt[conn[i]], 1u);
-}
-
-// Bitonic sort of BLOCK * I keys held I per thread (key I*t + j in v[j] of
-// thread t), ascending.  Compare-exchanges with partners in the same thread
-// run in registers, those within a warp by shuffles, and only the strides
-// that cross warps go through shared memory (`stage`, BLOCK * I keys).
-template <typename K>
-__device__ __forceinline__ K keep_of(K mine, K other, bool keep_min) {
-  return keep_min ? (other < mine ? other : mine) : (other > mine ? other : mine);
-}
-
-template <typename K, int I, int BLOCK>
-__device__ void block_sort_regs(K (&v)[I], K *stage) {
-  constexpr int N = BLOCK * I;
-  const int t = threadIdx.x;
-  for (int s = 2; s <= N; s <<= 1) {
-    int d = s >> 1;
-    for (; d >= 32 * I; d >>= 1) {  // across warps
-#pragma unroll
-      for (int j = 0; j < I; j++) stage[I * t + j] = v[j];
-      __syncthreads();
-#pragma unroll
-      for (int j = 0; j < I; j++) {
-        const int i = I * t + j;
-        v[j] = keep_of(v[j], stage[i ^ d], ((i & d) == 0) == ((i & s) == 0));
-      }
-      __syncthreads();
-    }
-    for (; d >= I; d >>= 1) {  // within a warp
-#pragma unroll
-      for (int j = 0; j < I; j++) {
-        const int i = I * t + j;
-        const K o = __shfl_xor_sync(0xffffffffu, v[j], d / I);
-        v[j] = keep_of(v[j], o, ((i & d) == 0) == ((i & s) == 0));
-      }
-    }
-#pragma unroll
-    for (int dd = I / 2; dd > 0; dd >>= 1) {  // within the thread
-      if (dd < s) {
-#pragma unroll
-        for (int j = 0; j < I; j++) {
-          if (j & dd) continue;
-          const bool up = (((I * t + j) & s) == 0);
-          const K a = v[j], b = v[j | dd];
-          if ((a > b) == up) {
-            v[j] = b;
-            v[j | dd] = a;
-          }
+// a family's first element: the lowest child of its parent that is a leaf
+// (children before e: e - 1 in the usual case, else look-ups)
+__global__ void k_family_heads(const Key128 *__restrict__ keys, size_t n, const uint32_t *__restrict__ tab,
+                               uint64_t mask, unsigned D, uint32_t *__restrict__ head) {
+  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const Key128 ke = keys[e];
+  const unsigned l = tag_level(ke);
+  bool first = true;
+  if (l > 0) {
+    const Key128 a = tag_anchor(ke);
+    const unsigned sh = 3 * (D - l);
+    const unsigned c = (unsigned)(key_shr(a, sh).lo & 7u);
+    if (c > 0 && e > 0) {
+      const Key128 kp = keys[e - 1];
+      first = !(tag_level(kp) == l && key_eq(key_shr(tag_anchor(kp), sh + 3), key_shr(a, sh + 3)));
+      if (first) {
+        for (unsigned q = 0; q < c && first; q++) {
+          const uint32_t j =
+              anchor_find(keys, tab, mask, key_xor(a, key_shl(Key128{(uint64_t)(q ^ c), 0}, sh)));
+          first = !(j != AH_EMPTY && tag_level(keys[j]) == l);
         }
       }
     }
   }
+  head[e] = first ? 1u : 0u;
 }
 
-// one block per patch: the patch's elements ordered by (type, level, index);
-// then its (element, vertex) pairs grouped by node with a shared-memory hash
-// table (one run per distinct node; the pairs of a run ordered by slot, so
-// sums over a run are reproducible), run starts, and whether each run holds
-// every pair of its node in the mesh.  The element loop needs the pairs of a
-// node together, not the runs in any order.
-constexpr int PS_HT = PATCH_ENT;  // hash slots (>= distinct nodes of a patch)
-constexpr uint32_t PS_EMPTY = 0xffffffffu;
+__global__ void k_family_list(const uint32_t *__restrict__ head, const uint32_t *__restrict__ pos, size_t n,
+                              uint32_t *__restrict__ first) {
+  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < n && head[e]) first[pos[e]] = (uint32_t)e;
+}
 
-struct PatchSortSmem {
-  uint32_t hkey[PS_HT];        // node of each hash slot
-  uint16_t hrun[PS_HT];        // run of each hash slot
-  uint16_t hcnt[PS_HT];        // pairs per hash slot, then placement cursor per run
-  uint16_t roff[PATCH_ENT + 1];  // run offsets
-  uint32_t rnode[PATCH_ENT];   // node of each run
-  uint16_t ent[PATCH_ENT];     // slots grouped by run
-  uint8_t rflag[PATCH_ENT];    // bit 0: a run starts here; bit 1 (per run): complete
-  uint32_t ek[PATCH];
-  uint16_t rank[PATCH];
+// One block per patch.  Thread t finds family t's children (the element after
+// a child is its next sibling, or a look-up tells); complete families move to
+// the front; then thread t builds lattice t from the elements' node ids and
+// the nodes are numbered through a shared-memory hash table.  The nodes are
+// numbered in claim order, for the element loop's shared-memory banks (number
+// mod 32; shared FP32 atomic adds at random banks cost about four times those
+// at distinct banks, measured 13.7 against 3.3 cycles per warp instruction on
+// an SM): the nodes that a warp claims at one lattice point take consecutive
+// numbers, so they fall on distinct banks when that warp touches them
+// together.  Patches append their nodes to one list (any order).
+constexpr int PF_HT = 4096;  // hash slots, more than FAM_MAX_RUN
+constexpr uint32_t PF_EMPTY = 0xffffffffu;
+static_assert(FAM_MAX_RUN < PF_HT, "a patch's nodes must fit the hash table");
+
+struct PatchFamSmem {
+  uint32_t hkey[PF_HT];          // node of each hash slot
+  uint32_t node[FAM_MAX_RUN];    // node of each number
+  uint16_t num[PF_HT];           // number of each hash slot
+  uint32_t child[8][FAM];        // elements of the reordered families
+  uint32_t cmask[FAM];
+  uint32_t minlev;
+  int counter;
+  unsigned long long base;
 };
 
-__global__ void __launch_bounds__(PATCH) k_patch_sort(const uint32_t *__restrict__ conn,
-                                                      const uint32_t *__restrict__ meta, size_t E,
-                                                      const uint32_t *__restrict__ node_pairs,
-                                                      uint16_t *__restrict__ pinc, uint16_t *__restrict__ pexc,
-                                                      uint32_t *__restrict__ pmeta, uint16_t *__restrict__ pkeys,
-                                                      uint16_t *__restrict__ pkcount, uint32_t *__restrict__ run_node,
-                                                      uint32_t *__restrict__ n_run, uint16_t *__restrict__ pperm) {
-  extern __shared__ __align__(16) unsigned char ps_raw[];
-  PatchSortSmem &S = *reinterpret_cast<PatchSortSmem *>(ps_raw);
-  const int tid = threadIdx.x;
-  const size_t p = blockIdx.x;
-  const size_t e0 = p * PATCH;
-  const int ne = (int)((E - e0) < (size_t)PATCH ? (E - e0) : (size_t)PATCH);
-  for (int i = tid; i < PS_HT; i += PATCH) {
-    S.hkey[i] = PS_EMPTY;
-    S.hcnt[i] = 0;
-  }
-  for (int i = tid; i < PATCH_ENT; i += PATCH) S.rflag[i] = 0;
-  // element order: (type, level, index); missing elements last
-  {
-    uint32_t k1[1];
-    if (tid < ne) {
-      const uint32_t me = meta[e0 + tid];
-      k1[0] = ((me >> 24) << 5 | (me & 31u)) << 9 | (uint32_t)tid;
-    } else {
-      k1[0] = 0xffffffffu;
-    }
-    block_sort_regs<uint32_t, 1, PATCH>(k1, S.ek);
-    __syncthreads();
-    S.ek[tid] = k1[0];
-    __syncthreads();
-  }
-  // (type, level) groups of the ordered elements: the patch's stencil keys
-  const uint32_t grp = S.ek[tid] >> 9;
-  const int gstart = tid < ne && (tid == 0 || (S.ek[tid - 1] >> 9) != grp) ? 1 : 0;
-  int nkeys;
-  const int kidx = block_excl_scan<int, PATCH>(gstart, nkeys) + gstart - 1;
-  if (tid < ne) {
-    const uint32_t eo = S.ek[tid] & (PATCH - 1);
-    S.rank[eo] = (uint16_t)tid;
-    if (pperm) pperm[p * PATCH + tid] = (uint16_t)eo;
-    const uint32_t mo = meta[e0 + eo];
-    pmeta[p * PATCH + tid] = (mo & 0xff00ffffu) | (uint32_t)(kidx < PKEY_MAX ? kidx : 0) << 16;
-    if (gstart && kidx < PKEY_MAX) pkeys[p * PKEY_MAX + kidx] = (uint16_t)grp;
-  }
-  if (tid == 0) pkcount[p] = (uint16_t)nkeys;
-  __syncthreads();
-  // 1. one hash slot per distinct node; pairs counted per slot
-  uint16_t hpos[8];
-  uint16_t slot[8];
-  const bool have = tid < ne;
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    hpos[k] = 0;
-    slot[k] = (uint16_t)(k * PATCH + (have ? S.rank[tid] : 0));
-    if (have) {
-      const uint32_t g = conn[(size_t)k * E + e0 + tid];
-      uint32_t h = (g * 2654435761u) >> (32 - 12);  // PS_HT = 2^12
-      for (int probe = 0; probe < PS_HT; probe++) {
-        const uint32_t cur = atomicCAS(&S.hkey[h], PS_EMPTY, g);
-        if (cur == PS_EMPTY || cur == g) break;
-        h = (h + 1) & (PS_HT - 1);
-      }
-      hpos[k] = (uint16_t)h;
-      atomicAdd(reinterpret_cast<unsigned int *>(&S.hcnt[h & ~1u]), (h & 1u) ? 0x10000u : 1u);
-    }
-  }
-  __syncthreads();
-  // 2. runs in hash-slot order: run index and offset of each occupied slot
-  {
-    constexpr int PER = PS_HT / PATCH;  // slots per thread
-    int nr = 0, np = 0;
-#pragma unroll
-    for (int q = 0; q < PER; q++) {
-      const int h = tid * PER + q;
-      nr += S.hkey[h] != PS_EMPTY ? 1 : 0;
-      np += S.hcnt[h];
-    }
-    int tot_runs, tot_pairs;
-    int ur = block_excl_scan<int, PATCH>(nr, tot_runs);
-    int up = block_excl_scan<int, PATCH>(np, tot_pairs);
-#pragma unroll
-    for (int q = 0; q < PER; q++) {
-      const int h = tid * PER + q;
-      if (S.hkey[h] != PS_EMPTY) {
-        S.hrun[h] = (uint16_t)ur;
-        S.roff[ur] = (uint16_t)up;
-        S.rnode[ur] = S.hkey[h];
-        S.rflag[up] = 1;
-        up += S.hcnt[h];
-        ur++;
-      }
-    }
-    if (tid == 0) {
-      S.roff[tot_runs] = (uint16_t)tot_pairs;
-      n_run[p] = (uint32_t)tot_runs;
-    }
-    __syncthreads();
-    for (int i = tid; i < PS_HT; i += PATCH) S.hcnt[i] = 0;  // becomes the placement cursor per run
-    __syncthreads();
-    // 3. place the pairs (any order), then order each run by slot
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-      if (have) {
-        const int u = S.hrun[hpos[k]];
-        const unsigned old = atomicAdd(reinterpret_cast<unsigned int *>(&S.hcnt[u & ~1]), (u & 1) ? 0x10000u : 1u);
-        const int at = (int)S.roff[u] + (int)((old >> ((u & 1) ? 16 : 0)) & 0xffffu);
-        S.ent[at] = slot[k];
-      }
-    __syncthreads();
-    for (int u = tid; u < tot_runs; u += PATCH) {
-      const int b = S.roff[u], e = S.roff[u + 1];
-      for (int i = b + 1; i < e; i++) {  // insertion sort: runs are short
-        const uint16_t v = S.ent[i];
-        int j = i - 1;
-        while (j >= b && S.ent[j] > v) {
-          S.ent[j + 1] = S.ent[j];
-          j--;
-        }
-        S.ent[j + 1] = v;
-      }
-      const uint32_t g = S.rnode[u];
-      run_node[p * PATCH_ENT + u] = g;
-      if ((uint32_t)(e - b) == node_pairs[g]) S.rflag[b] |= 2;
-    }
-    __syncthreads();
-  }
-  // 4. the packed entries, 8 per thread, and runs starting before each thread
-  const int nent = 8 * ne;
-  int nst = 0;
-#pragma unroll
-  for (int j = 0; j < 8; j++) nst += (8 * tid + j < nent && (S.rflag[8 * tid + j] & 1)) ? 1 : 0;
-  int total;
-  const int ex = block_excl_scan<int, PATCH>(nst, total);
-  pexc[p * PATCH + tid] = (uint16_t)ex;
-  uint32_t e[8];
-  uint8_t comp = 0;
-  if (ex > 0) {  // the run in progress at this thread's first pair started earlier
-    int i = 8 * tid;
-    while (i > 0 && !(S.rflag[i] & 1)) i--;
-    comp = S.rflag[i] & 2;
-  }
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    const int i = 8 * tid + j;
-    e[j] = 0;
-    if (i < nent) {
-      const uint8_t f = S.rflag[i];
-      if (f & 1) comp = f & 2;
-      e[j] = (uint32_t)S.ent[i] | ((f & 1) ? ENT_START : 0u) | (comp ? ENT_COMPLETE : 0u);
-    }
-  }
-  reinterpret_cast<uint4 *>(pinc + p * PATCH_ENT)[tid] =
-      make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
-}
-
-__global__ void k_patch_nodes(const uint32_t *__restrict__ run_node, const uint32_t *__restrict__ n_run,
-                              const uint64_t *__restrict__ poff, uint32_t *__restrict__ pnode) {
-  const size_t p = blockIdx.x;
-  const uint32_t nr = n_run[p];
-  for (uint32_t i = threadIdx.x; i < nr; i += blockDim.x) pnode[poff[p] + i] = run_node[p * PATCH_ENT + i];
-}
-
-// run-form tables from the pair tables: every pair's run index (run starts
-// counted from pexc) per slot in shared memory, then per (type, level)
-// position the runs of its vertices in the canonical order of its stencil
-// (vertex cperm[c][t] digit m at canonical position m), and per run its node
-// with the complete flag of its pairs and the domain-boundary flag of the
-// node (the Dirichlet rows and columns).
-// The runs are numbered in claim order, for the element loop's shared
-// memory banks (a run's index mod 32; shared FP32 atomic adds at random
-// banks cost about four times those at distinct banks, measured 13.7
-// against 3.3 cycles per warp instruction on an SM): in round m = 0..7
-// every element claims the run at its canonical position m if no element
-// has yet, and the runs a warp claims in one round take consecutive
-// indices, so that they fall on distinct banks when that warp touches them
-// together.  (A greedy colouring that also avoided the banks of a run's
-// other groups gave the same element-loop time at 4 to 7 times the cost.)
-__global__ void __launch_bounds__(PATCH) k_patch_runs(const uint16_t *__restrict__ pinc,
-                                                      const uint16_t *__restrict__ pexc,
-                                                      const uint32_t *__restrict__ pnode,
-                                                      const uint64_t *__restrict__ poff,
-                                                      const uint32_t *__restrict__ pmeta,
-                                                      const uint32_t *__restrict__ cperm, size_t E,
-                                                      const uint32_t *__restrict__ node_xyz, size_t V,
-                                                      uint32_t dom, uint4 *__restrict__ plid,
-                                                      uint32_t *__restrict__ prun) {
-  __shared__ uint16_t run_of[PATCH_ENT];
-  __shared__ unsigned short newidx[PATCH_ENT];
-  __shared__ uint32_t word[PATCH_ENT];
-  __shared__ int counter;
-  const size_t p = blockIdx.x;
+__global__ void __launch_bounds__(FAM)
+    k_patch_families(const Key128 *__restrict__ keys, size_t n, const uint32_t *__restrict__ tab, uint64_t tmask,
+                     unsigned D, const uint32_t *__restrict__ first, size_t n_fam, const uint32_t *__restrict__ meta,
+                     const uint32_t *__restrict__ conn, uint4 *__restrict__ fam, uint4 *__restrict__ pinfo,
+                     uint32_t *__restrict__ fchild, uint32_t *__restrict__ run_node,
+                     uint32_t *__restrict__ node_patches, unsigned long long *__restrict__ n_run,
+                     uint32_t *__restrict__ max_run) {
+  extern __shared__ __align__(16) unsigned char pf_raw[];
+  PatchFamSmem &S = *reinterpret_cast<PatchFamSmem *>(pf_raw);
   const int t = threadIdx.x, lane = t & 31;
-  const size_t e0 = p * PATCH;
-  const int ne = (int)((E - e0) < (size_t)PATCH ? (E - e0) : (size_t)PATCH);
-  const uint64_t ub = poff[p];
-  const int nr = (int)(poff[p + 1] - ub);
-  for (int i = t; i < nr; i += PATCH) newidx[i] = 0xffff;
-  if (t == 0) counter = 0;
-  if (t < ne) {
-    int r = (int)pexc[p * PATCH + t] - 1;
-    for (int i = 8 * t; i < 8 * t + 8; i++) {
-      const uint32_t ent = pinc[p * PATCH_ENT + i];
-      if (ent & ENT_START) {
-        r++;
-        const uint32_t g = pnode[ub + r];
-        const uint32_t cx = node_xyz[g], cy = node_xyz[V + g], cz = node_xyz[2 * V + g];
-        const bool on_bdy = cx == 0 || cy == 0 || cz == 0 || cx == dom || cy == dom || cz == dom;
-        word[r] = g | ((ent & ENT_COMPLETE) ? PRUN_COMPLETE : 0u) | (on_bdy ? PRUN_BDY : 0u);
+  const size_t p = blockIdx.x, f = p * FAM + t;
+  const bool have = f < n_fam;
+  for (int i = t; i < PF_HT; i += FAM) S.hkey[i] = PF_EMPTY;
+  if (t == 0) {
+    S.counter = 0;
+    S.minlev = 31;
+  }
+  // 1. the family's children
+  uint32_t el[8], mask = 0;
+#pragma unroll
+  for (int c = 0; c < 8; c++) el[c] = 0;
+  if (have) {
+    const uint32_t e0 = first[f];
+    const Key128 a = tag_anchor(keys[e0]);
+    const unsigned l = tag_level(keys[e0]);
+    if (l == 0) {
+      el[0] = e0;
+      mask = 1;
+    } else {
+      const unsigned sh = 3 * (D - l);
+      const unsigned c0 = (unsigned)(key_shr(a, sh).lo & 7u);
+      const Key128 par = key_shr(a, sh + 3);
+      uint32_t prev = e0;
+#pragma unroll
+      for (unsigned c = 0; c < 8; c++) {
+        if (c < c0) continue;
+        uint32_t e = c == c0 ? e0 : prev + 1;
+        bool ok = c == c0;
+        if (!ok && e < n) {
+          const Key128 k = keys[e];
+          const Key128 s = key_shr(tag_anchor(k), sh);
+          ok = tag_level(k) == l && (unsigned)(s.lo & 7u) == c && key_eq(key_shr(s, 3), par);
+        }
+        if (!ok) {
+          e = anchor_find(keys, tab, tmask, key_xor(a, key_shl(Key128{(uint64_t)(c ^ c0), 0}, sh)));
+          ok = e != AH_EMPTY && tag_level(keys[e]) == l;
+        }
+        if (ok) {
+          el[c] = e;
+          mask |= 1u << c;
+          prev = e;
+        }
       }
-      run_of[ent & ENT_SLOT] = (uint16_t)r;
+    }
+  }
+  // 2. complete families first
+  int n_whole;
+  const int whole = have && mask == 255u ? 1 : 0;
+  const int before = block_excl_scan<int, FAM>(whole, n_whole);
+  const int at = whole ? before : n_whole + (t - before);
+  S.cmask[at] = mask;
+#pragma unroll
+  for (int c = 0; c < 8; c++) S.child[c][at] = el[c];
+  __syncthreads();
+  mask = S.cmask[t];
+#pragma unroll
+  for (int c = 0; c < 8; c++) el[c] = S.child[c][t];
+  // 3. the lattice: node ids and hanging points
+  uint32_t lat[27], hang = 0, lev = 0;
+#pragma unroll
+  for (int i = 0; i < 27; i++) lat[i] = PF_EMPTY;
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    if (!(mask >> c & 1u)) continue;
+    const uint32_t me = meta[el[c]];
+    lev = me & 255u;
+    const uint32_t hm = me >> 16 & 255u;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int bit = hang_bit(lat_vertex(c, k));
+      if (bit >= 0 && (hm >> k & 1u)) {
+        hang |= 1u << (bit & 31);
+        if (lat[lat_corner(k)] == PF_EMPTY) lat[lat_corner(k)] = conn[(size_t)k * n + el[c]];
+      } else if (lat[lat_vertex(c, k)] == PF_EMPTY) {
+        lat[lat_vertex(c, k)] = conn[(size_t)k * n + el[c]];
+      }
+    }
+  }
+  if (mask) atomicMin(&S.minlev, lev);
+  if (have) {
+    uint4 *fc = reinterpret_cast<uint4 *>(fchild + 8 * f);
+    fc[0] = make_uint4(el[0], el[1], el[2], el[3]);
+    fc[1] = make_uint4(el[4], el[5], el[6], el[7]);
+  }
+  // 4. number the nodes
+  uint16_t slot[27];
+#pragma unroll
+  for (int i = 0; i < 27; i++) {
+    const uint32_t g = lat[i];
+    uint32_t h = (g * 2654435761u) >> (32 - 12);  // PF_HT = 2^12
+    bool won = false;
+    if (g != PF_EMPTY) {
+      for (int probe = 0; probe < PF_HT; probe++) {
+        const uint32_t cur = atomicCAS(&S.hkey[h], PF_EMPTY, g);
+        won = cur == PF_EMPTY;
+        if (won || cur == g) break;
+        h = (h + 1) & (PF_HT - 1);
+      }
+    }
+    slot[i] = (uint16_t)h;
+    const unsigned claims = __ballot_sync(0xffffffffu, won);
+    if (claims) {
+      const int leader = __ffs(claims) - 1;
+      int at0 = 0;
+      if (lane == leader) at0 = atomicAdd(&S.counter, __popc(claims));
+      at0 = __shfl_sync(0xffffffffu, at0, leader);
+      if (won) {
+        const int u = at0 + __popc(claims & ((1u << lane) - 1u));
+        S.num[h] = (uint16_t)(u + 1);
+        S.node[u] = g;
+      }
     }
   }
   __syncthreads();
-  uint32_t lid[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  if (t < ne) {
-    const uint32_t me = pmeta[p * PATCH + t];
-    const uint32_t sig = cperm[((me >> 8) & 7u) * 18 + (me >> 24)];
-#pragma unroll
-    for (int m = 0; m < 8; m++) lid[m] = run_of[((sig >> (3 * m)) & 7u) * PATCH + t];
+  const int nr = S.counter;
+  if (t == 0) {
+    S.base = atomicAdd(n_run, (unsigned long long)nr);
+    atomicMax(max_run, (uint32_t)nr);
+    pinfo[p] = make_uint4((uint32_t)S.base, (uint32_t)(S.base >> 32), (uint32_t)nr, S.minlev);
   }
-#pragma unroll 1
-  for (int m = 0; m < 8; m++) {
-    uint32_t r = 0;
+  uint32_t w[16];
 #pragma unroll
-    for (int k = 0; k < 8; k++) r = k == m ? lid[k] : r;
-    const bool won = t < ne && atomicCAS(&newidx[r], (unsigned short)0xffff, (unsigned short)0xfffe) == 0xffff;
-    const unsigned bal = __ballot_sync(0xffffffffu, won);
-    if (bal) {
-      const int leader = __ffs(bal) - 1;
-      int base = 0;
-      if (lane == leader) base = atomicAdd(&counter, __popc(bal));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (won) newidx[r] = (unsigned short)(base + __popc(bal & ((1u << lane) - 1u)));
-    }
-    __syncthreads();
-  }
-  if (t < ne) {
-    uint32_t w[4];
+  for (int i = 0; i < 16; i++) w[i] = 0;
 #pragma unroll
-    for (int m = 0; m < 8; m += 2) w[m >> 1] = (uint32_t)newidx[lid[m]] | (uint32_t)newidx[lid[m + 1]] << 16;
-    plid[p * PATCH + t] = make_uint4(w[0], w[1], w[2], w[3]);
+  for (int i = 0; i < 27; i++)
+    if (lat[i] != PF_EMPTY) w[i >> 1] |= (uint32_t)S.num[slot[i]] << (i & 1 ? 16 : 0);
+  w[13] |= lev << 16;
+  w[14] = mask | (hang & 0xffffu) << 16;
+  w[15] = hang >> 16;
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    fam[(p * 4 + q) * FAM + t] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+  __syncthreads();
+  for (int u = t; u < nr; u += FAM) {
+    const uint32_t g = S.node[u];
+    run_node[S.base + u] = g;
+    atomicAdd(&node_patches[g], 1u);
   }
-  for (int u = t; u < nr; u += PATCH) prun[ub + newidx[u]] = word[u];
 }
 
-// conn from the patch tables: pair i of patch p belongs to the run counted
-// by the run starts up to i (pexc gives the count before pair 8t), its slot
-// names the vertex and the element's (type, level) position
-__global__ void __launch_bounds__(PATCH) k_conn_from_patches(const uint16_t *__restrict__ pinc,
-                                                             const uint16_t *__restrict__ pexc,
-                                                             const uint32_t *__restrict__ pnode,
-                                                             const uint64_t *__restrict__ poff,
-                                                             const uint16_t *__restrict__ pperm, size_t E,
-                                                             uint32_t *__restrict__ conn) {
+// the run words: node, "no other patch touches it", "on the domain boundary"
+__global__ void k_run_flags(const uint32_t *__restrict__ run_node, size_t n_run,
+                            const uint32_t *__restrict__ node_patches, const uint32_t *__restrict__ node_xyz, size_t V,
+                            uint32_t dom, uint32_t *__restrict__ prun) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_run) return;
+  const uint32_t g = run_node[i];
+  const uint32_t x = node_xyz[g], y = node_xyz[V + g], z = node_xyz[2 * V + g];
+  const bool bdy = x == 0 || y == 0 || z == 0 || x == dom || y == dom || z == dom;
+  prun[i] = g | (node_patches[g] == 1u ? PRUN_COMPLETE : 0u) | (bdy ? PRUN_BDY : 0u);
+}
+
+// conn from the family tables: child c's vertex k is its lattice point, or
+// the parent's corner k where that point hangs
+__global__ void __launch_bounds__(FAM) k_conn_from_families(const uint4 *__restrict__ fam,
+                                                            const uint4 *__restrict__ pinfo,
+                                                            const uint32_t *__restrict__ prun,
+                                                            const uint32_t *__restrict__ fchild, size_t n_fam,
+                                                            size_t E, uint32_t *__restrict__ conn) {
   const size_t p = blockIdx.x;
   const int t = threadIdx.x;
-  const size_t e0 = p * PATCH;
-  const int ne = (int)((E - e0) < (size_t)PATCH ? (E - e0) : (size_t)PATCH);
-  if (t >= ne) return;  // the pairs of a patch's ne elements are its first 8 ne entries
-  uint32_t r = pexc[p * PATCH + t];
-  const uint64_t ub = poff[p];
-  for (int i = 8 * t; i < 8 * t + 8; i++) {
-    const uint32_t ent = pinc[p * PATCH_ENT + i];
-    if (ent & ENT_START) r++;
-    const uint32_t slot = ent & ENT_SLOT;
-    const uint32_t v = slot / PATCH, pos = slot % PATCH;
-    conn[(size_t)v * E + e0 + pperm[p * PATCH + pos]] = pnode[ub + r - 1];
+  if (p * FAM + t >= n_fam) return;
+  const uint4 info = pinfo[p];
+  const uint32_t *run = prun + ((size_t)info.x | (size_t)info.y << 32);
+  uint4 w[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) w[q] = fam[(p * 4 + q) * FAM + t];
+  const uint32_t mask = fam_mask(w), hang = fam_hang(w);
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    if (!(mask >> c & 1u)) continue;
+    const size_t e = fchild[8 * (p * FAM + t) + c];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int bit = hang_bit(lat_vertex(c, k));
+      const bool h = bit >= 0 && (hang >> (bit & 31) & 1u);
+      const uint32_t u = h ? fam_u16(w, lat_corner(k)) : fam_u16(w, lat_vertex(c, k));
+      conn[(size_t)k * E + e] = run[u - 1] & PRUN_NODE;
+    }
   }
 }
 
 const uint32_t *mesh_conn(Context &ctx, const Mesh &m, DBuf<uint32_t> &tmp) {
   if (!m.compressed) return m.conn;
   tmp.alloc(8 * m.n_elem, ctx.stream);
-  ProfScope _prof(ctx, "da_conn_decode", (double)m.n_elem * (16 + 2 + 32) + (double)m.n_elem * 6);
-  k_conn_from_patches<<<(unsigned)m.n_patch, PATCH, 0, ctx.stream>>>(m.pinc, m.pexc, m.pnode, m.poff, m.pperm,
-                                                                     m.n_elem, tmp.get());
+  ProfScope _prof(ctx, "da_conn_decode", (double)m.n_elem * 32 + (double)m.n_fam * 96 + (double)m.n_run * 4);
+  k_conn_from_families<<<(unsigned)m.n_patch, FAM, 0, ctx.stream>>>(m.fam, m.pinfo, m.prun, m.fchild, m.n_fam,
+                                                                    m.n_elem, tmp.get());
   DG_LAUNCH_CHECK();
   return tmp.get();
 }
 
 size_t mesh_bytes(const Mesh &m) {
-  const size_t E = m.n_elem, V = m.n_node, np = m.n_patch;
-  size_t runs = 0;
-  if (np && m.poff) {
-    uint64_t r = 0;
-    if (cudaMemcpy(&r, m.poff + np, sizeof(uint64_t), cudaMemcpyDeviceToHost) == cudaSuccess) runs = r;
-  }
-  size_t b = E * 4 + V * 12;                                    // meta, node coordinates
-  if (m.conn) b += 8 * E * 4;                                   // conn
-  b += np * (PATCH_ENT * 2 + PATCH * 2 + PATCH * 4 + PKEY_MAX * 2 + 2) + (np + 1) * 8 + runs * 4;  // patches
-  if (m.pperm) b += np * PATCH * 2;
-  if (m.plid) b += np * PATCH * 16 + runs * 4;  // run-form tables
+  size_t b = m.n_elem * 4 + m.n_node * 12;  // meta, node coordinates
+  if (m.conn) b += 8 * m.n_elem * 4;
+  b += m.n_patch * (4 * FAM + 1) * sizeof(uint4) + m.n_run * 4 + m.n_fam * 32;  // family tables
   return b;
 }
 
-static void mesh_patches(Context &ctx, Mesh &m) {
+static void mesh_families(Context &ctx, Mesh &m, const Key128 *keys, const uint32_t *atab, uint64_t amask) {
   cudaStream_t s = ctx.stream;
-  const size_t n = m.n_elem, np = (n + PATCH - 1) / PATCH;
+  const size_t n = m.n_elem;
   if (m.n_node >= (size_t)PRUN_BDY) fail(DG_ERR_INVALID_ARG, "DA: too many nodes for the element loop tables");
-  DBuf<uint32_t> pairs(m.n_node, s), run_node(np * PATCH_ENT, s), n_run(np, s);
-  DBuf<uint16_t> pinc(np * PATCH_ENT, s), pexc(np * PATCH, s);
-  DBuf<uint32_t> pmeta(np * PATCH, s);
-  DBuf<uint16_t> pkeys(np * PKEY_MAX, s), pkcount(np, s);
-  DBuf<uint64_t> poff(np + 1, s);
-  DBuf<uint16_t> pperm(np * PATCH, s);
-  DG_CUDA(cudaMemsetAsync(pairs.get(), 0, m.n_node * sizeof(uint32_t), s));
+  DBuf<uint32_t> head(n, s), pos(n, s);
   {
-    ProfScope _prof(ctx, "da_node_pairs", (double)n * 8 * 8);
-    k_node_incidence<<<grid_for(8 * n, 256, (unsigned)ctx.num_sms * 16), 256, 0, s>>>(m.conn, 8 * n, pairs.get());
+    ProfScope _prof(ctx, "da_family_heads", (double)n * 20);
+    k_family_heads<<<grid_for(n, 256), 256, 0, s>>>(keys, n, atab, amask, m.max_depth, head.get());
     DG_LAUNCH_CHECK();
   }
+  uint32_t *d_total = reinterpret_cast<uint32_t *>(ctx.d_scratch);
+  exclusive_scan<uint32_t, uint32_t>(head.get(), pos.get(), n, d_total, s);
+  const size_t nf = read_scalar(ctx, d_total);
+  const size_t np = (nf + FAM - 1) / FAM;
+  DBuf<uint32_t> first(nf, s), fchild(8 * nf, s), run_node(27 * nf, s), npatch(m.n_node, s);
   {
-    ProfScope _prof(ctx, "da_patch_sort", (double)n * 8 * 14);
-    ensure_smem_attr(ctx, k_patch_sort, (int)sizeof(PatchSortSmem));
-    k_patch_sort<<<(unsigned)np, PATCH, sizeof(PatchSortSmem), s>>>(m.conn, m.meta, n, pairs.get(), pinc.get(),
-                                                                    pexc.get(), pmeta.get(), pkeys.get(),
-                                                                    pkcount.get(), run_node.get(), n_run.get(),
-                                                                    pperm.get());
+    ProfScope _prof(ctx, "da_family_list", (double)n * 8 + (double)nf * 4);
+    k_family_list<<<grid_for(n, 256), 256, 0, s>>>(head.get(), pos.get(), n, first.get());
     DG_LAUNCH_CHECK();
   }
-  exclusive_scan<uint32_t, uint64_t>(n_run.get(), poff.get(), np, poff.get() + np, s);
-  uint64_t nruns = 0;
-  DG_CUDA(cudaMemcpyAsync(&nruns, poff.get() + np, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+  head.release();
+  pos.release();
+  DBuf<uint4> fam(np * 4 * FAM, s), pinfo(np, s);
+  DG_CUDA(cudaMemsetAsync(npatch.get(), 0, m.n_node * sizeof(uint32_t), s));
+  unsigned long long *d_run = ctx.d_scratch;  // {nodes of all patches, most of one}
+  DG_CUDA(cudaMemsetAsync(d_run, 0, 2 * sizeof(unsigned long long), s));
+  {
+    ProfScope _prof(ctx, "da_patch_families", (double)n * (16 + 4 + 32) + (double)nf * 100);
+    ensure_smem_attr(ctx, k_patch_families, (int)sizeof(PatchFamSmem));
+    k_patch_families<<<(unsigned)np, FAM, sizeof(PatchFamSmem), s>>>(
+        keys, n, atab, amask, m.max_depth, first.get(), nf, m.meta, m.conn, fam.get(), pinfo.get(), fchild.get(),
+        run_node.get(), npatch.get(), d_run, reinterpret_cast<uint32_t *>(d_run + 1));
+    DG_LAUNCH_CHECK();
+  }
+  DG_CUDA(cudaMemcpyAsync(ctx.h_scratch, d_run, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
   DG_CUDA(cudaStreamSynchronize(s));
-  DBuf<uint32_t> pnode(nruns ? nruns : 1, s);
+  const size_t nruns = (size_t)ctx.h_scratch[0];
+  m.max_run = (int)(uint32_t)ctx.h_scratch[1];
+  DBuf<uint32_t> prun(nruns ? nruns : 1, s);
   {
-    ProfScope _prof(ctx, "da_patch_nodes", (double)nruns * 8);
-    k_patch_nodes<<<(unsigned)np, 256, 0, s>>>(run_node.get(), n_run.get(), poff.get(), pnode.get());
+    ProfScope _prof(ctx, "da_run_flags", (double)nruns * 24);
+    k_run_flags<<<grid_for(nruns, 256), 256, 0, s>>>(run_node.get(), nruns, npatch.get(), m.node_xyz, m.n_node,
+                                                     1u << m.max_depth, prun.get());
     DG_LAUNCH_CHECK();
   }
-  if (!m.compressed) {  // a compressed DA keeps the pair tables only
-    DBuf<uint4> plid(np * PATCH, s);
-    DBuf<uint32_t> prun(nruns ? nruns : 1, s);
-    {
-      ProfScope _prof(ctx, "da_patch_runs", (double)n * (16 + 2 + 4 + 16) + (double)nruns * 8);
-      k_patch_runs<<<(unsigned)np, PATCH, 0, s>>>(pinc.get(), pexc.get(), pnode.get(), poff.get(), pmeta.get(),
-                                                  ctx.d_cperm, n, m.node_xyz, m.n_node, 1u << m.max_depth,
-                                                  plid.get(), prun.get());
-      DG_LAUNCH_CHECK();
-    }
-    m.plid = plid.release_ptr();
-    m.prun = prun.release_ptr();
-  }
+  m.n_fam = nf;
   m.n_patch = np;
-  m.pinc = pinc.release_ptr();
-  m.pexc = pexc.release_ptr();
-  m.pmeta = pmeta.release_ptr();
-  m.pkeys = pkeys.release_ptr();
-  m.pkcount = pkcount.release_ptr();
-  m.pnode = pnode.release_ptr();
-  m.poff = poff.release_ptr();
-  m.pperm = pperm.release_ptr();
+  m.n_run = nruns;
+  m.fam = fam.release_ptr();
+  m.pinfo = pinfo.release_ptr();
+  m.prun = prun.release_ptr();
+  m.fchild = fchild.release_ptr();
 }
 
 void mesh_build(Context &ctx, const Octree &bal, Mesh &m, bool compress) {
@@ -875,8 +713,8 @@ void mesh_build(Context &ctx, const Octree &bal, Mesh &m, bool compress) {
   m.conn = conn.release_ptr();
   m.node_xyz = nxyz.release_ptr();
   m.compressed = compress;
-  mesh_patches(ctx, m);
-  if (compress) {  // the element loop needs only the patch tables
+  mesh_families(ctx, m, bal.keys, atab.get(), amask);
+  if (compress) {  // the element loop needs only the family tables
     cudaFreeAsync(m.conn, s);
     m.conn = nullptr;
   }
@@ -886,186 +724,86 @@ void mesh_free(Context &ctx, Mesh &m) {
   if (m.meta) cudaFreeAsync(m.meta, ctx.stream);
   if (m.conn) cudaFreeAsync(m.conn, ctx.stream);
   if (m.node_xyz) cudaFreeAsync(m.node_xyz, ctx.stream);
-  if (m.pinc) cudaFreeAsync(m.pinc, ctx.stream);
-  if (m.pexc) cudaFreeAsync(m.pexc, ctx.stream);
-  if (m.pmeta) cudaFreeAsync(m.pmeta, ctx.stream);
-  if (m.pkeys) cudaFreeAsync(m.pkeys, ctx.stream);
-  if (m.pkcount) cudaFreeAsync(m.pkcount, ctx.stream);
-  if (m.pnode) cudaFreeAsync(m.pnode, ctx.stream);
-  if (m.poff) cudaFreeAsync(m.poff, ctx.stream);
-  if (m.pperm) cudaFreeAsync(m.pperm, ctx.stream);
-  if (m.plid) cudaFreeAsync(m.plid, ctx.stream);
+  if (m.fam) cudaFreeAsync(m.fam, ctx.stream);
+  if (m.pinfo) cudaFreeAsync(m.pinfo, ctx.stream);
   if (m.prun) cudaFreeAsync(m.prun, ctx.stream);
+  if (m.fchild) cudaFreeAsync(m.fchild, ctx.stream);
   m = Mesh();
 }
 
 // ------------------------------------------------------------------------
 // element loop
 // ------------------------------------------------------------------------
+// the diagonal table of the element loop for these factors (kept on the
+// context until a call with others)
 template <typename T>
-const T *comb_table(Context &ctx, double lap_fac, double mass_fac) {
-  ensure_stencils(ctx);
+static const T *diag_table(Context &ctx, double lap_fac, double mass_fac) {
   const bool dbl = std::is_same<T, double>::value;
-  T **tab = reinterpret_cast<T **>(dbl ? (void *)&ctx.d_comb64 : (void *)&ctx.d_comb32);
-  double *f = dbl ? ctx.comb64_f : ctx.comb32_f;
-  bool &ok = dbl ? ctx.comb64_ok : ctx.comb32_ok;
-  if (!*tab) DG_CUDA(cudaMalloc((void **)tab, COMB_ENTRIES * sizeof(T)));
-  if (!ok || f[0] != lap_fac || f[1] != mass_fac) {
-    const T *cs = dbl ? reinterpret_cast<const T *>(ctx.d_csten64) : reinterpret_cast<const T *>(ctx.d_csten32);
-    k_comb_table<T><<<(COMB_ENTRIES + 255) / 256, 256, 0, ctx.stream>>>(cs, (T)lap_fac, (T)mass_fac, *tab);
+  Context::DiagTable &t = dbl ? ctx.dtab64 : ctx.dtab32;
+  if (!t.p) DG_CUDA(cudaMalloc(&t.p, DTAB_ENTRIES * sizeof(T)));
+  if (!t.ok || t.lap != lap_fac || t.mass != mass_fac) {
+    k_dtab<T><<<(DTAB_ENTRIES + 127) / 128, 128, 0, ctx.stream>>>(static_cast<T *>(t.p), lap_fac, mass_fac);
     DG_LAUNCH_CHECK();
-    f[0] = lap_fac;
-    f[1] = mass_fac;
-    ok = true;
+    t.lap = lap_fac;
+    t.mass = mass_fac;
+    t.ok = true;
   }
-  return *tab;
-}
-template const float *comb_table<float>(Context &, double, double);
-template const double *comb_table<double>(Context &, double, double);
-
-// the FP64 combined stencils as (hi, lo) FP32 pairs, per (type, level) laid
-// out by (row pair p, column j): (hi[2p][j], hi[2p+1][j], lo[2p][j], lo[2p+1][j])
-__global__ void k_split_pairs(const double *__restrict__ in, size_t n_stencils, float4 *__restrict__ out) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_stencils * 32) return;
-  const size_t st = i / 32;
-  const int p = (int)(i % 32) / 8, j = (int)(i % 8);
-  const double a = in[st * 64 + (2 * p) * 8 + j], b = in[st * 64 + (2 * p + 1) * 8 + j];
-  const float ah = __double2float_rn(a), bh = __double2float_rn(b);
-  out[i] = make_float4(ah, bh, __double2float_rn(a - (double)ah), __double2float_rn(b - (double)bh));
+  return static_cast<const T *>(t.p);
 }
 
-__global__ void k_row_abs_max(const double *__restrict__ comb, float *__restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;  // (type, level)
-  if (i >= COMB_ENTRIES / 64) return;
-  double m = 0.0;
-  for (int k = 0; k < 8; k++) {
-    double r = 0.0;
-    for (int j = 0; j < 8; j++) r += fabs(comb[i * 64 + 8 * k + j]);
-    m = fmax(m, r);
-  }
-  out[i] = __double2float_ru(m * (1.0 + 1e-12));
-}
-
-const float4 *comb_table_ds(Context &ctx, double lap_fac, double mass_fac) {
-  if (!ctx.d_comb_ds) DG_CUDA(cudaMalloc((void **)&ctx.d_comb_ds, COMB_ENTRIES / 2 * sizeof(float4)));
-  if (!ctx.d_comb_rowabs) DG_CUDA(cudaMalloc((void **)&ctx.d_comb_rowabs, COMB_ENTRIES / 64 * sizeof(float)));
-  if (!ctx.comb_ds_ok || ctx.comb_ds_f[0] != lap_fac || ctx.comb_ds_f[1] != mass_fac) {
-    const double *d = comb_table<double>(ctx, lap_fac, mass_fac);
-    k_split_pairs<<<(COMB_ENTRIES / 2 + 255) / 256, 256, 0, ctx.stream>>>(d, COMB_ENTRIES / 64, ctx.d_comb_ds);
-    DG_LAUNCH_CHECK();
-    k_row_abs_max<<<(COMB_ENTRIES / 64 + 127) / 128, 128, 0, ctx.stream>>>(d, ctx.d_comb_rowabs);
-    DG_LAUNCH_CHECK();
-    ctx.comb_ds_f[0] = lap_fac;
-    ctx.comb_ds_f[1] = mass_fac;
-    ctx.comb_ds_ok = true;
-  }
-  return ctx.d_comb_ds;
-}
-
-// the double-single run-form loop (k_patch_matvec_runs_ds): FP64 vectors
-template <bool DIR>
-void launch_matvec_runs_ds(Context &ctx, const Mesh &m, const double *x, double *y, double lap_fac,
-                           double mass_fac, int scale_exp, const char *name, double bytes) {
-  const size_t smem = patch_runs_ds_smem();
-  ensure_smem_attr(ctx, k_patch_matvec_runs_ds<DIR>, (int)smem);
+// blocks of a grid-strided patch kernel
+template <typename F>
+static unsigned patch_grid(Context &ctx, F *kernel, size_t smem, size_t n_patch) {
+  ensure_smem_attr(ctx, kernel, 227 * 1024 - 1024);
   int per_sm = 1;
-  DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_patch_matvec_runs_ds<DIR>, PATCH, smem));
-  if (per_sm < 1) per_sm = 1;
-  const unsigned grid = (unsigned)std::min<size_t>(m.n_patch, (size_t)per_sm * ctx.num_sms);
-  const float4 *ctab = comb_table_ds(ctx, lap_fac, mass_fac);
-  ProfScope _prof(ctx, name, bytes);
-  k_patch_matvec_runs_ds<DIR><<<grid, PATCH, smem, ctx.stream>>>(m.pmeta, m.plid, m.prun, m.poff, m.pkeys,
-                                                                 m.pkcount, m.n_elem, m.n_patch, ctab,
-                                                                 ctx.d_comb_rowabs, x, y,
-                                                                 std::ldexp(1.0, scale_exp), -scale_exp);
-  DG_LAUNCH_CHECK();
+  DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, FAM, smem));
+  return (unsigned)std::min<size_t>(n_patch, (size_t)std::max(per_sm, 1) * ctx.num_sms);
 }
-template void launch_matvec_runs_ds<true>(Context &, const Mesh &, const double *, double *, double, double, int,
-                                          const char *, double);
-template void launch_matvec_runs_ds<false>(Context &, const Mesh &, const double *, double *, double, double, int,
-                                           const char *, double);
 
-// the run-form element loop (k_patch_matvec_runs); DIR: the Dirichlet
-// form (boundary rows and columns from the run words' boundary flag)
 template <typename T, bool DIR>
-void launch_matvec_runs(Context &ctx, const Mesh &m, const T *x, T *y, double lap_fac,
-                        double mass_fac, const char *name, double bytes) {
-  const size_t smem = patch_runs_smem<T>();
-  ensure_smem_attr(ctx, k_patch_matvec_runs<T, DIR>, (int)smem);
-  int per_sm = 1;
-  DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_patch_matvec_runs<T, DIR>, PATCH, smem));
-  if (per_sm < 1) per_sm = 1;
-  const unsigned grid = (unsigned)std::min<size_t>(m.n_patch, (size_t)per_sm * ctx.num_sms);
-  const T *cs = std::is_same<T, double>::value ? reinterpret_cast<const T *>(ctx.d_csten64)
-                                               : reinterpret_cast<const T *>(ctx.d_csten32);
-  const T *ctab = std::is_same<T, double>::value ? comb_table<T>(ctx, lap_fac, mass_fac) : nullptr;
+void launch_family_matvec(Context &ctx, const Mesh &m, const T *x, T *y, double lap_fac, double mass_fac,
+                          const char *name, double bytes) {
+  const size_t smem = family_smem<T>(m.max_run);
+  const unsigned grid = patch_grid(ctx, k_family_matvec<T, DIR, false>, smem, m.n_patch);
+  const T *dtab = diag_table<T>(ctx, lap_fac, mass_fac);
   ProfScope _prof(ctx, name, bytes);
-  k_patch_matvec_runs<T, DIR><<<grid, PATCH, smem, ctx.stream>>>(m.pmeta, m.plid, m.prun, m.poff, m.pkeys,
-                                                                m.pkcount, m.n_elem, m.n_patch, cs, ctab, x, y,
-                                                                (T)lap_fac, (T)mass_fac);
+  k_family_matvec<T, DIR, false><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch,
+                                                                  m.max_run, dtab, x, y, nullptr, nullptr);
   DG_LAUNCH_CHECK();
 }
-template void launch_matvec_runs<float, true>(Context &, const Mesh &, const float *, float *,
-                                              double, double, const char *, double);
-template void launch_matvec_runs<float, false>(Context &, const Mesh &, const float *, float *,
-                                               double, double, const char *, double);
-template void launch_matvec_runs<double, true>(Context &, const Mesh &, const double *, double *,
-                                               double, double, const char *, double);
-template void launch_matvec_runs<double, false>(Context &, const Mesh &, const double *,
-                                                double *, double, double, const char *, double);
+template void launch_family_matvec<float, true>(Context &, const Mesh &, const float *, float *, double, double,
+                                                const char *, double);
+template void launch_family_matvec<double, true>(Context &, const Mesh &, const double *, double *, double, double,
+                                                 const char *, double);
+
+void launch_family_matvec_fix(Context &ctx, const Mesh &m, const double *x, double *y, const char *name,
+                              double bytes) {
+  const size_t smem = 2 * ((size_t)m.max_run + 1) * sizeof(long long);
+  const unsigned grid = patch_grid(ctx, k_family_matvec_fix<true>, smem, m.n_patch);
+  ProfScope _prof(ctx, name, bytes);
+  k_family_matvec_fix<true><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch, m.max_run,
+                                                             x, y);
+  DG_LAUNCH_CHECK();
+}
 
 template <typename T>
 void mesh_matvec(Context &ctx, const Mesh &m, const T *x, T *y, double lap_fac, double mass_fac) {
-  ensure_stencils(ctx);
-  cudaStream_t s = ctx.stream;
-  DG_CUDA(cudaMemsetAsync(y, 0, m.n_node * sizeof(T), s));
-  if (m.plid && ctx.matvec_form != 1) {
-    launch_matvec_runs<T, false>(ctx, m, x, y, lap_fac, mass_fac,
-                                 sizeof(T) == 4 ? "matvec_fp32" : "matvec_fp64",
+  DG_CUDA(cudaMemsetAsync(y, 0, m.n_node * sizeof(T), ctx.stream));
+  launch_family_matvec<T, false>(ctx, m, x, y, lap_fac, mass_fac, sizeof(T) == 4 ? "matvec_fp32" : "matvec_fp64",
                                  (double)m.n_elem * 36 + (double)m.n_node * 3 * sizeof(T));
-    return;
-  }
-  const size_t smem = patch_smem<T>();
-  ensure_smem_attr(ctx, k_patch_matvec<T, false>, (int)smem);
-  int per_sm = 1;
-  DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_patch_matvec<T, false>, PATCH, smem));
-  if (per_sm < 1) per_sm = 1;
-  const unsigned grid = (unsigned)std::min<size_t>(m.n_patch, (size_t)per_sm * ctx.num_sms);
-  const T *cs = std::is_same<T, double>::value ? reinterpret_cast<const T *>(ctx.d_csten64)
-                                               : reinterpret_cast<const T *>(ctx.d_csten32);
-  const T *ctab = comb_table<T>(ctx, lap_fac, mass_fac);
-  {
-    ProfScope _prof(ctx, sizeof(T) == 4 ? "matvec_fp32" : "matvec_fp64",
-                    (double)m.n_elem * 36 + (double)m.n_node * 3 * sizeof(T));
-    k_patch_matvec<T, false><<<grid, PATCH, smem, s>>>(m.pmeta, m.pinc, m.pexc, m.pnode, m.poff, m.pkeys,
-                                                       m.pkcount, m.n_elem, m.n_patch, cs, ctab, ctx.d_cperm, nullptr,
-                                                       x, y, (T)lap_fac, (T)mass_fac);
-    DG_LAUNCH_CHECK();
-  }
 }
-
 template void mesh_matvec<float>(Context &, const Mesh &, const float *, float *, double, double);
 template void mesh_matvec<double>(Context &, const Mesh &, const double *, double *, double, double);
 
 template <typename T>
 void mesh_matvec_coef(Context &ctx, const Mesh &m, const double *coef, const T *x, T *y) {
-  ensure_stencils(ctx);
-  cudaStream_t s = ctx.stream;
-  DG_CUDA(cudaMemsetAsync(y, 0, m.n_node * sizeof(T), s));
-  const size_t smem = patch_smem<T>();
-  ensure_smem_attr(ctx, k_patch_matvec<T, false, true>, (int)smem);
-  int per_sm = 1;
-  DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_patch_matvec<T, false, true>, PATCH, smem));
-  if (per_sm < 1) per_sm = 1;
-  const unsigned grid = (unsigned)std::min<size_t>(m.n_patch, (size_t)per_sm * ctx.num_sms);
-  const T *cs = std::is_same<T, double>::value ? reinterpret_cast<const T *>(ctx.d_csten64)
-                                               : reinterpret_cast<const T *>(ctx.d_csten32);
+  DG_CUDA(cudaMemsetAsync(y, 0, m.n_node * sizeof(T), ctx.stream));
+  const size_t smem = family_smem<T>(m.max_run);
+  const unsigned grid = patch_grid(ctx, k_family_matvec<T, false, true>, smem, m.n_patch);
   ProfScope _prof(ctx, sizeof(T) == 4 ? "matvec_coef_fp32" : "matvec_coef_fp64",
                   (double)m.n_elem * (36 + 16 + 2) + (double)m.n_node * 3 * sizeof(T));
-  k_patch_matvec<T, false, true><<<grid, PATCH, smem, s>>>(m.pmeta, m.pinc, m.pexc, m.pnode, m.poff, m.pkeys,
-                                                           m.pkcount, m.n_elem, m.n_patch, cs, nullptr, ctx.d_cperm,
-                                                           nullptr, x, y, (T)1, (T)1, coef, m.pperm);
+  k_family_matvec<T, false, true><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch,
+                                                                   m.max_run, nullptr, x, y, coef, m.fchild);
   DG_LAUNCH_CHECK();
 }
 template void mesh_matvec_coef<float>(Context &, const Mesh &, const double *, const float *, float *);

@@ -21,31 +21,20 @@ struct Mesh {
   uint32_t *meta = nullptr;
   uint32_t *conn = nullptr;      // 8 * n_elem, vertex-major
   uint32_t *node_xyz = nullptr;  // 3 * n_node, coordinate-major
-  // element loop tables (dg_elem.cuh): n_patch patches of PATCH elements
-  size_t n_patch = 0;
-  uint16_t *pinc = nullptr;   // PATCH_ENT per patch, node-sorted pairs
-  uint16_t *pexc = nullptr;   // PATCH per patch: runs starting before pair 8t
-  uint32_t *pmeta = nullptr;  // PATCH per patch: meta in the patch's element order,
-                              // bits 16..23 = the element's stencil key index
-  uint16_t *pkeys = nullptr;  // PKEY_MAX per patch: (type << 5 | level) of each key
-  uint16_t *pkcount = nullptr;  // keys per patch (> PKEY_MAX: per-element L, M path)
-  uint32_t *pnode = nullptr;  // node of each run, patch after patch
-  uint64_t *poff = nullptr;   // n_patch + 1 run offsets into pnode
-  // pperm maps a patch's (type, level) order back to its element order
-  uint16_t *pperm = nullptr;  // PATCH per patch
-  // run form of the FP32 element loop (dg_elem.cuh, k_patch_matvec_runs):
-  // per (type, level) position the 8 patch-local run indices of its
-  // vertices in the canonical stencil order (8 x 16 bits), and per run its
-  // node with bit 31 set when the run holds all the node's pairs
-  uint4 *plid = nullptr;      // PATCH per patch
-  uint32_t *prun = nullptr;   // one per run, at poff
+  // element loop tables (dg_elem.cuh): families of siblings, FAM to a patch
+  size_t n_fam = 0, n_patch = 0, n_run = 0;
+  int max_run = 0;             // most nodes of a patch
+  uint4 *fam = nullptr;        // 4 x FAM words per patch
+  uint4 *pinfo = nullptr;      // per patch: offset in prun (64 bits), nodes, coarsest level
+  uint32_t *prun = nullptr;    // nodes of each patch with two flags
+  uint32_t *fchild = nullptr;  // 8 per family: the element of each child that is a leaf
   // compressed mode (the reference's compressLut): conn is released once the
-  // patch tables exist and decoded from them on demand (mesh_conn)
+  // family tables exist and decoded from them on demand (mesh_conn)
   bool compressed = false;
 };
 
 void mesh_build(Context &ctx, const Octree &bal, Mesh &m, bool compress = false);
-// the 8 x n_elem vertex-major node ids: m.conn, or decoded from the patch
+// the 8 x n_elem vertex-major node ids: m.conn, or decoded from the family
 // tables into tmp when the mesh is compressed
 const uint32_t *mesh_conn(Context &ctx, const Mesh &m, DBuf<uint32_t> &tmp);
 // device bytes the mesh holds
@@ -121,20 +110,15 @@ constexpr int STEN_ENTRIES = 8 * 18 * 128;
 
 // stencil tables on the device, generated on first use
 void ensure_stencils(Context &ctx);
-// the combined-stencil table of the element loop for these factors
-// (rebuilt on ctx's stream when they differ from the last call's)
-template <typename T>
-const T *comb_table(Context &ctx, double lap_fac, double mass_fac);
 
-// the double-single run-form loop (FP64 vectors, FP32-pair arithmetic; x
-// scaled by 2^scale_exp inside, the result by 2^-scale_exp)
-template <bool DIR>
-void launch_matvec_runs_ds(Context &ctx, const Mesh &m, const double *x, double *y, double lap_fac,
-                           double mass_fac, int scale_exp, const char *name, double bytes);
-// the run-form element loop on a mesh with run tables (m.plid)
+// the element loop on a zeroed y; DIR: the Dirichlet form (boundary rows and
+// columns from the run words' boundary flag)
 template <typename T, bool DIR>
-void launch_matvec_runs(Context &ctx, const Mesh &m, const T *x, T *y, double lap_fac,
-                        double mass_fac, const char *name, double bytes);
+void launch_family_matvec(Context &ctx, const Mesh &m, const T *x, T *y, double lap_fac, double mass_fac,
+                          const char *name, double bytes);
+// the Dirichlet K + M on FP64 vectors in 64-bit fixed point
+void launch_family_matvec_fix(Context &ctx, const Mesh &m, const double *x, double *y, const char *name,
+                              double bytes);
 
 // host-side generators (same mathematics as the reference's .inp tables)
 void gen_etype_masks(uint8_t masks[8 * 18]);

@@ -1,687 +1,532 @@
-// Element-loop building blocks shared by the matVec kernels.
+// The element loop y = (lapf K + massf M) x, by sibling families.
 //
-// Canonical stencils: every (child, type) stencil is a relabelling of the
-// child-0 stencil of the same type by one of the 48 symmetries of the cube,
-// S(c,t)[k][j] = S(0,t)[p[k]][p[j]] (equal to rounding), so 18 full 8x8
-// Laplacian + mass stencils (18 KB in FP64, 9 KB in FP32) and one 8-entry
-// relabelling per (child, type) stand for all 144.  Full rows load as
-// 16-byte vectors; the elements of a patch are ordered by (type, level), so
-// the threads of a warp mostly read the same stencil (a broadcast).
+// A family is one parent octant with those of its 8 children that are
+// leaves.  Its elements only ever refer to the 27 points of the 3x3x3
+// lattice that the children's vertices form: a vertex that does not hang is
+// a lattice point, and a hanging one refers to the parent's corner, the
+// lattice corner of its child.  So a family is the unit of work of one
+// thread: gather its lattice once, apply its elements in registers, add the
+// lattice out once.  An octree has (E - 1) / 7 internal octants, so a family
+// holds 7.4 elements on the workloads' meshes and touches 18 mesh nodes:
+// 2.5 gathers and adds per element against 8 for an element-wise loop.
 //
-// Patches: PATCH consecutive elements form a patch.  Its incidence table
-// lists the 8 x PATCH (element, vertex) pairs grouped by node (one run per
-// node, runs in the order of a per-patch hash table, the pairs of a run by
-// slot), 16 bits each:
-//   bits 0..11  slot = vertex * PATCH + element within the patch
-//   bit 12      first pair of a node's run
-//   bit 13      the run holds every pair of its node in the whole mesh, so
-//               the node's sum is complete in this patch (stored, not added)
-// pnode[poff[p] + u] is the node of run u of patch p, pexc[p][t] the number
-// of runs that start before pair 8t, and pmeta[p][t] the meta word of the
-// patch's element t in (type, level) order (the order slots use).  An element loop over a patch
-// gathers x once per node into the slots, applies the element stencils
-// slot-to-slot in shared memory, and sums each run with a segmented scan:
-// no shared-memory atomics, and global atomics only for nodes that other
-// patches also touch.
+// Hanging points: an edge midpoint of the parent that hangs takes the mean of
+// its edge's two corners, a face centre that hangs the mean of two opposite
+// edge midpoints of its face (which then hang too), and the results at
+// hanging points are passed back by the transpose.  That is the P^T S P of
+// the reference's 18 element types, so the elements themselves are all the
+// plain trilinear one, and no stencil table is read.
+//
+// Elements: K and M are tensor products, diagonal in a basis of sums and
+// differences.  For the assembled 2x2x2 family, per axis
+//   M = 1/4 s s^T + 1/3 o o^T + 1/12 q q^T,  A = 1/4 o o^T + 1/4 q q^T
+// with s = (1,2,1), o = (1,0,-1), q = (1,-2,1); for one element
+//   M = 1/2 s s^T + 1/6 d d^T,  A = 1/2 d d^T,  s = (1,1), d = (1,-1).
+// So a complete family (3 of 4) costs 27 lines each way (4 and 5 operations a
+// line, all coefficients 1 or 2) and 27 multiplications: 262 operations for 8
+// elements, where 8 dense 8x8 stencils cost 512 multiply-adds.  A family with
+// subdivided children is applied element by element: 397 operations.
+//
+// What bounds it (1.1e7 elements of a Gaussian cloud, GB300): FP32 143 us,
+// instruction issue and the latency of the gathers (DRAM traffic alone would
+// take 34 us; without the shared-memory atomics 116 us, without the x gather
+// 124 us); FP64 1,270 us, the FP64 pipe, which issues 2 operations per clock
+// per SM; fixed point 293 us, integer issue.  An element-wise loop over dense
+// stencils, 8 gathers and 8 atomics per element, took 348, 1,820 and 873 us
+// (the last in double-single arithmetic).  128 families per patch: 64 and 256
+// measured 152 / 150 us in FP32 and 1,296 / 1,481 us in FP64; a patch of 256
+// leaves too few blocks on small meshes.
+//
+// Patches: FAM consecutive families (in element order) make a patch, one
+// thread block's work at a time.  fam[(p * 4 + w) * FAM + t] is word w of the
+// patch's family t: 27 x 16 bits, the patch-local number of the node at each
+// lattice point (0: no node there), then 16 bits level and 8 bits mask of the
+// children that are leaves, then 18 bits of hanging points.  Complete families
+// come first, so that most warps hold one kind.  pinfo[p] = {offset of the
+// patch's nodes in prun (64 bits), their number, the level of its coarsest
+// element}; prun holds the nodes, number 1 first, with two flags.
 #pragma once
 
 #include "dg_prims.cuh"
 
 namespace dg {
 
-// per type: 8x8 Laplacian rows, then 8x8 mass rows, then 16 bytes of padding
-// so that the same row of two neighbouring types sits in different banks
-template <typename T>
-constexpr int fsten_stride() {
-  return 128 + 16 / (int)sizeof(T);
+constexpr int FAM = 128;                // families per patch, threads per block
+constexpr int FAM_MAX_RUN = 27 * FAM;  // most nodes a patch can touch
+constexpr uint32_t PRUN_COMPLETE = 1u << 31;  // no other patch touches the node: its sum is stored, not added
+constexpr uint32_t PRUN_BDY = 1u << 30;       // the node lies on the domain boundary
+constexpr uint32_t PRUN_NODE = PRUN_BDY - 1;
+
+// lattice point of child c's vertex k
+__host__ __device__ constexpr int lat_vertex(int c, int k) {
+  return ((c & 1) + (k & 1)) + 3 * ((c >> 1 & 1) + (k >> 1 & 1)) + 9 * ((c >> 2 & 1) + (k >> 2 & 1));
 }
-template <typename T>
-constexpr int fsten_entries() {
-  return 18 * fsten_stride<T>();
+// lattice point of the parent's corner k
+__host__ __device__ constexpr int lat_corner(int k) { return 2 * (k & 1) + 6 * (k >> 1 & 1) + 18 * (k >> 2 & 1); }
+
+// the 18 lattice points that can hang: edge midpoints (i = 0..11, along axis
+// i / 4) with the two corners of their edge, face centres (i = 12..17, normal
+// to axis (i - 12) / 2) with two opposite edge midpoints of their face
+__host__ __device__ constexpr int lat_stride(int ax) { return ax % 3 == 0 ? 1 : ax % 3 == 1 ? 3 : 9; }
+__host__ __device__ constexpr int hang_pos(int i) {
+  return i < 12 ? lat_stride(i / 4) + 2 * (i & 1) * lat_stride(i / 4 + 1) + 2 * (i >> 1 & 1) * lat_stride(i / 4 + 2)
+                : 2 * (i & 1) * lat_stride((i - 12) / 2) + lat_stride((i - 12) / 2 + 1) + lat_stride((i - 12) / 2 + 2);
 }
-constexpr int PATCH = 512;
-constexpr int PATCH_ENT = 8 * PATCH;
-// per-patch combined stencils: one 8x8 S = f1(l) L_t + f2(l) M_t per
-// (type, level) present in the patch, up to PKEY_MAX of them; rows padded by
-// 16 bytes so neighbouring keys sit in different banks
-constexpr int PKEY_MAX = 64;
-template <typename T>
-constexpr int sstride() {
-  return 64 + 16 / (int)sizeof(T);
+__host__ __device__ constexpr int hang_step(int i) {
+  return i < 12 ? lat_stride(i / 4) : lat_stride((i - 12) / 2 + 1);
 }
-constexpr uint32_t ENT_SLOT = 0xfffu, ENT_START = 1u << 12, ENT_COMPLETE = 1u << 13;
-constexpr uint32_t RUN_BDY = 1u << 31;  // run node flag in shared memory (Dirichlet)
+__host__ __device__ constexpr int hang_a(int i) { return hang_pos(i) - hang_step(i); }
+__host__ __device__ constexpr int hang_b(int i) { return hang_pos(i) + hang_step(i); }
+__host__ __device__ constexpr int hang_bit(int pos) {
+  for (int i = 0; i < 18; i++)
+    if (hang_pos(i) == pos) return i;
+  return -1;
+}
+
+// Diagonal of the operator in the sum / difference basis, per level: entry
+// dfam(o, q) for a family mode with o factors o and q factors q, entry
+// DCHILD + p for an element mode with p factors d.  Rows are padded so that
+// neighbouring levels fall in different shared-memory banks.
+constexpr int DTAB_CHILD = 10, DTAB_STRIDE = 15, DTAB_LEVELS = 31;
+constexpr int DTAB_ENTRIES = DTAB_LEVELS * DTAB_STRIDE;
+__host__ __device__ constexpr int dfam(int o, int q) { return o == 0 ? q : o == 1 ? 4 + q : o == 2 ? 7 + q : 9; }
 
 // 2^-l exactly, from the exponent bits (0 <= l <= 30)
 __device__ __forceinline__ float exp2_neg(float, unsigned l) { return __int_as_float((int)(127u - l) << 23); }
 __device__ __forceinline__ double exp2_neg(double, unsigned l) {
   return __longlong_as_double((long long)(1023u - l) << 52);
 }
+__device__ __forceinline__ bool is_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) != 0x7f800000u; }
+__device__ __forceinline__ bool is_finite(double v) {
+  return ((uint32_t)__double2hiint(v) & 0x7ff00000u) != 0x7ff00000u;
+}
 
-// combined stencils of every (type, level), 32 levels per type:
-// comb[(t * 32 + l) * 64 + q] = lapf 2^-l / 2 L_t[q] + massf 2^-3l / 8 M_t[q]
-// (the element loop copies the ones a patch uses into shared memory)
-constexpr int COMB_LEVELS = 32;
-constexpr int COMB_ENTRIES = 18 * COMB_LEVELS * 64;
+// entry i of the table: lap and mass already scaled by h / 2 and h^3 / 8
 template <typename T>
-__global__ void k_comb_table(const T *__restrict__ cs, T lapf, T massf, T *__restrict__ out) {
+__device__ __forceinline__ T dtab_entry(int i, T lap, T mass) {
+  double m[3], a[3];  // mode weights of the three axes
+  if (i < DTAB_CHILD) {
+    const int o = i < 4 ? 0 : i < 7 ? 1 : i < 9 ? 2 : 3;
+    const int q = i - (i < 4 ? 0 : i < 7 ? 4 : i < 9 ? 7 : 9);
+    for (int k = 0; k < 3; k++) {
+      m[k] = k < o ? 1.0 / 3.0 : k < o + q ? 1.0 / 12.0 : 0.25;
+      a[k] = k < o + q ? 0.25 : 0.0;
+    }
+  } else {
+    for (int k = 0; k < 3; k++) {
+      m[k] = k < i - DTAB_CHILD ? 1.0 / 6.0 : 0.5;
+      a[k] = k < i - DTAB_CHILD ? 0.5 : 0.0;
+    }
+  }
+  return lap * (T)(a[0] * m[1] * m[2] + m[0] * a[1] * m[2] + m[0] * m[1] * a[2]) + mass * (T)(m[0] * m[1] * m[2]);
+}
+
+template <typename T>
+__global__ void k_dtab(T *__restrict__ out, double lapf, double massf) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= COMB_ENTRIES) return;
-  const int t = i / (COMB_LEVELS * 64), l = (i / 64) % COMB_LEVELS, q = i % 64;
-  const T h = exp2_neg((T)0, (unsigned)l);
-  const T *st = cs + t * fsten_stride<T>();
-  out[i] = lapf * h * (T)0.5 * st[q] + massf * h * h * h * (T)0.125 * st[64 + q];
+  if (i >= DTAB_ENTRIES) return;
+  const double h = ldexp(1.0, -(i / DTAB_STRIDE));
+  const int q = i % DTAB_STRIDE;
+  out[i] = q < DTAB_CHILD + 4 ? (T)dtab_entry<double>(q, lapf * h * 0.5, massf * h * h * h * 0.125) : (T)0;
 }
 
-// two FP32 fused multiply-adds in one instruction (Blackwell f32x2)
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\t"
-      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
-      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return d;
-}
-
-// paired FP32 add, subtract and multiply (Blackwell f32x2), round to nearest
-__device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
-      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-      "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-__device__ __forceinline__ float2 fsub2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
-      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-      "sub.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n\t.reg .b64 ra, rb, rd;\n\t"
-      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-      "mul.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-
-// y_k = f1 sum_j L[k][j] x_j + f2 sum_j M[k][j] x_j (full-row stencil S),
-// handing each y_k to emit(k, y_k)
-template <typename Emit>
-__device__ __forceinline__ void apply_full(const float *__restrict__ S, float f1, float f2, const float (&xv)[8],
-                                           Emit &&emit) {
-  const float2 x0 = make_float2(xv[0], xv[1]), x1 = make_float2(xv[2], xv[3]);
-  const float2 x2 = make_float2(xv[4], xv[5]), x3 = make_float2(xv[6], xv[7]);
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const float4 l0 = reinterpret_cast<const float4 *>(S + 8 * k)[0];
-    const float4 l1 = reinterpret_cast<const float4 *>(S + 8 * k)[1];
-    const float4 m0 = reinterpret_cast<const float4 *>(S + 64 + 8 * k)[0];
-    const float4 m1 = reinterpret_cast<const float4 *>(S + 64 + 8 * k)[1];
-    float2 aL = ffma2(make_float2(l0.x, l0.y), x0, make_float2(0.f, 0.f));
-    aL = ffma2(make_float2(l0.z, l0.w), x1, aL);
-    aL = ffma2(make_float2(l1.x, l1.y), x2, aL);
-    aL = ffma2(make_float2(l1.z, l1.w), x3, aL);
-    float2 aM = ffma2(make_float2(m0.x, m0.y), x0, make_float2(0.f, 0.f));
-    aM = ffma2(make_float2(m0.z, m0.w), x1, aM);
-    aM = ffma2(make_float2(m1.x, m1.y), x2, aM);
-    aM = ffma2(make_float2(m1.z, m1.w), x3, aM);
-    emit(k, f1 * (aL.x + aL.y) + f2 * (aM.x + aM.y));
-  }
-}
-
-template <typename Emit>
-__device__ __forceinline__ void apply_full(const double *__restrict__ S, double f1, double f2, const double (&xv)[8],
-                                           Emit &&emit) {
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    double aL = 0, aM = 0;
-#pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-      const double2 l = reinterpret_cast<const double2 *>(S + 8 * k + j)[0];
-      const double2 m = reinterpret_cast<const double2 *>(S + 64 + 8 * k + j)[0];
-      aL = fma(l.x, xv[j], aL);
-      aL = fma(l.y, xv[j + 1], aL);
-      aM = fma(m.x, xv[j], aM);
-      aM = fma(m.y, xv[j + 1], aM);
+// The table entries of K + M as fractions: entry i is
+// (alpha fix_lap(i) + beta fix_mass(i)) / (27 * 2^fix_shift(i)) with
+// alpha = h / 2, beta = h^3 / 8
+__host__ __device__ constexpr int fix_weight(int i, bool lap) {
+  int m[3] = {}, a[3] = {};  // mode weights times 12 (a family's) or 6 (an element's)
+  if (i < DTAB_CHILD) {
+    const int o = i < 4 ? 0 : i < 7 ? 1 : i < 9 ? 2 : 3;
+    const int q = i - (i < 4 ? 0 : i < 7 ? 4 : i < 9 ? 7 : 9);
+    for (int k = 0; k < 3; k++) {
+      m[k] = k < o ? 4 : k < o + q ? 1 : 3;
+      a[k] = k < o + q ? 3 : 0;
     }
-    emit(k, f1 * aL + f2 * aM);
-  }
-}
-
-// y'_k = sum_j S[k][j] x_j with a combined, already scaled stencil S
-template <typename Emit>
-__device__ __forceinline__ void apply_comb(const float *__restrict__ S, const float (&xv)[8], Emit &&emit) {
-  const float2 x0 = make_float2(xv[0], xv[1]), x1 = make_float2(xv[2], xv[3]);
-  const float2 x2 = make_float2(xv[4], xv[5]), x3 = make_float2(xv[6], xv[7]);
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const float4 s0 = reinterpret_cast<const float4 *>(S + 8 * k)[0];
-    const float4 s1 = reinterpret_cast<const float4 *>(S + 8 * k)[1];
-    float2 a = ffma2(make_float2(s0.x, s0.y), x0, make_float2(0.f, 0.f));
-    a = ffma2(make_float2(s0.z, s0.w), x1, a);
-    a = ffma2(make_float2(s1.x, s1.y), x2, a);
-    a = ffma2(make_float2(s1.z, s1.w), x3, a);
-    emit(k, a.x + a.y);
-  }
-}
-
-template <typename Emit>
-__device__ __forceinline__ void apply_comb(const double *__restrict__ S, const double (&xv)[8], Emit &&emit) {
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    double a = 0;
-#pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-      const double2 sv = reinterpret_cast<const double2 *>(S + 8 * k + j)[0];
-      a = fma(sv.x, xv[j], a);
-      a = fma(sv.y, xv[j + 1], a);
+  } else {
+    for (int k = 0; k < 3; k++) {
+      m[k] = k < i - DTAB_CHILD ? 1 : 3;
+      a[k] = k < i - DTAB_CHILD ? 3 : 0;
     }
-    emit(k, a);
+  }
+  return lap ? a[0] * m[1] * m[2] + m[0] * a[1] * m[2] + m[0] * m[1] * a[2] : m[0] * m[1] * m[2];
+}
+__host__ __device__ constexpr int fix_shift(int i) { return i < DTAB_CHILD ? 6 : 3; }
+
+// arithmetic of one lattice value: FP32, FP64 or 64-bit fixed point
+template <typename V>
+struct LatOps {
+  static __device__ __forceinline__ V add_twice(V a, V b) { return a + (V)2 * b; }
+  static __device__ __forceinline__ V sub_twice(V a, V b) { return a - (V)2 * b; }
+  static __device__ __forceinline__ V half_add(V v, V half_of) { return v + (V)0.5 * half_of; }
+  static __device__ __forceinline__ V mean(V a, V b) { return (V)0.5 * (a + b); }
+};
+template <>
+struct LatOps<long long> {
+  static __device__ __forceinline__ long long add_twice(long long a, long long b) { return a + 2 * b; }
+  static __device__ __forceinline__ long long sub_twice(long long a, long long b) { return a - 2 * b; }
+  static __device__ __forceinline__ long long half_add(long long v, long long half_of) { return v + (half_of >> 1); }
+  static __device__ __forceinline__ long long mean(long long a, long long b) { return (a + b) >> 1; }
+};
+
+// values at hanging points from the points they depend on
+template <typename V>
+__device__ __forceinline__ void lat_interpolate(V (&u)[27], uint32_t hang) {
+#pragma unroll
+  for (int i = 0; i < 18; i++)
+    if (hang >> i & 1u) u[hang_pos(i)] = LatOps<V>::mean(u[hang_a(i)], u[hang_b(i)]);
+}
+// the transpose: results at hanging points passed back (faces first)
+template <typename V>
+__device__ __forceinline__ void lat_distribute(V (&v)[27], uint32_t hang) {
+#pragma unroll
+  for (int i = 17; i >= 0; i--)
+    if (hang >> i & 1u) {
+      v[hang_a(i)] = LatOps<V>::half_add(v[hang_a(i)], v[hang_pos(i)]);
+      v[hang_b(i)] = LatOps<V>::half_add(v[hang_b(i)], v[hang_pos(i)]);
+    }
+}
+
+// a complete family: to the sum / difference basis and back, in place
+template <typename V>
+__device__ __forceinline__ void lat_forward(V (&u)[27]) {
+#pragma unroll
+  for (int ax = 0; ax < 3; ax++) {
+    const int st = ax == 0 ? 1 : ax == 1 ? 3 : 9;
+#pragma unroll
+    for (int n = 0; n < 9; n++) {
+      const int i = ax == 0 ? 3 * n : ax == 1 ? n % 3 + 9 * (n / 3) : n;
+      const V e = u[i] + u[i + 2 * st], o = u[i] - u[i + 2 * st], b = u[i + st];
+      u[i] = LatOps<V>::add_twice(e, b);
+      u[i + st] = o;
+      u[i + 2 * st] = LatOps<V>::sub_twice(e, b);
+    }
+  }
+}
+template <typename V>
+__device__ __forceinline__ void lat_backward(V (&u)[27]) {
+#pragma unroll
+  for (int ax = 0; ax < 3; ax++) {
+    const int st = ax == 0 ? 1 : ax == 1 ? 3 : 9;
+#pragma unroll
+    for (int n = 0; n < 9; n++) {
+      const int i = ax == 0 ? 3 * n : ax == 1 ? n % 3 + 9 * (n / 3) : n;
+      const V t = u[i] + u[i + 2 * st], r = u[i] - u[i + 2 * st], o = u[i + st];
+      u[i] = t + o;
+      u[i + st] = r + r;
+      u[i + 2 * st] = t - o;
+    }
+  }
+}
+// the modes times their table entries; mul(t, i): t times entry i
+template <typename V, typename Mul>
+__device__ __forceinline__ void lat_scale(V (&u)[27], Mul &&mul) {
+#pragma unroll
+  for (int i = 0; i < 27; i++) {
+    const int x = i % 3, y = i / 3 % 3, z = i / 9;
+    u[i] = mul(u[i], dfam((x == 1) + (y == 1) + (z == 1), (x == 2) + (y == 2) + (z == 2)));
   }
 }
 
-// y = (lapf K + massf M) x over the elements of every patch; with DIR the
-// Dirichlet form: boundary rows are the identity (y = x), boundary columns
-// are dropped.  One block of PATCH threads per patch, grid-strided; thread t
-// holds pairs 8t..8t+7 of the patch's table and is element t of the patch.
-// The slot buffer and the run-node array are single (a patch costs four
-// barriers) so that more blocks fit an SM: three in FP32 (40 registers per
-// thread), two in FP64; one block's gathers and sums overlap another's
-// stencil phase.  (Double-buffering them by patch parity saves a barrier
-// but halves the blocks; measured slower.)  The next patch's table words are
-// loaded one patch ahead.
-template <typename T>
-constexpr int patch_nbuf() {
-  return 1;
+// any family, v = sum over its elements of S u, element by element in the
+// basis of one element, the sums and differences of shared edges and faces
+// formed once: 148 operations in, 64 multiplications, 185 out for 8 elements
+// (333 for each on its own: 512).  begin(c) before child c; mul(t, p): t times
+// its entry for p factors d.  A child that is not there gets no value.
+template <typename V, typename Begin, typename Mul>
+__device__ __forceinline__ void lat_elements(const V (&u)[27], V (&v)[27], uint32_t mask, Begin &&begin, Mul &&mul) {
+#pragma unroll
+  for (int cx = 0; cx < 2; cx++) {
+    V a[2][9], sum_x[2][9];  // [factor along x][y + 3 z]
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+      a[0][i] = u[3 * i + cx] + u[3 * i + cx + 1];
+      a[1][i] = u[3 * i + cx] - u[3 * i + cx + 1];
+    }
+#pragma unroll
+    for (int cy = 0; cy < 2; cy++) {
+      V b[4][3], sum_y[4][3];  // [factors along x, y][z]
+#pragma unroll
+      for (int z = 0; z < 3; z++)
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+          b[m][z] = a[m][3 * z + cy] + a[m][3 * z + cy + 1];
+          b[m + 2][z] = a[m][3 * z + cy] - a[m][3 * z + cy + 1];
+        }
+#pragma unroll
+      for (int cz = 0; cz < 2; cz++) {
+        const int c = cx + 2 * cy + 4 * cz;
+        const bool there = mask >> c & 1u;
+        begin(c);
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+          const int p = (m & 1) + (m >> 1);
+          V s = mul(b[m][cz] + b[m][cz + 1], p), d = mul(b[m][cz] - b[m][cz + 1], p + 1);
+          s = there ? s : (V)0;
+          d = there ? d : (V)0;
+          sum_y[m][cz] = cz == 0 ? s + d : sum_y[m][cz] + (s + d);
+          sum_y[m][cz + 1] = s - d;
+        }
+      }
+#pragma unroll
+      for (int z = 0; z < 3; z++)
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+          const V s = sum_y[m][z], d = sum_y[m + 2][z];
+          sum_x[m][3 * z + cy] = cy == 0 ? s + d : sum_x[m][3 * z + cy] + (s + d);
+          sum_x[m][3 * z + cy + 1] = s - d;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+      const V s = sum_x[0][i], d = sum_x[1][i];
+      v[3 * i + cx] = cx == 0 ? s + d : v[3 * i + cx] + (s + d);
+      v[3 * i + cx + 1] = s - d;
+    }
+  }
 }
 
-// With COEF, element e's factors are coef[2e] (Laplacian) and coef[2e + 1]
-// (mass) instead of lapf and massf (pperm gives e from the patch order).
-template <typename T, bool DIR, bool COEF = false>
-__global__ void __launch_bounds__(PATCH, sizeof(T) == 4 ? 3 : 2)
-    k_patch_matvec(const uint32_t *__restrict__ pmeta, const uint16_t *__restrict__ pinc,
-                   const uint16_t *__restrict__ pexc, const uint32_t *__restrict__ pnode,
-                   const uint64_t *__restrict__ poff, const uint16_t *__restrict__ pkeys,
-                   const uint16_t *__restrict__ pkcount, size_t E, size_t n_patch, const T *__restrict__ fsten,
-                   const T *__restrict__ ctab, const uint32_t *__restrict__ cperm, const uint8_t *__restrict__ bdy,
-                   const T *__restrict__ x, T *__restrict__ y, T lapf, T massf,
-                   const double *__restrict__ coef = nullptr, const uint16_t *__restrict__ pperm = nullptr) {
-  constexpr int NW = PATCH / 32;
+// the 16-bit number i of a family's four words
+__device__ __forceinline__ uint32_t fam_u16(const uint4 (&w)[4], int i) {
+  const uint4 q = w[i >> 3];
+  const uint32_t word = (i >> 1 & 3) == 0 ? q.x : (i >> 1 & 3) == 1 ? q.y : (i >> 1 & 3) == 2 ? q.z : q.w;
+  return (i & 1) ? word >> 16 : word & 0xffffu;
+}
+__device__ __forceinline__ uint32_t fam_level(const uint4 (&w)[4]) { return fam_u16(w, 27) & 31u; }
+__device__ __forceinline__ uint32_t fam_mask(const uint4 (&w)[4]) { return fam_u16(w, 28) & 255u; }
+__device__ __forceinline__ uint32_t fam_hang(const uint4 (&w)[4]) {
+  return fam_u16(w, 29) | fam_u16(w, 30) << 16;
+}
+
+// One block per patch, grid-strided, three barriers per patch:
+//   1. x of the patch's nodes into xs (node ids read coalesced), ys = 0;
+//   2. thread t = family t: its lattice from xs, its elements in registers,
+//      its lattice added into ys with shared-memory atomics;
+//   3. each node's sum stored (nodes of this patch alone) or added to y.
+// DIR, the Dirichlet form: boundary rows are the identity (y = x), boundary
+// columns are dropped.  COEF: element e's factors are coef[2e] (Laplacian)
+// and coef[2e + 1] (mass) instead of the table's; fchild[8 f + c] gives e.
+// A family whose values are not all finite takes the element path, so that a
+// non-finite x reaches exactly the rows of the elements that hold it.
+// Blocks per SM (registers): FP32 at 4 to 8 blocks 158, 152, 143, 145, 151 us on
+// 1.1e7 elements; FP64 at 2, 3, 4 blocks 1,350, 1,279, 1,267 us (4 spills).
+template <typename T, bool DIR, bool COEF>
+__global__ void __launch_bounds__(FAM, sizeof(T) == 4 ? 6 : 3)
+    k_family_matvec(const uint4 *__restrict__ fam, const uint32_t *__restrict__ prun, const uint4 *__restrict__ pinfo,
+                    size_t n_fam, size_t n_patch, int max_run, const T *__restrict__ dtab, const T *__restrict__ x,
+                    T *__restrict__ y, const double *__restrict__ coef, const uint32_t *__restrict__ fchild) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *cs = reinterpret_cast<T *>(smem_raw);
-  constexpr int NBUF = patch_nbuf<T>();
-  T *bufs = cs + fsten_entries<T>();
-  uint32_t *gns = reinterpret_cast<uint32_t *>(bufs + NBUF * PATCH_ENT);
-  uint32_t *cp = gns + NBUF * PATCH_ENT;
-  T *sc = reinterpret_cast<T *>(cp + 8 * 18 + 4);  // PKEY_MAX combined stencils (16-byte aligned)
-  __shared__ T ws_v[2][NW];
-  __shared__ int ws_f[2][NW];
-  __shared__ int ws_first[2][NW + 1];
-  for (int i = threadIdx.x; i < fsten_entries<T>(); i += PATCH) cs[i] = fsten[i];
-  for (int i = threadIdx.x; i < 8 * 18; i += PATCH) cp[i] = cperm[i];
-  __syncthreads();  // step 1 of the first patch already reads cs
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-
-  auto patch_ne = [&](size_t q) { return (int)((E - q * PATCH) < (size_t)PATCH ? (E - q * PATCH) : (size_t)PATCH); };
-  size_t p = blockIdx.x;
-  uint4 w = make_uint4(0, 0, 0, 0);
-  uint32_t ex = 0, me = 0, kc = 0;
-  uint64_t ub = 0;
-  if (p < n_patch) {
-    ub = poff[p];
-    kc = pkcount[p];
-    if (tid < patch_ne(p)) {
-      w = reinterpret_cast<const uint4 *>(pinc + p * PATCH_ENT)[tid];
-      ex = pexc[p * PATCH + tid];
-      me = pmeta[p * PATCH + tid];
-    }
-  }
-  int par = 0;
-  for (; p < n_patch; p += gridDim.x, par ^= (NBUF - 1)) {
-    const int ne = patch_ne(p);
-    const bool have = tid < ne;
-    const uint4 cw = w;
-    const uint32_t cex = ex, cme = me, ckc = kc;
-    const uint64_t cub = ub;
-    // the next patch's table words, one patch ahead
-    const size_t pn = p + gridDim.x;
-    if (pn < n_patch) {
-      ub = poff[pn];
-      kc = pkcount[pn];
-      if (tid < patch_ne(pn)) {
-        w = reinterpret_cast<const uint4 *>(pinc + pn * PATCH_ENT)[tid];
-        ex = pexc[pn * PATCH + tid];
-        me = pmeta[pn * PATCH + tid];
-      }
-    }
-    auto ent = [&](int j) -> uint32_t {
-      const uint32_t word = j < 2 ? cw.x : j < 4 ? cw.y : j < 6 ? cw.z : cw.w;
-      return (j & 1) ? word >> 16 : word & 0xffffu;
-    };
-    T *buf = bufs + par * PATCH_ENT;
-    uint32_t *gn = gns + par * PATCH_ENT;
-    // 1. x of each run's node into its slots; the run's node into gn
-    if (have) {
-      int u = (int)cex - 1;
-      T xv = (T)0;
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const uint32_t e = ent(j);
-        if (e & ENT_START) {
-          u++;
-          const uint32_t g = pnode[cub + u];
-          xv = x[g];
-          uint32_t tag = g;
-          if (DIR && bdy[g]) {
-            xv = (T)0;
-            tag |= RUN_BDY;
-          }
-          gn[u] = tag;
-        } else if (j == 0) {
-          xv = x[pnode[cub + u]];  // the run began in an earlier thread
-          if (DIR && bdy[pnode[cub + u]]) xv = (T)0;
-        }
-        buf[e & ENT_SLOT] = xv;
-      }
-    }
-    // the patch's combined stencils (read only in step 2 of this patch, and
-    // rewritten only after every thread has passed that step's barrier)
-    const bool comb = !COEF && ckc <= (uint32_t)PKEY_MAX;
-    if (comb) {
-      for (int i = tid; i < (int)ckc * 64; i += PATCH) {
-        const uint32_t key = pkeys[p * PKEY_MAX + (i >> 6)];
-        const unsigned t = key >> 5, l = key & 31u;
-        if constexpr (sizeof(T) == 8) {
-          // FP64 issue is scarce: copy the precomputed entry
-          sc[(i >> 6) * sstride<T>() + (i & 63)] = ctab[(t * COMB_LEVELS + l) * 64 + (i & 63)];
-        } else {
-          const T h = exp2_neg((T)0, l);
-          const T *st = cs + t * fsten_stride<T>();
-          sc[(i >> 6) * sstride<T>() + (i & 63)] =
-              lapf * h * (T)0.5 * st[i & 63] + massf * h * h * h * (T)0.125 * st[64 + (i & 63)];
-        }
-      }
-    }
-    if (lane == 0) ws_first[par][wid] = (ent(0) & ENT_START) ? 1 : 0;
-    if (tid == 0) ws_first[par][NW] = 1;
-    __syncthreads();
-    // 2. element stencils, slot to slot (canonical stencil, relabelled slots)
-    if (have) {
-      const unsigned l = cme & 255u, c = (cme >> 8) & 7u, t = cme >> 24;
-      const uint32_t sig = cp[c * 18 + t];
-      T xv[8];
-#pragma unroll
-      for (int m = 0; m < 8; m++) xv[m] = buf[((sig >> (3 * m)) & 7u) * PATCH + tid];
-      auto put = [&](int m, T ym) { buf[((sig >> (3 * m)) & 7u) * PATCH + tid] = ym; };
-      if (comb) {
-        apply_comb(sc + ((cme >> 16) & 255u) * sstride<T>(), xv, put);
-      } else {
-        const T h = exp2_neg((T)0, l);
-        T lf = lapf, mf = massf;
-        if constexpr (COEF) {
-          const size_t e = p * PATCH + pperm[p * PATCH + tid];
-          lf = (T)coef[2 * e];
-          mf = (T)coef[2 * e + 1];
-        }
-        apply_full(cs + t * fsten_stride<T>(), lf * h * (T)0.5, mf * h * h * h * (T)0.125, xv, put);
-      }
-    }
-    __syncthreads();
-    // 3. run sums: segmented scan of the threads' trailing partial sums
-    T v[8];
-    T tail = (T)0;
-    int head = 0;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      const uint32_t e = ent(j);
-      v[j] = have ? buf[e & ENT_SLOT] : (T)0;
-      if (e & ENT_START) {
-        head = 1;
-        tail = (T)0;
-      }
-      tail += v[j];
-    }
-    T s = tail;
-    int f = head;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const T s2 = __shfl_up_sync(0xffffffffu, s, o);
-      const int f2 = __shfl_up_sync(0xffffffffu, f, o);
-      if (lane >= o) {
-        if (!f) s += s2;
-        f |= f2;
-      }
-    }
-    if (lane == 31) {
-      ws_v[par][wid] = s;
-      ws_f[par][wid] = f;
-    }
-    __syncthreads();
-    T wv = lane < NW ? ws_v[par][lane] : (T)0;
-    int wf = lane < NW ? ws_f[par][lane] : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const T s2 = __shfl_up_sync(0xffffffffu, wv, o);
-      const int f2 = __shfl_up_sync(0xffffffffu, wf, o);
-      if (lane >= o) {
-        if (!wf) wv += s2;
-        wf |= f2;
-      }
-    }
-    const T wpre = __shfl_sync(0xffffffffu, wv, wid > 0 ? wid - 1 : 0);
-    const T wprefix = wid > 0 ? wpre : (T)0;
-    const T ex_s = __shfl_up_sync(0xffffffffu, s, 1);
-    const int ex_f = __shfl_up_sync(0xffffffffu, f, 1);
-    const T carry = (lane == 0) ? wprefix : (ex_f ? ex_s : wprefix + ex_s);
-    const int nxt = __shfl_down_sync(0xffffffffu, (ent(0) & ENT_START) ? 1 : 0, 1);
-    if (have) {
-      const bool last_run_ends = tid + 1 >= ne || (lane < 31 ? nxt : ws_first[par][wid + 1]);
-      auto emit = [&](int u, T acc, uint32_t e) {
-        const uint32_t tag = gn[u];
-        const uint32_t g = tag & ~RUN_BDY;
-        if (DIR && (tag & RUN_BDY)) y[g] = x[g];
-        else if (e & ENT_COMPLETE) y[g] = acc;
-        else atomicAdd(&y[g], acc);
-      };
-      int u = (int)cex - 1;
-      T acc = carry;
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const uint32_t e = ent(j);
-        if (e & ENT_START) {
-          if (j > 0) emit(u, acc, ent(j - 1));
-          u++;
-          acc = (T)0;
-        }
-        acc += v[j];
-      }
-      if (last_run_ends) emit(u, acc, ent(7));
-    }
-    if (NBUF == 1) __syncthreads();  // the next patch rewrites buf and gn
-  }
-}
-
-// The same operator from run-indexed tables (run form).  Per
-// patch: plid[p][t] holds, for the element at (type, level) position t, the
-// patch-local run (node) index of each of its 8 vertices in the canonical
-// (relabelled) order of its stencil, and prun[poff[p] + u] the node of run u
-// with bit 31 set when the run holds every pair of its node in the mesh.
-// One block of PATCH threads per patch, grid-strided, three barriers per
-// patch:
-//   1. x of every run's node into xs[u] (runs spread over the threads, so
-//      the node ids are read coalesced), ys[u] = 0;
-//   2. thread t = element t: x from xs through its 8 run indices, the
-//      element stencil, the 8 results added into ys with shared-memory
-//      atomics;
-//   3. each run's sum stored (complete runs) or added atomically to y.
-// No per-pair slots and no segmented scan: the shared traffic per element
-// is 8 loads and 8 atomic adds, against 8 stores, 16 loads and 8 stores in
-// the pair form above.
-constexpr uint32_t PRUN_COMPLETE = 1u << 31;
-constexpr uint32_t PRUN_BDY = 1u << 30;  // the run's node lies on the domain boundary
-constexpr uint32_t PRUN_NODE = PRUN_BDY - 1;
-
-template <typename T, bool DIR>
-__global__ void __launch_bounds__(PATCH, sizeof(T) == 4 ? 3 : 2)
-    k_patch_matvec_runs(const uint32_t *__restrict__ pmeta, const uint4 *__restrict__ plid,
-                        const uint32_t *__restrict__ prun, const uint64_t *__restrict__ poff,
-                        const uint16_t *__restrict__ pkeys, const uint16_t *__restrict__ pkcount, size_t E,
-                        size_t n_patch, const T *__restrict__ fsten, const T *__restrict__ ctab,
-                        const T *__restrict__ x, T *__restrict__ y, T lapf, T massf) {
-  // FP32 keeps the canonical stencils in shared memory and forms the
-  // patch's combined stencils from them; FP64 (whose arithmetic is the
-  // scarce resource) copies the combined stencils from the (type, level)
-  // table and reads the canonical ones from global memory on the rare
-  // patches with more than PKEY_MAX keys
-  constexpr bool F32 = sizeof(T) == 4;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *cs = reinterpret_cast<T *>(smem_raw);
-  T *xs = cs + (F32 ? fsten_entries<T>() : 0);
-  T *ys = xs + PATCH_ENT;
-  T *sc = ys + PATCH_ENT;  // PKEY_MAX combined stencils (16-byte aligned)
-  if (F32)
-    for (int i = threadIdx.x; i < fsten_entries<T>(); i += PATCH) cs[i] = fsten[i];
-  const T *gst = F32 ? cs : fsten;
+  T *xs = reinterpret_cast<T *>(smem_raw);
+  T *ys = xs + (max_run + 1);
+  T *dt = ys + (max_run + 1);
   const int tid = threadIdx.x;
+  if (!COEF)
+    for (int i = tid; i < DTAB_ENTRIES; i += FAM) dt[i] = dtab[i];
+  if (tid == 0) xs[0] = (T)0;
   for (size_t p = blockIdx.x; p < n_patch; p += gridDim.x) {
-    const int ne = (int)((E - p * PATCH) < (size_t)PATCH ? (E - p * PATCH) : (size_t)PATCH);
-    const uint64_t ub = poff[p];
-    const int nr = (int)(poff[p + 1] - ub);
-    const uint32_t kc = pkcount[p];
-    const bool comb = kc <= (uint32_t)PKEY_MAX;
-    // this element's tables, loaded before the gather so that their latency
-    // overlaps it
-    uint32_t me = 0;
-    uint4 lw = make_uint4(0, 0, 0, 0);
-    if (tid < ne) {
-      me = pmeta[p * PATCH + tid];
-      lw = plid[p * PATCH + tid];
-    }
-    __syncthreads();  // the previous patch is done with xs, ys and sc (and cs is loaded)
-    // 1. gather
-    for (int u = tid; u < nr; u += PATCH) {
-      const uint32_t r = prun[ub + u];
-      xs[u] = (DIR && (r & PRUN_BDY)) ? (T)0 : x[r & PRUN_NODE];
-      ys[u] = (T)0;
-    }
-    if (comb) {
-      for (int i = tid; i < (int)kc * 64; i += PATCH) {
-        const uint32_t key = pkeys[p * PKEY_MAX + (i >> 6)];
-        const unsigned t = key >> 5, l = key & 31u;
-        if constexpr (F32) {
-          const T h = exp2_neg((T)0, l);
-          const T *st = cs + t * fsten_stride<T>();
-          sc[(i >> 6) * sstride<T>() + (i & 63)] =
-              lapf * h * (T)0.5 * st[i & 63] + massf * h * h * h * (T)0.125 * st[64 + (i & 63)];
-        } else {
-          sc[(i >> 6) * sstride<T>() + (i & 63)] = ctab[(t * COMB_LEVELS + l) * 64 + (i & 63)];
-        }
-      }
+    const bool have = p * FAM + tid < n_fam;
+    const uint4 info = pinfo[p];
+    const size_t base = (size_t)info.x | (size_t)info.y << 32;
+    const int nr = (int)info.z;
+    uint4 w[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) w[q] = have ? fam[(p * 4 + q) * FAM + tid] : make_uint4(0, 0, 0, 0);
+    __syncthreads();  // the previous patch is done with xs and ys
+#pragma unroll 4
+    for (int u = tid; u < nr; u += FAM) {
+      const uint32_t r = prun[base + u];
+      xs[u + 1] = (DIR && (r & PRUN_BDY)) ? (T)0 : x[r & PRUN_NODE];
+      ys[u + 1] = (T)0;
     }
     __syncthreads();
-    // 2. element stencils
-    if (tid < ne) {
-      const uint32_t lv[4] = {lw.x, lw.y, lw.z, lw.w};
-      int lid[8];
+    if (have) {
+      const uint32_t mask = fam_mask(w), hang = fam_hang(w);
+      T u[27];
+      auto gather = [&]() {
 #pragma unroll
-      for (int m = 0; m < 8; m++) lid[m] = (int)((lv[m >> 1] >> ((m & 1) * 16)) & 0xffffu);
-      T xv[8];
-#pragma unroll
-      for (int m = 0; m < 8; m++) xv[m] = xs[lid[m]];
-      auto put = [&](int m, T ym) { atomicAdd(&ys[lid[m]], ym); };
-      if (comb) {
-        apply_comb(sc + ((me >> 16) & 255u) * sstride<T>(), xv, put);
+        for (int i = 0; i < 27; i++) u[i] = xs[fam_u16(w, i)];
+        lat_interpolate(u, hang);
+      };
+      gather();
+      bool regather = false;
+      // a warp takes one path: both cost more than the dearer one
+      bool whole = !COEF && __all_sync(__activemask(), mask == 255u);
+      if (whole) {
+        lat_forward(u);
+        regather = !is_finite(u[0]);  // the weighted sum of all 27
+        whole = !regather;
+      }
+      if (whole) {
+        const T *d = dt + fam_level(w) * DTAB_STRIDE;
+        lat_scale(u, [&](T t, int i) { return t * d[i]; });
+        lat_backward(u);
       } else {
-        const unsigned l = me & 255u, t = me >> 24;
-        const T h = exp2_neg((T)0, l);
-        apply_full(gst + t * fsten_stride<T>(), lapf * h * (T)0.5, massf * h * h * h * (T)0.125, xv, put);
+        if (regather) gather();
+        T v[27], d[4];
+        if constexpr (!COEF) {
+#pragma unroll
+          for (int k = 0; k < 4; k++) d[k] = dt[fam_level(w) * DTAB_STRIDE + DTAB_CHILD + k];
+        }
+        lat_elements(
+            u, v, mask,
+            [&](int c) {
+              if constexpr (COEF) {
+                const size_t e = fchild[8 * (p * FAM + tid) + c];  // 0 where there is none
+                const T h = exp2_neg((T)0, fam_level(w));
+                const T lf = (T)coef[2 * e] * h * (T)0.5, mf = (T)coef[2 * e + 1] * h * h * h * (T)0.125;
+#pragma unroll
+                for (int k = 0; k < 4; k++) d[k] = dtab_entry(DTAB_CHILD + k, lf, mf);
+              }
+            },
+            [&](T t, int q) { return t * d[q]; });
+#pragma unroll
+        for (int i = 0; i < 27; i++) u[i] = v[i];
+      }
+      lat_distribute(u, hang);
+#pragma unroll
+      for (int i = 0; i < 27; i++) {
+        const uint32_t n = fam_u16(w, i);
+        if (n) atomicAdd(&ys[n], u[i]);
       }
     }
     __syncthreads();
-    // 3. run sums out (the run words are read again: cached since step 1)
-    for (int u = tid; u < nr; u += PATCH) {
-      const uint32_t r = prun[ub + u], g = r & PRUN_NODE;
+#pragma unroll 4
+    for (int u = tid; u < nr; u += FAM) {
+      const uint32_t r = prun[base + u], g = r & PRUN_NODE;
       if (DIR && (r & PRUN_BDY)) y[g] = x[g];
-      else if (r & PRUN_COMPLETE) y[g] = ys[u];
-      else atomicAdd(&y[g], ys[u]);
+      else if (r & PRUN_COMPLETE) y[g] = ys[u + 1];
+      else atomicAdd(&y[g], ys[u + 1]);
     }
   }
 }
 
-// ---- double-single (FP32 pair) form of the run-form loop: the CG operator
-// of the FP32-V-cycle solve.  GB300 issues FP64 at 2 multiply-adds per
-// clock per SM, and the FP64 loop is bound by that.  Here each stencil
-// entry a and each gathered x are pairs (hi, lo) of FP32 values with
-// hi + lo equal to the FP64 value to about 2^-48; each product is formed
-// exactly (hi * hi and its rounding error by an FMA, plus the two cross
-// terms) and the 8 products of a row are summed with an error-free sum
-// (TwoSum) into a (hi, lo) pair, so a row is exact to about 2^-46 of the
-// sum of its terms' magnitudes.  The row results are summed per run in
-// 64-bit fixed point (below), so an element costs no FP64 operation at all;
-// only the split of each gathered x and each run's final sum use the FP64
-// pipe.  The paired instructions (f32x2) keep the compiler from fusing the
-// sums with the products, as the explicit FMAs do for the exact products.
-//
-// ds_term2: two rows k, k + 1 at once; a = (hi_k, hi_k+1, lo_k, lo_k+1) of
-// column j, x = (hi, lo) of x_j; (sh, sl) hold the two rows' running
-// (hi, lo) sums
-__device__ __forceinline__ void ds_term2(float2 &sh, float2 &sl, float4 a, float2 x) {
-  const float2 ah = make_float2(a.x, a.y), al = make_float2(a.z, a.w);
-  const float2 xh = make_float2(x.x, x.x), xl = make_float2(x.y, x.y);
-  const float2 ph = fmul2(ah, xh);
-  float2 pl = make_float2(fmaf(a.x, x.x, -ph.x), fmaf(a.y, x.x, -ph.y));  // exact: hi * hi - ph
-  pl = ffma2(ah, xl, pl);
-  pl = ffma2(al, xh, pl);
-  const float2 s = fadd2(sh, ph);
-  const float2 v = fsub2(s, sh);
-  const float2 e = fadd2(fsub2(sh, fsub2(s, v)), fsub2(ph, v));
-  sl = fadd2(sl, fadd2(e, pl));
-  sh = s;
+template <typename T>
+inline size_t family_smem(int max_run) {
+  return (2 * (size_t)(max_run + 1) + DTAB_ENTRIES) * sizeof(T);
 }
 
-// round(f * 2^s) as a 64-bit integer, by integer operations (the ALU
-// pipe): FP32 normal and subnormal values; the caller keeps |f| * 2^s below
-// 2^62
-__device__ __forceinline__ long long f2fix(float f, int s) {
-  const uint32_t u = __float_as_uint(f);
-  if (!(u & 0x7fffffffu)) return 0;
-  const int e = (int)((u >> 23) & 0xffu);
-  const long long m = e ? (long long)((u & 0x7fffffu) | 0x800000u) : (long long)(u & 0x7fffffu);
-  const int sh = (e ? e : 1) - 150 + s;  // f * 2^s = m * 2^sh
-  long long r;
-  if (sh >= 0) r = m << (sh < 39 ? sh : 39);
-  else if (sh > -63) r = (m + (1ll << (-sh - 1))) >> (-sh);
+// ---- fixed-point form for FP64 vectors: the CG operator (K + M, Dirichlet)
+// of the FP32-V-cycle solve.  GB300 issues FP64 at 2 multiply-adds per clock
+// per SM, and the FP64 loop is bound by that.  In the sum / difference basis
+// the operator is additions and one factor per mode, a small integer over
+// 27 * 2^k times powers of two of the level, so integers do all of it: each
+// patch takes its x as 51-bit fixed point relative to the patch's largest
+// entry, the sums and differences are exact, a mode's product is exact before
+// its shift, and the node sums are integer atomic adds; 1/27 is applied to
+// each node's sum.  With |x| < 2^51 a mode's product stays below 2^62
+// (1728 + 144 times |x| at the most) and a node's sum too (at most 75 alpha
+// times 27 |x|).  The rounding of x is 2^-52 of the patch's largest entry and
+// that of the modes smaller.  Conversions are integer operations as well, so
+// the loop issues one FP64 multiplication per node and the global adds.
+// Against FP64 on uniform random x the result is off by 1.4e-16 of its norm
+// (1.4e-15 for the FP32-pair arithmetic it replaces).  Blocks per SM: at 3, 4, 5,
+// 6 blocks 367, 319, 293, 293 us on 1.1e7 elements.
+
+// x * 2^s rounded to an integer (|x| * 2^s < 2^51)
+__device__ __forceinline__ long long double_to_fix(unsigned long long bits, int s) {
+  const int e = (int)(bits >> 52) & 0x7ff;
+  unsigned long long m = bits & 0xfffffffffffffull;
+  if (e) m |= 1ull << 52;
+  const int sh = (e ? e : 1) - 1075 + s;
+  unsigned long long r;
+  if (sh >= 0) r = m << sh;
+  else if (sh > -55) r = (m + (1ull << (-sh - 1))) >> -sh;
   else r = 0;
-  return (u >> 31) ? -r : r;
+  return (bits >> 63) ? -(long long)r : (long long)r;
 }
 
-constexpr int DS_STRIDE = 32;  // float4 entries per combined stencil: (row pair, column)
+// f * 2^-s as FP64, rounded
+__device__ __forceinline__ double fix_to_double(long long f, int s) {
+  const unsigned long long a = f < 0 ? 0ull - (unsigned long long)f : (unsigned long long)f;
+  if (!a) return 0.0;
+  const int lz = __clzll((long long)a);
+  const int e = 1023 + 63 - lz - s;  // biased exponent before rounding
+  if (e < 1 || e > 2045) return ldexp((double)f, -s);
+  // 53 bits with the leading one, which adds 1 to the exponent field
+  const unsigned long long m = lz <= 10 ? (a + (1ull << (10 - lz))) >> (11 - lz) : a << (lz - 11);
+  return __longlong_as_double((long long)((((unsigned long long)(e - 1)) << 52) + m) |
+                              (f < 0 ? (long long)(1ull << 63) : 0ll));
+}
 
-// ctab: the combined stencils of every (type, level) as (hi, lo) pairs,
-// laid out per (row pair p, column j) as (hi[2p][j], hi[2p+1][j],
-// lo[2p][j], lo[2p+1][j]);
-// rowabs: per (type, level) the largest row sum of |entries| (rounded up).
-// x is scaled by xscale = 2^k on the way in and the results by 2^yshift =
-// 2^-k on the way out (both exact), so that the FP32 parts stay far from
-// FP32's underflow whatever the vectors' magnitude.  The row results are
-// summed per run in 64-bit fixed point (shared-memory integer atomic adds;
-// FP64 shared-memory atomic adds cost about three FP64 operations each on
-// GB300's narrow FP64 pipe): the patch's scale 2^s makes (largest |x| of
-// the patch) x (largest row sum of its stencils) x 4096 (the most pairs a
-// run can have) smaller than 2^62, so no sum overflows, and a row result is
-// kept to 2^-50 of that bound.
 template <bool DIR>
-__global__ void __launch_bounds__(PATCH, 2)
-    k_patch_matvec_runs_ds(const uint32_t *__restrict__ pmeta, const uint4 *__restrict__ plid,
-                           const uint32_t *__restrict__ prun, const uint64_t *__restrict__ poff,
-                           const uint16_t *__restrict__ pkeys, const uint16_t *__restrict__ pkcount, size_t E,
-                           size_t n_patch, const float4 *__restrict__ ctab, const float *__restrict__ rowabs,
-                           const double *__restrict__ x, double *__restrict__ y, double xscale, int yshift) {
+__global__ void __launch_bounds__(FAM, 5)
+    k_family_matvec_fix(const uint4 *__restrict__ fam, const uint32_t *__restrict__ prun,
+                        const uint4 *__restrict__ pinfo, size_t n_fam, size_t n_patch, int max_run,
+                        const double *__restrict__ x, double *__restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2 *xs = reinterpret_cast<float2 *>(smem_raw);
-  unsigned long long *ys = reinterpret_cast<unsigned long long *>(xs + PATCH_ENT);
-  float4 *sc = reinterpret_cast<float4 *>(ys + PATCH_ENT);  // PKEY_MAX combined stencils
-  __shared__ uint32_t xmax_bits[2], smax_bits[2];  // per patch parity: largest |x|, largest row sum
+  long long *xs = reinterpret_cast<long long *>(smem_raw);
+  long long *ys = xs + (max_run + 1);
+  __shared__ uint32_t s_emax[2];  // largest biased exponent of the patch's x, by patch parity
   const int tid = threadIdx.x;
-  if (tid < 2) xmax_bits[tid] = smax_bits[tid] = 0;
+  if (tid < 2) s_emax[tid] = 0;
+  if (tid == 0) xs[0] = 0;
   int par = 0;
   for (size_t p = blockIdx.x; p < n_patch; p += gridDim.x, par ^= 1) {
-    const int ne = (int)((E - p * PATCH) < (size_t)PATCH ? (E - p * PATCH) : (size_t)PATCH);
-    const uint64_t ub = poff[p];
-    const int nr = (int)(poff[p + 1] - ub);
-    const uint32_t kc = pkcount[p];
-    const bool comb = kc <= (uint32_t)PKEY_MAX;
-    uint32_t me = 0;
-    uint4 lw = make_uint4(0, 0, 0, 0);
-    float rmax = 0.f;
-    if (tid < ne) {
-      me = pmeta[p * PATCH + tid];
-      lw = plid[p * PATCH + tid];
-      rmax = rowabs[(me >> 24) * COMB_LEVELS + (me & 31u)];
+    const bool have = p * FAM + tid < n_fam;
+    const uint4 info = pinfo[p];
+    const size_t base = (size_t)info.x | (size_t)info.y << 32;
+    const int nr = (int)info.z;
+    uint4 w[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) w[q] = have ? fam[(p * 4 + q) * FAM + tid] : make_uint4(0, 0, 0, 0);
+    __syncthreads();  // the previous patch is done with xs, ys and its exponent
+    uint32_t emax = 0;
+#pragma unroll 4
+    for (int u = tid; u < nr; u += FAM) {
+      const uint32_t r = prun[base + u];
+      const long long b = (DIR && (r & PRUN_BDY)) ? 0ll : __double_as_longlong(x[r & PRUN_NODE]);
+      xs[u + 1] = b;
+      ys[u + 1] = 0;
+      emax = max(emax, (uint32_t)((unsigned long long)b >> 52) & 0x7ffu);
     }
-    __syncthreads();  // the previous patch is done with xs, ys, sc and its bounds
-    // 1. gather, each x split into (hi, lo); the patch's bounds
-    float xmax = 0.f;
-    for (int u = tid; u < nr; u += PATCH) {
-      const uint32_t r = prun[ub + u];
-      const double xv = (DIR && (r & PRUN_BDY)) ? 0.0 : x[r & PRUN_NODE] * xscale;
-      const float hi = __double2float_rn(xv);
-      xs[u] = make_float2(hi, __double2float_rn(xv - (double)hi));
-      ys[u] = 0ull;
-      xmax = fmaxf(xmax, fabsf(hi));
-    }
-    const uint32_t wx = __reduce_max_sync(0xffffffffu, __float_as_uint(xmax));  // non-negative: bits order as values
-    const uint32_t ws = __reduce_max_sync(0xffffffffu, __float_as_uint(rmax));
-    if ((tid & 31) == 0) {
-      atomicMax(&xmax_bits[par], wx);
-      atomicMax(&smax_bits[par], ws);
-    }
-    if (comb) {
-      for (int i = tid; i < (int)kc * DS_STRIDE; i += PATCH) {
-        const uint32_t key = pkeys[p * PKEY_MAX + i / DS_STRIDE];
-        sc[i] = ctab[((key >> 5) * COMB_LEVELS + (key & 31u)) * DS_STRIDE + i % DS_STRIDE];
+    emax = __reduce_max_sync(0xffffffffu, emax);
+    if ((tid & 31) == 0) atomicMax(&s_emax[par], emax);
+    __syncthreads();
+    emax = s_emax[par];
+    if (tid == 0) s_emax[par ^ 1] = 0;  // for the next patch
+    const bool finite = emax < 0x7ffu;
+    const int s = 1073 - (int)(emax ? emax : 1u);  // |x| * 2^s < 2^51
+    for (int u = tid; u < nr; u += FAM) xs[u + 1] = double_to_fix((unsigned long long)xs[u + 1], s);
+    __syncthreads();
+    if (have) {
+      const uint32_t mask = fam_mask(w), hang = fam_hang(w);
+      // in units of alpha / 27 of the patch's coarsest level
+      const int finer = (int)fam_level(w) - (int)info.w, mass = 2 * (int)fam_level(w) + 2;
+      long long u[27];
+#pragma unroll
+      for (int i = 0; i < 27; i++) u[i] = xs[fam_u16(w, i)];
+      lat_interpolate(u, hang);
+      auto mul = [&](long long t, int i) {
+        return (t * fix_weight(i, true) + (t >> mass) * fix_weight(i, false)) >> (finer + fix_shift(i));
+      };
+      if (__all_sync(__activemask(), mask == 255u)) {
+        lat_forward(u);
+        lat_scale(u, mul);
+        lat_backward(u);
+      } else {
+        long long v[27];
+        lat_elements(u, v, mask, [](int) {}, [&](long long t, int q) { return mul(t, DTAB_CHILD + q); });
+#pragma unroll
+        for (int i = 0; i < 27; i++) u[i] = v[i];
+      }
+      lat_distribute(u, hang);
+#pragma unroll
+      for (int i = 0; i < 27; i++) {
+        const uint32_t n = fam_u16(w, i);
+        if (n) atomicAdd(reinterpret_cast<unsigned long long *>(&ys[n]), (unsigned long long)u[i]);
       }
     }
     __syncthreads();
-    const double bound = (double)__uint_as_float(xmax_bits[par]) * (double)__uint_as_float(smax_bits[par]);
-    const int fs = bound > 0.0 ? 49 - ilogb(bound) : 0;  // the fixed-point scale 2^fs
-    const double out_scale = ldexp(1.0, yshift - fs);
-    if (tid == 0) xmax_bits[par ^ 1] = smax_bits[par ^ 1] = 0;  // for the next patch
-    // 2. element stencils
-    if (tid < ne) {
-      const uint32_t lv[4] = {lw.x, lw.y, lw.z, lw.w};
-      int lid[8];
-#pragma unroll
-      for (int m = 0; m < 8; m++) lid[m] = (int)((lv[m >> 1] >> ((m & 1) * 16)) & 0xffffu);
-      float2 xv[8];
-#pragma unroll
-      for (int m = 0; m < 8; m++) xv[m] = xs[lid[m]];
-      const float4 *S = comb ? sc + ((me >> 16) & 255u) * DS_STRIDE
-                             : ctab + ((me >> 24) * COMB_LEVELS + (me & 31u)) * DS_STRIDE;
-#pragma unroll
-      for (int pr = 0; pr < 4; pr++) {
-        float2 sh = make_float2(0.f, 0.f), sl = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < 8; j++) ds_term2(sh, sl, S[pr * 8 + j], xv[j]);
-        atomicAdd(&ys[lid[2 * pr]], (unsigned long long)(f2fix(sh.x, fs) + f2fix(sl.x, fs)));
-        atomicAdd(&ys[lid[2 * pr + 1]], (unsigned long long)(f2fix(sh.y, fs) + f2fix(sl.y, fs)));
-      }
-    }
-    __syncthreads();
-    // 3. run sums out
-    for (int u = tid; u < nr; u += PATCH) {
-      const uint32_t r = prun[ub + u], g = r & PRUN_NODE;
-      const double v = (double)(long long)ys[u] * out_scale;
+    const int sy = s + (int)info.w + 1;
+#pragma unroll 4
+    for (int u = tid; u < nr; u += FAM) {
+      const uint32_t r = prun[base + u], g = r & PRUN_NODE;
+      // a patch with a non-finite x: all its rows are NaN
+      const double v = finite ? fix_to_double(ys[u + 1], sy) * (1.0 / 27.0) : __longlong_as_double(0x7ff8000000000000ll);
       if (DIR && (r & PRUN_BDY)) y[g] = x[g];
       else if (r & PRUN_COMPLETE) y[g] = v;
       else atomicAdd(&y[g], v);
     }
   }
-}
-
-constexpr size_t patch_runs_ds_smem() {
-  return PATCH_ENT * sizeof(float2) + PATCH_ENT * sizeof(unsigned long long) + PKEY_MAX * DS_STRIDE * sizeof(float4);
-}
-
-template <typename T>
-constexpr size_t patch_runs_smem() {
-  return (sizeof(T) == 4 ? fsten_entries<T>() * sizeof(T) : 0) + 2 * PATCH_ENT * sizeof(T) +
-         PKEY_MAX * sstride<T>() * sizeof(T);
-}
-
-template <typename T>
-constexpr size_t patch_smem() {
-  return fsten_entries<T>() * sizeof(T) + patch_nbuf<T>() * PATCH_ENT * (sizeof(T) + sizeof(uint32_t)) +
-         (8 * 18 + 4) * sizeof(uint32_t) + PKEY_MAX * sstride<T>() * sizeof(T);
 }
 
 }  // namespace dg

@@ -17,7 +17,6 @@
 // Pairs with a fine or a coarse boundary node carry no weight, as with the
 // reference's suppressed Dirichlet DOFs.
 #include "dg_mg.cuh"
-#include "dg_elem.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -401,33 +400,14 @@ __global__ void k_cg_p(double *__restrict__ p, const double *__restrict__ z, con
 
 // ------------------------------------------------------------------------
 // DirichletJacobianMatMult (omgJac.C:958-1057): boundary rows are the
-// identity, boundary columns are skipped (the patch element loop with DIR)
+// identity, boundary columns are skipped (the element loop with DIR)
 template <typename T>
 void dirichlet_matvec(Context &ctx, const MGLevel &L, const T *x, T *y) {
-  ensure_stencils(ctx);
-  cudaStream_t s = ctx.stream;
   const Mesh &m = L.mesh;
-  DG_CUDA(cudaMemsetAsync(y, 0, m.n_node * sizeof(T), s));
-  if (m.plid && ctx.matvec_form != 1) {
-    launch_matvec_runs<T, true>(ctx, m, x, y, 1.0, 1.0,
+  DG_CUDA(cudaMemsetAsync(y, 0, m.n_node * sizeof(T), ctx.stream));
+  launch_family_matvec<T, true>(ctx, m, x, y, 1.0, 1.0,
                                 sizeof(T) == 4 ? "dirichlet_matvec_fp32" : "dirichlet_matvec_fp64",
                                 (double)m.n_elem * 36 + (double)m.n_node * (3 * sizeof(T) + 1));
-    return;
-  }
-  const size_t smem = patch_smem<T>();
-  ensure_smem_attr(ctx, k_patch_matvec<T, true>, (int)smem);
-  int per_sm = 1;
-  DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_patch_matvec<T, true>, PATCH, smem));
-  const unsigned grid = (unsigned)std::min<size_t>(m.n_patch, (size_t)std::max(per_sm, 1) * ctx.num_sms);
-  const T *cs = std::is_same<T, double>::value ? reinterpret_cast<const T *>(ctx.d_csten64)
-                                               : reinterpret_cast<const T *>(ctx.d_csten32);
-  ProfScope _prof(ctx, sizeof(T) == 4 ? "dirichlet_matvec_fp32" : "dirichlet_matvec_fp64",
-                  (double)m.n_elem * 36 + (double)m.n_node * (3 * sizeof(T) + 1));
-  const T *ctab = comb_table<T>(ctx, 1.0, 1.0);
-  k_patch_matvec<T, true><<<grid, PATCH, smem, s>>>(m.pmeta, m.pinc, m.pexc, m.pnode, m.poff, m.pkeys, m.pkcount,
-                                                    m.n_elem, m.n_patch, cs, ctab, ctx.d_cperm, L.bdy, x, y, (T)1,
-                                                    (T)1);
-  DG_LAUNCH_CHECK();
 }
 
 void dirichlet_diagonal(Context &ctx, const MGLevel &L, double *diag) {
@@ -701,10 +681,10 @@ void mg_solve(Context &ctx, MG &mg, const double *b, double *x, int precision, d
     k_sum<<<1, 256, 0, s>>>(part.get(), nparts, out);
     DG_LAUNCH_CHECK();
   };
-  // the CG vectors scale with b: the FP32 V-cycle, the FP32 and the
-  // double-single operators work on them scaled by 2^ds_exp (exact), of
-  // order one, away from FP32's underflow (a fine mesh's load vector is of
-  // order h^3, and the residual falls by the tolerance on top)
+  // the CG vectors scale with b: the FP32 V-cycle and the FP32 operator
+  // work on them scaled by 2^ds_exp (exact), of order one, away from FP32's
+  // underflow (a fine mesh's load vector is of order h^3, and the residual
+  // falls by the tolerance on top)
   int ds_exp = 0;
   auto precond = [&](const double *rin, double *zout) {
     if (precision == 32) {
@@ -742,7 +722,7 @@ void mg_solve(Context &ctx, MG &mg, const double *b, double *x, int precision, d
       k_to_double<<<g, 256, 0, s>>>(q32.get(), n, q.get(), std::ldexp(1.0, -ds_exp));
       DG_LAUNCH_CHECK();
     } else if (precision == 32 && mg.cg_operator == 48) {
-      dirichlet_matvec_ds(ctx, L0, p.get(), q.get(), ds_exp);
+      dirichlet_matvec_ds(ctx, L0, p.get(), q.get());
     } else {
       dirichlet_matvec<double>(ctx, L0, p.get(), q.get());
     }
@@ -814,32 +794,11 @@ void mg_solve(Context &ctx, MG &mg, const double *b, double *x, int precision, d
   res.relres = std::sqrt(read_scalar(ctx, d_rr)) / bnorm;
 }
 
-__global__ void k_absmax_bits(const double *__restrict__ x, size_t n, unsigned long long *__restrict__ out) {
-  unsigned long long m = 0;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    m = max(m, (unsigned long long)__double_as_longlong(fabs(x[i])));  // non-negative: bits order as values
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
-}
-
-void dirichlet_matvec_ds(Context &ctx, const MGLevel &L, const double *x, double *y, int scale_exp) {
+void dirichlet_matvec_ds(Context &ctx, const MGLevel &L, const double *x, double *y) {
   const Mesh &m = L.mesh;
-  if (!m.plid) {
-    dirichlet_matvec<double>(ctx, L, x, y);
-    return;
-  }
-  ensure_stencils(ctx);
-  if (scale_exp == DS_SCALE_AUTO) {  // from the largest entry of x
-    DG_CUDA(cudaMemsetAsync(ctx.d_scratch, 0, sizeof(unsigned long long), ctx.stream));
-    k_absmax_bits<<<grid_for(m.n_node, 256, (unsigned)ctx.num_sms * 4), 256, 0, ctx.stream>>>(x, m.n_node,
-                                                                                         ctx.d_scratch);
-    DG_LAUNCH_CHECK();
-    const double xmax = __builtin_bit_cast(double, (unsigned long long)read_scalar(ctx, ctx.d_scratch));
-    scale_exp = xmax > 0 && std::isfinite(xmax) ? std::max(-900, std::min(900, -std::ilogb(xmax))) : 0;
-  }
   DG_CUDA(cudaMemsetAsync(y, 0, m.n_node * sizeof(double), ctx.stream));
-  launch_matvec_runs_ds<true>(ctx, m, x, y, 1.0, 1.0, scale_exp, "dirichlet_matvec_ds",
-                              (double)m.n_elem * 36 + (double)m.n_node * (3 * sizeof(double) + 1));
+  launch_family_matvec_fix(ctx, m, x, y, "dirichlet_matvec_ds",
+                           (double)m.n_elem * 36 + (double)m.n_node * (3 * sizeof(double) + 1));
 }
 
 template void dirichlet_matvec<float>(Context &, const MGLevel &, const float *, float *);

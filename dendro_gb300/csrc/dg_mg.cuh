@@ -36,8 +36,7 @@ struct MG {
   double omega = 0.667;  // Jacobi damping (bin/options:190)
   int nu_pre = 2, nu_post = 2;
   // CG operator with an FP32 V-cycle: 48 (the default) applies A p in
-  // double-single arithmetic on FP64 vectors (about 2^-46 relative per
-  // element row); 64 in FP64; 32 in FP32, with the recurrence residual
+  // 64-bit fixed point on FP64 vectors (dg_elem.cuh); 64 in FP64; 32 in FP32, with the recurrence residual
   // replaced by the FP64 residual b - A x whenever it has fallen by
   // reliable_delta since the last replacement (and before stopping)
   int cg_operator = 48;
@@ -65,13 +64,8 @@ void mg_solve(Context &ctx, MG &mg, const double *b, double *x, int precision, d
 // building blocks (level operators), exposed for tests and callers
 template <typename T>
 void dirichlet_matvec(Context &ctx, const MGLevel &L, const T *x, T *y);  // DirichletJacobianMatMult
-// the same operator on FP64 vectors in double-single arithmetic (FP32
-// pairs, about 2^-46 relative per element row; the FP64 loop where a mesh
-// has no run tables)
-// (scale_exp: x is multiplied by 2^scale_exp inside the loop, chosen so
-// that x is of order one; DS_SCALE_AUTO takes it from x's largest entry)
-constexpr int DS_SCALE_AUTO = -100000;
-void dirichlet_matvec_ds(Context &ctx, const MGLevel &L, const double *x, double *y, int scale_exp = DS_SCALE_AUTO);
+// the same operator on FP64 vectors in 64-bit fixed point (dg_elem.cuh)
+void dirichlet_matvec_ds(Context &ctx, const MGLevel &L, const double *x, double *y);
 // DirichletJacobianMatGetDiagonal (omgJac.C:1111): 1 on boundary nodes
 void dirichlet_diagonal(Context &ctx, const MGLevel &L, double *diag);
 template <typename T>

@@ -52,21 +52,13 @@ struct Context {
   float *d_sten32 = nullptr;
   uint8_t *d_etype_of = nullptr;   // [8][256] -> element type or 255
   uint8_t *d_etype_mask = nullptr; // [8][18] -> hanging mask
-  double *d_csten64 = nullptr;     // canonical full stencils, 18 types (dg_elem.cuh)
-  float *d_csten32 = nullptr;
-  uint32_t *d_cperm = nullptr;     // [8][18] vertex relabelling, 3 bits each
-  // combined stencils lapf 2^-l/2 L_t + massf 2^-3l/8 M_t per (type, level)
-  // for the factors of the last element loop (dg_elem.cuh, comb_table)
-  double *d_comb64 = nullptr;
-  float *d_comb32 = nullptr;
-  double comb64_f[2] = {0, 0}, comb32_f[2] = {0, 0};
-  bool comb64_ok = false, comb32_ok = false;
-  // the FP64 combined stencils as (hi, lo) FP32 pairs, two rows per float4
-  // (double-single loop)
-  float4 *d_comb_ds = nullptr;
-  float *d_comb_rowabs = nullptr;  // per (type, level): largest row sum of |combined stencil entries|
-  double comb_ds_f[2] = {0, 0};
-  bool comb_ds_ok = false;
+  // diagonal tables of the element loop (dg_elem.cuh) for the factors of its
+  // last call
+  struct DiagTable {
+    void *p = nullptr;
+    double lap = 0, mass = 0;
+    bool ok = false;
+  } dtab64, dtab32;
   bool prof = false;
   std::map<std::string, ProfStat> prof_stats;
   std::vector<ProfPending> prof_pending;
@@ -83,9 +75,6 @@ struct Context {
   // 0 Morton, 1 Hilbert (the reference's HILBERT_ORDERING builds); the
   // octrees themselves are always kept in Morton order on the device
   int order = 0;
-  // FP32 element loop form: 0 the run form where the mesh has its tables,
-  // 1 the pair form (dg_ctx_set_matvec_form)
-  int matvec_form = 0;
 };
 
 // thrown inside the library, converted to a status code at the C ABI

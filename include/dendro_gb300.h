@@ -84,12 +84,9 @@ const char *dg_status_string(int status);
 int dg_version(void);
 
 /* Form of the element loop (dg_matvec, dg_mg_matvec, the V-cycle and the
- * CG operator, FP32 and FP64): DG_MATVEC_RUNS (the default) sums each
- * element's results into patch-local node slots, DG_MATVEC_PAIRS sums them
- * through per-pair slots and a segmented scan.  Both give the same operator
- * (to the rounding of the precision); a compressed DA and the
- * per-element-factor loop always use the pair form.  No counterpart in the
- * reference. */
+ * CG operator, FP32 and FP64).  One loop over families of sibling elements
+ * now serves every mesh, precision and option; both values are accepted and
+ * select it.  No counterpart in the reference. */
 #define DG_MATVEC_RUNS 0
 #define DG_MATVEC_PAIRS 1
 int dg_ctx_set_matvec_form(dg_ctx ctx, int form);
@@ -265,8 +262,8 @@ int dg_octree_read_binary(dg_ctx ctx, const char *path, dg_octree *out);
 int dg_da_build(dg_ctx ctx, dg_octree balanced, dg_da *out);
 /* ot::DA with compressLut (include/oda/oda.h:622, decoded by
  * getNodeIndices, include/oda/oda.tcc:1304-1420): compressLut = 1 keeps only
- * the element loop's per-patch tables (16-bit slots per element vertex and
- * one node id per node run) and releases the plain 8 x u32 node list; the
+ * the element loop's family tables (a 16-bit node number per lattice point of
+ * 8 siblings and the nodes of each patch) and releases the plain 8 x u32 node list; the
  * node list is decoded from the tables when a call needs it
  * (dg_da_download, dg_da_assemble).  Results are identical in both modes.
  * dg_da_memory: device bytes the DA holds. */
@@ -323,7 +320,7 @@ int dg_mg_level_nodes(dg_ctx ctx, dg_mg mg, size_t level, uint32_t *node_xyz, in
 int dg_mg_level_octree(dg_ctx ctx, dg_mg mg, size_t level, uint32_t *xyzl, int dst_on_device);
 /* DirichletJacobianMatMult on a level: boundary rows identity, boundary
  * columns skipped.  precision 32 / 64 as dg_matvec; 48: FP64 vectors in
- * double-single arithmetic (the CG operator of dg_mg_set_cg_operator 48). */
+ * 64-bit fixed point (the CG operator of dg_mg_set_cg_operator 48). */
 int dg_mg_matvec(dg_ctx ctx, dg_mg mg, size_t level, const void *in, void *out, int precision, int on_device);
 /* restrictMatVecType1: out (level+1) = R in (level); prolongMatVecType1:
  * out (level) = P in (level+1), P = R^T. */
@@ -334,10 +331,9 @@ int dg_mg_prolong(dg_ctx ctx, dg_mg mg, size_t fine_level, const void *in, void 
 int dg_mg_set_smoother(dg_mg mg, double omega, int nu_pre, int nu_post);
 /* The CG's own operator application q = A p when the V-cycle runs in FP32
  * (precision 32 of dg_mg_solve).  48 (the default): A p on the FP64
- * vectors in double-single arithmetic (stencil entries and x as FP32 pairs,
- * each element row exact to about 2^-46 of its terms, summed across
- * elements in FP64; GB300's FP64 pipe issues 2 multiply-adds per clock per
- * SM).  64: A p in FP64 every iteration.  32: A p in FP32
+ * vectors in 64-bit fixed point (x to 2^-52 of the largest entry of its
+ * patch of about 950 elements, the sums in integers; GB300's FP64 pipe issues
+ * 2 multiply-adds per clock per SM).  64: A p in FP64 every iteration.  32: A p in FP32
  * (the FP32 element loop), and the recurrence
  * residual replaced by the FP64 residual b - A x whenever it has fallen by
  * reliable_delta since the last replacement, and before the stopping test
