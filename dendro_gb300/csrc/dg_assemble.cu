@@ -197,6 +197,7 @@ void assemble_csr(Context &ctx, const Mesh &m, const uint8_t *bdy, double lap_fa
     DG_LAUNCH_CHECK();
   }
   uint64_t *key = radix_sort<uint64_t>(ctx, ka.get(), kb.get(), np, 32 + (int)bits_of(V));
+  check_device_flags(ctx, "radix sort");
   DBuf<uint64_t> start(V + 1, s);
   DBuf<uint32_t> len(V, s);
   DBuf<unsigned> dmax(1, s);

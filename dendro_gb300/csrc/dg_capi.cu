@@ -144,8 +144,8 @@ int dg_ctx_create(int device, dg_ctx *out) {
     ctx->c.own_stream = true;
     DG_CUDA(cudaMalloc((void **)&ctx->c.d_flags, sizeof(uint32_t)));
     DG_CUDA(cudaMemset(ctx->c.d_flags, 0, sizeof(uint32_t)));
-    DG_CUDA(cudaMalloc((void **)&ctx->c.d_scratch, 64 * sizeof(unsigned long long)));
-    DG_CUDA(cudaMallocHost((void **)&ctx->c.h_scratch, 64 * sizeof(unsigned long long)));
+    DG_CUDA(cudaMalloc((void **)&ctx->c.d_scratch, 96 * sizeof(unsigned long long)));
+    DG_CUDA(cudaMallocHost((void **)&ctx->c.h_scratch, 96 * sizeof(unsigned long long)));
     DG_CUDA(cudaDeviceGetAttribute(&ctx->c.num_sms, cudaDevAttrMultiProcessorCount, device));
     DG_CUDA(cudaEventCreate(&ctx->ev0));
     DG_CUDA(cudaEventCreate(&ctx->ev1));

@@ -108,6 +108,8 @@ enum {
   DGF_TIMEOUT = 4u,        // a bounded spin gave up
   DGF_INTERNAL = 8u,       // internal consistency check failed
   DGF_ORDER = 16u,         // input not sorted / unique as the caller declared
+  DGF_LONG_RUN = 32u,      // a run of keys with one sorted prefix is too long to order in place
+  DGF_CAPACITY = 64u,      // a table sized by estimate is full (the host retries with a larger one)
 };
 
 }  // namespace dg

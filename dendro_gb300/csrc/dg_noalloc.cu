@@ -38,7 +38,6 @@ struct NaHeader {
   uint32_t active;        // bit p: digit pass p has more than one occupied bin
   uint32_t count;         // unique keys
   unsigned tile_counter;  // onesweep tile tickets
-  int shifts[OS_MAX_PASSES];
 };
 static_assert(sizeof(NaHeader) <= NA_ALIGN, "header fits its slot");
 
@@ -103,10 +102,6 @@ __global__ void k_na_quantize(const double *__restrict__ xyz, size_t n, double s
     atomicOr(flags, DGF_DOMAIN);
   }
   keys[i] = make_tagged(morton3(ux, uy, uz), D);
-}
-
-__global__ void k_na_shifts(int *shifts, int npass) {
-  if ((int)threadIdx.x < npass) shifts[threadIdx.x] = 8 * (int)threadIdx.x;
 }
 
 // per digit pass: exclusive scan of the 256 bins into digit offsets, and the
@@ -196,10 +191,8 @@ extern "C" int dg_sort_unique_points_noalloc(const double *xyz, size_t n, const 
   // digits of the anchor bits [0, 3D); the level byte is D for every key
   const int npass = (3 * (int)maxDepth + 7) / 8;
   if (npass > 0) {
-    k_na_shifts<<<1, 32, 0, s>>>(hdr->shifts, npass);
-    NA_TRY(cudaGetLastError());
     k_rs_digit_hists<Key128><<<grid_for(n, RS_BLOCK, (unsigned)(nd.num_sms * 4)), RS_BLOCK, 0, s>>>(
-        keys_a, n, npass, hdr->shifts, ghist);
+        keys_a, n, npass, 0, ghist);
     NA_TRY(cudaGetLastError());
     k_na_plan<<<1, 256, 0, s>>>(ghist, npass, offs, &hdr->active);
     NA_TRY(cudaGetLastError());

@@ -5,28 +5,34 @@
 // segment s lives in key bits [3D, 3D + seg_bits) (dg_octree.cuh), so every
 // sort, NCA and gap computation below stays inside its own cloud.
 //
+// Both pipelines describe an octree by its internal octants ("nodes"), sorted
+// in preorder, and write the leaves from them (k_emit_leaves): with i the
+// preorder index of a node of level d and digits(.) the sum of its path's
+// child numbers, 7 (i - d) + digits leaves precede it, so every leaf's place
+// follows from the nodes before it and no leaf is sorted or counted.
+//
 // Construction (unique points, reference p2oLocal, src/construct.cpp:976):
 // the leaf that holds point i is the child of its deepest ancestor that
 // contains more than maxPts points.  With the points in Morton order that
 // ancestor's level is max_j NCA(p_j, p_{j+m}) over the windows j in
-// [i-m, i] (m = maxPts), so every point's leaf is computed independently;
-// the empty leaves between consecutive point leaves are the maximal aligned
-// Morton blocks of the gap.  Inputs with repeated points take the
-// reference's sequential walk verbatim (a single-thread kernel), because its
-// point bookkeeping then departs from the rule above.
+// [i-m, i] (m = maxPts), and the nodes on the way to that leaf that do not
+// hold point i-1 are new at i: each point emits its nodes independently, in
+// preorder.  Inputs with repeated points take the reference's sequential walk
+// verbatim (a single-thread kernel), because its point bookkeeping then
+// departs from the rule above.
 //
 // Balance (reference comboRipple, src/balance.cpp:801): the coarsest 2:1
-// balanced refinement is unique.  With I_l the internal nodes at level l,
+// balanced refinement is unique.  With I_l the nodes at level l,
 //   I_{l-1} = parent(input leaves at level l) U parents of the 3x3x3 blocks
-//             around every q in I_l (8 octants per q, clipped to the domain)
-// and the balanced leaves at level l are children(I_{l-1}) \ I_l.  Each
-// level is one generate + radix sort + unique; the leaves are then placed in
-// Morton order by a bottom-up leaf count and a top-down offset pass.
+//             around every q in I_l (8 octants per q, clipped to the domain).
+// The sets grow in one hash table, level by level from the deepest, without
+// a read-back between levels; one radix sort puts all nodes in preorder.
 #include "dg_octree.cuh"
 #include "dg_walk.cuh"
 
 #include <algorithm>
 #include <array>
+#include <climits>
 #include <cmath>
 #include <vector>
 
@@ -55,49 +61,109 @@ __host__ __device__ __forceinline__ Key128 seg_key(uint64_t seg, unsigned D) {
 // ------------------------------------------------------------------------
 // quantize + Morton key (construct.cpp:930-942)
 // ------------------------------------------------------------------------
-// (unsigned int)(x * (double)(1u << D) / gLen): multiply, divide, truncate.
-// When every gLen is a power of two (the unit cube of the workloads), its
-// reciprocal is exact and x * 2^D * (1 / gLen) is the same correctly rounded
-// value as the division (both round the same exact quotient), without the
-// FP64 divide.
+// (unsigned int)(x * (double)(1u << D) / gLen): multiply, divide, truncate;
+// valid iff the value before truncation lies in (-1, 2^D).  False otherwise.
+//
+// When gLen is a power of two 2^e (the unit cube of the workloads) both
+// operations only move the exponent, so the value is x * 2^(D - e), truncated
+// from the bits of x by integer shifts: GB300's narrow FP64 pipe, which the
+// multiplications, comparisons and conversions of three coordinates kept busy,
+// does nothing (16e6 points: 0.45 -> 0.14 ms).  Where x * 2^D would leave the
+// normal range the value is 0 or out of the domain either way.
+__device__ __forceinline__ bool quantize_pow2(double x, int shift, unsigned D, uint32_t &q) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int e = (int)(b >> 52 & 0x7ffu) - 1023 + shift;  // |value| in [2^e, 2^(e+1)), or below 2^e for subnormals
+  q = 0;
+  if (e < 0) return true;  // in (-1, 1)
+  if ((long long)b < 0 || e >= (int)D) return false;  // also infinities and NaN: e >= 1024 + shift > D
+  q = (uint32_t)((b & 0xfffffffffffffull | 1ull << 52) >> (52 - e));
+  return true;
+}
+__device__ __forceinline__ bool quantize_div(double x, double scale, double g, uint32_t &q) {
+  const double v = __ddiv_rn(__dmul_rn(x, scale), g);
+  q = 0;
+  if (!(v > -1.0 && v < scale)) return false;
+  q = (uint32_t)__double2uint_rz(v);
+  return true;
+}
+
+// gx, gy, gz: the domain's lengths, or with POW2 the exponents D - e of the
+// shifts.  vary collects the bits on which the keys differ from the first
+// point's (two 64-bit words) where it is wanted.
 template <bool POW2>
 __global__ void k_quantize(const double *__restrict__ xyz, size_t n, double scale, double gx, double gy, double gz,
                            unsigned D, const uint64_t *__restrict__ seg_start, size_t nseg, Key128 *__restrict__ keys,
-                           uint32_t *flags) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
-  double qx, qy, qz;
-  if constexpr (POW2) {  // gx, gy, gz hold the exact reciprocals here
-    qx = __dmul_rn(__dmul_rn(x, scale), gx);
-    qy = __dmul_rn(__dmul_rn(y, scale), gy);
-    qz = __dmul_rn(__dmul_rn(z, scale), gz);
-  } else {
-    qx = __ddiv_rn(__dmul_rn(x, scale), gx);
-    qy = __ddiv_rn(__dmul_rn(y, scale), gy);
-    qz = __ddiv_rn(__dmul_rn(z, scale), gz);
-  }
-  // valid iff the truncated value lies in [0, 2^D): q in (-1, 2^D); NaN fails
-  bool ok = (qx > -1.0) && (qx < scale) && (qy > -1.0) && (qy < scale) && (qz > -1.0) && (qz < scale);
-  uint32_t ux = 0, uy = 0, uz = 0;
-  if (ok) {
-    ux = (uint32_t)__double2uint_rz(qx);
-    uy = (uint32_t)__double2uint_rz(qy);
-    uz = (uint32_t)__double2uint_rz(qz);
-  } else {
-    set_flag(flags, DGF_DOMAIN);
-  }
-  Key128 k = morton3(ux, uy, uz);
-  if (seg_start) {  // segment of point i: last s with seg_start[s] <= i
-    size_t lo = 0, hi = nseg;
-    while (hi - lo > 1) {
-      size_t mid = (lo + hi) / 2;
-      if (seg_start[mid] <= i) lo = mid;
-      else hi = mid;
+                           unsigned long long *__restrict__ vary, uint32_t *flags) {
+  __shared__ Key128 first;
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  auto key_of = [&](size_t j, bool &ok) {
+    uint32_t u[3];
+    ok = true;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      const double g = a == 0 ? gx : a == 1 ? gy : gz;
+      if constexpr (POW2) ok = quantize_pow2(xyz[3 * j + a], (int)g, D, u[a]) && ok;
+      else ok = quantize_div(xyz[3 * j + a], scale, g, u[a]) && ok;
     }
-    k = key_or(k, seg_key(lo, D));
+    if (!ok) u[0] = u[1] = u[2] = 0;
+    return morton3(u[0], u[1], u[2]);
+  };
+  Key128 diff{0, 0};
+  bool ok;
+  if (vary) {
+    if (threadIdx.x == 0) first = key_of(0, ok);
+    __syncthreads();
   }
-  keys[i] = make_tagged(k, D);
+  if (i < n) {
+    Key128 k = key_of(i, ok);
+    if (!ok) set_flag(flags, DGF_DOMAIN);
+    if (seg_start) {  // segment of point i: last s with seg_start[s] <= i
+      size_t lo = 0, hi = nseg;
+      while (hi - lo > 1) {
+        size_t mid = (lo + hi) / 2;
+        if (seg_start[mid] <= i) lo = mid;
+        else hi = mid;
+      }
+      k = key_or(k, seg_key(lo, D));
+    }
+    keys[i] = make_tagged(k, D);
+    if (vary) diff = key_xor(k, first);
+  }
+  if (vary) {
+#pragma unroll
+    for (int h = 0; h < 4; h++) {
+      const uint64_t w = h < 2 ? diff.lo : diff.hi;
+      const uint32_t v = __reduce_or_sync(0xffffffffu, (uint32_t)(h & 1 ? w >> 32 : w));
+      if ((threadIdx.x & 31) == 0 && v) {
+        const unsigned long long bits = (unsigned long long)v << (h & 1 ? 32 : 0);
+        if (bits & ~__ldcg(vary + (h >> 1))) atomicOr(vary + (h >> 1), bits);
+      }
+    }
+  }
+}
+
+// Orders runs of keys that agree above `begin` bits by the bits below, in
+// place, one thread per run (an insertion sort); a run longer than RUN_MAX
+// raises DGF_LONG_RUN.
+constexpr int RUN_MAX = 32;
+__global__ void k_sort_runs(Key128 *__restrict__ k, size_t n, unsigned begin, uint32_t *flags) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i + 1 >= n) return;
+  const Key128 pre = key_shr(tag_anchor(k[i]), begin);
+  if (!key_eq(key_shr(tag_anchor(k[i + 1]), begin), pre)) return;
+  if (i > 0 && key_eq(key_shr(tag_anchor(k[i - 1]), begin), pre)) return;  // not the run's first
+  size_t e = i + 2;
+  while (e < n && e - i <= RUN_MAX && key_eq(key_shr(tag_anchor(k[e]), begin), pre)) e++;
+  if (e - i > RUN_MAX) {
+    set_flag(flags, DGF_LONG_RUN);
+    return;
+  }
+  for (size_t a = i + 1; a < e; a++) {
+    const Key128 v = k[a];
+    size_t b = a;
+    for (; b > i && key_lt(v, k[b - 1]); b--) k[b] = k[b - 1];
+    k[b] = v;
+  }
 }
 
 // NCA level of two points of the same cloud; -1 across clouds
@@ -106,15 +172,6 @@ __device__ __forceinline__ int nca_level(Key128 a, Key128 b, unsigned D) {
   if (!x.lo && !x.hi) return (int)D;
   int lz = key_clz(x, 3 * (int)D);
   return lz < 0 ? -1 : lz / 3;
-}
-
-// dupseg[s] = 1 when cloud s holds a repeated point
-__global__ void k_flag_dups(const Key128 *__restrict__ p, size_t n, unsigned D, uint32_t *dupseg, uint32_t *flags) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 1 && i < n && key_eq(p[i], p[i - 1])) {
-    dupseg[seg_of(p[i], D)] = 1u;
-    set_flag(flags, 0x100u);
-  }
 }
 
 __device__ __forceinline__ unsigned leaf_level(const Key128 *__restrict__ p, size_t n, size_t i, unsigned m,
@@ -127,21 +184,201 @@ __device__ __forceinline__ unsigned leaf_level(const Key128 *__restrict__ p, siz
   return (unsigned)min(best + 1, (int)D);
 }
 
-// leaf of every point and the flag "first point of its leaf"
-__global__ void k_p2o_seeds(const Key128 *__restrict__ p, size_t n, unsigned m, unsigned D,
-                            Key128 *__restrict__ seeds, uint32_t *__restrict__ first) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  unsigned L = leaf_level(p, n, i, m, D);
-  Key128 a = key_shl(key_shr(tag_anchor(p[i]), 3 * (D - L)), 3 * (D - L));
-  seeds[i] = make_tagged(a, L);
-  bool f = true;
-  if (i > 0) {
-    unsigned L2 = leaf_level(p, n, i - 1, m, D);
-    Key128 a2 = key_shl(key_shr(tag_anchor(p[i - 1]), 3 * (D - L2)), 3 * (D - L2));
-    f = !(L2 == L && key_eq(a2, a));
+// Node counts: point i adds the nodes on the way to its leaf (levels up to
+// leaf level - 1) that do not hold point i-1, those below level NCA(i-1, i).
+// path[i] = leaf level | (first new level) << 8, sums[b] = new nodes of block
+// b's points; dupseg[s] = 1 where cloud s repeats a point (and 0x100 in
+// flags); max_level = largest leaf level.
+constexpr int P2O_BLOCK = 256, P2O_PER = 4, P2O_TILE = P2O_BLOCK * P2O_PER;
+__global__ void __launch_bounds__(P2O_BLOCK) k_p2o_count(const Key128 *__restrict__ p, size_t n, unsigned m,
+                                                         unsigned D, size_t nseg, uint16_t *__restrict__ path,
+                                                         uint64_t *__restrict__ sums, uint32_t *__restrict__ dupseg,
+                                                         unsigned long long *__restrict__ max_level, uint32_t *flags) {
+  uint64_t total = 0;
+  unsigned top = 0;
+#pragma unroll
+  for (int r = 0; r < P2O_PER; r++) {
+    const size_t i = (size_t)blockIdx.x * P2O_TILE + r * P2O_BLOCK + threadIdx.x;
+    if (i >= n) continue;
+    const unsigned L = leaf_level(p, n, i, m, D);
+    int a = -1;
+    if (i > 0) {
+      a = nca_level(p[i - 1], p[i], D);
+      if (key_eq(p[i - 1], p[i])) {
+        const uint64_t sg = seg_of(p[i], D);
+        if (sg < nseg) dupseg[sg] = 1u;
+        set_flag(flags, 0x100u);
+      }
+    }
+    path[i] = (uint16_t)(L | (unsigned)(a + 1) << 8);
+    if ((int)L > a + 1) total += L - (unsigned)(a + 1);
+    top = max(top, L);
   }
-  first[i] = f ? 1u : 0u;
+  uint64_t sum;
+  block_excl_scan<uint64_t, P2O_BLOCK>(total, sum);
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0 && (unsigned long long)top > __ldcg(max_level)) atomicMax(max_level, (unsigned long long)top);
+  if (threadIdx.x == 0) sums[blockIdx.x] = sum;
+}
+
+// ------------------------------------------------------------------------
+// nodes: an internal octant of level <= Lm as one sortable key, its path (3
+// bits per level to level Lm, the cloud index above) over 5 bits of level:
+// preorder is key order.  64-bit keys where they suffice, else 128-bit.
+// ------------------------------------------------------------------------
+__device__ __forceinline__ uint64_t node_wide(uint64_t k) { return k; }
+__device__ __forceinline__ u128 node_wide(Key128 k) { return to_u128(k); }
+template <typename K>
+struct NodeWide;
+template <>
+struct NodeWide<uint64_t> {
+  typedef uint64_t W;
+  __host__ __device__ __forceinline__ static uint64_t narrow(W w) { return w; }
+  __device__ __forceinline__ static W of(Key128 k) { return k.lo; }
+  __device__ __forceinline__ static Key128 key(W w) { return Key128{w, 0}; }
+};
+template <>
+struct NodeWide<Key128> {
+  typedef u128 W;
+  __host__ __device__ __forceinline__ static Key128 narrow(W w) { return from_u128(w); }
+  __device__ __forceinline__ static W of(Key128 k) { return to_u128(k); }
+  __device__ __forceinline__ static Key128 key(W w) { return from_u128(w); }
+};
+
+// the ancestor of level l (<= Lm) of a tagged anchor at depth D
+template <typename K>
+__device__ __forceinline__ K node_of(Key128 anchor, unsigned l, unsigned Lm, unsigned D) {
+  typedef NodeWide<K> N;
+  const typename N::W idx = N::of(key_shr(anchor, 3 * (D - l)));
+  return N::narrow(idx << (3 * (Lm - l)) << 5 | (typename N::W)l);
+}
+
+// sum of the octal digits of v
+__device__ __forceinline__ unsigned digit_sum(uint64_t v) {
+  const uint64_t m = 0x1249249249249249ull;  // bits 0, 3, ..., 60
+  return __popcll(v & m) + 2 * __popcll(v & m << 1) + 4 * __popcll(v & m << 2) + (unsigned)(v >> 63);
+}
+__device__ __forceinline__ unsigned digit_sum(u128 v) {
+  return digit_sum((uint64_t)((uint64_t)v & 0x7fffffffffffffffull)) + digit_sum((uint64_t)(v >> 63));
+}
+
+template <typename K>
+__global__ void __launch_bounds__(P2O_BLOCK) k_p2o_nodes(const Key128 *__restrict__ p, size_t n, unsigned D,
+                                                         unsigned Lm, const uint16_t *__restrict__ path,
+                                                         const uint64_t *__restrict__ sums, K *__restrict__ out) {
+  uint64_t at = sums[blockIdx.x];
+#pragma unroll
+  for (int r = 0; r < P2O_PER; r++) {
+    const size_t i = (size_t)blockIdx.x * P2O_TILE + r * P2O_BLOCK + threadIdx.x;
+    unsigned L = 0, l = 0;
+    if (i < n) {
+      L = path[i] & 255u;
+      l = path[i] >> 8;
+    }
+    const uint32_t c = L > l ? L - l : 0u;
+    uint32_t all;
+    const uint32_t before = block_excl_scan<uint32_t, P2O_BLOCK>(c, all);
+    if (c) {
+      const Key128 a = tag_anchor(p[i]);
+      for (uint64_t w = at + before; l < L; l++) out[w++] = node_of<K>(a, l, Lm, D);
+    }
+    at += all;
+  }
+}
+
+// The leaves of the octrees whose nodes are given (sorted), 8 threads per
+// node: child c of the node at index i is a leaf unless it is a node itself,
+// which is searched where the node has descendants (from i + 1, galloping).
+// The leaf's place is 7 (j - level) + digits + cloud, j the number of nodes
+// before it in preorder (every cloud before it has one leaf more than 7 per
+// node).
+template <typename K>
+__global__ void k_emit_leaves(const K *__restrict__ nodes, size_t nn, unsigned Lm, unsigned D,
+                              Key128 *__restrict__ out, size_t total) {
+  typedef NodeWide<K> N;
+  typedef typename N::W W;
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t i = t >> 3;
+  const unsigned c = (unsigned)(t & 7u);
+  if (i >= nn) return;
+  const W k = node_wide(nodes[i]);
+  const unsigned d = (unsigned)k & 31u;
+  const W path = k >> 5;
+  const W sub = (W)1 << (3 * (Lm - d));  // paths below the node
+  size_t j = i + 1;
+  Key128 anchor;  // child c, at depth D
+  if (d == Lm) {
+    anchor = key_or(key_shl(N::key(path), 3 * (D - Lm)), key_shl(Key128{c, 0}, 3 * (D - Lm - 1)));
+  } else {
+    const W child = path + (W)c * (sub >> 3);
+    anchor = key_shl(N::key(child), 3 * (D - Lm));
+    if (j < nn && (node_wide(nodes[j]) >> 5) < path + sub) {
+      const W ck = child << 5 | (W)(d + 1);
+      // first node at or after ck
+      size_t step = 1, lo = j, hi = nn;
+      while (lo < nn && node_wide(nodes[lo]) < ck) {
+        j = lo + 1;
+        lo += step;
+        step <<= 1;
+      }
+      if (lo < hi) hi = lo;
+      while (j < hi) {
+        const size_t mid = j + (hi - j) / 2;
+        if (node_wide(nodes[mid]) < ck) j = mid + 1;
+        else hi = mid;
+      }
+      if (j < nn && node_wide(nodes[j]) == ck) return;  // a node itself
+    }
+  }
+  const W in_cloud = path & (((W)1 << (3 * Lm)) - 1);
+  const size_t pos = 7 * (j - (d + 1)) + digit_sum(in_cloud) + c + (size_t)(path >> (3 * Lm));
+  if (pos < total) out[pos] = make_tagged(anchor, d + 1);
+}
+
+// per cloud: its first leaf's place, and its root where the root is a leaf
+// (seg_off may be null)
+template <typename K>
+__global__ void k_emit_clouds(const K *__restrict__ nodes, size_t nn, unsigned Lm, unsigned D, size_t nseg,
+                              Key128 *__restrict__ out, uint64_t *__restrict__ seg_off) {
+  typedef typename NodeWide<K>::W W;
+  const size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s > nseg) return;
+  size_t lo = 0, hi = nn;
+  if (s == nseg) {
+    lo = nn;
+  } else {
+    const W root = (W)s << (3 * Lm) << 5;
+    while (lo < hi) {
+      const size_t mid = lo + (hi - lo) / 2;
+      if (node_wide(nodes[mid]) < root) lo = mid + 1;
+      else hi = mid;
+    }
+    if (lo == nn || node_wide(nodes[lo]) != root) out[7 * lo + s] = make_tagged(seg_key(s, D), 0);
+  }
+  if (seg_off) seg_off[s] = 7 * lo + s;
+}
+
+// whether node keys of octrees with leaves to level top (> 0) fit 64 bits
+inline bool nodes_fit_64(unsigned top, unsigned seg_bits) { return 3 * (top - 1) + seg_bits + 5 <= 64; }
+
+// all leaves of nn sorted nodes of nseg clouds (7 nn + nseg octants)
+template <typename K>
+static void emit_octree(Context &ctx, const K *nodes, size_t nn, unsigned Lm, unsigned D, size_t nseg,
+                        DBuf<Key128> &leaves, DBuf<uint64_t> &seg_off) {
+  cudaStream_t s = ctx.stream;
+  const size_t total = 7 * nn + nseg;
+  leaves.alloc(total, s);
+  if (nseg > 1) seg_off.alloc(nseg + 1, s);
+  if (nseg > 1 || nn == 0) {
+    ProfScope _prof(ctx, "emit_clouds", (double)nseg * 24);
+    k_emit_clouds<K><<<grid_for(nseg + 1, 256), 256, 0, s>>>(nodes, nn, Lm, D, nseg, leaves.get(), seg_off.get());
+    DG_LAUNCH_CHECK();
+  }
+  if (nn) {
+    ProfScope _prof(ctx, "emit_leaves", (double)nn * sizeof(K) + (double)total * 16);
+    k_emit_leaves<K><<<grid_for(8 * nn, 256), 256, 0, s>>>(nodes, nn, Lm, D, leaves.get(), total);
+    DG_LAUNCH_CHECK();
+  }
 }
 
 __device__ __forceinline__ u128 kpos(Key128 k) { return to_u128(tag_anchor(k)); }
@@ -227,21 +464,6 @@ __global__ void k_p2o_walk_segments(const Key128 *__restrict__ pk, const uint64_
   if (outside && batched) counts[blockIdx.x] = (unsigned long long)P2O_WALK_OUTSIDE;
 }
 
-// first index of each cloud in a sorted key array (lower bound of s << 3D)
-__global__ void k_seg_bounds(const Key128 *__restrict__ keys, size_t n, unsigned D, size_t nseg,
-                             uint64_t *__restrict__ off) {
-  size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s > nseg) return;
-  Key128 v = seg_key(s, D);
-  size_t lo = 0, hi = n;
-  while (lo < hi) {
-    size_t mid = lo + (hi - lo) / 2;
-    if (key_lt(tag_anchor(keys[mid]), v)) lo = mid + 1;
-    else hi = mid;
-  }
-  off[s] = lo;
-}
-
 // place each cloud's octants at their final offsets: clouds with repeated
 // points take the walk's output, the others the parallel construction's.
 // The walk outputs are stored cloud after cloud in dup-list order; a walk
@@ -284,37 +506,81 @@ void check_device_flags(Context &ctx, const char *where) {
   }
 }
 
-static void quantize_sorted(Context &ctx, const double *d_xyz, size_t n, const double g[3], unsigned D,
-                            const uint64_t *d_seg_start, size_t nseg, unsigned seg_bits, DBuf<Key128> &keys,
-                            DBuf<Key128> &tmp, Key128 **sorted) {
-  keys.alloc(n, ctx.stream);
-  tmp.alloc(n, ctx.stream);
+// The points as sorted tagged keys.  LSD passes over all 3D key bits cost 12
+// reads and writes of the keys, while log2(n) + PREFIX_EXTRA leading bits
+// leave few points together: only those are sorted (5 passes for 16e6
+// points), from the highest bit on which the keys differ (read back for large
+// inputs, where the wait costs little), and k_sort_runs orders the short runs
+// left.  With `full` every bit is sorted: the caller's answer to
+// DGF_LONG_RUN (points clustered within a few tiny cells).  ctx.d_flags
+// collects what the kernels raise; sorted_flags() reads it.
+constexpr int PREFIX_EXTRA = 16;
+constexpr size_t VARY_MIN = size_t(1) << 18;
+
+// flags raised by quantize_sorted's kernels, after a wait for the stream;
+// throws on all but DGF_LONG_RUN and the repeated-points bit
+static uint32_t sorted_flags(Context &ctx) {
+  const uint32_t f = read_scalar(ctx, ctx.d_flags), keep = DGF_LONG_RUN | 0x100u;
+  if (f & ~keep) check_device_flags(ctx, "points2Octree");
+  if (f) DG_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), ctx.stream));
+  return f;
+}
+
+static Key128 *quantize_sorted(Context &ctx, const double *d_xyz, size_t n, const double g[3], unsigned D,
+                               const uint64_t *d_seg_start, size_t nseg, unsigned seg_bits, bool full,
+                               DBuf<Key128> &keys, DBuf<Key128> &tmp) {
+  cudaStream_t s = ctx.stream;
+  keys.alloc(n, s);
+  tmp.alloc(n, s);
+  unsigned long long *d_vary = n >= VARY_MIN && !full ? ctx.d_scratch + 4 : nullptr;
+  DG_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), s));
+  if (d_vary) DG_CUDA(cudaMemsetAsync(d_vary, 0, 2 * sizeof(unsigned long long), s));
   {
     ProfScope _prof(ctx, "quantize", (double)n * 40);
-    // a power of two whose reciprocal is a normal double
+    // e where v = 2^e, else INT_MIN
     auto pow2 = [](double v) {
       int e = 0;
-      return std::frexp(v, &e) == 0.5 && e > -1020 && e < 1020;
+      return std::frexp(v, &e) == 0.5 && e > -900 && e < 900 ? e - 1 : INT_MIN;
     };
-    if (pow2(g[0]) && pow2(g[1]) && pow2(g[2]))
-      k_quantize<true><<<grid_for(n, 256), 256, 0, ctx.stream>>>(d_xyz, n, (double)(1u << D), 1.0 / g[0], 1.0 / g[1],
-                                                                 1.0 / g[2], D, d_seg_start, nseg, keys.get(),
-                                                                 ctx.d_flags);
+    const int e[3] = {pow2(g[0]), pow2(g[1]), pow2(g[2])};
+    if (e[0] != INT_MIN && e[1] != INT_MIN && e[2] != INT_MIN)
+      k_quantize<true><<<grid_for(n, 256), 256, 0, s>>>(d_xyz, n, 0.0, (double)((int)D - e[0]),
+                                                        (double)((int)D - e[1]), (double)((int)D - e[2]), D,
+                                                        d_seg_start, nseg, keys.get(), d_vary, ctx.d_flags);
     else
-      k_quantize<false><<<grid_for(n, 256), 256, 0, ctx.stream>>>(d_xyz, n, (double)(1u << D), g[0], g[1], g[2], D,
-                                                                  d_seg_start, nseg, keys.get(), ctx.d_flags);
+      k_quantize<false><<<grid_for(n, 256), 256, 0, s>>>(d_xyz, n, (double)(1u << D), g[0], g[1], g[2], D, d_seg_start,
+                                                         nseg, keys.get(), d_vary, ctx.d_flags);
     DG_LAUNCH_CHECK();
   }
-  check_device_flags(ctx, "points2Octree");
-  *sorted = radix_sort<Key128>(ctx, keys.get(), tmp.get(), n, 3 * (int)D + (int)seg_bits);
+  int hi = 3 * (int)D + (int)seg_bits;
+  if (d_vary) {
+    DG_CUDA(cudaMemcpyAsync(ctx.h_scratch + 4, d_vary, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    sorted_flags(ctx);
+    const unsigned long long lo = ctx.h_scratch[4], up = ctx.h_scratch[5];
+    const int bits = up ? 128 - __builtin_clzll(up) : lo ? 64 - __builtin_clzll(lo) : 0;
+    hi = std::min(hi, bits);
+  }
+  int want = PREFIX_EXTRA;
+  while (want < 63 && ((size_t)1 << (want - PREFIX_EXTRA)) < n) want++;
+  const int begin = full ? 0 : std::max(0, hi - (want + 7) / 8 * 8);
+  Key128 *sorted = radix_sort<Key128>(ctx, keys.get(), tmp.get(), n, hi, begin);
+  if (begin > 0) {
+    ProfScope _prof(ctx, "sort_runs", (double)n * 16);
+    k_sort_runs<<<grid_for(n, 256), 256, 0, s>>>(sorted, n, (unsigned)begin, ctx.d_flags);
+    DG_LAUNCH_CHECK();
+  }
+  return sorted;
 }
 
 size_t sort_points(Context &ctx, const double *d_xyz, size_t n, const double g[3], unsigned D, Key128 *d_out,
                    bool *has_dups) {
   if (n == 0) return 0;
   DBuf<Key128> keys, tmp;
-  Key128 *sorted;
-  quantize_sorted(ctx, d_xyz, n, g, D, nullptr, 1, 0, keys, tmp, &sorted);
+  Key128 *sorted = quantize_sorted(ctx, d_xyz, n, g, D, nullptr, 1, 0, false, keys, tmp);
+  if (sorted_flags(ctx) & DGF_LONG_RUN) {
+    sorted = quantize_sorted(ctx, d_xyz, n, g, D, nullptr, 1, 0, true, keys, tmp);
+    sorted_flags(ctx);
+  }
   DBuf<uint32_t> flags(n, ctx.stream);
   {
     ProfScope _prof(ctx, "flag_unique", (double)n * 20);
@@ -357,7 +623,7 @@ void points_to_octree(Context &ctx, const double *d_xyz, size_t n, const double 
       {
         ProfScope _prof(ctx, "quantize", (double)n * 40);
         k_quantize<false><<<grid_for(n, 256), 256, 0, s>>>(d_xyz, n, (double)(1u << D), g[0], g[1], g[2], D, nullptr,
-                                                           1, keys.get(), ctx.d_flags);
+                                                           1, keys.get(), nullptr, ctx.d_flags);
         DG_LAUNCH_CHECK();
       }
       check_device_flags(ctx, "points2Octree");
@@ -377,68 +643,49 @@ void points_to_octree(Context &ctx, const double *d_xyz, size_t n, const double 
     return;
   }
   DBuf<Key128> keys, tmp;
-  Key128 *p;
-  quantize_sorted(ctx, d_xyz, n, g, D, d_seg_start.get(), nseg, SB, keys, tmp, &p);
-  Key128 *other = (p == keys.get()) ? tmp.get() : keys.get();
-
-  // clouds with repeated points
-  DBuf<uint32_t> dupseg(nseg, s);
-  DG_CUDA(cudaMemsetAsync(dupseg.get(), 0, nseg * sizeof(uint32_t), s));
-  DG_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), s));
-  {
-    ProfScope _prof(ctx, "flag_dups", (double)n * 16);
-    k_flag_dups<<<grid_for(n, 256), 256, 0, s>>>(p, n, D, dupseg.get(), ctx.d_flags);
-    DG_LAUNCH_CHECK();
-  }
-  uint32_t dupflag = read_scalar(ctx, ctx.d_flags);
-  DG_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), s));
-
-  // parallel construction over all points (clouds with repeated points are
-  // replaced below)
-  DBuf<uint32_t> first(n, s);
-  {
-    ProfScope _prof(ctx, "p2o_seeds", (double)n * 36);
-    k_p2o_seeds<<<grid_for(n, 256), 256, 0, s>>>(p, n, m, D, other, first.get());
-    DG_LAUNCH_CHECK();
-  }
-  DBuf<Key128> walk_keys;  // keeps p alive for the walk when needed
-  Key128 *seeds = other;
-  if (dupflag) {
-    // the walk needs the sorted points: compact the seeds into a new buffer
-    walk_keys.alloc(n, s);
-    seeds = walk_keys.get();
-  }
-  size_t ns = compact<Key128>(ctx, other, first.get(), n, dupflag ? seeds : p);
-  if (!dupflag) seeds = p;
-  first.release();
-  DBuf<uint32_t> cnt(ns, s);
-  {
-    ProfScope _prof(ctx, "fill_count", (double)ns * 20);
-    k_fill_count<<<grid_for(ns, 256), 256, 0, s>>>(seeds, ns, D, total, cnt.get());
-    DG_LAUNCH_CHECK();
-  }
-  DBuf<uint64_t> off(ns, s);
-  uint64_t *d_total = reinterpret_cast<uint64_t *>(ctx.d_scratch);
-  exclusive_scan<uint32_t, uint64_t>(cnt.get(), off.get(), ns, d_total, s);
-  size_t npar = (size_t)read_scalar(ctx, d_total);
-  DBuf<Key128> res(npar, s);
-  {
-    ProfScope _prof(ctx, "fill_emit", (double)ns * 24);
-    k_fill_emit<<<grid_for(ns, 256), 256, 0, s>>>(seeds, ns, D, total, off.get(), res.get());
-    DG_LAUNCH_CHECK();
-  }
-  cnt.release();
-  off.release();
-
-  DBuf<uint64_t> seg_off;
-  if (nseg > 1 || dupflag) {
-    seg_off.alloc(nseg + 1, s);
+  Key128 *p = nullptr;
+  const size_t nblocks = (n + P2O_TILE - 1) / P2O_TILE;
+  DBuf<uint32_t> dupseg(nseg, s);  // clouds with repeated points
+  DBuf<uint16_t> path(n, s);
+  DBuf<uint64_t> sums(nblocks, s);
+  unsigned long long *d_info = ctx.d_scratch;  // {nodes, largest leaf level}
+  uint32_t dupflag = 0;
+  for (bool full : {false, true}) {
+    p = quantize_sorted(ctx, d_xyz, n, g, D, d_seg_start.get(), nseg, SB, full, keys, tmp);
+    DG_CUDA(cudaMemsetAsync(dupseg.get(), 0, nseg * sizeof(uint32_t), s));
+    DG_CUDA(cudaMemsetAsync(d_info, 0, 2 * sizeof(unsigned long long), s));
     {
-      ProfScope _prof(ctx, "seg_bounds", (double)(nseg + 1) * 16);
-      k_seg_bounds<<<grid_for(nseg + 1, 256), 256, 0, s>>>(res.get(), npar, D, nseg, seg_off.get());
+      ProfScope _prof(ctx, "p2o_count", (double)n * 18);
+      k_p2o_count<<<(unsigned)nblocks, P2O_BLOCK, 0, s>>>(p, n, m, D, nseg, path.get(), sums.get(), dupseg.get(),
+                                                          d_info + 1, ctx.d_flags);
       DG_LAUNCH_CHECK();
     }
+    exclusive_scan<uint64_t, uint64_t>(sums.get(), sums.get(), nblocks, reinterpret_cast<uint64_t *>(d_info), s);
+    DG_CUDA(cudaMemcpyAsync(ctx.h_scratch + 4, d_info, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    const uint32_t f = sorted_flags(ctx);
+    dupflag = f & 0x100u;
+    if (!(f & DGF_LONG_RUN)) break;
   }
+  const size_t nn = (size_t)ctx.h_scratch[4];
+  const unsigned top = std::max(1u, (unsigned)ctx.h_scratch[5]);  // deepest leaf level
+
+  // parallel construction over all points (clouds with repeated points are
+  // replaced below): the nodes in preorder, then their leaves
+  DBuf<Key128> res;
+  DBuf<uint64_t> seg_off;
+  auto construct = [&](auto tag) {
+    typedef decltype(tag) K;
+    DBuf<K> nodes(nn ? nn : 1, s);
+    {
+      ProfScope _prof(ctx, "p2o_nodes", (double)n * 18 + (double)nn * sizeof(K));
+      k_p2o_nodes<K><<<(unsigned)nblocks, P2O_BLOCK, 0, s>>>(p, n, D, top - 1, path.get(), sums.get(), nodes.get());
+      DG_LAUNCH_CHECK();
+    }
+    emit_octree<K>(ctx, nodes.get(), nn, top - 1, D, nseg, res, seg_off);
+  };
+  if (nodes_fit_64(top, SB)) construct(uint64_t());
+  else construct(Key128());
+  const size_t npar = 7 * nn + nseg;
   if (!dupflag) {
     out.n = npar;
     out.keys = res.release_ptr();
@@ -451,6 +698,11 @@ void points_to_octree(Context &ctx, const double *d_xyz, size_t n, const double 
   std::vector<uint32_t> h_dup(nseg);
   DG_CUDA(cudaMemcpyAsync(h_dup.data(), dupseg.get(), nseg * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   std::vector<uint64_t> h_par_off(nseg + 1);
+  if (nseg == 1) {
+    seg_off.alloc(2, s);
+    const uint64_t one[2] = {0, npar};
+    DG_CUDA(cudaMemcpyAsync(seg_off.get(), one, sizeof(one), cudaMemcpyHostToDevice, s));
+  }
   DG_CUDA(cudaMemcpyAsync(h_par_off.data(), seg_off.get(), (nseg + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
   DG_CUDA(cudaStreamSynchronize(s));
   std::vector<uint32_t> dup_list, walk_slot(nseg, 0xffffffffu);
@@ -540,338 +792,355 @@ void octree_segment_offsets(Context &ctx, const Octree &o, uint64_t *h_off) {
 // ------------------------------------------------------------------------
 // balance
 // ------------------------------------------------------------------------
-// level histogram; flags octants that are not aligned octants of the
-// domain of their cloud (the reference asserts on those,
-// octFunctions.cpp:310)
-__global__ void k_level_hist(const Key128 *__restrict__ k, size_t n, unsigned D, uint64_t nseg,
-                             unsigned long long *hist, uint32_t *flags) {
+// Flags octants that are not aligned octants of the domain of their cloud
+// (the reference asserts on those, octFunctions.cpp:310) and counts, per level
+// of the parent, the leaves that bring a parent: all but those whose
+// predecessor has the same one.
+__device__ __forceinline__ bool brings_parent(const Key128 *__restrict__ k, size_t i, Key128 ki, unsigned D) {
+  const unsigned l = tag_level(ki);
+  if (l == 0) return false;
+  if (i == 0) return true;
+  const Key128 kp = k[i - 1];
+  const unsigned sh = 3 * (D - l + 1);
+  return !(tag_level(kp) == l && key_eq(key_shr(tag_anchor(kp), sh), key_shr(tag_anchor(ki), sh)));
+}
+
+__global__ void k_bal_scan(const Key128 *__restrict__ k, size_t n, unsigned D, uint64_t nseg,
+                           unsigned long long *hist, uint32_t *flags) {
   __shared__ unsigned int h[32];
   if (threadIdx.x < 32) h[threadIdx.x] = 0;
   __syncthreads();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    Key128 ki = k[i];
-    unsigned l = tag_level(ki);
-    Key128 a = morton_part(ki, D);
+    const Key128 ki = k[i];
+    const unsigned l = tag_level(ki);
+    const Key128 a = morton_part(ki, D);
     bool ok = l <= D && seg_of(ki, D) < nseg;
     if (ok && l < D) ok = key_eq(key_shl(key_shr(a, 3 * (D - l)), 3 * (D - l)), a);
     if (!ok) atomicOr(flags, DGF_DOMAIN);
-    atomicAdd(&h[l & 31u], 1u);
+    else if (brings_parent(k, i, ki, D)) atomicAdd(&h[l - 1], 1u);
   }
   __syncthreads();
   if (threadIdx.x < 32 && h[threadIdx.x]) atomicAdd(&hist[threadIdx.x], (unsigned long long)h[threadIdx.x]);
 }
 
-// level-(l-1) index (cloud bits included) of the parent of every input leaf
-// at level l
-__device__ __forceinline__ void put_key(Key128 *out, size_t i, Key128 v) { out[i] = v; }
-__device__ __forceinline__ void put_key(uint64_t *out, size_t i, Key128 v) { out[i] = v.lo; }
+// ---- the set of all nodes: open addressing.  The eight children of one
+// octant share a group of eight slots (one cache line of 64-bit keys), as the
+// candidates around one octant do; probing steps by groups, a bounded number
+// of times (BAL_PROBES; then DGF_CAPACITY, and the host retries with a larger
+// table).
+constexpr int BAL_PROBES = 512;
 
+__device__ __forceinline__ uint64_t mix64(uint64_t x) {
+  x ^= x >> 32;
+  x *= 0xd6e8feb86659fd93ull;
+  x ^= x >> 32;
+  return x;
+}
+__device__ __forceinline__ uint64_t node_hash(uint64_t k, unsigned Lm) {
+  const unsigned l = (unsigned)k & 31u, sh = 5 + 3 * (Lm - l);
+  return mix64((k >> sh >> 3) * 32 + l) << 3 | (k >> sh & 7u);
+}
+__device__ __forceinline__ uint64_t node_hash(u128 k, unsigned Lm) {
+  const unsigned l = (unsigned)k & 31u, sh = 5 + 3 * (Lm - l);
+  const u128 par = k >> sh >> 3;
+  return mix64(((uint64_t)par ^ (uint64_t)(par >> 64) * 0x9e3779b97f4a7c15ull) * 32 + l) << 3 | ((uint64_t)(k >> sh) & 7u);
+}
+__device__ __forceinline__ uint64_t node_empty(uint64_t) { return ~0ull; }
+__device__ __forceinline__ u128 node_empty(u128) { return ~(u128)0; }
+
+// compare-and-swap of one slot, returning what it held
+__device__ __forceinline__ uint64_t slot_cas(uint64_t *slot, uint64_t key) {
+  const uint64_t cur = __ldcg(slot);  // a full slot never changes
+  if (cur != ~0ull) return cur;
+  return atomicCAS(reinterpret_cast<unsigned long long *>(slot), ~0ull, (unsigned long long)key);
+}
+__device__ __forceinline__ u128 slot_cas(Key128 *slot, u128 key) {
+  uint64_t lo, hi;
+  asm volatile("{\n\t.reg .b128 d, b, c;\n\t"
+               "mov.b128 b, {%3, %4};\n\tmov.b128 c, {%5, %6};\n\t"
+               "atom.relaxed.gpu.cas.b128 d, [%2], b, c;\n\tmov.b128 {%0, %1}, d;\n\t}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(slot), "l"(~0ull), "l"(~0ull), "l"((uint64_t)key), "l"((uint64_t)(key >> 64))
+               : "memory");
+  return (u128)hi << 64 | lo;
+}
+
+// true when this call put the key into the table
 template <typename K>
-__global__ void k_leaf_parents(const Key128 *__restrict__ k, size_t n, unsigned D, unsigned l, K *__restrict__ out) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) put_key(out, i, key_shr(tag_anchor(k[i]), 3 * (D - l + 1)));
+__device__ __forceinline__ bool node_insert(K *__restrict__ tab, uint64_t mask, typename NodeWide<K>::W key,
+                                            unsigned Lm, uint32_t *flags) {
+  uint64_t h = node_hash(key, Lm) & mask;
+  for (int probe = 0; probe < BAL_PROBES; probe++) {
+    const auto cur = slot_cas(tab + h, key);
+    if (cur == node_empty(key)) return true;
+    if (cur == key) return false;
+    h = (h + 8) & mask;
+  }
+  set_flag(flags, DGF_CAPACITY);
+  return false;
 }
 
-// for q at level l: the 8 level-(l-1) parents of q's 3x3x3 block; parents
-// outside the domain are replaced by q's own parent (removed by the unique).
-// Without corners (balanceOctree's incCorner = false: faces and edges only,
-// the 18 directions of TreeNode::addBalancingDescendants,
-// src/TreeNode.cpp:160-190) the parent that only q's corner neighbours
-// reach (outward on all three axes) is replaced the same way.
+// where the nodes go: those from the leaves at off[l] of `leafs`, level by
+// level, the others in the order of their making in `grown`
+struct BalLists {
+  unsigned long long off[32];
+};
+// counters on the device: nodes per level from the leaves, and grown
+struct BalCounts {
+  unsigned long long leaf[32], grown[32];
+};
+
+// the parents of the input leaves
 template <typename K>
-__global__ void k_block_parents(const Key128 *__restrict__ q, size_t nq, unsigned l, bool inc_corner,
-                                K *__restrict__ out) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nq) return;
-  const Key128 qi = q[i];
-  const Key128 segk = key_shl(key_shr(qi, 3 * l), 3 * (l - 1));  // cloud bits at level l-1
-  Key128 idx = qi;
-  if (3 * l < 64) {
-    idx.lo &= (1ull << (3 * l)) - 1;
-    idx.hi = 0;
-  } else {
-    idx.hi &= (1ull << (3 * l - 64)) - 1;
-  }
-  uint32_t c[3];
-  demorton3(idx, c[0], c[1], c[2]);  // level-l integer coordinates
-  const int64_t side = (int64_t)1 << (l - 1);  // parents per axis
-  int64_t opt[3][2];
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    int64_t par = c[a] >> 1;
-    opt[a][0] = par;
-    opt[a][1] = (c[a] & 1) ? par + 1 : par - 1;
-  }
-#pragma unroll
-  for (int t = 0; t < 8; t++) {
-    int64_t p0 = opt[0][t & 1], p1 = opt[1][(t >> 1) & 1], p2 = opt[2][(t >> 2) & 1];
-    if (p0 < 0 || p1 < 0 || p2 < 0 || p0 >= side || p1 >= side || p2 >= side || (t == 7 && !inc_corner)) {
-      p0 = opt[0][0];
-      p1 = opt[1][0];
-      p2 = opt[2][0];
-    }
-    put_key(out, 8 * i + t, key_or(morton3((uint32_t)p0, (uint32_t)p1, (uint32_t)p2), segk));
-  }
-}
-
-__global__ void k_widen(const uint64_t *__restrict__ in, size_t n, Key128 *__restrict__ out) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] = Key128{in[i], 0};
-}
-
-__device__ __forceinline__ size_t lower_bound_key(const Key128 *a, size_t n, Key128 v) {
-  size_t lo = 0, hi = n;
-  while (lo < hi) {
-    size_t mid = lo + (hi - lo) / 2;
-    if (key_lt(a[mid], v)) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// rank map: R[8*parent_index + child] = index of the internal child in I_l
-__global__ void k_mark_internal(const Key128 *__restrict__ Il, size_t nl, const Key128 *__restrict__ Ip, size_t np,
-                                uint32_t *__restrict__ R, uint32_t *flags) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nl) return;
-  Key128 par = key_shr(Il[i], 3);
-  size_t p = lower_bound_key(Ip, np, par);
-  if (p >= np || !key_eq(Ip[p], par)) {
-    atomicOr(flags, DGF_INTERNAL);
-    return;
-  }
-  R[8 * p + (Il[i].lo & 7u)] = (uint32_t)i;
-}
-
-// clouds whose root is internal: Rtop[cloud] = index of its root in I_0
-__global__ void k_mark_roots(const Key128 *__restrict__ I0, size_t n0, size_t nseg, uint32_t *__restrict__ Rtop,
-                             uint32_t *flags) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n0) return;
-  uint64_t sg = I0[i].lo;
-  if (I0[i].hi || sg >= nseg) {
-    atomicOr(flags, DGF_INTERNAL);
-    return;
-  }
-  Rtop[sg] = (uint32_t)i;
-}
-
-__global__ void k_subtree_count(const uint32_t *__restrict__ R, size_t np, const uint64_t *__restrict__ sub_child,
-                                uint64_t *__restrict__ sub) {
-  size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= np) return;
-  uint64_t c = 0;
-#pragma unroll
-  for (int q = 0; q < 8; q++) {
-    uint32_t x = R ? R[8 * r + q] : 0xffffffffu;
-    c += (x == 0xffffffffu) ? 1ull : sub_child[x];
-  }
-  sub[r] = c;
-}
-
-// leaf count of every cloud (1 when its root is a leaf)
-__global__ void k_cloud_count(const uint32_t *__restrict__ Rtop, size_t nseg, const uint64_t *__restrict__ sub0,
-                              uint64_t *__restrict__ cnt) {
-  size_t sg = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (sg >= nseg) return;
-  uint32_t x = Rtop[sg];
-  cnt[sg] = (x == 0xffffffffu) ? 1ull : sub0[x];
-}
-
-// place cloud roots: a leaf root is written out, an internal one passes its
-// offset to level 0
-__global__ void k_place_roots(const uint32_t *__restrict__ Rtop, size_t nseg, const uint64_t *__restrict__ cloud_off,
-                              unsigned D, uint64_t *__restrict__ off0, Key128 *__restrict__ out) {
-  size_t sg = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (sg >= nseg) return;
-  uint32_t x = Rtop[sg];
-  if (x == 0xffffffffu) out[cloud_off[sg]] = make_tagged(from_u128((u128)sg << (3 * D)), 0);
-  else off0[x] = cloud_off[sg];
-}
-
-__global__ void k_place(const Key128 *__restrict__ Ip, size_t np, unsigned l, unsigned D, const uint32_t *__restrict__ R,
-                        const uint64_t *__restrict__ sub_child, const uint64_t *__restrict__ off,
-                        uint64_t *__restrict__ off_child, Key128 *__restrict__ out) {
-  size_t r = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= np) return;
-  uint64_t run = off[r];
-  Key128 base = key_shl(Ip[r], 3);
-#pragma unroll
-  for (int q = 0; q < 8; q++) {
-    uint32_t x = R ? R[8 * r + q] : 0xffffffffu;
-    if (x == 0xffffffffu) {
-      Key128 ch = base;
-      ch.lo |= (uint64_t)q;
-      out[run] = make_tagged(key_shl(ch, 3 * (D - l - 1)), l + 1);
-      run += 1;
-    } else {
-      off_child[x] = run;
-      run += sub_child[x];
+__global__ void __launch_bounds__(256) k_bal_leaves(const Key128 *__restrict__ k, size_t n, unsigned D, unsigned Lm,
+                                                    K *__restrict__ tab, uint64_t mask, BalLists lists,
+                                                    K *__restrict__ leafs, BalCounts *__restrict__ cnt,
+                                                    uint32_t *flags) {
+  __shared__ unsigned num[32];
+  __shared__ unsigned long long base[32];
+  if (threadIdx.x < 32) num[threadIdx.x] = 0;
+  __syncthreads();
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  bool won = false;
+  K key{};
+  unsigned l = 0, rank = 0;
+  if (i < n) {
+    const Key128 ki = k[i];
+    if (brings_parent(k, i, ki, D)) {
+      l = tag_level(ki) - 1;
+      key = node_of<K>(tag_anchor(ki), l, Lm, D);
+      won = node_insert<K>(tab, mask, node_wide(key), Lm, flags);
+      if (won) rank = atomicAdd(&num[l], 1u);
     }
   }
+  __syncthreads();
+  if (threadIdx.x < 32 && num[threadIdx.x])
+    base[threadIdx.x] = lists.off[threadIdx.x] + atomicAdd(&cnt->leaf[threadIdx.x], (unsigned long long)num[threadIdx.x]);
+  __syncthreads();
+  if (won) leafs[base[l] + rank] = key;
+}
+
+// One level of the recursion: for every node q of level l the 8 parents (level
+// l - 1) of q's 3x3x3 block that lie in the domain.  Without corners
+// (balanceOctree's incCorner = false: faces and edges only, the 18 directions
+// of TreeNode::addBalancingDescendants, src/TreeNode.cpp:160-190) not the
+// parent that only q's corner neighbours reach (outward on all three axes).
+// A block takes 256 nodes at a time; its 2048 candidates are made unique in
+// shared memory first (the nodes of a block lie close together, and 3 of 4
+// candidates repeat), so the table in L2 sees each once per block.
+constexpr int BAL_TILE = 256, BAL_CAND = 8 * BAL_TILE, BAL_SLOTS = 2 * BAL_CAND;
+constexpr uint32_t BAL_FREE = 0xffffffffu;
+template <typename K>
+struct BalSmem {
+  K cand[BAL_CAND];
+  uint32_t slot[BAL_SLOTS];
+  uint16_t won[BAL_CAND];
+  unsigned n_won;
+  unsigned long long at;
+};
+
+template <typename K>
+__global__ void __launch_bounds__(BAL_TILE) k_bal_level(unsigned l, unsigned Lm, bool inc_corner, K *__restrict__ tab,
+                                                        uint64_t mask, BalLists lists, const K *__restrict__ leafs,
+                                                        K *grown, size_t grown_cap, BalCounts *__restrict__ cnt,
+                                                        uint32_t *flags) {
+  typedef NodeWide<K> N;
+  typedef typename N::W W;
+  extern __shared__ __align__(16) unsigned char bal_raw[];
+  BalSmem<K> &S = *reinterpret_cast<BalSmem<K> *>(bal_raw);
+  const int t = threadIdx.x;
+  const size_t n0 = cnt->leaf[l], n1 = cnt->grown[l];
+  size_t first = 0;  // grown nodes of the levels below
+  for (unsigned q = l + 1; q <= Lm; q++) first += cnt->grown[q];
+  if (first + n1 > grown_cap) return;  // the list overflowed (flagged): the host starts again
+  const size_t n = n0 + n1, next = first + n1;
+  for (size_t tile = blockIdx.x; tile * BAL_TILE < n; tile += gridDim.x) {
+    const size_t i = tile * BAL_TILE + t;
+    for (int q = t; q < BAL_SLOTS; q += BAL_TILE) S.slot[q] = BAL_FREE;
+    if (t == 0) S.n_won = 0;
+    uint32_t valid = 0;
+    if (i < n) {
+      const W k = node_wide(i < n0 ? leafs[lists.off[l] + i] : grown[first + (i - n0)]);
+      const W path = k >> 5;
+      const W cloud = path >> (3 * Lm);
+      const W idx = (path & (((W)1 << (3 * Lm)) - 1)) >> (3 * (Lm - l));
+      uint32_t c[3];
+      demorton3(N::key(idx), c[0], c[1], c[2]);  // level-l integer coordinates
+      const uint32_t side = 1u << (l - 1);  // parents per axis
+      uint32_t opt[3][2];
+      bool in[3];
+#pragma unroll
+      for (int a = 0; a < 3; a++) {
+        opt[a][0] = c[a] >> 1;
+        opt[a][1] = (c[a] & 1u) ? opt[a][0] + 1 : opt[a][0] - 1;
+        in[a] = opt[a][1] < side;  // -1 wraps round
+      }
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        if (((q & 1) && !in[0]) || ((q & 2) && !in[1]) || ((q & 4) && !in[2]) || (q == 7 && !inc_corner)) continue;
+        valid |= 1u << q;
+        const W par = cloud << (3 * (l - 1)) | N::of(morton3(opt[0][q & 1], opt[1][q >> 1 & 1], opt[2][q >> 2]));
+        S.cand[8 * t + q] = N::narrow(par << (3 * (Lm - l + 1)) << 5 | (W)(l - 1));
+      }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int q = 0; q < 8; q++) {
+      if (!(valid >> q & 1u)) continue;
+      const uint32_t me = 8 * t + q;
+      const W key = node_wide(S.cand[me]);
+      uint32_t h = (uint32_t)(node_hash(key, Lm) ^ node_hash(key, Lm) >> 24) & (BAL_SLOTS - 1);
+      bool mine = false;
+      for (int probe = 0; probe < BAL_SLOTS; probe++) {
+        const uint32_t cur = atomicCAS(&S.slot[h], BAL_FREE, me);
+        mine = cur == BAL_FREE;
+        if (mine || node_wide(S.cand[cur]) == key) break;
+        h = (h + 1) & (BAL_SLOTS - 1);
+      }
+      if (mine && node_insert<K>(tab, mask, key, Lm, flags)) S.won[atomicAdd(&S.n_won, 1u)] = (uint16_t)me;
+    }
+    __syncthreads();
+    const unsigned nw = S.n_won;
+    if (t == 0 && nw) S.at = next + atomicAdd(&cnt->grown[l - 1], (unsigned long long)nw);
+    __syncthreads();
+    for (unsigned q = t; q < nw; q += BAL_TILE) {
+      if (S.at + q < grown_cap) grown[S.at + q] = S.cand[S.won[q]];
+      else set_flag(flags, DGF_CAPACITY);
+    }
+    __syncthreads();
+  }
+}
+
+// all nodes side by side: the leaves' lists without the room their repeats
+// left, then the grown ones
+struct BalGather {
+  unsigned long long off[32], num[32], to[32];
+};
+template <typename K>
+__global__ void k_bal_gather(const K *__restrict__ leafs, BalGather g, size_t n_room, K *__restrict__ out) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_room) return;
+  int l = 0;
+  while (l < 31 && i >= g.off[l + 1]) l++;
+  const size_t r = i - g.off[l];
+  if (r < g.num[l]) out[g.to[l] + r] = leafs[i];
+}
+
+// the sorted nodes of the balanced refinement
+template <typename K>
+static size_t balance_nodes(Context &ctx, const Octree &in, unsigned top, const unsigned long long (&hist)[32],
+                            bool inc_corner, DBuf<K> &a, DBuf<K> &b, K **sorted) {
+  cudaStream_t s = ctx.stream;
+  const unsigned D = in.max_depth, Lm = top - 1;
+  BalLists lists;
+  size_t room = 0;  // parents from the leaves, repeats of far-away leaves included
+  for (int l = 0; l < 32; l++) {
+    lists.off[l] = room;
+    room += hist[l];
+  }
+  ensure_smem_attr(ctx, k_bal_level<K>, (int)sizeof(BalSmem<K>));
+  int per_sm = 1;
+  DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bal_level<K>, BAL_TILE, sizeof(BalSmem<K>)));
+  // counters and flags come back together
+  BalCounts *cnt = reinterpret_cast<BalCounts *>(ctx.d_scratch);
+  BalCounts *h = reinterpret_cast<BalCounts *>(ctx.h_scratch);
+  DBuf<K> leafs(room, s), grown;
+  size_t n0 = 0, n1 = 0;
+  // balanced octrees of the workloads' clouds have 1.3 to 1.9 times the nodes
+  // of their input: room for 3 times, and four times that on each retry
+  for (size_t grow = 2;; grow *= 4) {
+    const size_t cap = grow * room + 65536;
+    size_t slots = 1024;
+    while (slots < room + cap) slots <<= 1;
+    grown.alloc(cap, s);
+    DBuf<K> tab(slots, s);
+    DG_CUDA(cudaMemsetAsync(tab.get(), 0xff, slots * sizeof(K), s));
+    DG_CUDA(cudaMemsetAsync(cnt, 0, sizeof(BalCounts), s));
+    {
+      ProfScope _prof(ctx, "bal_leaves", (double)in.n * 16 + (double)room * 2 * sizeof(K));
+      k_bal_leaves<K><<<grid_for(in.n, 256), 256, 0, s>>>(in.keys, in.n, D, Lm, tab.get(), slots - 1, lists,
+                                                          leafs.get(), cnt, ctx.d_flags);
+      DG_LAUNCH_CHECK();
+    }
+    const unsigned grid =
+        grid_for(room + cap, BAL_TILE, (unsigned)(std::max(per_sm, 1) * ctx.num_sms));
+    for (unsigned l = Lm; l >= 1; l--) {
+      ProfScope _prof(ctx, "bal_level", 0.0);
+      k_bal_level<K><<<grid, BAL_TILE, sizeof(BalSmem<K>), s>>>(l, Lm, inc_corner, tab.get(), slots - 1, lists,
+                                                                leafs.get(), grown.get(), cap, cnt, ctx.d_flags);
+      DG_LAUNCH_CHECK();
+    }
+    DG_CUDA(cudaMemcpyAsync(h, cnt, sizeof(BalCounts), cudaMemcpyDeviceToHost, s));
+    DG_CUDA(cudaMemcpyAsync(h + 1, ctx.d_flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    DG_CUDA(cudaStreamSynchronize(s));
+    uint32_t f;
+    std::memcpy(&f, h + 1, sizeof(f));
+    if (!(f & DGF_CAPACITY)) break;
+    DG_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), s));
+    if (cap > ((size_t)1 << 40) / sizeof(K)) fail(DG_ERR_OUT_OF_MEMORY, "balanceOctree: too many octants");
+  }
+  BalGather g;
+  for (int l = 0; l < 32; l++) {
+    g.off[l] = lists.off[l];
+    g.num[l] = h->leaf[l];
+    g.to[l] = n0;
+    n0 += h->leaf[l];
+    n1 += h->grown[l];
+  }
+  const size_t nn = n0 + n1;
+  a.alloc(nn, s);
+  b.alloc(nn, s);
+  {
+    ProfScope _prof(ctx, "bal_gather", (double)nn * 2 * sizeof(K));
+    k_bal_gather<K><<<grid_for(room, 256), 256, 0, s>>>(leafs.get(), g, room, a.get());
+    DG_LAUNCH_CHECK();
+  }
+  if (n1) DG_CUDA(cudaMemcpyAsync(a.get() + n0, grown.get(), n1 * sizeof(K), cudaMemcpyDeviceToDevice, s));
+  *sorted = radix_sort<K>(ctx, a.get(), b.get(), nn, 3 * (int)Lm + 5 + (int)in.seg_bits);
+  return nn;
 }
 
 void balance_octree(Context &ctx, const Octree &in, Octree &out, bool inc_corner) {
   cudaStream_t s = ctx.stream;
   const unsigned D = in.max_depth;
   const size_t nseg = in.nseg;
-  const unsigned SB = in.seg_bits;
   out.max_depth = D;
   out.nseg = nseg;
-  out.seg_bits = SB;
+  out.seg_bits = in.seg_bits;
   const size_t n = in.n;
   if (n == 0) fail(DG_ERR_INVALID_ARG, "balanceOctree: empty input");
-  // level histogram + domain validation
+  // parents per level + domain validation
   unsigned long long *d_hist = ctx.d_scratch + 16;
   DG_CUDA(cudaMemsetAsync(d_hist, 0, 32 * sizeof(unsigned long long), s));
   DG_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), s));
   {
-    ProfScope _prof(ctx, "bal_level_hist", (double)n * 16);
-    k_level_hist<<<grid_for(n, 256, ctx.num_sms * 4), 256, 0, s>>>(in.keys, n, D, nseg, d_hist, ctx.d_flags);
+    ProfScope _prof(ctx, "bal_scan", (double)n * 16);
+    k_bal_scan<<<grid_for(n, 256, ctx.num_sms * 8), 256, 0, s>>>(in.keys, n, D, nseg, d_hist, ctx.d_flags);
     DG_LAUNCH_CHECK();
   }
+  DG_CUDA(cudaMemcpyAsync(ctx.h_scratch + 16, d_hist, 32 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
   check_device_flags(ctx, "balanceOctree (octant outside the domain or misaligned)");
-  unsigned long long hcnt[32];
-  DG_CUDA(cudaMemcpyAsync(ctx.h_scratch + 16, d_hist, sizeof(hcnt), cudaMemcpyDeviceToHost, s));
-  DG_CUDA(cudaStreamSynchronize(s));
-  std::memcpy(hcnt, ctx.h_scratch + 16, sizeof(hcnt));
-  unsigned maxL = 0;
+  unsigned long long hist[32];
+  std::memcpy(hist, ctx.h_scratch + 16, sizeof(hist));
+  unsigned top = 0;  // deepest leaf level
   for (unsigned l = 0; l < 32; l++)
-    if (hcnt[l]) maxL = l;
-
-  // bucket the leaves by level (one stable radix pass on the level byte);
-  // every bucket stays in (cloud, Morton) order
-  DBuf<Key128> bucketed(n, s);
-  {
-    size_t ntiles = (n + RS_TILE - 1) / RS_TILE;
-    DBuf<uint32_t> hist(256 * ntiles, s);
-    {
-      ProfScope _prof(ctx, "rs_hist", (double)n * 16);
-      k_rs_hist<Key128><<<(unsigned)ntiles, RS_BLOCK, 0, s>>>(in.keys, n, 120, hist.get(), ntiles);
-      DG_LAUNCH_CHECK();
-    }
-    exclusive_scan<uint32_t, uint32_t>(hist.get(), hist.get(), 256 * ntiles, (uint32_t *)nullptr, s);
-    {
-      ProfScope _prof(ctx, "rs_scatter", (double)n * 32);
-      k_rs_scatter<Key128><<<(unsigned)ntiles, RS_BLOCK, 0, s>>>(in.keys, bucketed.get(), n, 120, hist.get(), ntiles);
-      DG_LAUNCH_CHECK();
-    }
-  }
-  std::vector<size_t> boff(33, 0);
-  for (unsigned l = 0; l < 32; l++) boff[l + 1] = boff[l] + hcnt[l];
-
-  std::vector<DBuf<Key128>> I(maxL + 1);
-  std::vector<size_t> nI(maxL + 1, 0);
-  for (int l = (int)maxL; l >= 1; l--) {
-    size_t nt = hcnt[l], nq = nI[l];
-    size_t nc = nt + 8 * nq;
-    if (nc == 0) continue;
-    const int kbits = 3 * (l - 1) + (int)SB;
-    if (kbits <= 64) {
-      // level-(l-1) indices fit one word: sort 8-byte keys
-      DBuf<uint64_t> cand(nc, s), ctmp(nc, s);
-      if (nt) {
-        ProfScope _prof(ctx, "bal_leaf_parents", (double)nt * 24);
-        k_leaf_parents<uint64_t><<<grid_for(nt, 256), 256, 0, s>>>(bucketed.get() + boff[l], nt, D, (unsigned)l,
-                                                                   cand.get());
-        DG_LAUNCH_CHECK();
-      }
-      if (nq) {
-        ProfScope _prof(ctx, "bal_block_parents", (double)nq * 80);
-        k_block_parents<uint64_t><<<grid_for(nq, 256), 256, 0, s>>>(I[l].get(), nq, (unsigned)l, inc_corner, cand.get() + nt);
-        DG_LAUNCH_CHECK();
-      }
-      uint64_t *res;
-      size_t nu = sort_unique<uint64_t>(ctx, cand.get(), ctmp.get(), nc, kbits, &res);
-      DBuf<Key128> Il(nu, s);
-      {
-        ProfScope _prof(ctx, "bal_widen", (double)nu * 24);
-        k_widen<<<grid_for(nu, 256), 256, 0, s>>>(res, nu, Il.get());
-        DG_LAUNCH_CHECK();
-      }
-      I[l - 1] = std::move(Il);
-      nI[l - 1] = nu;
-    } else {
-      DBuf<Key128> cand(nc, s), ctmp(nc, s);
-      if (nt) {
-        ProfScope _prof(ctx, "bal_leaf_parents", (double)nt * 32);
-        k_leaf_parents<Key128><<<grid_for(nt, 256), 256, 0, s>>>(bucketed.get() + boff[l], nt, D, (unsigned)l,
-                                                                 cand.get());
-        DG_LAUNCH_CHECK();
-      }
-      if (nq) {
-        ProfScope _prof(ctx, "bal_block_parents", (double)nq * 144);
-        k_block_parents<Key128><<<grid_for(nq, 256), 256, 0, s>>>(I[l].get(), nq, (unsigned)l, inc_corner, cand.get() + nt);
-        DG_LAUNCH_CHECK();
-      }
-      Key128 *res;
-      size_t nu = sort_unique<Key128>(ctx, cand.get(), ctmp.get(), nc, kbits, &res);
-      DBuf<Key128> Il(nu, s);
-      DG_CUDA(cudaMemcpyAsync(Il.get(), res, nu * sizeof(Key128), cudaMemcpyDeviceToDevice, s));
-      I[l - 1] = std::move(Il);
-      nI[l - 1] = nu;
-    }
-  }
-  bucketed.release();
-
-  // rank maps R_l (l = 0..maxL-1): children of I_l that are internal
-  std::vector<DBuf<uint32_t>> R(maxL + 1);
-  for (unsigned l = 0; l + 1 <= maxL; l++) {
-    if (!nI[l] || !nI[l + 1]) continue;
-    R[l].alloc(8 * nI[l], s);
-    DG_CUDA(cudaMemsetAsync(R[l].get(), 0xff, 8 * nI[l] * sizeof(uint32_t), s));
-    {
-      ProfScope _prof(ctx, "bal_mark_internal", (double)nI[l + 1] * 20);
-      k_mark_internal<<<grid_for(nI[l + 1], 256), 256, 0, s>>>(I[l + 1].get(), nI[l + 1], I[l].get(), nI[l],
-                                                               R[l].get(), ctx.d_flags);
-      DG_LAUNCH_CHECK();
-    }
-  }
-  DBuf<uint32_t> Rtop(nseg, s);
-  DG_CUDA(cudaMemsetAsync(Rtop.get(), 0xff, nseg * sizeof(uint32_t), s));
-  if (maxL > 0 && nI[0]) {
-    k_mark_roots<<<grid_for(nI[0], 256), 256, 0, s>>>(I[0].get(), nI[0], nseg, Rtop.get(), ctx.d_flags);
-    DG_LAUNCH_CHECK();
-  }
+    if (hist[l]) top = l + 1;
+  DBuf<Key128> res;
+  DBuf<uint64_t> seg_off;
+  size_t nn = 0;
+  auto run = [&](auto tag) {
+    typedef decltype(tag) K;
+    DBuf<K> a, b;
+    K *nodes = nullptr;
+    if (top) nn = balance_nodes<K>(ctx, in, top, hist, inc_corner, a, b, &nodes);
+    emit_octree<K>(ctx, nodes, nn, top ? top - 1 : 0, D, nseg, res, seg_off);
+  };
+  if (top == 0 || nodes_fit_64(top, in.seg_bits)) run(uint64_t());
+  else run(Key128());
   check_device_flags(ctx, "balanceOctree");
-  // bottom-up leaf counts
-  std::vector<DBuf<uint64_t>> sub(maxL + 1);
-  for (int l = (int)maxL - 1; l >= 0; l--) {
-    if (!nI[l]) continue;
-    sub[l].alloc(nI[l], s);
-    {
-      ProfScope _prof(ctx, "bal_subtree_count", (double)nI[l] * 72);
-      k_subtree_count<<<grid_for(nI[l], 256), 256, 0, s>>>(R[l].get(), nI[l], sub[l + 1].get(), sub[l].get());
-      DG_LAUNCH_CHECK();
-    }
-  }
-  DBuf<uint64_t> ccnt(nseg, s), coff(nseg + 1, s);
-  k_cloud_count<<<grid_for(nseg, 256), 256, 0, s>>>(Rtop.get(), nseg, sub[0].get(), ccnt.get());
-  DG_LAUNCH_CHECK();
-  uint64_t *d_total = reinterpret_cast<uint64_t *>(ctx.d_scratch);
-  exclusive_scan<uint64_t, uint64_t>(ccnt.get(), coff.get(), nseg, d_total, s);
-  size_t total = (size_t)read_scalar(ctx, d_total);
-  DG_CUDA(cudaMemcpyAsync(coff.get() + nseg, d_total, sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
-  DBuf<Key128> res(total, s);
-  // top-down placement
-  DBuf<uint64_t> off_cur(nI[0] ? nI[0] : 1, s);
-  k_place_roots<<<grid_for(nseg, 256), 256, 0, s>>>(Rtop.get(), nseg, coff.get(), D, off_cur.get(), res.get());
-  DG_LAUNCH_CHECK();
-  for (unsigned l = 0; l < maxL; l++) {
-    if (!nI[l]) break;
-    DBuf<uint64_t> off_next(nI[l + 1] ? nI[l + 1] : 1, s);
-    {
-      ProfScope _prof(ctx, "bal_place", (double)nI[l] * 24);
-      k_place<<<grid_for(nI[l], 256), 256, 0, s>>>(I[l].get(), nI[l], l, D, R[l].get(), sub[l + 1].get(),
-                                                   off_cur.get(), off_next.get(), res.get());
-      DG_LAUNCH_CHECK();
-    }
-    off_cur = std::move(off_next);
-  }
-  DG_CUDA(cudaStreamSynchronize(s));
-  out.n = total;
+  out.n = 7 * nn + nseg;
   out.keys = res.release_ptr();
-  out.seg_off = nseg > 1 ? coff.release_ptr() : nullptr;
+  out.seg_off = nseg > 1 ? seg_off.release_ptr() : nullptr;
 }
 
 // ------------------------------------------------------------------------
@@ -1177,6 +1446,7 @@ static void octree_to_xyzl_hilbert(Context &ctx, const Octree &o, uint32_t *d_xy
     k_hilbert_keys<<<grid_for(n, 256), 256, 0, s>>>(o.keys + off[g], n, D, o.nseg > 1, tab, a.get() + off[g]);
     DG_LAUNCH_CHECK();
     Key128 *srt = radix_sort<Key128>(ctx, a.get() + off[g], b.get() + off[g], n, 3 * (int)D + 5 + 32);
+    check_device_flags(ctx, "Hilbert order");
     k_gather_xyzl<<<grid_for(n, 256), 256, 0, s>>>(o.keys + off[g], srt, n, D, o.nseg > 1,
                                                    reinterpret_cast<uint4 *>(d_xyzl) + off[g]);
     DG_LAUNCH_CHECK();
@@ -1214,6 +1484,7 @@ void octree_from_xyzl(Context &ctx, const uint32_t *d_xyzl, size_t n, unsigned D
       k_to_sortform<<<grid_for(n, 256), 256, 0, ctx.stream>>>(k.get(), n, a.get());
       DG_LAUNCH_CHECK();
       Key128 *srt = radix_sort<Key128>(ctx, a.get(), b.get(), n, 3 * (int)D + 5);
+      check_device_flags(ctx, "Hilbert order");
       k_from_sortform<<<grid_for(n, 256), 256, 0, ctx.stream>>>(srt, n, k.get());
       DG_LAUNCH_CHECK();
     }
@@ -1308,7 +1579,10 @@ void sort_octants(Context &ctx, const uint32_t *d_xyzl, size_t n, unsigned D, in
   Key128 *srt = a.get();
   size_t m = n;
   if (unique) m = sort_unique<Key128>(ctx, a.get(), b.get(), n, bits, &srt);
-  else srt = radix_sort<Key128>(ctx, a.get(), b.get(), n, bits);
+  else {
+    srt = radix_sort<Key128>(ctx, a.get(), b.get(), n, bits);
+    check_device_flags(ctx, "sortOctants");
+  }
   if (mode == 2) {
     // tagged keys of the octants not followed by a descendant
     Key128 *other = (srt == a.get()) ? b.get() : a.get();

@@ -1,11 +1,5 @@
 // Device-wide primitives: exclusive scan, stream compaction and a stable
-// LSD radix sort of 64- or 128-bit keys that skips the digits on which all
-// keys agree.
-//
-// Radix sort, per 8-bit digit: (1) per-tile 256-bin histograms (shared
-// atomics), (2) one exclusive scan of the digit-major histogram matrix,
-// (3) a stable scatter in which each warp ranks its keys in order with
-// __match_any_sync and per-warp running digit counters in shared memory.
+// LSD radix sort ("onesweep") of 64- or 128-bit keys.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -194,93 +188,12 @@ size_t compact(Context &ctx, const T *in, const uint32_t *flags, size_t n, T *ou
 // ------------------------------------------------------------------------
 constexpr int RS_BLOCK = 256;
 constexpr int RS_WARPS = RS_BLOCK / 32;
-constexpr int RS_ITEMS = 8;
-constexpr int RS_TILE = RS_BLOCK * RS_ITEMS;
-constexpr int RS_WARP_KEYS = RS_TILE / RS_WARPS;
-
-template <typename K>
-__global__ void __launch_bounds__(RS_BLOCK) k_rs_hist(const K *__restrict__ keys, size_t n, int shift,
-                                                      uint32_t *__restrict__ hist, size_t ntiles) {
-  __shared__ uint32_t h[256];
-  h[threadIdx.x] = 0;
-  __syncthreads();
-  size_t base = (size_t)blockIdx.x * RS_TILE;
-#pragma unroll
-  for (int i = 0; i < RS_ITEMS; i++) {
-    size_t idx = base + (size_t)i * RS_BLOCK + threadIdx.x;
-    if (idx < n) atomicAdd(&h[KeyOps<K>::digit(keys[idx], shift)], 1u);
-  }
-  __syncthreads();
-  hist[(size_t)threadIdx.x * ntiles + blockIdx.x] = h[threadIdx.x];
-}
-
-template <typename K>
-__global__ void __launch_bounds__(RS_BLOCK) k_rs_scatter(const K *__restrict__ in, K *__restrict__ out, size_t n,
-                                                         int shift, const uint32_t *__restrict__ offs,
-                                                         size_t ntiles) {
-  __shared__ K tk[RS_TILE];
-  __shared__ uint32_t wh[RS_WARPS][256];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const size_t base = (size_t)blockIdx.x * RS_TILE;
-#pragma unroll
-  for (int i = 0; i < RS_ITEMS; i++) {
-    size_t idx = base + (size_t)i * RS_BLOCK + threadIdx.x;
-    if (idx < n) tk[i * RS_BLOCK + threadIdx.x] = in[idx];
-  }
-#pragma unroll
-  for (int i = 0; i < 256 / 32; i++) wh[wid][i * 32 + lane] = 0;
-  __syncthreads();
-  const unsigned lt_mask = (1u << lane) - 1u;
-  // phase A: per-warp digit counts over the warp's contiguous key range
-#pragma unroll
-  for (int r = 0; r < RS_WARP_KEYS / 32; r++) {
-    int t = wid * RS_WARP_KEYS + r * 32 + lane;
-    bool valid = base + (size_t)t < n;
-    unsigned d = valid ? KeyOps<K>::digit(tk[t], shift) : 256u + lane;
-    unsigned peers = __match_any_sync(0xffffffffu, d);
-    if (valid && (peers & lt_mask) == 0) wh[wid][d] += __popc(peers);
-  }
-  __syncthreads();
-  // phase B: turn counts into global write positions, warp order within tile
-  {
-    unsigned d = threadIdx.x;
-    uint32_t run = offs[(size_t)d * ntiles + blockIdx.x];
-#pragma unroll
-    for (int w = 0; w < RS_WARPS; w++) {
-      uint32_t c = wh[w][d];
-      wh[w][d] = run;
-      run += c;
-    }
-  }
-  __syncthreads();
-  // phase C: stable ranks, scatter
-#pragma unroll
-  for (int r = 0; r < RS_WARP_KEYS / 32; r++) {
-    int t = wid * RS_WARP_KEYS + r * 32 + lane;
-    bool valid = base + (size_t)t < n;
-    K k;
-    unsigned d;
-    if (valid) {
-      k = tk[t];
-      d = KeyOps<K>::digit(k, shift);
-    } else {
-      d = 256u + lane;
-    }
-    unsigned peers = __match_any_sync(0xffffffffu, d);
-    uint32_t pos = 0;
-    if (valid) pos = wh[wid][d] + __popc(peers & lt_mask);
-    __syncwarp();
-    if (valid && (peers & lt_mask) == 0) wh[wid][d] += __popc(peers);
-    __syncwarp();
-    if (valid) out[pos] = k;
-  }
-}
 
 // ------------------------------------------------------------------------
 // single-pass-per-digit ("onesweep") radix sort
 //   1. one read of all keys builds the 256-bin histogram of every digit
-//      position that is sorted; digits with a single occupied bin are
-//      skipped; the digit offsets come from these histograms
+//      position that is sorted; one block per digit turns it into offsets
+//      (on the device: the sort is launched without a read-back)
 //   2. per digit, one kernel: a block takes the next tile (ticket order),
 //      counts its digits, publishes the counts, looks back over the
 //      preceding tiles' published counts (decoupled look-back) for its
@@ -289,9 +202,13 @@ __global__ void __launch_bounds__(RS_BLOCK) k_rs_scatter(const K *__restrict__ i
 // DGF_TIMEOUT and the host reports DG_ERR_TIMEOUT.
 // ------------------------------------------------------------------------
 constexpr int OS_MAX_PASSES = 16;
-constexpr uint64_t OS_FLAG_AGG = 1ull << 62;
-constexpr uint64_t OS_FLAG_INCL = 2ull << 62;
-constexpr uint64_t OS_VALUE = (1ull << 62) - 1;
+// a look-back word: two flag bits above a count; 32-bit words for sorts of
+// fewer than 2^30 keys (half the words to clear and read), else 64-bit
+template <typename S>
+struct OsWord {
+  static constexpr int SHIFT = 8 * sizeof(S) - 2;
+  static constexpr S AGG = (S)1 << SHIFT, INCL = (S)2 << SHIFT, VALUE = ((S)1 << SHIFT) - 1;
+};
 constexpr unsigned OS_SPIN_LIMIT = 1u << 22;
 
 // tile of one onesweep block: ITEMS keys per thread (the default; the
@@ -316,30 +233,44 @@ __device__ __forceinline__ uint64_t ld_relaxed(const uint64_t *p) {
 __device__ __forceinline__ void st_relaxed(uint64_t *p, uint64_t v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+__device__ __forceinline__ uint32_t ld_relaxed(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed(uint32_t *p, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 
 // Histograms of every sorted digit position in one read of the keys.  Two
 // shared copies (even / odd lanes) halve the same-address contention that
 // skewed high digits cause.
 template <typename K>
 __global__ void __launch_bounds__(RS_BLOCK) k_rs_digit_hists(const K *__restrict__ keys, size_t n, int npass,
-                                                              const int *__restrict__ shifts,
-                                                              unsigned long long *__restrict__ ghist) {
+                                                              int shift0, unsigned long long *__restrict__ ghist) {
   __shared__ uint32_t h[2][OS_MAX_PASSES * 256];
-  __shared__ int sh[OS_MAX_PASSES];
-  for (int i = threadIdx.x; i < 2 * OS_MAX_PASSES * 256; i += blockDim.x) (&h[0][0])[i] = 0;
-  if (threadIdx.x < npass) sh[threadIdx.x] = shifts[threadIdx.x];
+  for (int i = threadIdx.x; i < npass * 256; i += blockDim.x) h[0][i] = h[1][i] = 0;
   __syncthreads();
   uint32_t *mine = h[threadIdx.x & 1];
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     K k = keys[i];
-    for (int p = 0; p < npass; p++) atomicAdd(&mine[p * 256 + KeyOps<K>::digit(k, sh[p])], 1u);
+    for (int p = 0; p < npass; p++) atomicAdd(&mine[p * 256 + KeyOps<K>::digit(k, shift0 + 8 * p)], 1u);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < npass * 256; i += blockDim.x) {
     uint32_t v = h[0][i] + h[1][i];
     if (v) atomicAdd(&ghist[i], (unsigned long long)v);
   }
+}
+
+// digit offsets: exclusive scan of each pass's 256 bins (one block per pass)
+template <int UNUSED = 0>
+__global__ void __launch_bounds__(256) k_rs_offsets(const unsigned long long *__restrict__ ghist,
+                                                    uint64_t *__restrict__ offs) {
+  const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+  unsigned long long total;
+  offs[i] = block_excl_scan<unsigned long long, 256>(ghist[i], total);
 }
 
 // One digit pass.  Keys are ranked in registers (warp-striped tile layout:
@@ -349,11 +280,12 @@ __global__ void __launch_bounds__(RS_BLOCK) k_rs_digit_hists(const K *__restrict
 // addresses of each digit's run.
 // MINB: blocks per SM the kernel is compiled for (register budget); the
 // autotuner picks the tile and MINB per size class.
-template <typename K, int ITEMS = OsCfg<K>::ITEMS, int MINB = 4>
+template <typename K, int ITEMS = OsCfg<K>::ITEMS, int MINB = 4, typename S = uint64_t>
 __global__ void __launch_bounds__(RS_BLOCK, MINB) k_rs_onesweep(const K *__restrict__ in, K *__restrict__ out, size_t n,
                                                           int shift, const uint64_t *__restrict__ digit_off,
-                                                          uint64_t *__restrict__ status, unsigned *tile_counter,
+                                                          S *__restrict__ status, unsigned *tile_counter,
                                                           uint32_t *flags) {
+  using W = OsWord<S>;
   constexpr int TILE = RS_BLOCK * ITEMS, WK = TILE / RS_WARPS;
   __shared__ K tk[TILE];
   __shared__ uint32_t wh[RS_WARPS][256];
@@ -405,27 +337,27 @@ __global__ void __launch_bounds__(RS_BLOCK, MINB) k_rs_onesweep(const K *__restr
     uint32_t total_unused;
     const uint32_t local = block_excl_scan<uint32_t, RS_BLOCK>(run, total_unused);
     s_local[dg] = local;
-    uint64_t *my = status + (size_t)tile * 256 + dg;
+    S *my = status + (size_t)tile * 256 + dg;
     uint64_t excl = 0;
     if (tile == 0) {
-      st_relaxed(my, OS_FLAG_INCL | (uint64_t)run);
+      st_relaxed(my, W::INCL | (S)run);
     } else {
-      st_relaxed(my, OS_FLAG_AGG | (uint64_t)run);
+      st_relaxed(my, W::AGG | (S)run);
       // look back four predecessors per round trip: their words are read
       // together, then summed newest first until an inclusive one; a word
       // not yet published is waited for (bounded) and the walk resumes there
       long t = (long)tile - 1;
       unsigned spins = 0;
       while (t >= 0) {
-        uint64_t v[4];
+        S v[4];
 #pragma unroll
-        for (int q = 0; q < 4; q++) v[q] = (t - q >= 0) ? ld_relaxed(status + (size_t)(t - q) * 256 + dg) : 0;
+        for (int q = 0; q < 4; q++) v[q] = (t - q >= 0) ? ld_relaxed(status + (size_t)(t - q) * 256 + dg) : (S)0;
         int q = 0;
         bool done = false;
         for (; q < 4 && t - q >= 0; q++) {
-          if ((v[q] & ~OS_VALUE) == 0) break;
-          excl += v[q] & OS_VALUE;
-          if (v[q] & OS_FLAG_INCL) {
+          if ((v[q] & (S)~W::VALUE) == 0) break;
+          excl += v[q] & W::VALUE;
+          if (v[q] & W::INCL) {
             done = true;
             break;
           }
@@ -440,7 +372,7 @@ __global__ void __launch_bounds__(RS_BLOCK, MINB) k_rs_onesweep(const K *__restr
           __nanosleep(32);
         }
       }
-      st_relaxed(my, OS_FLAG_INCL | (excl + run));
+      st_relaxed(my, W::INCL | (S)(excl + run));
     }
     s_glob[dg] = digit_off[dg] + excl - (uint64_t)local;
   }
@@ -460,21 +392,16 @@ __global__ void __launch_bounds__(RS_BLOCK, MINB) k_rs_onesweep(const K *__restr
   }
 }
 
-// Sort n keys (stable) on the digits of bits [0, end_bit) (8-bit digits;
-// end_bit must not cut into bits that vary above it).  Digits on which all
-// keys agree are skipped.  Returns the buffer that holds the result (keys or
-// tmp).
+// Sort n keys (stable) on the 8-bit digits of bits [begin_bit, end_bit) (the
+// last digit may reach past end_bit: bits there must agree or be part of the
+// order).  Returns the buffer that holds the result (keys or tmp).  Launches
+// only: nothing is read back, and DGF_TIMEOUT in ctx.d_flags tells a failed
+// look-back, which the caller checks before it uses the keys as indices.
 template <typename K>
-K *radix_sort(Context &ctx, K *keys, K *tmp, size_t n, int end_bit) {
-  if (n < 2 || end_bit <= 0) return keys;
+K *radix_sort(Context &ctx, K *keys, K *tmp, size_t n, int end_bit, int begin_bit = 0) {
+  if (n < 2 || end_bit <= begin_bit) return keys;
   cudaStream_t s = ctx.stream;
-  int shifts[OS_MAX_PASSES];
-  int npass = 0;
-  for (int sh = 0; sh < end_bit && sh < KeyOps<K>::BITS && npass < OS_MAX_PASSES; sh += 8) shifts[npass++] = sh;
-  // histograms of every digit position, one read of the keys
-  DBuf<unsigned long long> ghist(npass * 256, s);
-  DBuf<int> dshifts(npass, s);
-  DG_CUDA(cudaMemcpyAsync(dshifts.get(), shifts, npass * sizeof(int), cudaMemcpyHostToDevice, s));
+  const int npass = (std::min(end_bit, KeyOps<K>::BITS) - begin_bit + 7) / 8;
   // launch shape of this size class: the context's decision, else the
   // disk cache's, else tuned below
   const int width = sizeof(K) == 16 ? 1 : 0;
@@ -489,6 +416,20 @@ K *radix_sort(Context &ctx, K *keys, K *tmp, size_t n, int end_bit) {
     ctx.tune_log += line;
   }
   const bool tuning = tunable && tn.items == 0;
+  // one cleared buffer: histograms, tile tickets and every pass's look-back words
+  const bool wide = n >= ((size_t)1 << 30);
+  const size_t max_tile = RS_BLOCK * (size_t)(tuning || (tn.items && tn.items != OsCfg<K>::ITEMS) ? OsAlt<K>::ITEMS
+                                                                                                  : OsCfg<K>::ITEMS);
+  const size_t max_tiles = (n + max_tile - 1) / max_tile;
+  if (max_tiles >= 0xffffffffull) fail(DG_ERR_INVALID_ARG, "radix sort: too many keys");
+  const size_t word = wide ? 8 : 4, pass_bytes = max_tiles * 256 * word;
+  const size_t head = (size_t)npass * 256 * 8 + OS_MAX_PASSES * sizeof(unsigned);
+  DBuf<unsigned char> work(head + npass * pass_bytes, s);
+  DBuf<uint64_t> doffs(npass * 256, s);
+  auto *ghist = reinterpret_cast<unsigned long long *>(work.get());
+  auto *tickets = reinterpret_cast<unsigned *>(work.get() + (size_t)npass * 256 * 8);
+  unsigned char *status = work.get() + head;
+  DG_CUDA(cudaMemsetAsync(work.get(), 0, head + npass * pass_bytes, s));
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (tuning) {
     DG_CUDA(cudaEventCreate(&e0));
@@ -509,10 +450,9 @@ K *radix_sort(Context &ctx, K *keys, K *tmp, size_t n, int end_bit) {
     return best;
   };
   auto hists = [&](int mul) {
-    DG_CUDA(cudaMemsetAsync(ghist.get(), 0, npass * 256 * sizeof(unsigned long long), s));
     ProfScope _prof(ctx, "rs_digit_hists", (double)n * sizeof(K));
     unsigned g = grid_for(n, RS_BLOCK, (unsigned)(ctx.num_sms * mul));
-    k_rs_digit_hists<K><<<g, RS_BLOCK, 0, s>>>(keys, n, npass, dshifts.get(), ghist.get());
+    k_rs_digit_hists<K><<<g, RS_BLOCK, 0, s>>>(keys, n, npass, begin_bit, ghist);
     DG_LAUNCH_CHECK();
   };
   float hist_ms[3] = {0.f, 0.f, 0.f};
@@ -523,61 +463,42 @@ K *radix_sort(Context &ctx, K *keys, K *tmp, size_t n, int end_bit) {
     for (int c = 1; c < 3; c++)
       if (hist_ms[c] < hist_ms[b]) b = c;
     tn.hist_mul = hist_cand[b];
+    DG_CUDA(cudaMemsetAsync(ghist, 0, (size_t)npass * 256 * 8, s));
   }
   hists(tn.hist_mul ? tn.hist_mul : 4);
-  std::vector<unsigned long long> h(npass * 256);
-  DG_CUDA(cudaMemcpyAsync(h.data(), ghist.get(), h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-  DG_CUDA(cudaStreamSynchronize(s));
-  std::vector<int> active;
-  std::vector<uint64_t> offs;
-  for (int p = 0; p < npass; p++) {
-    int occupied = 0;
-    for (int d = 0; d < 256; d++) occupied += h[p * 256 + d] != 0;
-    if (occupied <= 1) continue;  // every key has the same digit here
-    active.push_back(p);
-    uint64_t run = 0;
-    for (int d = 0; d < 256; d++) {
-      offs.push_back(run);
-      run += h[p * 256 + d];
-    }
+  {
+    ProfScope _prof(ctx, "rs_offsets", (double)npass * 4096);
+    k_rs_offsets<><<<npass, 256, 0, s>>>(ghist, doffs.get());
+    DG_LAUNCH_CHECK();
   }
-  if (active.empty()) {
-    if (tuning) {
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      tn = Context::Tune();  // nothing to sort here: decide on a later sort of this size
-    }
-    return keys;
-  }
-  DBuf<uint64_t> doffs(offs.size(), s);
-  DG_CUDA(cudaMemcpyAsync(doffs.get(), offs.data(), offs.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
-  const size_t max_tiles = (n + RS_BLOCK * OsAlt<K>::ITEMS - 1) / (RS_BLOCK * OsAlt<K>::ITEMS);
-  if (max_tiles >= 0xffffffffull) fail(DG_ERR_INVALID_ARG, "radix sort: too many keys");
-  DBuf<uint64_t> status(max_tiles * 256, s);
-  unsigned *d_counter = reinterpret_cast<unsigned *>(ctx.d_scratch + 12);
   // one digit pass with `items` keys per thread, compiled for `minb` blocks
   // per SM
-  auto pass = [&](int items, int minb, const K *src, K *dst, size_t a) {
+  auto pass = [&](int items, int minb, const K *src, K *dst, int a) {
     if (items != OsCfg<K>::ITEMS) items = OsAlt<K>::ITEMS;  // the two compiled tiles
-    const size_t tile = (size_t)RS_BLOCK * items, ntiles = (n + tile - 1) / tile;
-    DG_CUDA(cudaMemsetAsync(status.get(), 0, ntiles * 256 * sizeof(uint64_t), s));
-    DG_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(unsigned), s));
-    ProfScope _prof(ctx, "rs_onesweep", (double)n * sizeof(K) * 2);
-    const int sh = shifts[active[a]];
+    const size_t tile = (size_t)RS_BLOCK * items;
+    const unsigned g = (unsigned)((n + tile - 1) / tile);
+    const int sh = begin_bit + 8 * a;
     const uint64_t *off = doffs.get() + 256 * a;
-    const unsigned g = (unsigned)ntiles;
-    if (items == OsCfg<K>::ITEMS && minb == 3)
-      k_rs_onesweep<K, OsCfg<K>::ITEMS, 3><<<g, RS_BLOCK, 0, s>>>(src, dst, n, sh, off, status.get(), d_counter,
-                                                                  ctx.d_flags);
-    else if (items == OsCfg<K>::ITEMS && minb == 5)
-      k_rs_onesweep<K, OsCfg<K>::ITEMS, 5><<<g, RS_BLOCK, 0, s>>>(src, dst, n, sh, off, status.get(), d_counter,
-                                                                  ctx.d_flags);
-    else if (items == OsCfg<K>::ITEMS)
-      k_rs_onesweep<K, OsCfg<K>::ITEMS, 4><<<g, RS_BLOCK, 0, s>>>(src, dst, n, sh, off, status.get(), d_counter,
-                                                                  ctx.d_flags);
-    else
-      k_rs_onesweep<K, OsAlt<K>::ITEMS, 4><<<g, RS_BLOCK, 0, s>>>(src, dst, n, sh, off, status.get(), d_counter,
-                                                                  ctx.d_flags);
+    unsigned char *st = status + a * pass_bytes;
+    ProfScope _prof(ctx, "rs_onesweep", (double)n * sizeof(K) * 2);
+    auto run = [&](auto word_tag) {
+      using S = decltype(word_tag);
+      S *w = reinterpret_cast<S *>(st);
+      if (items == OsCfg<K>::ITEMS && minb == 3)
+        k_rs_onesweep<K, OsCfg<K>::ITEMS, 3, S><<<g, RS_BLOCK, 0, s>>>(src, dst, n, sh, off, w, tickets + a,
+                                                                       ctx.d_flags);
+      else if (items == OsCfg<K>::ITEMS && minb == 5)
+        k_rs_onesweep<K, OsCfg<K>::ITEMS, 5, S><<<g, RS_BLOCK, 0, s>>>(src, dst, n, sh, off, w, tickets + a,
+                                                                       ctx.d_flags);
+      else if (items == OsCfg<K>::ITEMS)
+        k_rs_onesweep<K, OsCfg<K>::ITEMS, 4, S><<<g, RS_BLOCK, 0, s>>>(src, dst, n, sh, off, w, tickets + a,
+                                                                       ctx.d_flags);
+      else
+        k_rs_onesweep<K, OsAlt<K>::ITEMS, 4, S><<<g, RS_BLOCK, 0, s>>>(src, dst, n, sh, off, w, tickets + a,
+                                                                       ctx.d_flags);
+    };
+    if (wide) run(uint64_t());
+    else run(uint32_t());
     DG_LAUNCH_CHECK();
   };
   // autotuner: the first sort of each size class (log2 of the key count)
@@ -585,7 +506,7 @@ K *radix_sort(Context &ctx, K *keys, K *tmp, size_t n, int end_bit) {
   // so every run writes the same output) and keeps the fastest for every
   // later pass and sort of that class
   K *src = keys, *dst = tmp;
-  size_t a0 = 0;
+  int a0 = 0;
   if (tuning) {
     struct Cand {
       int items, minb;
@@ -594,7 +515,11 @@ K *radix_sort(Context &ctx, K *keys, K *tmp, size_t n, int end_bit) {
     float ms[4];
     int b = 0;
     for (int c = 0; c < 4; c++) {
-      ms[c] = time2([&]() { pass(cand[c].items, cand[c].minb, src, dst, 0); });
+      ms[c] = time2([&]() {
+        DG_CUDA(cudaMemsetAsync(tickets, 0, sizeof(unsigned), s));
+        DG_CUDA(cudaMemsetAsync(status, 0, pass_bytes, s));
+        pass(cand[c].items, cand[c].minb, src, dst, 0);
+      });
       if (ms[c] < ms[b]) b = c;
     }
     cudaEventDestroy(e0);
@@ -614,13 +539,10 @@ K *radix_sort(Context &ctx, K *keys, K *tmp, size_t n, int end_bit) {
     a0 = 1;
   }
   const int use = tn.items ? tn.items : OsCfg<K>::ITEMS, use_minb = tn.minb ? tn.minb : 4;
-  for (size_t a = a0; a < active.size(); a++) {
+  for (int a = a0; a < npass; a++) {
     pass(use, use_minb, src, dst, a);
-    K *t = src;
-    src = dst;
-    dst = t;
+    std::swap(src, dst);
   }
-  check_device_flags(ctx, "radix sort");
   return src;
 }
 
@@ -740,6 +662,7 @@ size_t sort_unique(Context &ctx, K *keys, K *tmp, size_t n, int end_bit, K **res
     return (size_t)read_scalar(ctx, d_count);
   }
   K *sorted = radix_sort<K>(ctx, keys, tmp, n, end_bit);
+  check_device_flags(ctx, "radix sort");
   K *out = (sorted == keys) ? tmp : keys;
   DBuf<uint32_t> flags(n, ctx.stream);
   {
