@@ -228,6 +228,9 @@ __global__ void __launch_bounds__(P2O_BLOCK) k_p2o_count(const Key128 *__restric
 // ------------------------------------------------------------------------
 __device__ __forceinline__ uint64_t node_wide(uint64_t k) { return k; }
 __device__ __forceinline__ u128 node_wide(Key128 k) { return to_u128(k); }
+// no node: the level bits of a node never are 31
+__device__ __forceinline__ uint64_t node_empty(uint64_t) { return ~0ull; }
+__device__ __forceinline__ u128 node_empty(u128) { return ~(u128)0; }
 template <typename K>
 struct NodeWide;
 template <>
@@ -286,50 +289,66 @@ __global__ void __launch_bounds__(P2O_BLOCK) k_p2o_nodes(const Key128 *__restric
   }
 }
 
+__device__ __forceinline__ uint64_t shfl_wide(uint64_t v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+__device__ __forceinline__ u128 shfl_wide(u128 v, int lane) {
+  return (u128)__shfl_sync(0xffffffffu, (uint64_t)(v >> 64), lane) << 64 | __shfl_sync(0xffffffffu, (uint64_t)v, lane);
+}
+
 // The leaves of the octrees whose nodes are given (sorted), 8 threads per
-// node: child c of the node at index i is a leaf unless it is a node itself,
-// which is searched where the node has descendants (from i + 1, galloping).
+// node: child c of the node at index i is a leaf unless it is a node itself.
 // The leaf's place is 7 (j - level) + digits + cloud, j the number of nodes
 // before it in preorder (every cloud before it has one leaf more than 7 per
-// node).
+// node).  A warp holds four nodes and the 32 nodes that follow the first of
+// them in its registers, so j comes from a search by shuffles; only a subtree
+// that reaches past those is searched in memory.
 template <typename K>
-__global__ void k_emit_leaves(const K *__restrict__ nodes, size_t nn, unsigned Lm, unsigned D,
-                              Key128 *__restrict__ out, size_t total) {
+__global__ void __launch_bounds__(256) k_emit_leaves(const K *__restrict__ nodes, size_t nn, unsigned Lm, unsigned D,
+                                                     Key128 *__restrict__ out, size_t total) {
   typedef NodeWide<K> N;
   typedef typename N::W W;
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t i = t >> 3;
-  const unsigned c = (unsigned)(t & 7u);
-  if (i >= nn) return;
-  const W k = node_wide(nodes[i]);
+  const int lane = threadIdx.x & 31;
+  const size_t i0 = ((size_t)blockIdx.x * 256 + threadIdx.x) >> 5 << 2;  // the warp's first node
+  if (i0 >= nn) return;
+  const size_t i = i0 + (lane >> 3);
+  const unsigned c = lane & 7;
+  const W follow = i0 + 1 + lane < nn ? node_wide(nodes[i0 + 1 + lane]) : node_empty(W());
+  const W k = i < nn ? node_wide(nodes[i]) : (W)0;
   const unsigned d = (unsigned)k & 31u;
   const W path = k >> 5;
-  const W sub = (W)1 << (3 * (Lm - d));  // paths below the node
-  size_t j = i + 1;
-  Key128 anchor;  // child c, at depth D
+  // child c, at depth D, and its key where it can be a node
+  Key128 anchor;
+  W ck = k + 1;  // level Lm: no node below
   if (d == Lm) {
     anchor = key_or(key_shl(N::key(path), 3 * (D - Lm)), key_shl(Key128{c, 0}, 3 * (D - Lm - 1)));
   } else {
-    const W child = path + (W)c * (sub >> 3);
+    const W child = path + ((W)c << (3 * (Lm - d - 1)));
     anchor = key_shl(N::key(child), 3 * (D - Lm));
-    if (j < nn && (node_wide(nodes[j]) >> 5) < path + sub) {
-      const W ck = child << 5 | (W)(d + 1);
-      // first node at or after ck
-      size_t step = 1, lo = j, hi = nn;
-      while (lo < nn && node_wide(nodes[lo]) < ck) {
-        j = lo + 1;
-        lo += step;
-        step <<= 1;
-      }
-      if (lo < hi) hi = lo;
-      while (j < hi) {
-        const size_t mid = j + (hi - j) / 2;
-        if (node_wide(nodes[mid]) < ck) j = mid + 1;
-        else hi = mid;
-      }
-      if (j < nn && node_wide(nodes[j]) == ck) return;  // a node itself
-    }
+    ck = child << 5 | (W)(d + 1);
   }
+  int at = 0;  // nodes of `follow` before ck
+#pragma unroll
+  for (int step = 16; step > 0; step >>= 1)
+    if (shfl_wide(follow, at + step - 1) < ck) at += step;
+  const W found = shfl_wide(follow, at);
+  if (i >= nn) return;
+  size_t j = i0 + 1 + at;
+  bool node = found == ck;
+  if (at == 31 && found < ck) {  // galloping past the 32
+    size_t lo = ++j, step = 1, hi;
+    while (lo < nn && node_wide(nodes[lo]) < ck) {
+      j = lo + 1;
+      lo += step;
+      step <<= 1;
+    }
+    hi = min(lo, nn);
+    while (j < hi) {
+      const size_t mid = j + (hi - j) / 2;
+      if (node_wide(nodes[mid]) < ck) j = mid + 1;
+      else hi = mid;
+    }
+    node = j < nn && node_wide(nodes[j]) == ck;
+  }
+  if (node && d != Lm) return;
   const W in_cloud = path & (((W)1 << (3 * Lm)) - 1);
   const size_t pos = 7 * (j - (d + 1)) + digit_sum(in_cloud) + c + (size_t)(path >> (3 * Lm));
   if (pos < total) out[pos] = make_tagged(anchor, d + 1);
@@ -845,9 +864,6 @@ __device__ __forceinline__ uint64_t node_hash(u128 k, unsigned Lm) {
   const u128 par = k >> sh >> 3;
   return mix64(((uint64_t)par ^ (uint64_t)(par >> 64) * 0x9e3779b97f4a7c15ull) * 32 + l) << 3 | ((uint64_t)(k >> sh) & 7u);
 }
-__device__ __forceinline__ uint64_t node_empty(uint64_t) { return ~0ull; }
-__device__ __forceinline__ u128 node_empty(u128) { return ~(u128)0; }
-
 // compare-and-swap of one slot, returning what it held
 __device__ __forceinline__ uint64_t slot_cas(uint64_t *slot, uint64_t key) {
   const uint64_t cur = __ldcg(slot);  // a full slot never changes
@@ -934,8 +950,8 @@ template <typename K>
 struct BalSmem {
   K cand[BAL_CAND];
   uint32_t slot[BAL_SLOTS];
-  uint16_t won[BAL_CAND];
-  unsigned n_won;
+  uint16_t list[BAL_CAND], won[BAL_CAND];
+  unsigned n_cand, n_won;
   unsigned long long at;
 };
 
@@ -954,12 +970,16 @@ __global__ void __launch_bounds__(BAL_TILE) k_bal_level(unsigned l, unsigned Lm,
   for (unsigned q = l + 1; q <= Lm; q++) first += cnt->grown[q];
   if (first + n1 > grown_cap) return;  // the list overflowed (flagged): the host starts again
   const size_t n = n0 + n1, next = first + n1;
-  for (size_t tile = blockIdx.x; tile * BAL_TILE < n; tile += gridDim.x) {
-    const size_t i = tile * BAL_TILE + t;
-    for (int q = t; q < BAL_SLOTS; q += BAL_TILE) S.slot[q] = BAL_FREE;
-    if (t == 0) S.n_won = 0;
-    uint32_t valid = 0;
-    if (i < n) {
+  // nodes per tile: all blocks get some, up to BAL_TILE
+  const unsigned per = (unsigned)min((size_t)BAL_TILE, max((size_t)16, (n + gridDim.x - 1) / gridDim.x));
+  unsigned slots = 32;
+  while (slots < 16 * per) slots <<= 1;
+  for (size_t base = (size_t)blockIdx.x * per; base < n; base += (size_t)gridDim.x * per) {
+    const unsigned here = (unsigned)min((size_t)per, n - base);
+    for (unsigned q = t; q < slots; q += BAL_TILE) S.slot[q] = BAL_FREE;
+    if (t == 0) S.n_cand = S.n_won = 0;
+    if (t < here) {
+      const size_t i = base + t;
       const W k = node_wide(i < n0 ? leafs[lists.off[l] + i] : grown[first + (i - n0)]);
       const W path = k >> 5;
       const W cloud = path >> (3 * Lm);
@@ -977,27 +997,31 @@ __global__ void __launch_bounds__(BAL_TILE) k_bal_level(unsigned l, unsigned Lm,
       }
 #pragma unroll
       for (int q = 0; q < 8; q++) {
-        if (((q & 1) && !in[0]) || ((q & 2) && !in[1]) || ((q & 4) && !in[2]) || (q == 7 && !inc_corner)) continue;
-        valid |= 1u << q;
+        const bool skip = ((q & 1) && !in[0]) || ((q & 2) && !in[1]) || ((q & 4) && !in[2]) || (q == 7 && !inc_corner);
         const W par = cloud << (3 * (l - 1)) | N::of(morton3(opt[0][q & 1], opt[1][q >> 1 & 1], opt[2][q >> 2]));
-        S.cand[8 * t + q] = N::narrow(par << (3 * (Lm - l + 1)) << 5 | (W)(l - 1));
+        S.cand[8 * t + q] = skip ? N::narrow(node_empty(k)) : N::narrow(par << (3 * (Lm - l + 1)) << 5 | (W)(l - 1));
       }
     }
     __syncthreads();
-#pragma unroll 1
-    for (int q = 0; q < 8; q++) {
-      if (!(valid >> q & 1u)) continue;
-      const uint32_t me = 8 * t + q;
+    for (unsigned me = t; me < 8 * here; me += BAL_TILE) {
       const W key = node_wide(S.cand[me]);
-      uint32_t h = (uint32_t)(node_hash(key, Lm) ^ node_hash(key, Lm) >> 24) & (BAL_SLOTS - 1);
+      if (key == node_empty(key)) continue;
+      const uint64_t hash = node_hash(key, Lm);
+      uint32_t h = (uint32_t)(hash ^ hash >> 24) & (slots - 1);
       bool mine = false;
-      for (int probe = 0; probe < BAL_SLOTS; probe++) {
+      for (unsigned probe = 0; probe < slots; probe++) {
         const uint32_t cur = atomicCAS(&S.slot[h], BAL_FREE, me);
         mine = cur == BAL_FREE;
         if (mine || node_wide(S.cand[cur]) == key) break;
-        h = (h + 1) & (BAL_SLOTS - 1);
+        h = (h + 1) & (slots - 1);
       }
-      if (mine && node_insert<K>(tab, mask, key, Lm, flags)) S.won[atomicAdd(&S.n_won, 1u)] = (uint16_t)me;
+      if (mine) S.list[atomicAdd(&S.n_cand, 1u)] = (uint16_t)me;
+    }
+    __syncthreads();
+    const unsigned nc = S.n_cand;
+    for (unsigned q = t; q < nc; q += BAL_TILE) {
+      const uint16_t me = S.list[q];
+      if (node_insert<K>(tab, mask, node_wide(S.cand[me]), Lm, flags)) S.won[atomicAdd(&S.n_won, 1u)] = me;
     }
     __syncthreads();
     const unsigned nw = S.n_won;
