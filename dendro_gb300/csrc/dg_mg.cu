@@ -346,12 +346,8 @@ __global__ void k_to_double(const float *__restrict__ a, size_t n, double *__res
   if (i < n) b[i] = (double)a[i] * scale;
 }
 
-// block partial sums of a.b (and of a.a when b is null)
-__global__ void k_dot_partial(const double *__restrict__ a, const double *__restrict__ b, size_t n,
-                              double *__restrict__ part) {
-  double acc = 0.0;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    acc += a[i] * (b ? b[i] : a[i]);
+// sum over a block of acc, to part[blockIdx.x]
+__device__ __forceinline__ void block_sum(double acc, double *__restrict__ part) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   __shared__ double ws[32];
@@ -363,6 +359,17 @@ __global__ void k_dot_partial(const double *__restrict__ a, const double *__rest
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (threadIdx.x == 0) part[blockIdx.x] = v;
   }
+}
+
+// block partial sums of a.b (and of a.a when b is null); B: FP32 entries are
+// taken times scale
+template <typename B>
+__global__ void k_dot_partial(const double *__restrict__ a, const B *__restrict__ b, size_t n, double scale,
+                              double *__restrict__ part) {
+  double acc = 0.0;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    acc += a[i] * (!b ? a[i] : sizeof(B) == 4 ? (double)b[i] * scale : (double)b[i]);
+  block_sum(acc, part);
 }
 __global__ void k_sum(const double *__restrict__ part, int np, double *__restrict__ out) {
   double acc = 0.0;
@@ -380,20 +387,33 @@ __global__ void k_sum(const double *__restrict__ part, int np, double *__restric
   }
 }
 
+// x += alpha p, r -= alpha q, block partial sums of r.r, and r32 = r * scale
+// in FP32 where it is given (the next V-cycle's right-hand side): one pass
+// over the vectors for the three
 __global__ void k_cg_xr(double *__restrict__ x, double *__restrict__ r, const double *__restrict__ p,
                         const double *__restrict__ q, const double *__restrict__ alpha_num,
-                        const double *__restrict__ alpha_den, size_t n) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+                        const double *__restrict__ alpha_den, size_t n, float *__restrict__ r32, double scale,
+                        double *__restrict__ part) {
   const double alpha = *alpha_num / *alpha_den;
-  x[i] += alpha * p[i];
-  r[i] -= alpha * q[i];
+  double acc = 0.0;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    x[i] += alpha * p[i];
+    const double v = r[i] - alpha * q[i];
+    r[i] = v;
+    if (r32) r32[i] = (float)(v * scale);
+    acc += v * v;
+  }
+  block_sum(acc, part);
 }
-__global__ void k_cg_p(double *__restrict__ p, const double *__restrict__ z, const double *__restrict__ rz_new,
-                       const double *__restrict__ rz_old, size_t n) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  p[i] = z[i] + (*rz_new / *rz_old) * p[i];
+// p = z + beta p, z FP64 or FP32 times scale; rz_old null: p = z
+template <typename Z>
+__global__ void k_cg_p(double *__restrict__ p, const Z *__restrict__ z, const double *__restrict__ rz_new,
+                       const double *__restrict__ rz_old, size_t n, double scale) {
+  const double beta = rz_old ? *rz_new / *rz_old : 0.0;  // once per thread: a division is some 20 FP64 operations
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const double zi = sizeof(Z) == 4 ? (double)z[i] * scale : (double)z[i];
+    p[i] = rz_old ? zi + beta * p[i] : zi;
+  }
 }
 
 }  // namespace
@@ -662,39 +682,53 @@ void mg_solve(Context &ctx, MG &mg, const double *b, double *x, int precision, d
   const MGLevel &L0 = mg.lv[0];
   const size_t n = L0.mesh.n_node;
   const unsigned g = grid_for(n, 256);
-  DBuf<double> r(n, s), z(n, s), p(n, s), q(n, s);
-  const int nparts = (int)std::min<size_t>(grid_for(n, 256), (size_t)(ctx.num_sms * 4));
+  const bool f32 = precision == 32;
+  DBuf<double> r(n, s), z(f32 ? 0 : n, s), p(n, s), q(n, s);
+  const int nparts = (int)std::min<size_t>(grid_for(n, 256), (size_t)(ctx.num_sms * 8));
   DBuf<double> part(nparts, s), sc(8, s);  // sc: rz, pq, rr, rz_new, bb
   VWork<float> w32;
   VWork<double> w64;
   DBuf<float> r32, z32;
-  if (precision == 32) {
+  if (f32) {
     w32 = make_work<float>(ctx, mg);
     r32.alloc(n, s);
     z32.alloc(n, s);
   } else {
     w64 = make_work<double>(ctx, mg);
   }
-  auto dot = [&](const double *a, const double *bb, double *out) {
-    ProfScope _prof(ctx, "cg_dot", (double)n * (bb ? 16 : 8));
-    k_dot_partial<<<nparts, 256, 0, s>>>(a, bb, n, part.get());
+  auto sum_to = [&](double *out) {
     k_sum<<<1, 256, 0, s>>>(part.get(), nparts, out);
     DG_LAUNCH_CHECK();
+  };
+  auto dot = [&](const double *a, const double *bb, double *out) {
+    ProfScope _prof(ctx, "cg_dot", (double)n * (bb ? 16 : 8));
+    k_dot_partial<double><<<nparts, 256, 0, s>>>(a, bb, n, 1.0, part.get());
+    sum_to(out);
   };
   // the CG vectors scale with b: the FP32 V-cycle and the FP32 operator
   // work on them scaled by 2^ds_exp (exact), of order one, away from FP32's
   // underflow (a fine mesh's load vector is of order h^3, and the residual
   // falls by the tolerance on top)
   int ds_exp = 0;
-  auto precond = [&](const double *rin, double *zout) {
-    if (precision == 32) {
-      k_to_float<<<g, 256, 0, s>>>(rin, n, r32.get(), std::ldexp(1.0, ds_exp));
-      vcycle_level<float>(ctx, mg, w32, 0, r32.get(), z32.get());
-      k_to_double<<<g, 256, 0, s>>>(z32.get(), n, zout, std::ldexp(1.0, -ds_exp));
-      DG_LAUNCH_CHECK();
-    } else {
-      vcycle_level<double>(ctx, mg, w64, 0, rin, zout);
-    }
+  auto to_r32 = [&]() {
+    k_to_float<<<g, 256, 0, s>>>(r.get(), n, r32.get(), std::ldexp(1.0, ds_exp));
+    DG_LAUNCH_CHECK();
+  };
+  // z = V-cycle(r) (FP32: z32 from r32, both scaled) and r.z
+  auto precond = [&](double *rz) {
+    if (f32) vcycle_level<float>(ctx, mg, w32, 0, r32.get(), z32.get());
+    else vcycle_level<double>(ctx, mg, w64, 0, r.get(), z.get());
+    ProfScope _prof(ctx, "cg_dot", (double)n * (f32 ? 12 : 16));
+    if (f32)
+      k_dot_partial<float><<<nparts, 256, 0, s>>>(r.get(), z32.get(), n, std::ldexp(1.0, -ds_exp), part.get());
+    else k_dot_partial<double><<<nparts, 256, 0, s>>>(r.get(), z.get(), n, 1.0, part.get());
+    sum_to(rz);
+  };
+  auto direction = [&](const double *rz_new, const double *rz_old) {
+    ProfScope _prof(ctx, "cg_p", (double)n * (f32 ? 20 : 24));
+    if (f32) k_cg_p<float><<<nparts, 256, 0, s>>>(p.get(), z32.get(), rz_new, rz_old, n, std::ldexp(1.0, -ds_exp));
+    else k_cg_p<double><<<nparts, 256, 0, s>>>(p.get(), z.get(), rz_new, rz_old, n, 1.0);
+    DG_LAUNCH_CHECK();
   };
   double *d_rz = sc.get(), *d_pq = sc.get() + 1, *d_rr = sc.get() + 2, *d_rzn = sc.get() + 3, *d_bb = sc.get() + 4;
   DG_CUDA(cudaMemsetAsync(x, 0, n * sizeof(double), s));
@@ -727,25 +761,25 @@ void mg_solve(Context &ctx, MG &mg, const double *b, double *x, int precision, d
       dirichlet_matvec<double>(ctx, L0, p.get(), q.get());
     }
     dot(p.get(), q.get(), d_pq);
-    k_cg_xr<<<g, 256, 0, s>>>(x, r.get(), p.get(), q.get(), d_rz, d_pq, n);
-    DG_LAUNCH_CHECK();
-    dot(r.get(), nullptr, d_rr);
+    ProfScope _prof(ctx, "cg_xr", (double)n * (f32 ? 52 : 48));
+    k_cg_xr<<<nparts, 256, 0, s>>>(x, r.get(), p.get(), q.get(), d_rz, d_pq, n, f32 ? r32.get() : nullptr,
+                                   std::ldexp(1.0, ds_exp), part.get());
+    sum_to(d_rr);
   };
   auto step_b = [&]() {
-    precond(r.get(), z.get());
-    dot(r.get(), z.get(), d_rzn);
-    k_cg_p<<<g, 256, 0, s>>>(p.get(), z.get(), d_rzn, d_rz, n);
-    DG_LAUNCH_CHECK();
+    precond(d_rzn);
+    direction(d_rzn, d_rz);
     DG_CUDA(cudaMemcpyAsync(d_rz, d_rzn, sizeof(double), cudaMemcpyDeviceToDevice, s));
   };
-  precond(r.get(), z.get());
-  DG_CUDA(cudaMemcpyAsync(p.get(), z.get(), n * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  dot(r.get(), z.get(), d_rz);
+  if (f32) to_r32();
+  precond(d_rz);
+  direction(d_rz, nullptr);
   // r = b - A x in FP64 (the reliable update of the FP32-operator form)
   auto true_residual = [&]() {
     dirichlet_matvec<double>(ctx, L0, x, q.get());
     k_residual<double><<<g, 256, 0, s>>>(b, q.get(), r.get(), n);
     DG_LAUNCH_CHECK();
+    if (f32) to_r32();
     dot(r.get(), nullptr, d_rr);
     return std::sqrt(read_scalar(ctx, d_rr)) / bnorm;
   };
