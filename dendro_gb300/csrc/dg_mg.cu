@@ -26,8 +26,6 @@
 
 namespace dg {
 
-void coarsen_octree(Context &ctx, const Octree &in, Octree &out);
-
 namespace {
 
 __global__ void k_node_bdy(const uint32_t *__restrict__ xyz, size_t V, unsigned D, uint8_t *__restrict__ bdy) {
@@ -583,6 +581,14 @@ static void copy_octree(Context &ctx, const Octree &in, Octree &out) {
   out.n = in.n;
   DG_CUDA(cudaMallocAsync((void **)&out.keys, in.n * sizeof(Key128), ctx.stream));
   DG_CUDA(cudaMemcpyAsync(out.keys, in.keys, in.n * sizeof(Key128), cudaMemcpyDeviceToDevice, ctx.stream));
+  if (in.nodes) {
+    const size_t bytes = in.n_node * (in.node_wide ? 16 : 8);
+    DG_CUDA(cudaMallocAsync(&out.nodes, bytes, ctx.stream));
+    DG_CUDA(cudaMemcpyAsync(out.nodes, in.nodes, bytes, cudaMemcpyDeviceToDevice, ctx.stream));
+    out.n_node = in.n_node;
+    out.top = in.top;
+    out.node_wide = in.node_wide;
+  }
 }
 
 void mg_setup(Context &ctx, const Octree &fine, size_t max_coarse_elem, MG &mg) {
@@ -597,7 +603,7 @@ void mg_setup(Context &ctx, const Octree &fine, size_t max_coarse_elem, MG &mg) 
     mesh_build(ctx, mg.lv[0].oct, mg.lv[0].mesh);
     while (mg.lv.back().mesh.n_elem > max_coarse_elem) {
       Octree c, b;
-      coarsen_octree(ctx, mg.lv.back().oct, c);
+      coarsen_octree(ctx, mg.lv.back().oct, c, false);
       if (c.n == mg.lv.back().oct.n) {
         octree_free(ctx, c);
         break;  // nothing left to coarsen

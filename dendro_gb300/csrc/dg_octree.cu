@@ -27,7 +27,7 @@
 //             around every q in I_l (8 octants per q, clipped to the domain).
 // The sets grow in one hash table, level by level from the deepest, without
 // a read-back between levels; one radix sort puts all nodes in preorder.
-#include "dg_octree.cuh"
+#include "dg_nodes.cuh"
 #include "dg_walk.cuh"
 
 #include <algorithm>
@@ -37,26 +37,6 @@
 #include <vector>
 
 namespace dg {
-
-__device__ __forceinline__ void set_flag(uint32_t *flags, uint32_t f) { atomicOr(flags, f); }
-
-// key with only the Morton bits of one cloud (bits [0, 3D))
-__host__ __device__ __forceinline__ Key128 morton_part(Key128 k, unsigned D) {
-  Key128 a = tag_anchor(k);
-  if (3 * D < 64) {
-    a.lo &= (3 * D) ? ((1ull << (3 * D)) - 1) : 0ull;
-    a.hi = 0;
-  } else {
-    a.hi &= (1ull << (3 * D - 64)) - 1;
-  }
-  return a;
-}
-__host__ __device__ __forceinline__ uint64_t seg_of(Key128 k, unsigned D) {
-  return to_u128(tag_anchor(k)) >> (3 * D) & 0xffffffffffull;
-}
-__host__ __device__ __forceinline__ Key128 seg_key(uint64_t seg, unsigned D) {
-  return from_u128((u128)seg << (3 * D));
-}
 
 // ------------------------------------------------------------------------
 // quantize + Morton key (construct.cpp:930-942)
@@ -166,14 +146,6 @@ __global__ void k_sort_runs(Key128 *__restrict__ k, size_t n, unsigned begin, ui
   }
 }
 
-// NCA level of two points of the same cloud; -1 across clouds
-__device__ __forceinline__ int nca_level(Key128 a, Key128 b, unsigned D) {
-  Key128 x = key_xor(tag_anchor(a), tag_anchor(b));
-  if (!x.lo && !x.hi) return (int)D;
-  int lz = key_clz(x, 3 * (int)D);
-  return lz < 0 ? -1 : lz / 3;
-}
-
 __device__ __forceinline__ unsigned leaf_level(const Key128 *__restrict__ p, size_t n, size_t i, unsigned m,
                                                unsigned D) {
   size_t lo = (i >= m) ? i - m : 0;
@@ -221,50 +193,6 @@ __global__ void __launch_bounds__(P2O_BLOCK) k_p2o_count(const Key128 *__restric
   if (threadIdx.x == 0) sums[blockIdx.x] = sum;
 }
 
-// ------------------------------------------------------------------------
-// nodes: an internal octant of level <= Lm as one sortable key, its path (3
-// bits per level to level Lm, the cloud index above) over 5 bits of level:
-// preorder is key order.  64-bit keys where they suffice, else 128-bit.
-// ------------------------------------------------------------------------
-__device__ __forceinline__ uint64_t node_wide(uint64_t k) { return k; }
-__device__ __forceinline__ u128 node_wide(Key128 k) { return to_u128(k); }
-// no node: the level bits of a node never are 31
-__device__ __forceinline__ uint64_t node_empty(uint64_t) { return ~0ull; }
-__device__ __forceinline__ u128 node_empty(u128) { return ~(u128)0; }
-template <typename K>
-struct NodeWide;
-template <>
-struct NodeWide<uint64_t> {
-  typedef uint64_t W;
-  __host__ __device__ __forceinline__ static uint64_t narrow(W w) { return w; }
-  __device__ __forceinline__ static W of(Key128 k) { return k.lo; }
-  __device__ __forceinline__ static Key128 key(W w) { return Key128{w, 0}; }
-};
-template <>
-struct NodeWide<Key128> {
-  typedef u128 W;
-  __host__ __device__ __forceinline__ static Key128 narrow(W w) { return from_u128(w); }
-  __device__ __forceinline__ static W of(Key128 k) { return to_u128(k); }
-  __device__ __forceinline__ static Key128 key(W w) { return from_u128(w); }
-};
-
-// the ancestor of level l (<= Lm) of a tagged anchor at depth D
-template <typename K>
-__device__ __forceinline__ K node_of(Key128 anchor, unsigned l, unsigned Lm, unsigned D) {
-  typedef NodeWide<K> N;
-  const typename N::W idx = N::of(key_shr(anchor, 3 * (D - l)));
-  return N::narrow(idx << (3 * (Lm - l)) << 5 | (typename N::W)l);
-}
-
-// sum of the octal digits of v
-__device__ __forceinline__ unsigned digit_sum(uint64_t v) {
-  const uint64_t m = 0x1249249249249249ull;  // bits 0, 3, ..., 60
-  return __popcll(v & m) + 2 * __popcll(v & m << 1) + 4 * __popcll(v & m << 2) + (unsigned)(v >> 63);
-}
-__device__ __forceinline__ unsigned digit_sum(u128 v) {
-  return digit_sum((uint64_t)((uint64_t)v & 0x7fffffffffffffffull)) + digit_sum((uint64_t)(v >> 63));
-}
-
 template <typename K>
 __global__ void __launch_bounds__(P2O_BLOCK) k_p2o_nodes(const Key128 *__restrict__ p, size_t n, unsigned D,
                                                          unsigned Lm, const uint16_t *__restrict__ path,
@@ -287,11 +215,6 @@ __global__ void __launch_bounds__(P2O_BLOCK) k_p2o_nodes(const Key128 *__restric
     }
     at += all;
   }
-}
-
-__device__ __forceinline__ uint64_t shfl_wide(uint64_t v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
-__device__ __forceinline__ u128 shfl_wide(u128 v, int lane) {
-  return (u128)__shfl_sync(0xffffffffu, (uint64_t)(v >> 64), lane) << 64 | __shfl_sync(0xffffffffu, (uint64_t)v, lane);
 }
 
 // The leaves of the octrees whose nodes are given (sorted), 8 threads per
@@ -377,8 +300,14 @@ __global__ void k_emit_clouds(const K *__restrict__ nodes, size_t nn, unsigned L
   if (seg_off) seg_off[s] = 7 * lo + s;
 }
 
-// whether node keys of octrees with leaves to level top (> 0) fit 64 bits
-inline bool nodes_fit_64(unsigned top, unsigned seg_bits) { return 3 * (top - 1) + seg_bits + 5 <= 64; }
+// out's sorted nodes, taken over from a buffer
+template <typename K>
+static void keep_nodes(Octree &out, DBuf<K> &nodes, size_t nn, unsigned top) {
+  out.nodes = nodes.release_ptr();
+  out.n_node = nn;
+  out.top = top;
+  out.node_wide = sizeof(K) == 16;
+}
 
 // all leaves of nn sorted nodes of nseg clouds (7 nn + nseg octants)
 template <typename K>
@@ -701,6 +630,7 @@ void points_to_octree(Context &ctx, const double *d_xyz, size_t n, const double 
       DG_LAUNCH_CHECK();
     }
     emit_octree<K>(ctx, nodes.get(), nn, top - 1, D, nseg, res, seg_off);
+    if (!dupflag) keep_nodes(out, nodes, nn, top);
   };
   if (nodes_fit_64(top, SB)) construct(uint64_t());
   else construct(Key128());
@@ -842,76 +772,36 @@ __global__ void k_bal_scan(const Key128 *__restrict__ k, size_t n, unsigned D, u
   if (threadIdx.x < 32 && h[threadIdx.x]) atomicAdd(&hist[threadIdx.x], (unsigned long long)h[threadIdx.x]);
 }
 
-// ---- the set of all nodes: open addressing.  The eight children of one
-// octant share a group of eight slots (one cache line of 64-bit keys), as the
-// candidates around one octant do; probing steps by groups, a bounded number
-// of times (BAL_PROBES; then DGF_CAPACITY, and the host retries with a larger
-// table).
-constexpr int BAL_PROBES = 512;
-
-__device__ __forceinline__ uint64_t mix64(uint64_t x) {
-  x ^= x >> 32;
-  x *= 0xd6e8feb86659fd93ull;
-  x ^= x >> 32;
-  return x;
-}
-__device__ __forceinline__ uint64_t node_hash(uint64_t k, unsigned Lm) {
-  const unsigned l = (unsigned)k & 31u, sh = 5 + 3 * (Lm - l);
-  return mix64((k >> sh >> 3) * 32 + l) << 3 | (k >> sh & 7u);
-}
-__device__ __forceinline__ uint64_t node_hash(u128 k, unsigned Lm) {
-  const unsigned l = (unsigned)k & 31u, sh = 5 + 3 * (Lm - l);
-  const u128 par = k >> sh >> 3;
-  return mix64(((uint64_t)par ^ (uint64_t)(par >> 64) * 0x9e3779b97f4a7c15ull) * 32 + l) << 3 | ((uint64_t)(k >> sh) & 7u);
-}
-// compare-and-swap of one slot, returning what it held
-__device__ __forceinline__ uint64_t slot_cas(uint64_t *slot, uint64_t key) {
-  const uint64_t cur = __ldcg(slot);  // a full slot never changes
-  if (cur != ~0ull) return cur;
-  return atomicCAS(reinterpret_cast<unsigned long long *>(slot), ~0ull, (unsigned long long)key);
-}
-__device__ __forceinline__ u128 slot_cas(Key128 *slot, u128 key) {
-  uint64_t lo, hi;
-  asm volatile("{\n\t.reg .b128 d, b, c;\n\t"
-               "mov.b128 b, {%3, %4};\n\tmov.b128 c, {%5, %6};\n\t"
-               "atom.relaxed.gpu.cas.b128 d, [%2], b, c;\n\tmov.b128 {%0, %1}, d;\n\t}"
-               : "=l"(lo), "=l"(hi)
-               : "l"(slot), "l"(~0ull), "l"(~0ull), "l"((uint64_t)key), "l"((uint64_t)(key >> 64))
-               : "memory");
-  return (u128)hi << 64 | lo;
-}
-
-// true when this call put the key into the table
-template <typename K>
-__device__ __forceinline__ bool node_insert(K *__restrict__ tab, uint64_t mask, typename NodeWide<K>::W key,
-                                            unsigned Lm, uint32_t *flags) {
-  uint64_t h = node_hash(key, Lm) & mask;
-  for (int probe = 0; probe < BAL_PROBES; probe++) {
-    const auto cur = slot_cas(tab + h, key);
-    if (cur == node_empty(key)) return true;
-    if (cur == key) return false;
-    h = (h + 8) & mask;
-  }
-  set_flag(flags, DGF_CAPACITY);
-  return false;
-}
-
-// where the nodes go: those from the leaves at off[l] of `leafs`, level by
-// level, the others in the order of their making in `grown`
-struct BalLists {
-  unsigned long long off[32];
-};
-// counters on the device: nodes per level from the leaves, and grown
+// Where the nodes go: those the balance starts from at off[l] of `start`, level
+// by level; the grown ones in the order of their making in `grown`.  Counters
+// on the device: room per level, nodes per level from the start, and grown.
 struct BalCounts {
-  unsigned long long leaf[32], grown[32];
+  unsigned long long room[32], start[32], grown[32];
 };
+__device__ __forceinline__ unsigned long long bal_off(const BalCounts *__restrict__ cnt, unsigned l) {
+  unsigned long long at = 0;
+  for (unsigned q = 0; q < l; q++) at += cnt->room[q];
+  return at;
+}
 
-// the parents of the input leaves
+// nodes per level of an octree that has them
 template <typename K>
-__global__ void __launch_bounds__(256) k_bal_leaves(const Key128 *__restrict__ k, size_t n, unsigned D, unsigned Lm,
-                                                    K *__restrict__ tab, uint64_t mask, BalLists lists,
-                                                    K *__restrict__ leafs, BalCounts *__restrict__ cnt,
-                                                    uint32_t *flags) {
+__global__ void k_bal_node_levels(const K *__restrict__ nodes, size_t nn, unsigned long long *__restrict__ hist) {
+  __shared__ unsigned h[32];
+  if (threadIdx.x < 32) h[threadIdx.x] = 0;
+  __syncthreads();
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += (size_t)gridDim.x * blockDim.x)
+    atomicAdd(&h[(unsigned)node_wide(nodes[i]) & 31u], 1u);
+  __syncthreads();
+  if (threadIdx.x < 32 && h[threadIdx.x]) atomicAdd(&hist[threadIdx.x], (unsigned long long)h[threadIdx.x]);
+}
+
+// the nodes that the balance starts from into the table and their level's
+// list: the input's own (sorted) nodes, or with LEAVES the parents of its leaves
+template <typename K, bool LEAVES>
+__global__ void __launch_bounds__(256) k_bal_start(const void *__restrict__ in, size_t n, unsigned D, unsigned Lm,
+                                                   K *__restrict__ tab, uint64_t mask, K *__restrict__ list,
+                                                   BalCounts *__restrict__ cnt, uint32_t *flags) {
   __shared__ unsigned num[32];
   __shared__ unsigned long long base[32];
   if (threadIdx.x < 32) num[threadIdx.x] = 0;
@@ -921,19 +811,28 @@ __global__ void __launch_bounds__(256) k_bal_leaves(const Key128 *__restrict__ k
   K key{};
   unsigned l = 0, rank = 0;
   if (i < n) {
-    const Key128 ki = k[i];
-    if (brings_parent(k, i, ki, D)) {
-      l = tag_level(ki) - 1;
-      key = node_of<K>(tag_anchor(ki), l, Lm, D);
-      won = node_insert<K>(tab, mask, node_wide(key), Lm, flags);
-      if (won) rank = atomicAdd(&num[l], 1u);
+    if constexpr (LEAVES) {
+      const Key128 *k = static_cast<const Key128 *>(in);
+      const Key128 ki = k[i];
+      won = brings_parent(k, i, ki, D);
+      if (won) {
+        l = tag_level(ki) - 1;
+        key = node_of<K>(tag_anchor(ki), l, Lm, D);
+      }
+    } else {
+      key = static_cast<const K *>(in)[i];
+      l = (unsigned)node_wide(key) & 31u;
+      won = true;
     }
+    if (won) won = node_insert<K>(tab, mask, node_wide(key), Lm, flags);
+    if (won) rank = atomicAdd(&num[l], 1u);
   }
   __syncthreads();
   if (threadIdx.x < 32 && num[threadIdx.x])
-    base[threadIdx.x] = lists.off[threadIdx.x] + atomicAdd(&cnt->leaf[threadIdx.x], (unsigned long long)num[threadIdx.x]);
+    base[threadIdx.x] =
+        bal_off(cnt, threadIdx.x) + atomicAdd(&cnt->start[threadIdx.x], (unsigned long long)num[threadIdx.x]);
   __syncthreads();
-  if (won) leafs[base[l] + rank] = key;
+  if (won) list[base[l] + rank] = key;
 }
 
 // One level of the recursion: for every node q of level l the 8 parents (level
@@ -957,7 +856,7 @@ struct BalSmem {
 
 template <typename K>
 __global__ void __launch_bounds__(BAL_TILE) k_bal_level(unsigned l, unsigned Lm, bool inc_corner, K *__restrict__ tab,
-                                                        uint64_t mask, BalLists lists, const K *__restrict__ leafs,
+                                                        uint64_t mask, const K *__restrict__ start,
                                                         K *grown, size_t grown_cap, BalCounts *__restrict__ cnt,
                                                         uint32_t *flags) {
   typedef NodeWide<K> N;
@@ -965,7 +864,7 @@ __global__ void __launch_bounds__(BAL_TILE) k_bal_level(unsigned l, unsigned Lm,
   extern __shared__ __align__(16) unsigned char bal_raw[];
   BalSmem<K> &S = *reinterpret_cast<BalSmem<K> *>(bal_raw);
   const int t = threadIdx.x;
-  const size_t n0 = cnt->leaf[l], n1 = cnt->grown[l];
+  const size_t n0 = cnt->start[l], n1 = cnt->grown[l], off = bal_off(cnt, l);
   size_t first = 0;  // grown nodes of the levels below
   for (unsigned q = l + 1; q <= Lm; q++) first += cnt->grown[q];
   if (first + n1 > grown_cap) return;  // the list overflowed (flagged): the host starts again
@@ -980,7 +879,7 @@ __global__ void __launch_bounds__(BAL_TILE) k_bal_level(unsigned l, unsigned Lm,
     if (t == 0) S.n_cand = S.n_won = 0;
     if (t < here) {
       const size_t i = base + t;
-      const W k = node_wide(i < n0 ? leafs[lists.off[l] + i] : grown[first + (i - n0)]);
+      const W k = node_wide(i < n0 ? start[off + i] : grown[first + (i - n0)]);
       const W path = k >> 5;
       const W cloud = path >> (3 * Lm);
       const W idx = (path & (((W)1 << (3 * Lm)) - 1)) >> (3 * (Lm - l));
@@ -1035,41 +934,35 @@ __global__ void __launch_bounds__(BAL_TILE) k_bal_level(unsigned l, unsigned Lm,
   }
 }
 
-// all nodes side by side: the leaves' lists without the room their repeats
+// all nodes side by side: the start's lists without the room their repeats
 // left, then the grown ones
 struct BalGather {
   unsigned long long off[32], num[32], to[32];
 };
 template <typename K>
-__global__ void k_bal_gather(const K *__restrict__ leafs, BalGather g, size_t n_room, K *__restrict__ out) {
+__global__ void k_bal_gather(const K *__restrict__ start, BalGather g, size_t n_room, K *__restrict__ out) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_room) return;
   int l = 0;
   while (l < 31 && i >= g.off[l + 1]) l++;
   const size_t r = i - g.off[l];
-  if (r < g.num[l]) out[g.to[l] + r] = leafs[i];
+  if (r < g.num[l]) out[g.to[l] + r] = start[i];
 }
 
-// the sorted nodes of the balanced refinement
+// the sorted nodes of the balanced refinement; d_hist: per level the nodes (an
+// input that has them) or the leaves' parents with repeats, `room` their sum
 template <typename K>
-static size_t balance_nodes(Context &ctx, const Octree &in, unsigned top, const unsigned long long (&hist)[32],
+static size_t balance_nodes(Context &ctx, const Octree &in, unsigned top, const unsigned long long *d_hist, size_t room,
                             bool inc_corner, DBuf<K> &a, DBuf<K> &b, K **sorted) {
   cudaStream_t s = ctx.stream;
   const unsigned D = in.max_depth, Lm = top - 1;
-  BalLists lists;
-  size_t room = 0;  // parents from the leaves, repeats of far-away leaves included
-  for (int l = 0; l < 32; l++) {
-    lists.off[l] = room;
-    room += hist[l];
-  }
   ensure_smem_attr(ctx, k_bal_level<K>, (int)sizeof(BalSmem<K>));
   int per_sm = 1;
   DG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bal_level<K>, BAL_TILE, sizeof(BalSmem<K>)));
-  // counters and flags come back together
-  BalCounts *cnt = reinterpret_cast<BalCounts *>(ctx.d_scratch);
-  BalCounts *h = reinterpret_cast<BalCounts *>(ctx.h_scratch);
-  DBuf<K> leafs(room, s), grown;
-  size_t n0 = 0, n1 = 0;
+  DBuf<BalCounts> counts(1, s);
+  BalCounts *cnt = counts.get();
+  BalCounts h;
+  DBuf<K> start(room, s), grown;
   // balanced octrees of the workloads' clouds have 1.3 to 1.9 times the nodes
   // of their input: room for 3 times, and four times that on each retry
   for (size_t grow = 2;; grow *= 4) {
@@ -1080,43 +973,51 @@ static size_t balance_nodes(Context &ctx, const Octree &in, unsigned top, const 
     DBuf<K> tab(slots, s);
     DG_CUDA(cudaMemsetAsync(tab.get(), 0xff, slots * sizeof(K), s));
     DG_CUDA(cudaMemsetAsync(cnt, 0, sizeof(BalCounts), s));
+    DG_CUDA(cudaMemcpyAsync(cnt->room, d_hist, sizeof(cnt->room), cudaMemcpyDeviceToDevice, s));
     {
-      ProfScope _prof(ctx, "bal_leaves", (double)in.n * 16 + (double)room * 2 * sizeof(K));
-      k_bal_leaves<K><<<grid_for(in.n, 256), 256, 0, s>>>(in.keys, in.n, D, Lm, tab.get(), slots - 1, lists,
-                                                          leafs.get(), cnt, ctx.d_flags);
+      ProfScope _prof(ctx, "bal_start", in.nodes ? (double)room * 3 * sizeof(K)
+                                                 : (double)in.n * 16 + (double)room * 2 * sizeof(K));
+      if (in.nodes)
+        k_bal_start<K, false><<<grid_for(in.n_node, 256), 256, 0, s>>>(in.nodes, in.n_node, D, Lm, tab.get(),
+                                                                       slots - 1, start.get(), cnt, ctx.d_flags);
+      else
+        k_bal_start<K, true><<<grid_for(in.n, 256), 256, 0, s>>>(in.keys, in.n, D, Lm, tab.get(), slots - 1,
+                                                                 start.get(), cnt, ctx.d_flags);
       DG_LAUNCH_CHECK();
     }
     const unsigned grid =
         grid_for(room + cap, BAL_TILE, (unsigned)(std::max(per_sm, 1) * ctx.num_sms));
     for (unsigned l = Lm; l >= 1; l--) {
       ProfScope _prof(ctx, "bal_level", 0.0);
-      k_bal_level<K><<<grid, BAL_TILE, sizeof(BalSmem<K>), s>>>(l, Lm, inc_corner, tab.get(), slots - 1, lists,
-                                                                leafs.get(), grown.get(), cap, cnt, ctx.d_flags);
+      k_bal_level<K><<<grid, BAL_TILE, sizeof(BalSmem<K>), s>>>(l, Lm, inc_corner, tab.get(), slots - 1, start.get(),
+                                                                grown.get(), cap, cnt, ctx.d_flags);
       DG_LAUNCH_CHECK();
     }
-    DG_CUDA(cudaMemcpyAsync(h, cnt, sizeof(BalCounts), cudaMemcpyDeviceToHost, s));
-    DG_CUDA(cudaMemcpyAsync(h + 1, ctx.d_flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    static_assert(sizeof(BalCounts) <= 96 * sizeof(unsigned long long), "the counts fit the pinned mirror");
+    DG_CUDA(cudaMemcpyAsync(ctx.h_scratch, cnt, sizeof(BalCounts), cudaMemcpyDeviceToHost, s));
     DG_CUDA(cudaStreamSynchronize(s));
-    uint32_t f;
-    std::memcpy(&f, h + 1, sizeof(f));
+    std::memcpy(&h, ctx.h_scratch, sizeof(h));
+    const uint32_t f = read_scalar(ctx, ctx.d_flags);
     if (!(f & DGF_CAPACITY)) break;
     DG_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), s));
     if (cap > ((size_t)1 << 40) / sizeof(K)) fail(DG_ERR_OUT_OF_MEMORY, "balanceOctree: too many octants");
   }
   BalGather g;
+  size_t off = 0, n0 = 0, n1 = 0;
   for (int l = 0; l < 32; l++) {
-    g.off[l] = lists.off[l];
-    g.num[l] = h->leaf[l];
+    g.off[l] = off;
+    g.num[l] = h.start[l];
     g.to[l] = n0;
-    n0 += h->leaf[l];
-    n1 += h->grown[l];
+    off += h.room[l];
+    n0 += h.start[l];
+    n1 += h.grown[l];
   }
   const size_t nn = n0 + n1;
   a.alloc(nn, s);
   b.alloc(nn, s);
   {
     ProfScope _prof(ctx, "bal_gather", (double)nn * 2 * sizeof(K));
-    k_bal_gather<K><<<grid_for(room, 256), 256, 0, s>>>(leafs.get(), g, room, a.get());
+    k_bal_gather<K><<<grid_for(room, 256), 256, 0, s>>>(start.get(), g, room, a.get());
     DG_LAUNCH_CHECK();
   }
   if (n1) DG_CUDA(cudaMemcpyAsync(a.get() + n0, grown.get(), n1 * sizeof(K), cudaMemcpyDeviceToDevice, s));
@@ -1133,22 +1034,34 @@ void balance_octree(Context &ctx, const Octree &in, Octree &out, bool inc_corner
   out.seg_bits = in.seg_bits;
   const size_t n = in.n;
   if (n == 0) fail(DG_ERR_INVALID_ARG, "balanceOctree: empty input");
-  // parents per level + domain validation
   unsigned long long *d_hist = ctx.d_scratch + 16;
   DG_CUDA(cudaMemsetAsync(d_hist, 0, 32 * sizeof(unsigned long long), s));
   DG_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), s));
-  {
-    ProfScope _prof(ctx, "bal_scan", (double)n * 16);
-    k_bal_scan<<<grid_for(n, 256, ctx.num_sms * 8), 256, 0, s>>>(in.keys, n, D, nseg, d_hist, ctx.d_flags);
+  unsigned top = in.top;  // deepest leaf level
+  size_t room = in.n_node;
+  if (in.nodes) {
+    ProfScope _prof(ctx, "bal_node_levels", (double)in.n_node * (in.node_wide ? 16 : 8));
+    const unsigned g = grid_for(in.n_node, 256, ctx.num_sms * 8);
+    if (in.node_wide)
+      k_bal_node_levels<Key128><<<g, 256, 0, s>>>(static_cast<const Key128 *>(in.nodes), in.n_node, d_hist);
+    else
+      k_bal_node_levels<uint64_t><<<g, 256, 0, s>>>(static_cast<const uint64_t *>(in.nodes), in.n_node, d_hist);
     DG_LAUNCH_CHECK();
+  } else {
+    // parents per level + domain validation
+    {
+      ProfScope _prof(ctx, "bal_scan", (double)n * 16);
+      k_bal_scan<<<grid_for(n, 256, ctx.num_sms * 8), 256, 0, s>>>(in.keys, n, D, nseg, d_hist, ctx.d_flags);
+      DG_LAUNCH_CHECK();
+    }
+    DG_CUDA(cudaMemcpyAsync(ctx.h_scratch + 16, d_hist, 32 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+    check_device_flags(ctx, "balanceOctree (octant outside the domain or misaligned)");
+    top = 0;
+    for (unsigned l = 0; l < 32; l++) {
+      room += ctx.h_scratch[16 + l];
+      if (ctx.h_scratch[16 + l]) top = l + 1;
+    }
   }
-  DG_CUDA(cudaMemcpyAsync(ctx.h_scratch + 16, d_hist, 32 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-  check_device_flags(ctx, "balanceOctree (octant outside the domain or misaligned)");
-  unsigned long long hist[32];
-  std::memcpy(hist, ctx.h_scratch + 16, sizeof(hist));
-  unsigned top = 0;  // deepest leaf level
-  for (unsigned l = 0; l < 32; l++)
-    if (hist[l]) top = l + 1;
   DBuf<Key128> res;
   DBuf<uint64_t> seg_off;
   size_t nn = 0;
@@ -1156,12 +1069,13 @@ void balance_octree(Context &ctx, const Octree &in, Octree &out, bool inc_corner
     typedef decltype(tag) K;
     DBuf<K> a, b;
     K *nodes = nullptr;
-    if (top) nn = balance_nodes<K>(ctx, in, top, hist, inc_corner, a, b, &nodes);
+    if (room) nn = balance_nodes<K>(ctx, in, top, d_hist, room, inc_corner, a, b, &nodes);
     emit_octree<K>(ctx, nodes, nn, top ? top - 1 : 0, D, nseg, res, seg_off);
+    check_device_flags(ctx, "balanceOctree");
+    if (nn) keep_nodes(out, nodes == a.get() ? a : b, nn, top);
   };
-  if (top == 0 || nodes_fit_64(top, in.seg_bits)) run(uint64_t());
+  if (in.nodes ? !in.node_wide : top == 0 || nodes_fit_64(top, in.seg_bits)) run(uint64_t());
   else run(Key128());
-  check_device_flags(ctx, "balanceOctree");
   out.n = 7 * nn + nseg;
   out.keys = res.release_ptr();
   out.seg_off = nseg > 1 ? seg_off.release_ptr() : nullptr;
@@ -1213,13 +1127,70 @@ __global__ void k_coarsen_apply(const Key128 *__restrict__ k, size_t n, unsigned
   val[i] = fam[i] ? key_parent(ki, D) : ki;
 }
 
-void coarsen_octree(Context &ctx, const Octree &in, Octree &out) {
+// the nodes that stay: those with a node among their children, which follows
+// them in preorder
+template <typename K>
+__global__ void k_coarsen_flags(const K *__restrict__ nodes, size_t nn, unsigned Lm, uint32_t *__restrict__ keep) {
+  typedef typename NodeWide<K>::W W;
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nn) return;
+  const W k = node_wide(nodes[i]);
+  const unsigned d = (unsigned)k & 31u;
+  keep[i] = i + 1 < nn && (node_wide(nodes[i + 1]) >> 5) < (k >> 5) + ((W)1 << (3 * (Lm - d))) ? 1u : 0u;
+}
+// ... with paths to one level less (the deepest nodes have no node below)
+template <typename K>
+__global__ void k_coarsen_nodes(const K *__restrict__ nodes, const uint32_t *__restrict__ keep,
+                                const uint32_t *__restrict__ pos, size_t nn, K *__restrict__ out) {
+  typedef NodeWide<K> N;
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nn || !keep[i]) return;
+  const typename N::W k = node_wide(nodes[i]);
+  out[pos[i]] = N::narrow(k >> 8 << 5 | (k & 31u));
+}
+
+template <typename K>
+static void coarsen_nodes(Context &ctx, const Octree &in, Octree &out, bool leaves) {
+  cudaStream_t s = ctx.stream;
+  const K *nodes = static_cast<const K *>(in.nodes);
+  const size_t nn = in.n_node;
+  DBuf<uint32_t> keep(nn, s), pos(nn, s);
+  uint32_t *d_total = reinterpret_cast<uint32_t *>(ctx.d_scratch);
+  {
+    ProfScope _prof(ctx, "coarsen_flags", (double)nn * (sizeof(K) + 4));
+    k_coarsen_flags<K><<<grid_for(nn, 256), 256, 0, s>>>(nodes, nn, in.top - 1, keep.get());
+    DG_LAUNCH_CHECK();
+  }
+  exclusive_scan<uint32_t, uint32_t>(keep.get(), pos.get(), nn, d_total, s);
+  const size_t nc = read_scalar(ctx, d_total);
+  DBuf<K> kept(nc ? nc : 1, s);
+  DBuf<Key128> res;
+  DBuf<uint64_t> seg_off;
+  if (nc) {
+    ProfScope _prof(ctx, "coarsen_nodes", (double)nn * 8 + (double)nc * 2 * sizeof(K));
+    k_coarsen_nodes<K><<<grid_for(nn, 256), 256, 0, s>>>(nodes, keep.get(), pos.get(), nn, kept.get());
+    DG_LAUNCH_CHECK();
+  }
+  if (leaves || !nc)
+    emit_octree<K>(ctx, kept.get(), nc, nc ? in.top - 2 : 0, in.max_depth, 1, res, seg_off);
+  out.n = 7 * nc + 1;
+  out.keys = res.release_ptr();
+  if (nc) keep_nodes(out, kept, nc, in.top - 1);
+}
+
+void coarsen_octree(Context &ctx, const Octree &in, Octree &out, bool leaves) {
   cudaStream_t s = ctx.stream;
   const size_t n = in.n;
+  out = Octree();
   out.max_depth = in.max_depth;
   out.nseg = in.nseg;
   out.seg_bits = in.seg_bits;
   if (in.nseg != 1) fail(DG_ERR_UNSUPPORTED, "coarsenOctree: one cloud per call");
+  if (in.nodes) {
+    if (in.node_wide) coarsen_nodes<Key128>(ctx, in, out, leaves);
+    else coarsen_nodes<uint64_t>(ctx, in, out, leaves);
+    return;
+  }
   DBuf<Key128> res(n ? n : 1, s);
   if (n < 8) {  // coarsen.cpp:66-70
     if (n) DG_CUDA(cudaMemcpyAsync(res.get(), in.keys, n * sizeof(Key128), cudaMemcpyDeviceToDevice, s));
@@ -1297,6 +1268,13 @@ __global__ void k_strip_cloud(const Key128 *__restrict__ in, size_t n, unsigned 
   if (i < n) out[i] = make_tagged(morton_part(in[i], D), tag_level(in[i]));
 }
 
+template <typename K>
+__global__ void k_strip_nodes(const K *__restrict__ in, size_t n, unsigned Lm, K *__restrict__ out) {
+  typedef NodeWide<K> N;
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = N::narrow(node_wide(in[i]) & (((typename N::W)1 << (3 * Lm + 5)) - 1));
+}
+
 void octree_extract(Context &ctx, const Octree &in, size_t seg, Octree &out) {
   if (seg >= in.nseg) fail(DG_ERR_INVALID_ARG, "octree: cloud index out of range");
   uint64_t off[2] = {0, in.n};
@@ -1312,6 +1290,20 @@ void octree_extract(Context &ctx, const Octree &in, size_t seg, Octree &out) {
     ProfScope _prof(ctx, "strip_cloud", (double)n * 32);
     k_strip_cloud<<<grid_for(n, 256), 256, 0, ctx.stream>>>(in.keys + off[0], n, in.max_depth, k.get());
     DG_LAUNCH_CHECK();
+  }
+  // the cloud's nodes: 7 leaves per node and one more per cloud lie before them
+  const size_t first = (off[0] - seg) / 7, nn = n ? (n - 1) / 7 : 0;
+  auto strip = [&](auto tag) {
+    typedef decltype(tag) K;
+    DBuf<K> nodes(nn, ctx.stream);
+    k_strip_nodes<K><<<grid_for(nn, 256), 256, 0, ctx.stream>>>(static_cast<const K *>(in.nodes) + first, nn,
+                                                                in.top - 1, nodes.get());
+    DG_LAUNCH_CHECK();
+    keep_nodes(out, nodes, nn, in.top);
+  };
+  if (in.nodes && nn) {
+    if (in.node_wide) strip(Key128());
+    else strip(uint64_t());
   }
   out.keys = k.release_ptr();
 }
@@ -1519,6 +1511,7 @@ void octree_from_xyzl(Context &ctx, const uint32_t *d_xyzl, size_t n, unsigned D
 void octree_free(Context &ctx, Octree &o) {
   if (o.keys) cudaFreeAsync(o.keys, ctx.stream);
   if (o.seg_off) cudaFreeAsync(o.seg_off, ctx.stream);
+  if (o.nodes) cudaFreeAsync(o.nodes, ctx.stream);
   o = Octree();
 }
 

@@ -28,6 +28,12 @@ struct Octree {
   size_t nseg = 1;
   unsigned seg_bits = 0;
   uint64_t *seg_off = nullptr;  // device, nseg + 1 (null for one segment)
+  // the internal octants in preorder (dg_nodes.cuh), where the octree was made
+  // from them: construction, balance, coarsening and the clouds of a batch
+  void *nodes = nullptr;  // uint64_t, or Key128 when node_wide
+  size_t n_node = 0;      // n = 7 n_node + nseg
+  unsigned top = 0;       // deepest leaf level (node keys reach level top - 1)
+  bool node_wide = false;
 };
 
 inline unsigned bits_for(size_t nseg) {
@@ -61,8 +67,10 @@ void balance_octree(Context &ctx, const Octree &in, Octree &out, bool inc_corner
 // cloud `seg` of a batched octree as a single-cloud octree
 void octree_extract(Context &ctx, const Octree &in, size_t seg, Octree &out);
 
-// ot::coarsenOctree (src/coarsen.cpp:53), one cloud.
-void coarsen_octree(Context &ctx, const Octree &in, Octree &out);
+// ot::coarsenOctree (src/coarsen.cpp:53), one cloud.  With leaves false an
+// input that has its nodes gives an octree of nodes alone (no keys), for a
+// balance that follows.
+void coarsen_octree(Context &ctx, const Octree &in, Octree &out, bool leaves = true);
 
 // ot::completeOctree (src/construct.cpp:518), one cloud: the octants of
 // d_xyzl (n records x y z level at max_depth), sorted and made unique and
