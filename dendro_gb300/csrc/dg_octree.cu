@@ -827,6 +827,7 @@ __global__ void __launch_bounds__(256) k_bal_start(const void *__restrict__ in, 
     if (won) won = node_insert<K>(tab, mask, node_wide(key), Lm, flags);
     if (won) rank = atomicAdd(&num[l], 1u);
   }
+  __syncwarp();
   __syncthreads();
   if (threadIdx.x < 32 && num[threadIdx.x])
     base[threadIdx.x] =
@@ -853,6 +854,22 @@ struct BalSmem {
   unsigned n_cand, n_won;
   unsigned long long at;
 };
+
+// appends v of the lanes that say so to a list in shared memory; all lanes of
+// the warp take part, which also brings them together again after the
+// diverging probes (with each lane adding to the counter where it left its
+// probes, entries were at times read across the next barrier before they were
+// written, with 128-bit keys)
+__device__ __forceinline__ void warp_append(bool mine, uint16_t v, unsigned *n, uint16_t *list) {
+  const unsigned m = __ballot_sync(0xffffffffu, mine);
+  if (!m) return;
+  const int lane = threadIdx.x & 31, leader = __ffs(m) - 1;
+  unsigned at = 0;
+  if (lane == leader) at = atomicAdd(n, (unsigned)__popc(m));
+  at = __shfl_sync(0xffffffffu, at, leader);
+  if (mine) list[at + __popc(m & ((1u << lane) - 1u))] = v;
+  __syncwarp();
+}
 
 template <typename K>
 __global__ void __launch_bounds__(BAL_TILE) k_bal_level(unsigned l, unsigned Lm, bool inc_corner, K *__restrict__ tab,
@@ -902,32 +919,35 @@ __global__ void __launch_bounds__(BAL_TILE) k_bal_level(unsigned l, unsigned Lm,
       }
     }
     __syncthreads();
-    for (unsigned me = t; me < 8 * here; me += BAL_TILE) {
-      const W key = node_wide(S.cand[me]);
-      if (key == node_empty(key)) continue;
-      const uint64_t hash = node_hash(key, Lm);
-      uint32_t h = (uint32_t)(hash ^ hash >> 24) & (slots - 1);
+    for (unsigned r = 0; r < 8 * here; r += BAL_TILE) {
+      const unsigned me = r + t;
       bool mine = false;
-      for (unsigned probe = 0; probe < slots; probe++) {
-        const uint32_t cur = atomicCAS(&S.slot[h], BAL_FREE, me);
-        mine = cur == BAL_FREE;
-        if (mine || node_wide(S.cand[cur]) == key) break;
-        h = (h + 1) & (slots - 1);
+      const W key = me < 8 * here ? node_wide(S.cand[me]) : node_empty(W());
+      if (key != node_empty(key)) {
+        const uint64_t hash = node_hash(key, Lm);
+        uint32_t h = (uint32_t)(hash ^ hash >> 24) & (slots - 1);
+        for (unsigned probe = 0; probe < slots; probe++) {
+          const uint32_t cur = atomicCAS(&S.slot[h], BAL_FREE, me);
+          mine = cur == BAL_FREE;
+          if (mine || node_wide(S.cand[cur]) == key) break;
+          h = (h + 1) & (slots - 1);
+        }
       }
-      if (mine) S.list[atomicAdd(&S.n_cand, 1u)] = (uint16_t)me;
+      warp_append(mine, (uint16_t)me, &S.n_cand, S.list);
     }
     __syncthreads();
     const unsigned nc = S.n_cand;
-    for (unsigned q = t; q < nc; q += BAL_TILE) {
-      const uint16_t me = S.list[q];
-      if (node_insert<K>(tab, mask, node_wide(S.cand[me]), Lm, flags)) S.won[atomicAdd(&S.n_won, 1u)] = me;
+    for (unsigned r = 0; r < nc; r += BAL_TILE) {
+      const unsigned q = r + t, me = q < nc ? S.list[q] & (BAL_CAND - 1) : 0u;
+      const bool won = q < nc && node_insert<K>(tab, mask, node_wide(S.cand[me]), Lm, flags);
+      warp_append(won, (uint16_t)me, &S.n_won, S.won);
     }
     __syncthreads();
     const unsigned nw = S.n_won;
     if (t == 0 && nw) S.at = next + atomicAdd(&cnt->grown[l - 1], (unsigned long long)nw);
     __syncthreads();
     for (unsigned q = t; q < nw; q += BAL_TILE) {
-      if (S.at + q < grown_cap) grown[S.at + q] = S.cand[S.won[q]];
+      if (S.at + q < grown_cap) grown[S.at + q] = S.cand[S.won[q] & (BAL_CAND - 1)];
       else set_flag(flags, DGF_CAPACITY);
     }
     __syncthreads();
