@@ -193,6 +193,41 @@ __global__ void __launch_bounds__(P2O_BLOCK) k_p2o_count(const Key128 *__restric
   if (threadIdx.x == 0) sums[blockIdx.x] = sum;
 }
 
+// the same for the leaves of a sorted octree: a leaf adds the nodes above it
+// that do not hold its predecessor; leaves that are not aligned octants of the
+// domain in strictly ascending order raise DGF_NOT_BALANCED
+__global__ void __launch_bounds__(P2O_BLOCK) k_leaf_count(const Key128 *__restrict__ k, size_t n, unsigned D,
+                                                          uint16_t *__restrict__ path, uint64_t *__restrict__ sums,
+                                                          unsigned long long *__restrict__ max_level,
+                                                          uint32_t *flags) {
+  uint64_t total = 0;
+  unsigned top = 0;
+#pragma unroll
+  for (int r = 0; r < P2O_PER; r++) {
+    const size_t i = (size_t)blockIdx.x * P2O_TILE + r * P2O_BLOCK + threadIdx.x;
+    if (i >= n) continue;
+    const Key128 ki = k[i], a = tag_anchor(ki);
+    const unsigned L = tag_level(ki);
+    bool ok = L <= D && key_eq(morton_part(ki, D), a);
+    if (ok && L < D) ok = key_eq(key_shl(key_shr(a, 3 * (D - L)), 3 * (D - L)), a);
+    unsigned first = 0;
+    if (i > 0) {
+      const Key128 kp = k[i - 1];
+      ok = ok && key_lt(tag_anchor(kp), a);
+      first = min((unsigned)(nca_level(kp, ki, D) + 1), tag_level(kp));
+    }
+    if (!ok) set_flag(flags, DGF_NOT_BALANCED);
+    path[i] = ok ? (uint16_t)(L | first << 8) : (uint16_t)0;
+    if (ok && L > first) total += L - first;
+    if (ok) top = max(top, L);
+  }
+  uint64_t sum;
+  block_excl_scan<uint64_t, P2O_BLOCK>(total, sum);
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0 && (unsigned long long)top > __ldcg(max_level)) atomicMax(max_level, (unsigned long long)top);
+  if (threadIdx.x == 0) sums[blockIdx.x] = sum;
+}
+
 template <typename K>
 __global__ void __launch_bounds__(P2O_BLOCK) k_p2o_nodes(const Key128 *__restrict__ p, size_t n, unsigned D,
                                                          unsigned Lm, const uint16_t *__restrict__ path,
@@ -224,9 +259,10 @@ __global__ void __launch_bounds__(P2O_BLOCK) k_p2o_nodes(const Key128 *__restric
 // node).  A warp holds four nodes and the 32 nodes that follow the first of
 // them in its registers, so j comes from a search by shuffles; only a subtree
 // that reaches past those is searched in memory.
-template <typename K>
+// CHECK compares with the leaves that are there instead (DGF_NOT_BALANCED).
+template <typename K, bool CHECK>
 __global__ void __launch_bounds__(256) k_emit_leaves(const K *__restrict__ nodes, size_t nn, unsigned Lm, unsigned D,
-                                                     Key128 *__restrict__ out, size_t total) {
+                                                     Key128 *__restrict__ out, size_t total, uint32_t *flags) {
   typedef NodeWide<K> N;
   typedef typename N::W W;
   const int lane = threadIdx.x & 31;
@@ -274,7 +310,12 @@ __global__ void __launch_bounds__(256) k_emit_leaves(const K *__restrict__ nodes
   if (node && d != Lm) return;
   const W in_cloud = path & (((W)1 << (3 * Lm)) - 1);
   const size_t pos = 7 * (j - (d + 1)) + digit_sum(in_cloud) + c + (size_t)(path >> (3 * Lm));
-  if (pos < total) out[pos] = make_tagged(anchor, d + 1);
+  const Key128 leaf = make_tagged(anchor, d + 1);
+  if constexpr (CHECK) {
+    if (pos >= total || !key_eq(out[pos], leaf)) set_flag(flags, DGF_NOT_BALANCED);
+  } else {
+    if (pos < total) out[pos] = leaf;
+  }
 }
 
 // per cloud: its first leaf's place, and its root where the root is a leaf
@@ -324,7 +365,7 @@ static void emit_octree(Context &ctx, const K *nodes, size_t nn, unsigned Lm, un
   }
   if (nn) {
     ProfScope _prof(ctx, "emit_leaves", (double)nn * sizeof(K) + (double)total * 16);
-    k_emit_leaves<K><<<grid_for(8 * nn, 256), 256, 0, s>>>(nodes, nn, Lm, D, leaves.get(), total);
+    k_emit_leaves<K, false><<<grid_for(8 * nn, 256), 256, 0, s>>>(nodes, nn, Lm, D, leaves.get(), total, nullptr);
     DG_LAUNCH_CHECK();
   }
 }
@@ -726,6 +767,51 @@ void points_to_octree(Context &ctx, const double *d_xyz, size_t n, const double 
     out.seg_off = d_final.release_ptr();
   }
   DG_CUDA(cudaStreamSynchronize(s));
+}
+
+bool octree_nodes(Context &ctx, const Octree &in, Octree &out) {
+  cudaStream_t s = ctx.stream;
+  const size_t n = in.n, nblocks = (n + P2O_TILE - 1) / P2O_TILE;
+  const unsigned D = in.max_depth;
+  out = Octree();
+  out.max_depth = D;
+  out.n = n;
+  if (in.nseg != 1) fail(DG_ERR_UNSUPPORTED, "octree: one cloud per call");
+  auto in_order = [&] {
+    const uint32_t f = read_scalar(ctx, ctx.d_flags);
+    if (f & ~(uint32_t)DGF_NOT_BALANCED) check_device_flags(ctx, "octree");
+    if (f) DG_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), s));
+    return f == 0;
+  };
+  DBuf<uint16_t> path(n, s);
+  DBuf<uint64_t> sums(nblocks, s);
+  unsigned long long *d_info = ctx.d_scratch;  // {nodes, deepest leaf level}
+  DG_CUDA(cudaMemsetAsync(d_info, 0, 2 * sizeof(unsigned long long), s));
+  DG_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), s));
+  {
+    ProfScope _prof(ctx, "leaf_count", (double)n * 18);
+    k_leaf_count<<<(unsigned)nblocks, P2O_BLOCK, 0, s>>>(in.keys, n, D, path.get(), sums.get(), d_info + 1,
+                                                         ctx.d_flags);
+    DG_LAUNCH_CHECK();
+  }
+  exclusive_scan<uint64_t, uint64_t>(sums.get(), sums.get(), nblocks, reinterpret_cast<uint64_t *>(d_info), s);
+  DG_CUDA(cudaMemcpyAsync(ctx.h_scratch + 4, d_info, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+  if (!in_order()) return false;
+  const size_t nn = (size_t)ctx.h_scratch[4];
+  const unsigned top = (unsigned)ctx.h_scratch[5];
+  if (!nn || n != 7 * nn + 1) return false;
+  auto make = [&](auto tag) {
+    typedef decltype(tag) K;
+    DBuf<K> nodes(nn, s);
+    k_p2o_nodes<K><<<(unsigned)nblocks, P2O_BLOCK, 0, s>>>(in.keys, n, D, top - 1, path.get(), sums.get(), nodes.get());
+    DG_LAUNCH_CHECK();
+    k_emit_leaves<K, true><<<grid_for(8 * nn, 256), 256, 0, s>>>(nodes.get(), nn, top - 1, D, in.keys, n, ctx.d_flags);
+    DG_LAUNCH_CHECK();
+    if (!in_order()) return false;
+    keep_nodes(out, nodes, nn, top);
+    return true;
+  };
+  return nodes_fit_64(top, 0) ? make(uint64_t()) : make(Key128());
 }
 
 void octree_segment_offsets(Context &ctx, const Octree &o, uint64_t *h_off) {

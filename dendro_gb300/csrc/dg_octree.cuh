@@ -51,6 +51,10 @@ void octree_free(Context &ctx, Octree &o);
 void points_to_octree(Context &ctx, const double *d_xyz, size_t n, const double glens[3], unsigned max_depth,
                       unsigned max_pts, Octree &out, const uint64_t *h_seg_start = nullptr, size_t nseg = 1);
 
+// the nodes of an octree that came without them (out: nodes only); false
+// unless the leaves are those of a complete octree in order, with a node
+bool octree_nodes(Context &ctx, const Octree &in, Octree &out);
+
 // per-segment output offsets of a batched octree, on the host
 void octree_segment_offsets(Context &ctx, const Octree &o, uint64_t *h_off);
 
