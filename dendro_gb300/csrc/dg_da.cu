@@ -1199,14 +1199,20 @@ void mesh_free(Context &ctx, Mesh &m) {
 // ------------------------------------------------------------------------
 // the diagonal table of the element loop for these factors (kept on the
 // context until a call with others)
+// (FP64: the fixed-point table follows it)
 template <typename T>
 static const T *diag_table(Context &ctx, double lap_fac, double mass_fac) {
-  const bool dbl = std::is_same<T, double>::value;
+  constexpr bool dbl = std::is_same<T, double>::value;
   Context::DiagTable &t = dbl ? ctx.dtab64 : ctx.dtab32;
-  if (!t.p) DG_CUDA(cudaMalloc(&t.p, DTAB_ENTRIES * sizeof(T)));
+  if (!t.p) DG_CUDA(cudaMalloc(&t.p, DTAB_ENTRIES * (dbl ? sizeof(T) + sizeof(int2) : sizeof(T))));
   if (!t.ok || t.lap != lap_fac || t.mass != mass_fac) {
     k_dtab<T><<<(DTAB_ENTRIES + 127) / 128, 128, 0, ctx.stream>>>(static_cast<T *>(t.p), lap_fac, mass_fac);
     DG_LAUNCH_CHECK();
+    if (dbl) {
+      k_fix_table<<<(DTAB_ENTRIES + 127) / 128, 128, 0, ctx.stream>>>(
+          reinterpret_cast<int2 *>(static_cast<T *>(t.p) + DTAB_ENTRIES), lap_fac, mass_fac);
+      DG_LAUNCH_CHECK();
+    }
     t.lap = lap_fac;
     t.mass = mass_fac;
     t.ok = true;
@@ -1223,37 +1229,40 @@ static unsigned patch_grid(Context &ctx, F *kernel, size_t smem, size_t n_patch)
   return (unsigned)std::min<size_t>(n_patch, (size_t)std::max(per_sm, 1) * ctx.num_sms);
 }
 
-template <typename T, bool DIR>
-void launch_family_matvec(Context &ctx, const Mesh &m, const T *x, T *y, double lap_fac, double mass_fac,
+template <bool DIR>
+void launch_family_matvec(Context &ctx, const Mesh &m, const float *x, float *y, double lap_fac, double mass_fac,
                           const char *name, double bytes) {
-  const size_t smem = family_smem<T>(m.max_run);
-  const unsigned grid = patch_grid(ctx, k_family_matvec<T, DIR, false>, smem, m.n_patch);
-  const T *dtab = diag_table<T>(ctx, lap_fac, mass_fac);
+  const size_t smem = family_smem<float>(m.max_run);
+  const unsigned grid = patch_grid(ctx, k_family_matvec<float, DIR, false>, smem, m.n_patch);
+  const float *dtab = diag_table<float>(ctx, lap_fac, mass_fac);
   ProfScope _prof(ctx, name, bytes);
-  k_family_matvec<T, DIR, false><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch,
-                                                                  m.max_run, dtab, x, y, nullptr, nullptr);
+  k_family_matvec<float, DIR, false><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch,
+                                                                      m.max_run, dtab, x, y, nullptr, nullptr);
   DG_LAUNCH_CHECK();
 }
-template void launch_family_matvec<float, true>(Context &, const Mesh &, const float *, float *, double, double,
-                                                const char *, double);
-template void launch_family_matvec<double, true>(Context &, const Mesh &, const double *, double *, double, double,
-                                                 const char *, double);
 
-void launch_family_matvec_fix(Context &ctx, const Mesh &m, const double *x, double *y, const char *name,
-                              double bytes) {
-  const size_t smem = 2 * ((size_t)m.max_run + 1) * sizeof(long long);
-  const unsigned grid = patch_grid(ctx, k_family_matvec_fix<true>, smem, m.n_patch);
+template <bool DIR>
+void launch_family_matvec(Context &ctx, const Mesh &m, const double *x, double *y, double lap_fac, double mass_fac,
+                          const char *name, double bytes) {
+  const size_t smem = family_fix_smem(m.max_run);
+  const unsigned grid = patch_grid(ctx, k_family_matvec_fix<DIR>, smem, m.n_patch);
+  const double *dtab = diag_table<double>(ctx, lap_fac, mass_fac);
   ProfScope _prof(ctx, name, bytes);
-  k_family_matvec_fix<true><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch, m.max_run,
-                                                             x, y);
+  k_family_matvec_fix<DIR><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch, m.max_run,
+                                                            reinterpret_cast<const int2 *>(dtab + DTAB_ENTRIES), dtab,
+                                                            x, y);
   DG_LAUNCH_CHECK();
 }
+template void launch_family_matvec<true>(Context &, const Mesh &, const float *, float *, double, double, const char *,
+                                         double);
+template void launch_family_matvec<true>(Context &, const Mesh &, const double *, double *, double, double,
+                                         const char *, double);
 
 template <typename T>
 void mesh_matvec(Context &ctx, const Mesh &m, const T *x, T *y, double lap_fac, double mass_fac) {
   DG_CUDA(cudaMemsetAsync(y, 0, m.n_node * sizeof(T), ctx.stream));
-  launch_family_matvec<T, false>(ctx, m, x, y, lap_fac, mass_fac, sizeof(T) == 4 ? "matvec_fp32" : "matvec_fp64",
-                                 (double)m.n_elem * 36 + (double)m.n_node * 3 * sizeof(T));
+  launch_family_matvec<false>(ctx, m, x, y, lap_fac, mass_fac, sizeof(T) == 4 ? "matvec_fp32" : "matvec_fp64",
+                              (double)m.n_elem * 36 + (double)m.n_node * 3 * sizeof(T));
 }
 template void mesh_matvec<float>(Context &, const Mesh &, const float *, float *, double, double);
 template void mesh_matvec<double>(Context &, const Mesh &, const double *, double *, double, double);

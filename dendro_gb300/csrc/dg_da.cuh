@@ -113,12 +113,12 @@ void ensure_stencils(Context &ctx);
 
 // the element loop on a zeroed y; DIR: the Dirichlet form (boundary rows and
 // columns from the run words' boundary flag)
-template <typename T, bool DIR>
-void launch_family_matvec(Context &ctx, const Mesh &m, const T *x, T *y, double lap_fac, double mass_fac,
+template <bool DIR>
+void launch_family_matvec(Context &ctx, const Mesh &m, const float *x, float *y, double lap_fac, double mass_fac,
                           const char *name, double bytes);
-// the Dirichlet K + M on FP64 vectors in 64-bit fixed point
-void launch_family_matvec_fix(Context &ctx, const Mesh &m, const double *x, double *y, const char *name,
-                              double bytes);
+template <bool DIR>
+void launch_family_matvec(Context &ctx, const Mesh &m, const double *x, double *y, double lap_fac, double mass_fac,
+                          const char *name, double bytes);
 
 // host-side generators (same mathematics as the reference's .inp tables)
 void gen_etype_masks(uint8_t masks[8 * 18]);

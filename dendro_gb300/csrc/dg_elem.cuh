@@ -30,12 +30,10 @@
 // What bounds it (1.1e7 elements of a Gaussian cloud, GB300): FP32 143 us,
 // instruction issue and the latency of the gathers (DRAM traffic alone would
 // take 34 us; without the shared-memory atomics 116 us, without the x gather
-// 124 us); FP64 1,270 us, the FP64 pipe, which issues 2 operations per clock
-// per SM; fixed point 293 us, integer issue.  An element-wise loop over dense
-// stencils, 8 gathers and 8 atomics per element, took 348, 1,820 and 873 us
-// (the last in double-single arithmetic).  128 families per patch: 64 and 256
-// measured 152 / 150 us in FP32 and 1,296 / 1,481 us in FP64; a patch of 256
-// leaves too few blocks on small meshes.
+// 124 us); FP64 vectors 350 us, integer instructions (further down).  An
+// element-wise loop over dense stencils, 8 gathers and 8 atomics per element,
+// took 348 and 1,820 us.  128 families per patch: 64 and 256 measured 152 / 150
+// us in FP32; a patch of 256 leaves too few blocks on small meshes.
 //
 // Patches: FAM consecutive families (in element order) make a patch, one
 // thread block's work at a time.  fam[(p * 4 + w) * FAM + t] is word w of the
@@ -130,27 +128,30 @@ __global__ void k_dtab(T *__restrict__ out, double lapf, double massf) {
   out[i] = q < DTAB_CHILD + 4 ? (T)dtab_entry<double>(q, lapf * h * 0.5, massf * h * h * h * 0.125) : (T)0;
 }
 
-// The table entries of K + M as fractions: entry i is
-// (alpha fix_lap(i) + beta fix_mass(i)) / (27 * 2^fix_shift(i)) with
-// alpha = h / 2, beta = h^3 / 8
-__host__ __device__ constexpr int fix_weight(int i, bool lap) {
-  int m[3] = {}, a[3] = {};  // mode weights times 12 (a family's) or 6 (an element's)
-  if (i < DTAB_CHILD) {
-    const int o = i < 4 ? 0 : i < 7 ? 1 : i < 9 ? 2 : 3;
-    const int q = i - (i < 4 ? 0 : i < 7 ? 4 : i < 9 ? 7 : 9);
-    for (int k = 0; k < 3; k++) {
-      m[k] = k < o ? 4 : k < o + q ? 1 : 3;
-      a[k] = k < o + q ? 3 : 0;
-    }
-  } else {
-    for (int k = 0; k < 3; k++) {
-      m[k] = k < i - DTAB_CHILD ? 1 : 3;
-      a[k] = k < i - DTAB_CHILD ? 3 : 0;
-    }
+// The same table for 64-bit fixed point, a row per level: entry i times
+// 2^(63 - k), split into its upper bits and its 30 lowest, with 2^k the power
+// of two not below the level's |lap| + |mass| (so that |entry| <= 2^(k - 3));
+// k in the row's last place, FIX_NONE where it leaves the range that the element
+// loop's exponents have room for.
+constexpr int FIX_K = DTAB_STRIDE - 1, FIX_K_MAX = 400, FIX_NONE = 0x7fffffff;
+static_assert(DTAB_CHILD + 4 <= FIX_K, "a place for the exponent");
+static __global__ void k_fix_table(int2 *__restrict__ out, double lapf, double massf) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= DTAB_ENTRIES) return;
+  const double h = ldexp(1.0, -(i / DTAB_STRIDE)), lap = lapf * h * 0.5, mass = massf * h * h * h * 0.125;
+  const double most = fabs(lap) + fabs(mass);
+  int k = 0;
+  if (most > 0.0 && frexp(most, &k) == 0.5) k--;
+  const bool ok = is_finite(most) && k >= -FIX_K_MAX && k <= FIX_K_MAX && (most > 0.0 || (lapf == 0.0 && massf == 0.0));
+  const int q = i % DTAB_STRIDE;
+  int2 e = make_int2(0, 0);
+  if (q == FIX_K) e.x = ok ? k : FIX_NONE;
+  else if (ok) {
+    const long long f = __double2ll_rn(ldexp(dtab_entry<double>(q, lap, mass), 63 - k));
+    e = make_int2((int)(f & ((1 << 30) - 1)), (int)(f >> 30));
   }
-  return lap ? a[0] * m[1] * m[2] + m[0] * a[1] * m[2] + m[0] * m[1] * a[2] : m[0] * m[1] * m[2];
+  out[i] = e;
 }
-__host__ __device__ constexpr int fix_shift(int i) { return i < DTAB_CHILD ? 6 : 3; }
 
 // arithmetic of one lattice value: FP32, FP64 or 64-bit fixed point
 template <typename V>
@@ -297,18 +298,75 @@ __device__ __forceinline__ uint32_t fam_hang(const uint4 (&w)[4]) {
   return fam_u16(w, 29) | fam_u16(w, 30) << 16;
 }
 
+// Family f in floating point: its lattice from xs, its elements in registers,
+// its lattice added into ys with shared-memory atomics.  COEF: element e's
+// factors are coef[2e] (Laplacian) and coef[2e + 1] (mass) instead of the
+// table's; fchild[8 f + c] gives e.  A family whose values are not all finite
+// takes the element path, so that a non-finite x reaches exactly the rows of
+// the elements that hold it.
+template <typename T, bool COEF>
+__device__ __forceinline__ void family_floating(const uint4 (&w)[4], size_t f, const T *xs, T *ys, const T *dt,
+                                                const double *__restrict__ coef,
+                                                const uint32_t *__restrict__ fchild) {
+  const uint32_t mask = fam_mask(w), hang = fam_hang(w);
+  T u[27];
+  auto gather = [&]() {
+#pragma unroll
+    for (int i = 0; i < 27; i++) u[i] = xs[fam_u16(w, i)];
+    lat_interpolate(u, hang);
+  };
+  gather();
+  bool regather = false;
+  // a warp takes one path: both cost more than the dearer one
+  bool whole = !COEF && __all_sync(__activemask(), mask == 255u);
+  if (whole) {
+    lat_forward(u);
+    regather = !is_finite(u[0]);  // the weighted sum of all 27
+    whole = !regather;
+  }
+  if (whole) {
+    const T *d = dt + fam_level(w) * DTAB_STRIDE;
+    lat_scale(u, [&](T t, int i) { return t * d[i]; });
+    lat_backward(u);
+  } else {
+    if (regather) gather();
+    T v[27], d[4];
+    if constexpr (!COEF) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) d[k] = dt[fam_level(w) * DTAB_STRIDE + DTAB_CHILD + k];
+    }
+    lat_elements(
+        u, v, mask,
+        [&](int c) {
+          if constexpr (COEF) {
+            const size_t e = fchild[8 * f + c];  // 0 where there is none
+            const T h = exp2_neg((T)0, fam_level(w));
+            const T lf = (T)coef[2 * e] * h * (T)0.5, mf = (T)coef[2 * e + 1] * h * h * h * (T)0.125;
+#pragma unroll
+            for (int k = 0; k < 4; k++) d[k] = dtab_entry(DTAB_CHILD + k, lf, mf);
+          }
+        },
+        [&](T t, int q) { return t * d[q]; });
+#pragma unroll
+    for (int i = 0; i < 27; i++) u[i] = v[i];
+  }
+  lat_distribute(u, hang);
+#pragma unroll
+  for (int i = 0; i < 27; i++) {
+    const uint32_t n = fam_u16(w, i);
+    if (n) atomicAdd(&ys[n], u[i]);
+  }
+}
+
 // One block per patch, grid-strided, three barriers per patch:
 //   1. x of the patch's nodes into xs (node ids read coalesced), ys = 0;
 //   2. thread t = family t: its lattice from xs, its elements in registers,
 //      its lattice added into ys with shared-memory atomics;
 //   3. each node's sum stored (nodes of this patch alone) or added to y.
 // DIR, the Dirichlet form: boundary rows are the identity (y = x), boundary
-// columns are dropped.  COEF: element e's factors are coef[2e] (Laplacian)
-// and coef[2e + 1] (mass) instead of the table's; fchild[8 f + c] gives e.
-// A family whose values are not all finite takes the element path, so that a
-// non-finite x reaches exactly the rows of the elements that hold it.
+// columns are dropped.
 // Blocks per SM (registers): FP32 at 4 to 8 blocks 158, 152, 143, 145, 151 us on
-// 1.1e7 elements; FP64 at 2, 3, 4 blocks 1,350, 1,279, 1,267 us (4 spills).
+// 1.1e7 elements.
 template <typename T, bool DIR, bool COEF>
 __global__ void __launch_bounds__(FAM, sizeof(T) == 4 ? 6 : 3)
     k_family_matvec(const uint4 *__restrict__ fam, const uint32_t *__restrict__ prun, const uint4 *__restrict__ pinfo,
@@ -338,56 +396,7 @@ __global__ void __launch_bounds__(FAM, sizeof(T) == 4 ? 6 : 3)
       ys[u + 1] = (T)0;
     }
     __syncthreads();
-    if (have) {
-      const uint32_t mask = fam_mask(w), hang = fam_hang(w);
-      T u[27];
-      auto gather = [&]() {
-#pragma unroll
-        for (int i = 0; i < 27; i++) u[i] = xs[fam_u16(w, i)];
-        lat_interpolate(u, hang);
-      };
-      gather();
-      bool regather = false;
-      // a warp takes one path: both cost more than the dearer one
-      bool whole = !COEF && __all_sync(__activemask(), mask == 255u);
-      if (whole) {
-        lat_forward(u);
-        regather = !is_finite(u[0]);  // the weighted sum of all 27
-        whole = !regather;
-      }
-      if (whole) {
-        const T *d = dt + fam_level(w) * DTAB_STRIDE;
-        lat_scale(u, [&](T t, int i) { return t * d[i]; });
-        lat_backward(u);
-      } else {
-        if (regather) gather();
-        T v[27], d[4];
-        if constexpr (!COEF) {
-#pragma unroll
-          for (int k = 0; k < 4; k++) d[k] = dt[fam_level(w) * DTAB_STRIDE + DTAB_CHILD + k];
-        }
-        lat_elements(
-            u, v, mask,
-            [&](int c) {
-              if constexpr (COEF) {
-                const size_t e = fchild[8 * (p * FAM + tid) + c];  // 0 where there is none
-                const T h = exp2_neg((T)0, fam_level(w));
-                const T lf = (T)coef[2 * e] * h * (T)0.5, mf = (T)coef[2 * e + 1] * h * h * h * (T)0.125;
-#pragma unroll
-                for (int k = 0; k < 4; k++) d[k] = dtab_entry(DTAB_CHILD + k, lf, mf);
-              }
-            },
-            [&](T t, int q) { return t * d[q]; });
-#pragma unroll
-        for (int i = 0; i < 27; i++) u[i] = v[i];
-      }
-      lat_distribute(u, hang);
-#pragma unroll
-      for (int i = 0; i < 27; i++) {
-        const uint32_t n = fam_u16(w, i);
-        if (n) atomicAdd(&ys[n], u[i]);
-      }
-    }
+    if (have) family_floating<T, COEF>(w, p * FAM + tid, xs, ys, dt, coef, fchild);
     __syncthreads();
 #pragma unroll 4
     for (int u = tid; u < nr; u += FAM) {
@@ -404,63 +413,142 @@ inline size_t family_smem(int max_run) {
   return (2 * (size_t)(max_run + 1) + DTAB_ENTRIES) * sizeof(T);
 }
 
-// ---- fixed-point form for FP64 vectors: the CG operator (K + M, Dirichlet)
-// of the FP32-V-cycle solve.  GB300 issues FP64 at 2 multiply-adds per clock
-// per SM, and the FP64 loop is bound by that.  In the sum / difference basis
-// the operator is additions and one factor per mode, a small integer over
-// 27 * 2^k times powers of two of the level, so integers do all of it: each
-// patch takes its x as 51-bit fixed point relative to the patch's largest
-// entry, the sums and differences are exact, a mode's product is exact before
-// its shift, and the node sums are integer atomic adds; 1/27 is applied to
-// each node's sum.  With |x| < 2^51 a mode's product stays below 2^62
-// (1728 + 144 times |x| at the most) and a node's sum too (at most 75 alpha
-// times 27 |x|).  The rounding of x is 2^-52 of the patch's largest entry and
-// that of the modes smaller.  Conversions are integer operations as well, so
-// the loop issues one FP64 multiplication per node and the global adds.
-// Against FP64 on uniform random x the result is off by 1.4e-16 of its norm
-// (1.4e-15 for the FP32-pair arithmetic it replaces).  Blocks per SM: at 3, 4, 5,
-// 6 blocks 367, 319, 293, 293 us on 1.1e7 elements.
+// ---- FP64 vectors ----
+// GB300 issues FP64 at 2 multiply-adds per clock per SM, and an element loop in
+// FP64 is bound by that: 1,270 us on 1.1e7 elements.  In the sum / difference
+// basis the operator is additions and one factor per mode, so integers do all
+// of it, in 64-bit fixed point with an exponent per family:
+//   - x of the patch's nodes is kept as mantissa and exponent in one word; a
+//     family shifts its 27 values to its largest exponent: |u| < 2^55, cut
+//     below the last place (values within a factor of 4 are exact);
+//   - modes, |t| < 2^61, times table entries of 2^63 scale, rounded: results
+//     in units of 2^(k - 3) u.  A child's row sums |entries| to at most
+//     4/3 (|lap| + |mass|), a family's lattice point to 8 of them, so |v| <
+//     2^(55 + 3.42 + 3): sums in between may wrap, the results do not;
+//   - a node's sum is kept in half the finest unit of the families that touch
+//     it: at most 43 times 2^(55 + 2) < 2^63 (4 of 8 octants around it
+//     refined, all their edges and faces hanging).  The unit is the coarsest of
+//     those families', found by one more round of shared-memory atomics where
+//     the patch's families differ by more than FIX_EVEN binary places (without
+//     the rule 394 -> 357 us); the sum becomes FP64 once per node.
+// Errors in a family's result are a few units, 2^-57 of its largest value
+// times the level's |lap| + |mass|; those of the FP64 form in the same basis
+// are 2^-53 of that.  Measured against extended precision (norm; 1.6e5
+// elements): uniform random x 8.9e-17 (FP64 1.2e-16, dense stencils 1.4e-16),
+// products of sines 3.9e-16 (1.9e-15, 3.0e-15), a Gaussian 1.4e-15 (3.9e-15,
+// 7.0e-15), one node 7.9e-17 (5.1e-17, 2.2e-17).
+// Patches outside that range take floating point, all of it: values that are
+// not finite or not within 2^-511 .. 2^511, factors beyond 2^+-400, and
+// families with subdivided children where a child's values all lie below 2^-4
+// of the family's (those are applied child by child in FP64, so a child's
+// rows would be as exact as its own values there).
+// What bounds it: 350 us on 1.1e7 elements (DRAM traffic alone 50): 3,500
+// instructions per 32 families at 1.5 per clock per SM; warps wait for the
+// gathers (3.0 of 10.5 cycles per instruction), barriers (1.6) and
+// instructions (1.5: the code is long, so loops over nodes unroll no further
+// than they must: 4 and 1 times 350 us, 4 and 4 359, 8 and 8 405).  Blocks per
+// SM: at 3, 4, 5, 6 451, 387, 411, 480 us.  Small meshes are bound by latency
+// (2e4 elements 16 us).
+// x as one word: its 53-bit mantissa, signed, above a 10-bit exponent (0: zero)
+constexpr int FIX_EXP = 10, FIX_BIAS = 511;
+constexpr uint32_t FIX_EVEN = 2;
+constexpr uint32_t FIX_EMASK = (1u << FIX_EXP) - 1;
 
-// x * 2^s rounded to an integer (|x| * 2^s < 2^51)
-__device__ __forceinline__ long long double_to_fix(unsigned long long bits, int s) {
-  const int e = (int)(bits >> 52) & 0x7ff;
-  unsigned long long m = bits & 0xfffffffffffffull;
-  if (e) m |= 1ull << 52;
-  const int sh = (e ? e : 1) - 1075 + s;
-  unsigned long long r;
-  if (sh >= 0) r = m << sh;
-  else if (sh > -55) r = (m + (1ull << (-sh - 1))) >> -sh;
-  else r = 0;
-  return (bits >> 63) ? -(long long)r : (long long)r;
+__device__ __forceinline__ long long fix_pack(double v, bool &outside) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  if (!(b << 1)) return 0;
+  const int e = ((int)(b >> 52) & 0x7ff) - FIX_BIAS;
+  outside = outside || e < 1 || e > (int)FIX_EMASK;
+  const long long m = (long long)((b & 0xfffffffffffffull) | 1ull << 52);
+  return (long long)((unsigned long long)((long long)b < 0 ? -m : m) << FIX_EXP) | (e & (int)FIX_EMASK);
 }
 
-// f * 2^-s as FP64, rounded
+// t times the table entry d, over 2^60: |t| < 2^61, |d| <= 2^60.  The product
+// of the two low parts is replaced by its mean
+__device__ __forceinline__ long long fix_mul(long long t, int2 d) {
+  const int th = (int)(t >> 30), tl = (int)t & ((1 << 30) - 1);
+  const long long mid = (long long)th * d.x + ((long long)tl * d.y + ((1 << 29) + (d.x >> 1)));
+  return (long long)th * d.y + (mid >> 30);
+}
+
+// t / 2^n rounded down, also for n > 63
+__device__ __forceinline__ long long fix_shr(long long t, uint32_t n) {
+  long long r;
+  asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(t), "r"(n));
+  return r;
+}
+
+// adds v to a 64-bit sum in shared memory, as two words and a carry: the
+// 64-bit atomic is a loop there (382 -> 357 us on 1.1e7 elements; plain adds
+// would take 355)
+__device__ __forceinline__ void fix_add(long long *at, long long v) {
+  uint32_t *w = reinterpret_cast<uint32_t *>(at);
+  const uint32_t lo = (uint32_t)v, old = atomicAdd(w, lo);
+  atomicAdd(w + 1, (uint32_t)(v >> 32) + (old + lo < lo ? 1u : 0u));
+}
+
+// f * 2^-s as FP64, rounded (a normal number)
 __device__ __forceinline__ double fix_to_double(long long f, int s) {
   const unsigned long long a = f < 0 ? 0ull - (unsigned long long)f : (unsigned long long)f;
   if (!a) return 0.0;
   const int lz = __clzll((long long)a);
   const int e = 1023 + 63 - lz - s;  // biased exponent before rounding
-  if (e < 1 || e > 2045) return ldexp((double)f, -s);
   // 53 bits with the leading one, which adds 1 to the exponent field
   const unsigned long long m = lz <= 10 ? (a + (1ull << (10 - lz))) >> (11 - lz) : a << (lz - 11);
   return __longlong_as_double((long long)((((unsigned long long)(e - 1)) << 52) + m) |
                               (f < 0 ? (long long)(1ull << 63) : 0ll));
 }
 
+// a family of a patch that takes floating point (out of line, it is rare)
+__device__ __noinline__ void family_fp64(const uint4 *__restrict__ fw, const double *xs, double *ys,
+                                         const double *__restrict__ dtab) {
+  uint4 w[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) w[q] = fw[q * FAM];
+  family_floating<double, false>(w, 0, xs, ys, dtab, nullptr, nullptr);
+}
+
+// a child whose values, not all zero, lie below 2^-4 of the family's largest
+// (which is 2^54 or more)
+__device__ __forceinline__ bool fix_uneven(const long long (&u)[27], uint32_t mask) {
+  uint32_t m[27];  // upper words' magnitudes, then their unions over an element
+#pragma unroll
+  for (int i = 0; i < 27; i++) {
+    const int h = (int)(u[i] >> 32);
+    m[i] = (uint32_t)(h ^ h >> 31);
+  }
+  bool any = false;
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    uint32_t o = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) o |= m[lat_vertex(c, k)];
+    if ((mask >> c & 1u) && o < 1u << 18) {
+      long long nz = 0;
+#pragma unroll
+      for (int k = 0; k < 8; k++) nz |= u[lat_vertex(c, k)];
+      any = any || nz != 0;
+    }
+  }
+  return any;
+}
+
 template <bool DIR>
-__global__ void __launch_bounds__(FAM, 5)
+__global__ void __launch_bounds__(FAM, 4)
     k_family_matvec_fix(const uint4 *__restrict__ fam, const uint32_t *__restrict__ prun,
                         const uint4 *__restrict__ pinfo, size_t n_fam, size_t n_patch, int max_run,
+                        const int2 *__restrict__ ftab, const double *__restrict__ dtab,
                         const double *__restrict__ x, double *__restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   long long *xs = reinterpret_cast<long long *>(smem_raw);
   long long *ys = xs + (max_run + 1);
-  __shared__ uint32_t s_emax[2];  // largest biased exponent of the patch's x, by patch parity
+  int2 *ft = reinterpret_cast<int2 *>(ys + (max_run + 1));
+  uint32_t *unit = reinterpret_cast<uint32_t *>(ft + DTAB_ENTRIES);
+  __shared__ uint32_t s_q[2];  // most and least unit of the patch's families
   const int tid = threadIdx.x;
-  if (tid < 2) s_emax[tid] = 0;
+  for (int i = tid; i < DTAB_ENTRIES; i += FAM) ft[i] = ftab[i];
   if (tid == 0) xs[0] = 0;
-  int par = 0;
-  for (size_t p = blockIdx.x; p < n_patch; p += gridDim.x, par ^= 1) {
+  for (size_t p = blockIdx.x; p < n_patch; p += gridDim.x) {
     const bool have = p * FAM + tid < n_fam;
     const uint4 info = pinfo[p];
     const size_t base = (size_t)info.x | (size_t)info.y << 32;
@@ -468,65 +556,97 @@ __global__ void __launch_bounds__(FAM, 5)
     uint4 w[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) w[q] = have ? fam[(p * 4 + q) * FAM + tid] : make_uint4(0, 0, 0, 0);
-    __syncthreads();  // the previous patch is done with xs, ys and its exponent
-    uint32_t emax = 0;
+    __syncthreads();  // the previous patch is done with xs, ys and the units
+    if (tid < 2) s_q[tid] = tid ? 0xffffffffu : 0u;
+    bool plain = false;  // no fixed point
 #pragma unroll 4
     for (int u = tid; u < nr; u += FAM) {
       const uint32_t r = prun[base + u];
-      const long long b = (DIR && (r & PRUN_BDY)) ? 0ll : __double_as_longlong(x[r & PRUN_NODE]);
-      xs[u + 1] = b;
+      xs[u + 1] = (DIR && (r & PRUN_BDY)) ? 0ll : fix_pack(x[r & PRUN_NODE], plain);
       ys[u + 1] = 0;
-      emax = max(emax, (uint32_t)((unsigned long long)b >> 52) & 0x7ffu);
+      unit[u + 1] = 0;
     }
-    emax = __reduce_max_sync(0xffffffffu, emax);
-    if ((tid & 31) == 0) atomicMax(&s_emax[par], emax);
     __syncthreads();
-    emax = s_emax[par];
-    if (tid == 0) s_emax[par ^ 1] = 0;  // for the next patch
-    const bool finite = emax < 0x7ffu;
-    const int s = 1073 - (int)(emax ? emax : 1u);  // |x| * 2^s < 2^51
-    for (int u = tid; u < nr; u += FAM) xs[u + 1] = double_to_fix((unsigned long long)xs[u + 1], s);
-    __syncthreads();
+    const uint32_t mask = fam_mask(w), hang = fam_hang(w), level = fam_level(w);
+    const int k = ft[level * DTAB_STRIDE + FIX_K].x;
+    long long u[27];
+    uint32_t emax = 0;
     if (have) {
-      const uint32_t mask = fam_mask(w), hang = fam_hang(w);
-      // in units of alpha / 27 of the patch's coarsest level
-      const int finer = (int)fam_level(w) - (int)info.w, mass = 2 * (int)fam_level(w) + 2;
-      long long u[27];
 #pragma unroll
-      for (int i = 0; i < 27; i++) u[i] = xs[fam_u16(w, i)];
+      for (int i = 0; i < 27; i++) {
+        u[i] = xs[fam_u16(w, i)];
+        emax = max(emax, (uint32_t)u[i] & FIX_EMASK);
+      }
+      plain = plain || k == FIX_NONE;
+    }
+    const uint32_t q = emax ? emax + (uint32_t)k + 1024u : 0u;
+    const uint32_t hi = __reduce_max_sync(0xffffffffu, q), lo = __reduce_min_sync(0xffffffffu, q ? q : 0xffffffffu);
+    if ((tid & 31) == 0) {
+      atomicMax(&s_q[0], hi);
+      atomicMin(&s_q[1], lo);
+    }
+    if (emax) {
+#pragma unroll
+      for (int i = 0; i < 27; i++) {
+        const uint32_t e = (uint32_t)u[i] & FIX_EMASK;
+        u[i] = fix_shr(u[i] & ~(long long)FIX_EMASK, FIX_EXP - 2 + emax - e);
+      }
       lat_interpolate(u, hang);
-      auto mul = [&](long long t, int i) {
-        return (t * fix_weight(i, true) + (t >> mass) * fix_weight(i, false)) >> (finer + fix_shift(i));
-      };
+      const int2 *d = ft + level * DTAB_STRIDE;
       if (__all_sync(__activemask(), mask == 255u)) {
         lat_forward(u);
-        lat_scale(u, mul);
+        lat_scale(u, [&](long long t, int i) { return fix_mul(t, d[i]); });
         lat_backward(u);
       } else {
         long long v[27];
-        lat_elements(u, v, mask, [](int) {}, [&](long long t, int q) { return mul(t, DTAB_CHILD + q); });
+        plain = plain || fix_uneven(u, mask);
+        lat_elements(u, v, mask, [](int) {}, [&](long long t, int i) { return fix_mul(t, d[DTAB_CHILD + i]); });
 #pragma unroll
         for (int i = 0; i < 27; i++) u[i] = v[i];
       }
       lat_distribute(u, hang);
+    }
+    plain = __syncthreads_or(plain);
+    const uint32_t qmax = s_q[0], qmin = s_q[1];
+    const bool even = qmax - qmin <= FIX_EVEN;
+    if (!plain) {
+      if (!even) {
+        if (emax)
 #pragma unroll
-      for (int i = 0; i < 27; i++) {
-        const uint32_t n = fam_u16(w, i);
-        if (n) atomicAdd(reinterpret_cast<unsigned long long *>(&ys[n]), (unsigned long long)u[i]);
+          for (int i = 0; i < 27; i++) {
+            const uint32_t n = fam_u16(w, i);
+            if (n) atomicMax(&unit[n], q);
+          }
+        __syncthreads();
       }
+      if (emax)
+#pragma unroll
+        for (int i = 0; i < 27; i++) {
+          const uint32_t n = fam_u16(w, i);
+          if (n) fix_add(&ys[n], fix_shr(u[i], (even ? qmax : unit[n]) + 1 - q));
+        }
+    } else {
+      double *xd = reinterpret_cast<double *>(xs);
+      for (int u = tid; u < nr; u += FAM) {
+        const uint32_t r = prun[base + u];
+        xd[u + 1] = (DIR && (r & PRUN_BDY)) ? 0.0 : x[r & PRUN_NODE];
+      }
+      __syncthreads();
+      if (have) family_fp64(fam + p * 4 * FAM + tid, xd, reinterpret_cast<double *>(ys), dtab);
     }
     __syncthreads();
-    const int sy = s + (int)info.w + 1;
-#pragma unroll 4
+#pragma unroll 1
     for (int u = tid; u < nr; u += FAM) {
       const uint32_t r = prun[base + u], g = r & PRUN_NODE;
-      // a patch with a non-finite x: all its rows are NaN
-      const double v = finite ? fix_to_double(ys[u + 1], sy) * (1.0 / 27.0) : __longlong_as_double(0x7ff8000000000000ll);
+      const double v = plain ? __longlong_as_double(ys[u + 1])
+                             : fix_to_double(ys[u + 1], 1024 + 1079 - FIX_BIAS - (int)(even ? qmax : unit[u + 1]));
       if (DIR && (r & PRUN_BDY)) y[g] = x[g];
       else if (r & PRUN_COMPLETE) y[g] = v;
       else atomicAdd(&y[g], v);
     }
   }
 }
+
+inline size_t family_fix_smem(int max_run) { return ((size_t)max_run + 1) * 20 + DTAB_ENTRIES * sizeof(int2); }
 
 }  // namespace dg
