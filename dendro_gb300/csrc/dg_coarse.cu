@@ -9,15 +9,21 @@
 // In-place block Gauss-Jordan without pivoting (the operator is SPD).  For
 // the pivot block K = [k0, k0 + 64), R the other indices and P = inv(X_KK):
 //   X_RR -= X_RK (P X_KR),  X_KR = P X_KR,  X_RK = -(X_RK P),  X_KK = P;
-// after the last block X holds the inverse.  Three launches per block:
-//   k_gj_diag    P, one CTA (64 serial pivots held in registers);
-//   k_gj_strips  Cs = X_RK and Rs = P X_KR into scratch strips, and the new
-//                row and column blocks of X (2 * 64^2 * n multiply-adds on
-//                the CUDA cores);
-//   k_gj_update  X_RR -= Cs Rs: a rank-64 update, n^2 * 64 multiply-adds,
-//                on the tensor cores (tcgen05.mma kind::tf32, accumulators in
-//                tensor memory), 128 x 128 tiles of X, one persistent CTA
-//                per SM.
+// after the last block X holds the inverse.  Two launches per block, on two
+// streams:
+//   k_gj_block   brings the rows and columns of block K up to date with the
+//                block before it, inverts X_KK (64 serial pivots) and leaves
+//                Cs = X_RK and Rs = P X_KR in scratch strips, and the new row
+//                and column blocks in X: the chain from block to block;
+//   k_gj_update  X_RR -= Cs Rs but for the rows and columns of the next block:
+//                a rank-64 update, n^2 * 64 multiply-adds, on the tensor cores
+//                (tcgen05.mma kind::tf32, accumulators in tensor memory), 128
+//                x 128 tiles of X, persistent CTAs; beside the next k_gj_block.
+// 1,741 unknowns (28 blocks) take 0.84 ms and 2,400 take 1.38, host included: of
+// a block k_gj_block takes some 22 us (loads 2, X_KK 4, the inversion 9, the
+// products 5), the update beside it as long.  The next block's part of the
+// update, the inversion and the strips as three launches, the inversion over 20
+// us: 1.53 and 2.05 ms.
 // The update splits each operand entry a = a_hi + a_lo, a_hi the nearest
 // TF32 value and a_lo = a - a_hi (exact in FP32), and accumulates
 // lo * hi + hi * lo + hi * hi in FP32 ("3xTF32"): the dropped lo * lo term
@@ -45,64 +51,9 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
   return d;
 }
 
-// ---- k_gj_diag: P = inv(X_KK) for one diagonal block (one CTA of 256
-// threads): thread t holds 16 entries of row t / 4 in registers.  Per pivot
-// the pivot row's threads scale their row by the reciprocal of the pivot
-// (the pivot column entry becomes that reciprocal) and store it in shared
-// memory (double-buffered, one barrier per pivot); every other row zeroes
-// its pivot-column entry and subtracts its former value times the scaled
-// row.  A row's pivot-column entry comes by a shuffle within the row's four
-// threads.  A partial last block is padded with the identity; P is written
-// as a full GJB x GJB block.  The 64 pivots form a chain of dependent
-// steps (about 20 us); the host overlaps it with the previous block's
-// trailing update.
-__global__ void __launch_bounds__(256) k_gj_diag(const float *__restrict__ X, size_t n, size_t k0, int b,
-                                                 float *__restrict__ P) {
-  static_assert(GJB == 64, "one CTA of 256 threads covers a 64 x 64 block");
-  __shared__ __align__(16) float prow[2][GJB];
-  const int t = threadIdx.x, r = t >> 2, q = t & 3, c0 = q * 16;
-  const int lane = t & 31, base = lane & ~3;
-  float v[16];
-#pragma unroll
-  for (int i = 0; i < 16; i++) {
-    const int c = c0 + i;
-    v[i] = (r < b && c < b) ? X[(k0 + r) * n + k0 + c] : (r == c ? 1.f : 0.f);
-  }
-#pragma unroll
-  for (int p = 0; p < GJB; p++) {
-    float *pr = prow[p & 1];
-    const float f = __shfl_sync(0xffffffffu, v[p & 15], base | (p >> 4));  // this row's column-p entry
-    if (r == p) {
-      const float inv = 1.0f / f;
-#pragma unroll
-      for (int i = 0; i < 16; i++) v[i] *= inv;
-      if (q == (p >> 4)) v[p & 15] = inv;
-      float4 *dst = reinterpret_cast<float4 *>(pr + c0);
-#pragma unroll
-      for (int i = 0; i < 4; i++) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-    }
-    __syncthreads();
-    if (r != p) {
-      if (q == (p >> 4)) v[p & 15] = 0.f;
-      const float4 *src = reinterpret_cast<const float4 *>(pr + c0);
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const float4 s4 = src[i];
-        v[4 * i] -= f * s4.x;
-        v[4 * i + 1] -= f * s4.y;
-        v[4 * i + 2] -= f * s4.z;
-        v[4 * i + 3] -= f * s4.w;
-      }
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 16; i++) P[r * GJB + c0 + i] = v[i];
-}
-
-// acc[4][4] += L R over a 64-deep product, L given transposed (Lt[m][r]), R
-// as is (Rm[m][c]); thread (ty, tx) of 256 owns rows 4ty.., columns 4tx..
-__device__ __forceinline__ void gj_mma(const float *Lt, const float *Rm, float2 (&acc)[4][2]) {
-  const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
+// acc += L R over a 64-deep product, L given transposed (Lt[m][r]), R as is
+// (Rm[m][c]); a thread owns rows 4 ty.., columns 4 tx..
+__device__ __forceinline__ void gj_mma(const float *Lt, const float *Rm, int ty, int tx, float2 (&acc)[4][2]) {
 #pragma unroll 8
   for (int m = 0; m < 64; m++) {
     const float4 a = *reinterpret_cast<const float4 *>(&Lt[m * GJT + ty * 4]);
@@ -122,90 +73,204 @@ __device__ __forceinline__ float acc_at(const float2 (&acc)[4][2], int r, int c)
   return c < 2 ? (c == 0 ? acc[r][0].x : acc[r][0].y) : (c == 2 ? acc[r][1].x : acc[r][1].y);
 }
 
-// ---- k_gj_strips: CTA t takes index tile I = [64 t, 64 t + 64).  For
-// I != K: (a) rows I: Cs[I, :] = X_IK, X_IK = -(X_IK P); (b) columns I:
-// Rs[:, I] = P X_KI, X_KI = Rs[:, I].  For I = K: X_KK = P and Rs[:, K] = 0.
-// The tiles of different CTAs are disjoint, so no CTA reads what another
-// writes.  Columns k >= b of a partial last block are zero in Cs and Rs,
-// and so are the rows of K in Cs and the columns of K in Rs.
-__global__ void __launch_bounds__(256) k_gj_strips(float *__restrict__ X, size_t n, size_t k0, int b,
-                                                   const float *__restrict__ P, float *__restrict__ Cs,
-                                                   float *__restrict__ Rs) {
-  __shared__ __align__(16) float Lt[64 * GJT];
-  __shared__ __align__(16) float Rm[64 * GJT];
-  const size_t t = blockIdx.x, base = t * GJB;
-  const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-  if (base == k0) {
-    for (int q = threadIdx.x; q < GJB * GJB; q += 256) {
+// ---- k_gj_block: CTA t takes index tile I = [64 t, 64 t + 64): its rows in the
+// columns of K (X_IK, Cs) and its columns in the rows of K (X_KI, Rs).  Threads
+// 0..255 bring X_KK up to date (X_KK - Cs' Rs', the strips of the block before;
+// every CTA does, which costs less than waiting for one that would) and invert
+// it; meanwhile threads 256..511 bring the CTA's two tiles up to date; then all
+// form their products with P.  X_KK itself is read by every CTA and so not
+// written here: P goes to scratch, and the next launch (the CTA of that tile)
+// puts it in place.  A partial last block is padded with the identity; columns
+// k >= b are zero in Cs and Rs, and so are the rows of K in Cs and the columns
+// of K in Rs.
+//
+// The inversion: thread t holds 16 entries of row t / 4, columns 4 i + t % 4,
+// in registers, and two pivots go at a time: their rows to shared memory
+// (double-buffered, one barrier per pair), the 2 x 2 inverse by every thread;
+// every other row subtracts its entries in the pivot columns, times that
+// inverse, times the two rows.  The registers rotate by one place after four
+// pivots, so that a pivot's column is always the first: a loop of two pairs,
+// where 64 unrolled pivots were fetched from memory, instruction by
+// instruction (20 us).
+constexpr int GJ_THREADS = 512;
+struct GjSmem {
+  float lk[64 * GJT], rk[64 * GJT];  // Cs'_K transposed, Rs'_K
+  float lo[64 * GJT], ro[64 * GJT];  // Cs'_I transposed, Rs'_I
+  float ta[64 * GJT], tb[64 * GJT];  // X_IK transposed, X_KI
+  float p[64 * GJT], pt[64 * GJT];   // X_KK, then P; P transposed
+  float prow[2][2][4][20];           // two pivot rows, twice (20: distinct banks)
+};
+
+__global__ void __launch_bounds__(GJ_THREADS, 1)
+    k_gj_block(float *__restrict__ X, size_t n, size_t k0, int b, const float *__restrict__ Cp,
+               const float *__restrict__ Rp, const float *__restrict__ Pp, float *__restrict__ Cs,
+               float *__restrict__ Rs, float *__restrict__ P) {
+  extern __shared__ __align__(16) unsigned char gj_raw[];
+  GjSmem &S = *reinterpret_cast<GjSmem *>(gj_raw);
+  const size_t base = blockIdx.x * (size_t)GJB;
+  const bool diag = base == k0, first = k0 == 0;
+  const int t = threadIdx.x & 255, group = threadIdx.x >> 8, ty = t / 16, tx = t % 16;
+  const int have = (int)(n - base < (size_t)GJB ? n - base : (size_t)GJB);  // rows of I
+  // 64 rows of 64 transposed, 64 rows of Rs' from column c0 on
+  auto strip_t = [&](float *dst, size_t r0, int rows) {
+    const int r = t & 63, m0 = (t >> 6) * 16;
+    float4 v[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+      v[e] = r < rows ? *reinterpret_cast<const float4 *>(Cp + (r0 + r) * GJB + m0 + 4 * e)
+                      : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      float *d = dst + (m0 + 4 * e) * GJT + r;
+      d[0] = v[e].x;
+      d[GJT] = v[e].y;
+      d[2 * GJT] = v[e].z;
+      d[3 * GJT] = v[e].w;
+    }
+  };
+  auto strip = [&](float *dst, size_t c0, int cols) {
+    const int c = t & 63, m0 = (t >> 6) * 16;
+    float v[16];
+#pragma unroll
+    for (int e = 0; e < 16; e++) v[e] = c < cols ? Rp[(size_t)(m0 + e) * n + c0 + c] : 0.f;
+#pragma unroll
+    for (int e = 0; e < 16; e++) dst[(m0 + e) * GJT + c] = v[e];
+  };
+  // the thread's 4 x 4 entries of X from (r0, c0) on, 0 or `one` on the diagonal outside
+  auto tile = [&](float (&x)[16], size_t r0, int rows, size_t c0, int cols, float one) {
+#pragma unroll
+    for (int e = 0; e < 16; e++) {
+      const int r = ty * 4 + e / 4, c = tx * 4 + e % 4;
+      x[e] = r < rows && c < cols ? X[(r0 + r) * n + c0 + c] : (r == c ? one : 0.f);
+    }
+  };
+  auto minus = [&](float (&x)[16], const float *Lt, const float *Rm) {
+    float2 acc[4][2];
+#pragma unroll
+    for (int r = 0; r < 4; r++) acc[r][0] = acc[r][1] = make_float2(0.f, 0.f);
+    gj_mma(Lt, Rm, ty, tx, acc);
+#pragma unroll
+    for (int e = 0; e < 16; e++) x[e] -= acc_at(acc, e / 4, e % 4);
+  };
+  if (!first) {
+    if (group == 0) {
+      strip_t(S.lk, k0, b);
+      strip(S.rk, k0, b);
+    } else if (!diag) {
+      strip_t(S.lo, base, have);
+      strip(S.ro, base, have);
+    }
+  }
+  float xa[16], xb[16];
+  if (group == 0) {
+    tile(xa, k0, b, k0, b, 1.f);
+  } else if (!diag) {
+    tile(xa, base, have, k0, b, 0.f);
+    tile(xb, k0, b, base, have, 0.f);
+  }
+  __syncthreads();
+  if (group == 0) {
+    if (!first) minus(xa, S.lk, S.rk);
+#pragma unroll
+    for (int e = 0; e < 16; e++) S.p[(ty * 4 + e / 4) * GJT + tx * 4 + e % 4] = xa[e];
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    const int r = t >> 2, q = t & 3, at = (t & 31) & ~3;
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = S.p[r * GJT + 4 * i + q];
+#pragma unroll 1
+    for (int o = 0; o < 16; o++) {
+#pragma unroll
+      for (int s = 0; s < 4; s += 2) {
+        const int p = 4 * o + s;
+        const bool pivot = (r & ~1) == p;
+        auto &pr = S.prow[s >> 1];
+        const float f0 = __shfl_sync(0xffffffffu, v[0], at | s), f1 = __shfl_sync(0xffffffffu, v[0], at | s | 1);
+        if (pivot) {
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            reinterpret_cast<float4 *>(pr[r & 1][q])[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2],
+                                                                      v[4 * j + 3]);
+#pragma unroll
+          for (int i = 0; i < 16; i++) v[i] = 0.f;
+        }
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        const float a00 = pr[0][s][0], a01 = pr[0][s + 1][0], a10 = pr[1][s][0], a11 = pr[1][s + 1][0];
+        const float i0 = 1.0f / a00, l = a10 * i0, u = a01 * i0, i1 = 1.0f / (a11 - l * a01);
+        const float p01 = -u * i1, p10 = -l * i1, p00 = i0 + u * (l * i1);  // inverse of the two pivots' block
+        const float g0 = r == p ? p00 : r == p + 1 ? p10 : -(f0 * p00 + f1 * p10);
+        const float g1 = r == p ? p01 : r == p + 1 ? i1 : -(f0 * p01 + f1 * i1);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const float4 x = reinterpret_cast<const float4 *>(pr[0][q])[j];
+          const float4 y = reinterpret_cast<const float4 *>(pr[1][q])[j];
+          v[4 * j] = fmaf(g1, y.x, fmaf(g0, x.x, v[4 * j]));
+          v[4 * j + 1] = fmaf(g1, y.y, fmaf(g0, x.y, v[4 * j + 1]));
+          v[4 * j + 2] = fmaf(g1, y.z, fmaf(g0, x.z, v[4 * j + 2]));
+          v[4 * j + 3] = fmaf(g1, y.w, fmaf(g0, x.w, v[4 * j + 3]));
+        }
+        if (q == s) v[0] = g0;
+        if (q == s + 1) v[0] = g1;
+      }
+      const float head = v[0];
+#pragma unroll
+      for (int i = 0; i < 15; i++) v[i] = v[i + 1];
+      v[15] = head;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+      const int c = 4 * i + q;
+      S.p[r * GJT + c] = v[i];
+      S.pt[c * GJT + r] = v[i];
+      if (diag) P[r * GJB + c] = v[i];
+    }
+  } else if (!diag) {
+    if (!first) {
+      minus(xa, S.lo, S.rk);
+      minus(xb, S.lk, S.ro);
+    }
+#pragma unroll
+    for (int e = 0; e < 16; e++) {
+      const int r = ty * 4 + e / 4, c = tx * 4 + e % 4;
+      S.ta[c * GJT + r] = xa[e];
+      S.tb[r * GJT + c] = xb[e];
+      if (r < have) Cs[(base + r) * GJB + c] = xa[e];
+    }
+    if (base + GJB == k0)  // the block before, a full one
+      for (int q = t; q < GJB * GJB; q += 256) X[(base + q / GJB) * n + base + q % GJB] = Pp[q];
+  } else {
+    for (int q = t; q < GJB * GJB; q += 256) {
       const int r = q / GJB, c = q % GJB;
-      if (r < b && c < b) X[(k0 + r) * n + k0 + c] = P[q];
       if (c < b) Rs[(size_t)r * n + k0 + c] = 0.f;
       if (r < b) Cs[(k0 + r) * GJB + c] = 0.f;
     }
-    return;
   }
-  const int rows = (int)(n - base < (size_t)GJB ? n - base : (size_t)GJB);
+  __syncthreads();
+  if (diag) return;
+  // group 0: X_IK = -(X_IK P), group 1: X_KI = P X_KI
   float2 acc[4][2];
-  // (a) the rows of I in column block K (loads first, so that they overlap)
-  {
-    float xv[16], pv[16];
-#pragma unroll
-    for (int e = 0; e < 16; e++) {
-      const int q = threadIdx.x + e * 256, r = q / GJB, m = q % GJB;
-      xv[e] = (r < rows && m < b) ? X[(base + r) * n + k0 + m] : 0.f;
-      pv[e] = P[q];
-    }
-#pragma unroll
-    for (int e = 0; e < 16; e++) {
-      const int q = threadIdx.x + e * 256, r = q / GJB, m = q % GJB;
-      Lt[m * GJT + r] = xv[e];
-      if (r < rows) Cs[(base + r) * GJB + m] = xv[e];
-      Rm[r * GJT + m] = pv[e];
-    }
-  }
-  __syncthreads();
 #pragma unroll
   for (int r = 0; r < 4; r++) acc[r][0] = acc[r][1] = make_float2(0.f, 0.f);
-  gj_mma(Lt, Rm, acc);
+  gj_mma(group == 0 ? S.ta : S.pt, group == 0 ? S.p : S.tb, ty, tx, acc);
 #pragma unroll
   for (int r = 0; r < 4; r++)
 #pragma unroll
     for (int c = 0; c < 4; c++) {
       const int rr = ty * 4 + r, cc = tx * 4 + c;
-      if (rr < rows && cc < b) X[(base + rr) * n + k0 + cc] = -acc_at(acc, r, c);
-    }
-  __syncthreads();  // Lt and Rm are read again below
-  // (b) row block K in the columns of I
-  {
-    float xv[16], pv[16];
-#pragma unroll
-    for (int e = 0; e < 16; e++) {
-      const int q = threadIdx.x + e * 256, m = q / GJB, c = q % GJB;
-      xv[e] = (m < b && c < rows) ? X[(k0 + m) * n + base + c] : 0.f;
-      pv[e] = P[q];
-    }
-#pragma unroll
-    for (int e = 0; e < 16; e++) {
-      const int q = threadIdx.x + e * 256, m = q / GJB, c = q % GJB;
-      Lt[c * GJT + m] = pv[e];  // Lt[m'][r'] = P[r'][m']
-      Rm[m * GJT + c] = xv[e];
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < 4; r++) acc[r][0] = acc[r][1] = make_float2(0.f, 0.f);
-  gj_mma(Lt, Rm, acc);
-#pragma unroll
-  for (int r = 0; r < 4; r++)
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const int rr = ty * 4 + r, cc = tx * 4 + c;
-      if (cc < rows) {
-        const float v = acc_at(acc, r, c);
+      const float v = acc_at(acc, r, c);
+      if (group == 0) {
+        if (rr < have && cc < b) X[(base + rr) * n + k0 + cc] = -v;
+      } else if (cc < have) {
         Rs[(size_t)rr * n + base + cc] = v;  // rows rr >= b are zero (P is the identity there)
         if (rr < b) X[(k0 + rr) * n + base + cc] = v;
       }
     }
+}
+
+// the last block's P into place
+__global__ void k_gj_last(float *__restrict__ X, size_t n, size_t k0, int b, const float *__restrict__ P) {
+  for (int q = threadIdx.x; q < GJB * GJB; q += blockDim.x)
+    if (q / GJB < b && q % GJB < b) X[(k0 + q / GJB) * n + k0 + q % GJB] = P[q];
 }
 
 // ---- tensor-core helpers (tcgen05, tensor memory, mbarrier)
@@ -286,7 +351,8 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// ---- k_gj_update: X_ij -= sum_k Cs[i][k] Rs[k][j] for i, j outside K
+// ---- k_gj_update: X_ij -= sum_k Cs[i][k] Rs[k][j] for i, j outside K and the
+// next block K' = [k1, k1 + 64), which k_gj_block updates
 constexpr int TC_M = 128, TC_N = 128, TC_K = GJB;
 constexpr int TC_PROD_WARPS = 4, TC_CONS_WARPS = 8;
 constexpr int TC_THREADS = 32 * (TC_PROD_WARPS + TC_CONS_WARPS);
@@ -352,40 +418,10 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
       : "memory");
 }
 
-// The tiles one launch covers: every tile (GJ_ALL), the panel of the next
-// pivot block (GJ_PANEL: tile row tp and tile column tp, 2 nt - 1 tiles) or
-// the rest (GJ_REST: (nt - 1)^2 tiles); gj_tile maps a launch's tile number
-// to its tile row and column.
-enum GjTiles { GJ_ALL = 0, GJ_PANEL = 1, GJ_REST = 2 };
-
-__host__ __device__ inline size_t gj_tile_count(int mode, size_t nt) {
-  return mode == GJ_ALL ? nt * nt : mode == GJ_PANEL ? 2 * nt - 1 : (nt - 1) * (nt - 1);
-}
-
-__device__ __forceinline__ void gj_tile(int mode, size_t nt, size_t tp, size_t u, size_t &tr, size_t &tc) {
-  if (mode == GJ_ALL) {
-    tr = u / nt;
-    tc = u % nt;
-  } else if (mode == GJ_PANEL) {
-    if (u < nt) {
-      tr = tp;
-      tc = u;
-    } else {
-      const size_t w = u - nt;
-      tr = w < tp ? w : w + 1;
-      tc = tp;
-    }
-  } else {
-    const size_t a = u / (nt - 1), b = u % (nt - 1);
-    tr = a < tp ? a : a + 1;
-    tc = b < tp ? b : b + 1;
-  }
-}
-
 // Persistent and warp-specialised: CTA c of G takes the tiles
-// [c T / G, (c + 1) T / G) of the T tiles of its tile set (128 x 128 each,
-// row-major within the set, so that a CTA mostly stays in one tile row and
-// stages the A operand, rows of Cs, once per row).  The CTA's tile number
+// [c T / G, (c + 1) T / G) of the T tiles (128 x 128 each, row-major, so that
+// a CTA mostly stays in one tile row and stages the A operand, rows of Cs, once
+// per row).  The CTA's tile number
 // lt picks the B stage and the accumulator buffer (lt & 1).
 //   producers (warps 0-3): stage B[c][k] = Rs[k][j0 + c] (and A[r][k] =
 //     Cs[i0 + r][k] when the row changes) split into hi and lo, K-major;
@@ -400,9 +436,9 @@ __device__ __forceinline__ void gj_tile(int mode, size_t nt, size_t tp, size_t u
 // raised, both roles stop, and the tensor memory is freed after a last
 // bounded wait.
 __global__ void __launch_bounds__(TC_THREADS, 1) k_gj_update(float *__restrict__ X, size_t n, size_t k0,
-                                                             const float *__restrict__ Cs,
-                                                             const float *__restrict__ Rs, size_t nt, int mode,
-                                                             size_t tp, uint32_t *__restrict__ flags) {
+                                                             size_t k1, const float *__restrict__ Cs,
+                                                             const float *__restrict__ Rs, size_t nt,
+                                                             uint32_t *__restrict__ flags) {
   extern __shared__ __align__(1024) unsigned char tsm[];
   unsigned char *Ahi = tsm, *Alo = tsm + TC_OPER;
   unsigned char *Bst = tsm + 2 * TC_OPER;  // stage s: hi at Bst + 2 s TC_OPER, lo after it
@@ -411,7 +447,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gj_update(float *__restrict__
   uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 4);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(bar + 5);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const size_t ntile = gj_tile_count(mode, nt), G = gridDim.x;
+  const size_t ntile = nt * nt, G = gridDim.x;
   const size_t t_begin = blockIdx.x * ntile / G, t_end = (blockIdx.x + 1) * ntile / G;
   const size_t L = t_end - t_begin;
 
@@ -442,8 +478,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gj_update(float *__restrict__
     // ---- producers
     size_t a_row = ~(size_t)0;
     for (size_t lt = 0; lt < L; lt++) {
-      size_t tr, tc;
-      gj_tile(mode, nt, tp, t_begin + lt, tr, tc);
+      const size_t tr = (t_begin + lt) / nt, tc = (t_begin + lt) % nt;
       const size_t i0 = tr * TC_M, j0 = tc * TC_N;
       const int st = (int)(lt & 1);
       unsigned char *Bhi = Bst + 2 * st * TC_OPER, *Blo = Bhi + TC_OPER;
@@ -531,8 +566,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gj_update(float *__restrict__
         break;
       }
       tc_fence_after();
-      size_t tr, tc;
-      gj_tile(mode, nt, tp, t_begin + lt, tr, tc);
+      const size_t tr = (t_begin + lt) / nt, tc = (t_begin + lt) % nt;
       const size_t i0 = tr * TC_M, j0 = tc * TC_N;
       const uint32_t tbase = tmem + (uint32_t)st * TC_N + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * 64);
       // chunk 0 into the transpose scratch, chunk 1 held in registers; then
@@ -553,17 +587,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gj_update(float *__restrict__
           __syncwarp();
         }
         const size_t j = j0 + (size_t)(half * 64 + ch * 32 + lane);
-        const bool jok = j < n && (j < k0 || j >= k0 + GJB);
+        // outside K and K': unsigned differences, so that one comparison does
+        const bool jok = j < n && j - k0 >= (size_t)GJB && j - k1 >= (size_t)GJB;
         float xv[32];
 #pragma unroll
         for (int rr = 0; rr < 32; rr++) {
           const size_t i = i0 + (size_t)(q * 32 + rr);
-          xv[rr] = (jok && i < n && (i < k0 || i >= k0 + GJB)) ? X[i * n + j] : 0.f;
+          xv[rr] = (jok && i < n && i - k0 >= (size_t)GJB && i - k1 >= (size_t)GJB) ? X[i * n + j] : 0.f;
         }
 #pragma unroll
         for (int rr = 0; rr < 32; rr++) {
           const size_t i = i0 + (size_t)(q * 32 + rr);
-          if (jok && i < n && (i < k0 || i >= k0 + GJB)) X[i * n + j] = xv[rr] - T[rr * TC_TSTRIDE + lane];
+          if (jok && i < n && i - k0 >= (size_t)GJB && i - k1 >= (size_t)GJB)
+            X[i * n + j] = xv[rr] - T[rr * TC_TSTRIDE + lane];
         }
         __syncwarp();
       }
@@ -583,14 +619,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_gj_update(float *__restrict__
 
 }  // namespace
 
-// The host loop overlaps each block's serial part with the previous
-// block's update: the update of block k first covers the panel of block
-// k + 1 (its tile row and column); a side stream then runs k_gj_diag and
-// k_gj_strips for block k + 1 (they read and write only rows and columns
-// of block k + 1, final after the panel) while the main stream updates the
-// remaining tiles of block k.  The strips and P alternate between two
-// buffers; the main stream waits for block k + 1's strips before its
-// update.
+// k_gj_block of block k + 1 needs the strips of block k and the updates up to
+// block k - 1, and runs beside the update of block k: on the side stream, which
+// waits for the update before; the main stream waits for the strips.  Strips
+// and P alternate between two buffers.
 void coarse_inverse(Context &ctx, float *X, size_t n) {
   if (n == 0) return;
   cudaStream_t s = ctx.stream;
@@ -598,48 +630,45 @@ void coarse_inverse(Context &ctx, float *X, size_t n) {
   const size_t nb = (n + GJB - 1) / GJB, nt = (n + TC_M - 1) / TC_M;
   DBuf<float> P(2 * GJB * GJB, s), Cs(2 * n * GJB, s), Rs(2 * GJB * n, s);
   ensure_smem_attr(ctx, k_gj_update, TC_SMEM);
+  ensure_smem_attr(ctx, k_gj_block, (int)sizeof(GjSmem));
   if (!ctx.side) {
     DG_CUDA(cudaStreamCreateWithFlags(&ctx.side, cudaStreamNonBlocking));
     DG_CUDA(cudaEventCreateWithFlags(&ctx.side_ev[0], cudaEventDisableTiming));
     DG_CUDA(cudaEventCreateWithFlags(&ctx.side_ev[1], cudaEventDisableTiming));
   }
   cudaStream_t side = ctx.side;
-  cudaEvent_t ev_panel = ctx.side_ev[0], ev_strips = ctx.side_ev[1];
-  auto blk = [&](size_t k, cudaStream_t st) {  // diag + strips of block k into buffer k & 1
-    const size_t k0 = k * GJB, o = k & 1;
+  cudaEvent_t ev_block = ctx.side_ev[0], ev_update = ctx.side_ev[1];
+  auto block = [&](size_t k) {
+    const size_t k0 = k * GJB, o = k & 1, q = o ^ 1;
     const int b = (int)std::min<size_t>(GJB, n - k0);
-    k_gj_diag<<<1, 256, 0, st>>>(X, n, k0, b, P.get() + o * GJB * GJB);
-    k_gj_strips<<<(unsigned)nb, 256, 0, st>>>(X, n, k0, b, P.get() + o * GJB * GJB, Cs.get() + o * n * GJB,
-                                             Rs.get() + o * GJB * n);
-  };
-  // an update CTA fills its SM (shared memory), so the update of the
-  // remaining tiles leaves some SMs to the side stream's diag and strips
-  const size_t side_sms = std::min<size_t>(16, (size_t)ctx.num_sms / 8);
-  auto update = [&](size_t k, int mode, size_t tp) {
-    const size_t o = k & 1, cnt = gj_tile_count(mode, nt);
-    if (cnt == 0) return;
-    const size_t sms = mode == GJ_REST ? (size_t)ctx.num_sms - side_sms : (size_t)ctx.num_sms;
-    const unsigned grid = (unsigned)std::min<size_t>(cnt, sms);
-    k_gj_update<<<grid, TC_THREADS, TC_SMEM, s>>>(X, n, k * GJB, Cs.get() + o * n * GJB, Rs.get() + o * GJB * n,
-                                                  nt, mode, tp, ctx.d_flags);
-  };
-  try {
-    blk(0, s);
-    for (size_t k = 0; k < nb; k++) {
-      if (k + 1 < nb) {
-        const size_t tp = (k + 1) * GJB / TC_M;
-        update(k, GJ_PANEL, tp);
-        DG_CUDA(cudaEventRecord(ev_panel, s));
-        DG_CUDA(cudaStreamWaitEvent(side, ev_panel, 0));
-        blk(k + 1, side);
-        DG_CUDA(cudaEventRecord(ev_strips, side));
-        update(k, GJ_REST, tp);
-        DG_CUDA(cudaStreamWaitEvent(s, ev_strips, 0));
-      } else {
-        update(k, GJ_ALL, 0);
-      }
-    }
+    k_gj_block<<<(unsigned)nb, GJ_THREADS, sizeof(GjSmem), side>>>(
+        X, n, k0, b, Cs.get() + q * n * GJB, Rs.get() + q * GJB * n, P.get() + q * GJB * GJB, Cs.get() + o * n * GJB,
+        Rs.get() + o * GJB * n, P.get() + o * GJB * GJB);
     DG_LAUNCH_CHECK();
+    DG_CUDA(cudaEventRecord(ev_block, side));
+  };
+  // an update CTA fills its SM (shared memory), one of k_gj_block most of one
+  const size_t side_sms = std::min<size_t>(nb, (size_t)ctx.num_sms / 4);
+  const unsigned grid = (unsigned)std::min<size_t>(nt * nt, (size_t)ctx.num_sms - side_sms);
+  DG_CUDA(cudaEventRecord(ev_update, s));
+  try {
+    DG_CUDA(cudaStreamWaitEvent(side, ev_update, 0));
+    block(0);
+    for (size_t k = 0; k < nb; k++) {
+      DG_CUDA(cudaStreamWaitEvent(s, ev_block, 0));
+      if (k + 1 < nb) {
+        DG_CUDA(cudaStreamWaitEvent(side, ev_update, 0));  // of block k - 1
+        block(k + 1);
+      } else {
+        k_gj_last<<<1, 256, 0, s>>>(X, n, k * GJB, (int)(n - k * GJB), P.get() + (k & 1) * GJB * GJB);
+        DG_LAUNCH_CHECK();
+      }
+      const size_t o = k & 1;
+      k_gj_update<<<grid, TC_THREADS, TC_SMEM, s>>>(X, n, k * GJB, k + 1 < nb ? (k + 1) * GJB : n,
+                                                    Cs.get() + o * n * GJB, Rs.get() + o * GJB * n, nt, ctx.d_flags);
+      DG_LAUNCH_CHECK();
+      DG_CUDA(cudaEventRecord(ev_update, s));
+    }
   } catch (...) {
     cudaStreamSynchronize(side);  // the scratch buffers are freed on the main stream
     throw;
