@@ -1229,9 +1229,21 @@ static unsigned patch_grid(Context &ctx, F *kernel, size_t smem, size_t n_patch)
   return (unsigned)std::min<size_t>(n_patch, (size_t)std::max(per_sm, 1) * ctx.num_sms);
 }
 
+template <typename T, bool DIR>
+static bool elem_matvec(Context &ctx, const Mesh &m, const uint8_t *bdy, const T *x, T *y, double lap_fac,
+                        double mass_fac, const char *name, double bytes) {
+  if (!m.conn || m.n_elem > elem_wise_max<T> || (DIR && !bdy)) return false;
+  ProfScope _prof(ctx, name, bytes);
+  k_elem_matvec<T, DIR><<<grid_for(m.n_elem, 128), 128, 0, ctx.stream>>>(m.meta, m.conn, m.n_elem, bdy, (T)lap_fac,
+                                                                         (T)mass_fac, x, y);
+  DG_LAUNCH_CHECK();
+  return true;
+}
+
 template <bool DIR>
-void launch_family_matvec(Context &ctx, const Mesh &m, const float *x, float *y, double lap_fac, double mass_fac,
-                          const char *name, double bytes) {
+void launch_matvec(Context &ctx, const Mesh &m, const uint8_t *bdy, const float *x, float *y, double lap_fac,
+                          double mass_fac, const char *name, double bytes) {
+  if (elem_matvec<float, DIR>(ctx, m, bdy, x, y, lap_fac, mass_fac, name, bytes)) return;
   const size_t smem = family_smem<float>(m.max_run);
   const unsigned grid = patch_grid(ctx, k_family_matvec<float, DIR, false>, smem, m.n_patch);
   const float *dtab = diag_table<float>(ctx, lap_fac, mass_fac);
@@ -1242,8 +1254,9 @@ void launch_family_matvec(Context &ctx, const Mesh &m, const float *x, float *y,
 }
 
 template <bool DIR>
-void launch_family_matvec(Context &ctx, const Mesh &m, const double *x, double *y, double lap_fac, double mass_fac,
-                          const char *name, double bytes) {
+void launch_matvec(Context &ctx, const Mesh &m, const uint8_t *bdy, const double *x, double *y,
+                          double lap_fac, double mass_fac, const char *name, double bytes) {
+  if (elem_matvec<double, DIR>(ctx, m, bdy, x, y, lap_fac, mass_fac, name, bytes)) return;
   const size_t smem = family_fix_smem(m.max_run);
   const unsigned grid = patch_grid(ctx, k_family_matvec_fix<DIR>, smem, m.n_patch);
   const double *dtab = diag_table<double>(ctx, lap_fac, mass_fac);
@@ -1253,15 +1266,15 @@ void launch_family_matvec(Context &ctx, const Mesh &m, const double *x, double *
                                                             x, y);
   DG_LAUNCH_CHECK();
 }
-template void launch_family_matvec<true>(Context &, const Mesh &, const float *, float *, double, double, const char *,
-                                         double);
-template void launch_family_matvec<true>(Context &, const Mesh &, const double *, double *, double, double,
-                                         const char *, double);
+template void launch_matvec<true>(Context &, const Mesh &, const uint8_t *, const float *, float *, double,
+                                         double, const char *, double);
+template void launch_matvec<true>(Context &, const Mesh &, const uint8_t *, const double *, double *, double,
+                                         double, const char *, double);
 
 template <typename T>
 void mesh_matvec(Context &ctx, const Mesh &m, const T *x, T *y, double lap_fac, double mass_fac) {
   DG_CUDA(cudaMemsetAsync(y, 0, m.n_node * sizeof(T), ctx.stream));
-  launch_family_matvec<false>(ctx, m, x, y, lap_fac, mass_fac, sizeof(T) == 4 ? "matvec_fp32" : "matvec_fp64",
+  launch_matvec<false>(ctx, m, nullptr, x, y, lap_fac, mass_fac, sizeof(T) == 4 ? "matvec_fp32" : "matvec_fp64",
                               (double)m.n_elem * 36 + (double)m.n_node * 3 * sizeof(T));
 }
 template void mesh_matvec<float>(Context &, const Mesh &, const float *, float *, double, double);

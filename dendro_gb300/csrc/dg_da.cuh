@@ -112,13 +112,13 @@ constexpr int STEN_ENTRIES = 8 * 18 * 128;
 void ensure_stencils(Context &ctx);
 
 // the element loop on a zeroed y; DIR: the Dirichlet form (boundary rows and
-// columns from the run words' boundary flag)
+// columns; bdy flags the boundary nodes)
 template <bool DIR>
-void launch_family_matvec(Context &ctx, const Mesh &m, const float *x, float *y, double lap_fac, double mass_fac,
-                          const char *name, double bytes);
+void launch_matvec(Context &ctx, const Mesh &m, const uint8_t *bdy, const float *x, float *y, double lap_fac,
+                   double mass_fac, const char *name, double bytes);
 template <bool DIR>
-void launch_family_matvec(Context &ctx, const Mesh &m, const double *x, double *y, double lap_fac, double mass_fac,
-                          const char *name, double bytes);
+void launch_matvec(Context &ctx, const Mesh &m, const uint8_t *bdy, const double *x, double *y, double lap_fac,
+                   double mass_fac, const char *name, double bytes);
 
 // host-side generators (same mathematics as the reference's .inp tables)
 void gen_etype_masks(uint8_t masks[8 * 18]);

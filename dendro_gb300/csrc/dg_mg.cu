@@ -423,7 +423,7 @@ template <typename T>
 void dirichlet_matvec(Context &ctx, const MGLevel &L, const T *x, T *y) {
   const Mesh &m = L.mesh;
   DG_CUDA(cudaMemsetAsync(y, 0, m.n_node * sizeof(T), ctx.stream));
-  launch_family_matvec<true>(ctx, m, x, y, 1.0, 1.0,
+  launch_matvec<true>(ctx, m, L.bdy, x, y, 1.0, 1.0,
                              sizeof(T) == 4 ? "dirichlet_matvec_fp32" : "dirichlet_matvec_fp64",
                              (double)m.n_elem * 36 + (double)m.n_node * (3 * sizeof(T) + 1));
 }
@@ -837,7 +837,7 @@ void mg_solve(Context &ctx, MG &mg, const double *b, double *x, int precision, d
 void dirichlet_matvec_ds(Context &ctx, const MGLevel &L, const double *x, double *y) {
   const Mesh &m = L.mesh;
   DG_CUDA(cudaMemsetAsync(y, 0, m.n_node * sizeof(double), ctx.stream));
-  launch_family_matvec<true>(ctx, m, x, y, 1.0, 1.0, "dirichlet_matvec_ds",
+  launch_matvec<true>(ctx, m, L.bdy, x, y, 1.0, 1.0, "dirichlet_matvec_ds",
                              (double)m.n_elem * 36 + (double)m.n_node * (3 * sizeof(double) + 1));
 }
 
