@@ -1244,12 +1244,12 @@ template <bool DIR>
 void launch_matvec(Context &ctx, const Mesh &m, const uint8_t *bdy, const float *x, float *y, double lap_fac,
                           double mass_fac, const char *name, double bytes) {
   if (elem_matvec<float, DIR>(ctx, m, bdy, x, y, lap_fac, mass_fac, name, bytes)) return;
-  const size_t smem = family_smem<float>(m.max_run);
-  const unsigned grid = patch_grid(ctx, k_family_matvec<float, DIR, false>, smem, m.n_patch);
+  const size_t smem = family_smem(m.max_run);
+  const unsigned grid = patch_grid(ctx, k_family_matvec<DIR>, smem, m.n_patch);
   const float *dtab = diag_table<float>(ctx, lap_fac, mass_fac);
   ProfScope _prof(ctx, name, bytes);
-  k_family_matvec<float, DIR, false><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch,
-                                                                      m.max_run, dtab, x, y, nullptr, nullptr);
+  k_family_matvec<DIR><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch, m.max_run, dtab,
+                                                        x, y);
   DG_LAUNCH_CHECK();
 }
 
@@ -1283,12 +1283,12 @@ template void mesh_matvec<double>(Context &, const Mesh &, const double *, doubl
 template <typename T>
 void mesh_matvec_coef(Context &ctx, const Mesh &m, const double *coef, const T *x, T *y) {
   DG_CUDA(cudaMemsetAsync(y, 0, m.n_node * sizeof(T), ctx.stream));
-  const size_t smem = family_smem<T>(m.max_run);
-  const unsigned grid = patch_grid(ctx, k_family_matvec<T, false, true>, smem, m.n_patch);
+  const size_t smem = family_coef_smem<T>(m.max_run);
+  const unsigned grid = patch_grid(ctx, k_family_coef<T>, smem, m.n_patch);
   ProfScope _prof(ctx, sizeof(T) == 4 ? "matvec_coef_fp32" : "matvec_coef_fp64",
                   (double)m.n_elem * (36 + 16 + 2) + (double)m.n_node * 3 * sizeof(T));
-  k_family_matvec<T, false, true><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch,
-                                                                   m.max_run, nullptr, x, y, coef, m.fchild);
+  k_family_coef<T><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch, m.max_run, x, y, coef,
+                                                    m.fchild);
   DG_LAUNCH_CHECK();
 }
 template void mesh_matvec_coef<float>(Context &, const Mesh &, const double *, const float *, float *);

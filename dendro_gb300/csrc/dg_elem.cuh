@@ -27,13 +27,11 @@
 // elements, where 8 dense 8x8 stencils cost 512 multiply-adds.  A family with
 // subdivided children is applied element by element: 397 operations.
 //
-// What bounds it (1.1e7 elements of a Gaussian cloud, GB300): FP32 143 us,
-// instruction issue and the latency of the gathers (DRAM traffic alone would
-// take 34 us; without the shared-memory atomics 116 us, without the x gather
-// 124 us); FP64 vectors 350 us, integer instructions (further down).  An
-// element-wise loop over dense stencils, 8 gathers and 8 atomics per element,
-// took 348 and 1,820 us.  128 families per patch: 64 and 256 measured 152 / 150
-// us in FP32; a patch of 256 leaves too few blocks on small meshes.
+// On 1.1e7 elements of a Gaussian cloud (GB300) FP32 takes 109 us and FP64
+// vectors 350 us; what bounds them stands at the kernels.  An element-wise loop
+// over dense stencils, 8 gathers and 8 atomics per element, took 348 and 1,820
+// us.  128 families per patch: 64 and 256 measured 152 / 150 us where 128 took
+// 143 (FP32); a patch of 256 leaves too few blocks on small meshes.
 //
 // Patches: FAM consecutive families (in element order) make a patch, one
 // thread block's work at a time.  fam[(p * 4 + w) * FAM + t] is word w of the
@@ -358,32 +356,123 @@ __device__ __forceinline__ void family_floating(const uint4 (&w)[4], size_t f, c
   }
 }
 
-// One block per patch, grid-strided, three barriers per patch:
-//   1. x of the patch's nodes into xs (node ids read coalesced), ys = 0;
+// FP32: one block per patch, grid-strided, the next patch's x on its way while
+// this one is applied.  Per patch, two barriers:
+//   1. wait for x of this patch's nodes (and the words of the next one's), then
+//      start copying the next one's x into the other buffer (cp.async; boundary
+//      columns of the Dirichlet form are filled with zeros);
 //   2. thread t = family t: its lattice from xs, its elements in registers,
 //      its lattice added into ys with shared-memory atomics;
-//   3. each node's sum stored (nodes of this patch alone) or added to y.
+//   3. each node's sum stored (nodes of this patch alone) or added to y, and ys
+//      left zero; the first 8 words per thread are loaded before the barrier.
 // DIR, the Dirichlet form: boundary rows are the identity (y = x), boundary
 // columns are dropped.
-// Blocks per SM (registers): FP32 at 4 to 8 blocks 158, 152, 143, 145, 151 us on
-// 1.1e7 elements.
-template <typename T, bool DIR, bool COEF>
-__global__ void __launch_bounds__(FAM, sizeof(T) == 4 ? 6 : 3)
+//
+// 1.1e7 elements: 109 us.  With x gathered after each barrier 142 us (warps
+// waited 6.6 of 15.2 cycles per instruction for it), with the copies but the
+// words of step 3 loaded in step 3 118 us.  The shared-memory and load/store
+// pipe is two thirds busy; DRAM traffic alone would take 34.  Blocks per SM
+// (registers, shared memory): 3, 4, 5, 6 took 165, 135, 121, 118 us; 12 words
+// ahead 112, 4 words 115.
+__device__ __forceinline__ void async_word(void *dst, const void *src, bool zero) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(zero ? 0 : 4)
+               : "memory");
+}
+__device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ size_t run_base(uint4 info) { return (size_t)info.x | (size_t)info.y << 32; }
+
+template <bool DIR>
+__global__ void __launch_bounds__(FAM, 6)
     k_family_matvec(const uint4 *__restrict__ fam, const uint32_t *__restrict__ prun, const uint4 *__restrict__ pinfo,
-                    size_t n_fam, size_t n_patch, int max_run, const T *__restrict__ dtab, const T *__restrict__ x,
-                    T *__restrict__ y, const double *__restrict__ coef, const uint32_t *__restrict__ fchild) {
+                    size_t n_fam, size_t n_patch, int max_run, const float *__restrict__ dtab,
+                    const float *__restrict__ x, float *__restrict__ y) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float *xs = reinterpret_cast<float *>(smem_raw);  // two buffers
+  float *ys = xs + 2 * (max_run + 1);
+  uint32_t *ids = reinterpret_cast<uint32_t *>(ys + (max_run + 1));  // words of the next patch (a thread reads its own)
+  float *dt = reinterpret_cast<float *>(ids + (max_run + 1));
+  const int tid = threadIdx.x;
+  const uint4 none = make_uint4(0, 0, 0, 0);
+  for (int i = tid; i < DTAB_ENTRIES; i += FAM) dt[i] = dtab[i];
+  for (int i = tid; i <= max_run; i += FAM) ys[i] = 0.f;
+  if (tid == 0) xs[0] = xs[max_run + 1] = 0.f;
+  auto copy_ids = [&](uint4 info) {
+    const uint32_t *src = prun + run_base(info);
+    for (int u = tid; u < (int)info.z; u += FAM) async_word(ids + u, src + u, false);
+  };
+  auto copy_x = [&](uint4 info, int par) {
+    float *dst = xs + par * (max_run + 1) + 1;
+    for (int u = tid; u < (int)info.z; u += FAM) {
+      const uint32_t r = ids[u];
+      async_word(dst + u, x + (r & PRUN_NODE), DIR && (r & PRUN_BDY));
+    }
+  };
+  uint4 w[4];
+  auto load_w = [&](size_t p) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) w[q] = p * FAM + tid < n_fam ? fam[(p * 4 + q) * FAM + tid] : none;
+  };
+  const size_t G = gridDim.x;
+  size_t p = blockIdx.x;
+  uint4 info = p < n_patch ? pinfo[p] : none, next = p + G < n_patch ? pinfo[p + G] : none;
+  copy_ids(info);
+  async_wait();
+  copy_x(info, 0);
+  copy_ids(next);
+  load_w(p);
+  for (int par = 0; p < n_patch; p += G, par ^= 1) {
+    const uint4 after = p + 2 * G < n_patch ? pinfo[p + 2 * G] : none;
+    async_wait();
+    __syncthreads();  // x of this patch is there, ys is zero, the other buffer is free
+    copy_x(next, par ^ 1);
+    copy_ids(after);
+    if (p * FAM + tid < n_fam)
+      family_floating<float, false>(w, p * FAM + tid, xs + par * (max_run + 1), ys, dt, nullptr, nullptr);
+    const uint32_t *run = prun + run_base(info);
+    const int nr = (int)info.z;
+    constexpr int AHEAD = 8;
+    uint32_t r0[AHEAD];
+#pragma unroll
+    for (int k = 0; k < AHEAD; k++) r0[k] = tid + k * FAM < nr ? run[tid + k * FAM] : 0u;
+    load_w(p + G);
+    __syncthreads();
+    auto put = [&](int u, uint32_t r) {
+      const uint32_t g = r & PRUN_NODE;
+      const float v = ys[u + 1];
+      ys[u + 1] = 0.f;
+      if (DIR && (r & PRUN_BDY)) y[g] = x[g];
+      else if (r & PRUN_COMPLETE) y[g] = v;
+      else atomicAdd(&y[g], v);
+    };
+#pragma unroll
+    for (int k = 0; k < AHEAD; k++)
+      if (tid + k * FAM < nr) put(tid + k * FAM, r0[k]);
+#pragma unroll 2
+    for (int u = tid + AHEAD * FAM; u < nr; u += FAM) put(u, run[u]);
+    info = next;
+    next = after;
+  }
+}
+
+inline size_t family_smem(int max_run) { return (4 * (size_t)(max_run + 1) + DTAB_ENTRIES) * 4; }
+
+// Elements with factors of their own (FP32 and FP64): as above without the
+// copies ahead.
+template <typename T>
+__global__ void __launch_bounds__(FAM, sizeof(T) == 4 ? 6 : 3)
+    k_family_coef(const uint4 *__restrict__ fam, const uint32_t *__restrict__ prun, const uint4 *__restrict__ pinfo,
+                  size_t n_fam, size_t n_patch, int max_run, const T *__restrict__ x, T *__restrict__ y,
+                  const double *__restrict__ coef, const uint32_t *__restrict__ fchild) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *xs = reinterpret_cast<T *>(smem_raw);
   T *ys = xs + (max_run + 1);
-  T *dt = ys + (max_run + 1);
   const int tid = threadIdx.x;
-  if (!COEF)
-    for (int i = tid; i < DTAB_ENTRIES; i += FAM) dt[i] = dtab[i];
   if (tid == 0) xs[0] = (T)0;
   for (size_t p = blockIdx.x; p < n_patch; p += gridDim.x) {
     const bool have = p * FAM + tid < n_fam;
     const uint4 info = pinfo[p];
-    const size_t base = (size_t)info.x | (size_t)info.y << 32;
+    const size_t base = run_base(info);
     const int nr = (int)info.z;
     uint4 w[4];
 #pragma unroll
@@ -391,26 +480,24 @@ __global__ void __launch_bounds__(FAM, sizeof(T) == 4 ? 6 : 3)
     __syncthreads();  // the previous patch is done with xs and ys
 #pragma unroll 4
     for (int u = tid; u < nr; u += FAM) {
-      const uint32_t r = prun[base + u];
-      xs[u + 1] = (DIR && (r & PRUN_BDY)) ? (T)0 : x[r & PRUN_NODE];
+      xs[u + 1] = x[prun[base + u] & PRUN_NODE];
       ys[u + 1] = (T)0;
     }
     __syncthreads();
-    if (have) family_floating<T, COEF>(w, p * FAM + tid, xs, ys, dt, coef, fchild);
+    if (have) family_floating<T, true>(w, p * FAM + tid, xs, ys, nullptr, coef, fchild);
     __syncthreads();
 #pragma unroll 4
     for (int u = tid; u < nr; u += FAM) {
       const uint32_t r = prun[base + u], g = r & PRUN_NODE;
-      if (DIR && (r & PRUN_BDY)) y[g] = x[g];
-      else if (r & PRUN_COMPLETE) y[g] = ys[u + 1];
+      if (r & PRUN_COMPLETE) y[g] = ys[u + 1];
       else atomicAdd(&y[g], ys[u + 1]);
     }
   }
 }
 
 template <typename T>
-inline size_t family_smem(int max_run) {
-  return (2 * (size_t)(max_run + 1) + DTAB_ENTRIES) * sizeof(T);
+inline size_t family_coef_smem(int max_run) {
+  return 2 * (size_t)(max_run + 1) * sizeof(T);
 }
 
 // ---- FP64 vectors ----
@@ -551,7 +638,7 @@ __global__ void __launch_bounds__(FAM, 4)
   for (size_t p = blockIdx.x; p < n_patch; p += gridDim.x) {
     const bool have = p * FAM + tid < n_fam;
     const uint4 info = pinfo[p];
-    const size_t base = (size_t)info.x | (size_t)info.y << 32;
+    const size_t base = run_base(info);
     const int nr = (int)info.z;
     uint4 w[4];
 #pragma unroll

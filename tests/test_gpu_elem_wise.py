@@ -10,7 +10,7 @@ roundings)."""
 import numpy as np
 import pytest
 
-from dendro_gb300 import DA, MultiGrid, Octree
+from dendro_gb300 import DA, MultiGrid, Octree, balanceOctree, datagen, points2Octree
 from .test_gpu_families import DEPTH, _perm, _tree
 
 pytestmark = pytest.mark.gpu
@@ -39,3 +39,21 @@ def test_both_sides_of_the_limits(ctx, oracle, level, split):
     assert np.abs(mg.matvec(0, xg)[p] - want).max() <= 1e-12 * np.abs(want).max()
     got = mg.matvec(0, xg.astype(np.float32), precision=32)[p]
     assert np.linalg.norm(got - want) <= 1e-6 * np.linalg.norm(want)
+
+
+def test_blocks_that_take_several_patches(ctx, oracle):
+    """More patches than blocks fit the chip (a patch is 128 families): the
+    copies ahead run from patch to patch, over the last one's end."""
+    rng = np.random.Generator(np.random.PCG64(4))
+    bal = balanceOctree(points2Octree(datagen.mixture(400_000, rng), ctx=ctx))
+    da, oda = DA(bal), oracle.DA(bal.to_numpy(), DEPTH)
+    assert da.n_elem > 7 * 128 * 1500
+    p = _perm(da.download()["node_xyz"], oda.node_xyz)
+    x = rng.uniform(-1, 1, oda.n_node)
+    xg = np.empty_like(x)
+    xg[p] = x
+    mg = MultiGrid(bal)
+    for want, apply in ((oda.matvec(x), lambda v, q: da.matvec(v, precision=q)),
+                        (oda.dirichlet_matvec(x), lambda v, q: mg.matvec(0, v, precision=q))):
+        assert np.abs(apply(xg, 64)[p] - want).max() <= 1e-12 * np.abs(want).max()
+        assert np.linalg.norm(apply(xg.astype(np.float32), 32)[p] - want) <= 1e-6 * np.linalg.norm(want)
