@@ -526,14 +526,17 @@ inline size_t family_coef_smem(int max_run) {
 // 7.0e-15), one node 7.9e-17 (5.1e-17, 2.2e-17).
 // Patches outside that range take floating point, all of it: values that are
 // not finite or not within 2^-511 .. 2^511, factors beyond 2^+-400, and
-// families with subdivided children where a child's values all lie below 2^-4
-// of the family's (those are applied child by child in FP64, so a child's
-// rows would be as exact as its own values there).
+// families with subdivided children where a child's values, not all zero, lie
+// below 2^-8 of the family's: FP64 applies those child by child, and the rows
+// that only such a child touches would be less exact here (a bound of 2^-4
+// sent some patches at the domain's corners there in every solve: FP64 solve of
+// 5e5 points 9.37 -> 10.3 ms).
 // What bounds it: 350 us on 1.1e7 elements (DRAM traffic alone 50): 3,500
 // instructions per 32 families at 1.5 per clock per SM; warps wait for the
 // gathers (3.0 of 10.5 cycles per instruction), barriers (1.6) and
 // instructions (1.5: the code is long, so loops over nodes unroll no further
-// than they must: 4 and 1 times 350 us, 4 and 4 359, 8 and 8 405).  Blocks per
+// than they must: by 4 and 1 350 us, 4 and 4 359, 8 and 8 405).  Copying the next
+// patch's x ahead gains 3% here and loses as much on half as many elements.  Blocks per
 // SM: at 3, 4, 5, 6 451, 387, 411, 480 us.  Small meshes are bound by latency
 // (2e4 elements 16 us).
 // x as one word: its 53-bit mantissa, signed, above a 10-bit exponent (0: zero)
@@ -595,7 +598,7 @@ __device__ __noinline__ void family_fp64(const uint4 *__restrict__ fw, const dou
   family_floating<double, false>(w, 0, xs, ys, dtab, nullptr, nullptr);
 }
 
-// a child whose values, not all zero, lie below 2^-4 of the family's largest
+// a child whose values, not all zero, lie below 2^-8 of the family's largest
 // (which is 2^54 or more)
 __device__ __forceinline__ bool fix_uneven(const long long (&u)[27], uint32_t mask) {
   uint32_t m[27];  // upper words' magnitudes, then their unions over an element
@@ -610,7 +613,7 @@ __device__ __forceinline__ bool fix_uneven(const long long (&u)[27], uint32_t ma
     uint32_t o = 0;
 #pragma unroll
     for (int k = 0; k < 8; k++) o |= m[lat_vertex(c, k)];
-    if ((mask >> c & 1u) && o < 1u << 18) {
+    if ((mask >> c & 1u) && o < 1u << 14) {
       long long nz = 0;
 #pragma unroll
       for (int k = 0; k < 8; k++) nz |= u[lat_vertex(c, k)];
