@@ -61,6 +61,14 @@ def _ptr(a):
     return a.ctypes.data_as(ctypes.c_void_p)
 
 
+def _ptrs(a, b):
+    """Addresses of an input and an output, with one wait for torch's stream
+    where both are CUDA tensors of one device."""
+    p = _ptr(a)
+    same = _is_device(a) and _is_device(b) and a.device == b.device
+    return p, ctypes.c_void_p(b.data_ptr()) if same else _ptr(b)
+
+
 class Context:
     """One GPU, one CUDA stream (dg_ctx)."""
 
@@ -455,7 +463,7 @@ class Csr:
         else:
             x = np.ascontiguousarray(x, dtype=np.float64)
             out = np.empty_like(x) if out is None else out
-        check(self.ctx.handle, self.ctx._L.dg_csr_spmv(self.ctx.handle, self.handle, _ptr(x), _ptr(out), 1 if on_dev else 0),
+        check(self.ctx.handle, self.ctx._L.dg_csr_spmv(self.ctx.handle, self.handle, *_ptrs(x, out), 1 if on_dev else 0),
               "dg_csr_spmv")
         return out
 
@@ -515,7 +523,7 @@ class DA:
             out = np.empty_like(x) if out is None else out
             c = self._coef(coef)
         _check_len(x, self.n_node, "Jacobian2MatMult")
-        check(self.ctx.handle, self.ctx._L.dg_matvec_coef(self.ctx.handle, self.handle, _ptr(c), _ptr(x), _ptr(out),
+        check(self.ctx.handle, self.ctx._L.dg_matvec_coef(self.ctx.handle, self.handle, _ptr(c), *_ptrs(x, out),
                                                           precision, 1 if on_dev else 0), "dg_matvec_coef")
         return out
 
@@ -579,7 +587,7 @@ class DA:
         if (x.numel() if on_dev else x.size) != self.n_node:
             raise ValueError("vector length differs from the node count")
         check(self.ctx.handle,
-              self.ctx._L.dg_matvec(self.ctx.handle, self.handle, _ptr(x), _ptr(out), precision, lapFac, massFac, on_dev),
+              self.ctx._L.dg_matvec(self.ctx.handle, self.handle, *_ptrs(x, out), precision, lapFac, massFac, on_dev),
               "Jacobian1MatMult")
         return out
 
@@ -664,7 +672,7 @@ class MultiGrid:
         else:
             x = np.ascontiguousarray(x, dtype=np.float32 if precision == 32 else np.float64)
             out = np.empty(n_out, x.dtype)
-        check(self.ctx.handle, fn(self.ctx.handle, self.handle, level, _ptr(x), _ptr(out), precision, on_dev), fn.__name__)
+        check(self.ctx.handle, fn(self.ctx.handle, self.handle, level, *_ptrs(x, out), precision, on_dev), fn.__name__)
         return out
 
     def matvec(self, level: int, x, precision: int = 64):
@@ -702,7 +710,7 @@ class MultiGrid:
         else:
             f = np.ascontiguousarray(f, dtype=np.float64)
             out = np.empty_like(f)
-        check(self.ctx.handle, self.ctx._L.dg_mg_rhs(self.ctx.handle, self.handle, _ptr(f), _ptr(out), on_dev), "rhs")
+        check(self.ctx.handle, self.ctx._L.dg_mg_rhs(self.ctx.handle, self.handle, *_ptrs(f, out), on_dev), "rhs")
         return out
 
     def solve(self, b, precision: int = 32, rtol: float = 1e-8, maxit: int = 200, x=None):
@@ -721,7 +729,7 @@ class MultiGrid:
             x = np.empty_like(b) if x is None else x
         it, rr = ctypes.c_int(), ctypes.c_double()
         check(self.ctx.handle,
-              self.ctx._L.dg_mg_solve(self.ctx.handle, self.handle, _ptr(b), _ptr(x), precision, rtol, maxit, on_dev,
+              self.ctx._L.dg_mg_solve(self.ctx.handle, self.handle, *_ptrs(b, x), precision, rtol, maxit, on_dev,
                                       ctypes.byref(it), ctypes.byref(rr)), "solve")
         return x, it.value, rr.value
 

@@ -33,6 +33,8 @@ struct dg_csr_s {
 
 namespace {
 
+// runs f and waits for its work (the call's one wait at the end; buffers that f
+// frees are freed in stream order), status from what it throws
 template <typename F>
 int guarded(dg_ctx ctx, F &&f) {
   if (!ctx) return DG_ERR_INVALID_ARG;
@@ -340,7 +342,6 @@ int dg_sort_unique_points(dg_ctx ctx, const double *xyz, size_t n, const double 
       dg::DBuf<uint32_t> dx(4 * (nu ? nu : 1), ctx->c.stream);
       dg::octree_to_xyzl(ctx->c, tmp, dx.get());
       copy_out(ctx->c, out_xyzl, dx.get(), 4 * nu, 0);
-      DG_CUDA(cudaStreamSynchronize(ctx->c.stream));
     }
     *n_unique = nu;
   });
@@ -431,7 +432,6 @@ int dg_sort_octants(dg_ctx ctx, const uint32_t *xyzl, size_t n, unsigned maxDept
       dg::octree_to_xyzl(c, o, dx.get());
       copy_out(c, out_xyzl, dx.get(), 4 * o.n, 0);
     }
-    DG_CUDA(cudaStreamSynchronize(c.stream));
     *n_out = o.n;
   });
 }
@@ -458,7 +458,6 @@ int dg_tree_sort(dg_ctx ctx, const uint32_t *xyzl, size_t n, unsigned maxDepth, 
       dg::octree_to_xyzl(c, o, dx.get());
       copy_out(c, out_xyzl, dx.get(), 4 * o.n, 0);
     }
-    DG_CUDA(cudaStreamSynchronize(c.stream));
     *n_out = o.n;
   });
 }
@@ -608,7 +607,6 @@ int dg_da_download(dg_ctx ctx, dg_da da, uint32_t *meta, uint32_t *nodes, uint32
         DG_LAUNCH_CHECK();
       }
       copy_out(c, nodes, t.get(), 8 * E, dst_on_device);
-      DG_CUDA(cudaStreamSynchronize(c.stream));
     }
     if (node_xyz && V) {
       dg::DBuf<uint32_t> t(3 * V, c.stream);
@@ -618,7 +616,6 @@ int dg_da_download(dg_ctx ctx, dg_da da, uint32_t *meta, uint32_t *nodes, uint32
         DG_LAUNCH_CHECK();
       }
       copy_out(c, node_xyz, t.get(), 3 * V, dst_on_device);
-      DG_CUDA(cudaStreamSynchronize(c.stream));
     }
   });
 }
@@ -659,7 +656,6 @@ int level_op(dg_ctx ctx, dg_mg mg, size_t n_in, size_t n_out, const void *in, vo
     }
     op(c, x, y);
     if (!on_device) DG_CUDA(cudaMemcpyAsync(out, y, n_out * es, cudaMemcpyDeviceToHost, c.stream));
-    DG_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
 }  // namespace
@@ -824,7 +820,6 @@ int dg_matvec_coef(dg_ctx ctx, dg_da da, const double *coef, const void *in, voi
       }
       dg::mesh_matvec_coef<T>(c, da->m, dc, x, y);
       if (!on_device) copy_out(c, (T *)out, y, V, 0);
-      DG_CUDA(cudaStreamSynchronize(c.stream));
     };
     if (precision == 64) run(double());
     else run(float());
@@ -846,7 +841,6 @@ int dg_da_diagonal(dg_ctx ctx, dg_da da, const double *coef, double lapFac, doub
     }
     dg::mesh_diagonal(c, da->m, dc, lapFac, massFac, d);
     if (!on_device) copy_out(c, diag, d, V, 0);
-    DG_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
 
@@ -864,7 +858,6 @@ int dg_mg_diagonal(dg_ctx ctx, dg_mg mg, size_t level, double *diag, int on_devi
     }
     dg::dirichlet_diagonal(c, L, d);
     if (!on_device) copy_out(c, diag, d, V, 0);
-    DG_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
 
@@ -889,7 +882,6 @@ int dg_csr_download(dg_ctx ctx, dg_csr a, int64_t *row_ptr, uint32_t *col, doubl
     if (row_ptr) copy_out(ctx->c, row_ptr, c.row_ptr, c.n_rows + 1, dst_on_device);
     if (col && c.nnz) copy_out(ctx->c, col, c.col, c.nnz, dst_on_device);
     if (val && c.nnz) copy_out(ctx->c, val, c.val, c.nnz, dst_on_device);
-    DG_CUDA(cudaStreamSynchronize(ctx->c.stream));
   });
 }
 
@@ -907,7 +899,6 @@ int dg_csr_spmv(dg_ctx ctx, dg_csr a, const double *x, double *y, int on_device)
     }
     dg::csr_spmv(c, a->c, dx, dy);
     if (!on_device) copy_out(c, y, dy, V, 0);
-    DG_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
 
@@ -940,7 +931,6 @@ int dg_matvec(dg_ctx ctx, dg_da da, const void *in, void *out, int precision, do
       }
       dg::mesh_matvec<double>(c, da->m, x, y, lapFac, massFac);
       if (!on_device) copy_out(c, (double *)out, y, V, 0);
-      DG_CUDA(cudaStreamSynchronize(c.stream));
     } else {
       dg::DBuf<float> hin, hout;
       const float *x = device_input(c, (const float *)in, V, on_device, hin);
@@ -951,7 +941,6 @@ int dg_matvec(dg_ctx ctx, dg_da da, const void *in, void *out, int precision, do
       }
       dg::mesh_matvec<float>(c, da->m, x, y, lapFac, massFac);
       if (!on_device) copy_out(c, (float *)out, y, V, 0);
-      DG_CUDA(cudaStreamSynchronize(c.stream));
     }
   });
 }
