@@ -58,26 +58,30 @@ __host__ __device__ __forceinline__ uint32_t compact10(uint32_t v) {
 
 // Morton key of 32-bit coordinates (96 bits used)
 __host__ __device__ __forceinline__ Key128 morton3(uint32_t x, uint32_t y, uint32_t z) {
-  uint32_t p[4];
+  uint32_t p[3];
 #ifdef __CUDA_ARCH__
 #pragma unroll
 #endif
-  for (int i = 0; i < 4; i++)
+  for (int i = 0; i < 3; i++)
     p[i] = spread10(x >> 10 * i) | spread10(y >> 10 * i) << 1 | spread10(z >> 10 * i) << 2;
+  const uint32_t t = (x >> 30 & 1u) | (y >> 30 & 1u) << 1 | (z >> 30 & 1u) << 2 | (x >> 31) << 3 | (y >> 31) << 4 |
+                     (z >> 31) << 5;  // coordinate bits 30 and 31
   Key128 k;
   k.lo = (uint64_t)p[0] | (uint64_t)p[1] << 30 | (uint64_t)p[2] << 60;
-  k.hi = (uint64_t)p[2] >> 4 | (uint64_t)p[3] << 26;
+  k.hi = (uint64_t)p[2] >> 4 | (uint64_t)t << 26;
   return k;
 }
 
 __host__ __device__ __forceinline__ void demorton3(Key128 k, uint32_t &x, uint32_t &y, uint32_t &z) {
-  const uint32_t p[4] = {(uint32_t)k.lo, (uint32_t)(k.lo >> 30), (uint32_t)(k.lo >> 60) | (uint32_t)k.hi << 4,
-                         (uint32_t)(k.hi >> 26)};
-  x = y = z = 0;
+  const uint32_t p[3] = {(uint32_t)k.lo, (uint32_t)(k.lo >> 30), (uint32_t)(k.lo >> 60) | (uint32_t)k.hi << 4};
+  const uint32_t t = (uint32_t)(k.hi >> 26);
+  x = (t & 1u) << 30 | (t >> 3 & 1u) << 31;
+  y = (t >> 1 & 1u) << 30 | (t >> 4 & 1u) << 31;
+  z = (t >> 2 & 1u) << 30 | (t >> 5 & 1u) << 31;
 #ifdef __CUDA_ARCH__
 #pragma unroll
 #endif
-  for (int i = 0; i < 4; i++) {
+  for (int i = 0; i < 3; i++) {
     x |= compact10(p[i]) << 10 * i;
     y |= compact10(p[i] >> 1) << 10 * i;
     z |= compact10(p[i] >> 2) << 10 * i;

@@ -1422,7 +1422,7 @@ void octree_extract(Context &ctx, const Octree &in, size_t seg, Octree &out) {
 // anchor bits then run past 3D and are decoded as is)
 // Four records per thread, their keys loaded together: with one the loads in
 // flight and the operations of demorton3 (in 64-bit pieces) took 0.67 ms for
-// 8.8e7 records, with one and 32-bit pieces 0.57, now 0.48 ms (5.8 TB/s).
+// 8.8e7 records, with one and 32-bit pieces 0.57, now 0.51 ms (5.5 TB/s).
 constexpr int XYZL_PER = 4;
 __global__ void __launch_bounds__(256) k_to_xyzl(const Key128 *__restrict__ k, size_t n, unsigned D, bool batched,
                                                  uint4 *__restrict__ out) {
@@ -1434,10 +1434,8 @@ __global__ void __launch_bounds__(256) k_to_xyzl(const Key128 *__restrict__ k, s
 #pragma unroll
   for (int j = 0; j < XYZL_PER; j++) {
     if (i0 + 256 * j >= n) break;
-    Key128 a = batched ? morton_part(key[j], D) : tag_anchor(key[j]);
-    a.hi &= (1ull << 26) - 1;  // D <= 30: 90 bits, the fourth piece of demorton3 falls away
     uint32_t x, y, z;
-    demorton3(a, x, y, z);
+    demorton3(batched ? morton_part(key[j], D) : tag_anchor(key[j]), x, y, z);
     out[i0 + 256 * j] = make_uint4(x, y, z, tag_level(key[j]));
   }
 }
