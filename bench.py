@@ -596,10 +596,7 @@ def run_scale(args, dg, ctx, local):
         V, E = da.n_node, da.n_elem
         res["n_elem"], res["n_node"] = E, V
         mv = {}
-        # fp32 / fp64: the run form of the element loop (default); *_pairs: its pair form
-        for name, prec, dt, form in (("fp32", 32, torch.float32, "runs"), ("fp32_pairs", 32, torch.float32, "pairs"),
-                                     ("fp64", 64, torch.float64, "runs"), ("fp64_pairs", 64, torch.float64, "pairs")):
-            ctx.set_matvec_form(form)
+        for name, prec, dt in (("fp32", 32, torch.float32), ("fp64", 64, torch.float64)):
             x = torch.rand(V, dtype=dt, device=f"cuda:{local}") * 2 - 1
             y = torch.empty_like(x)
             for _ in range(3):
@@ -613,7 +610,6 @@ def run_scale(args, dg, ctx, local):
             nbytes = 36 * E + 3 * (prec // 8) * V
             mv[name] = {"ms": kms, "GB/s": nbytes / (kms * 1e-3) / 1e9,
                         "frac_of_measured_peak": nbytes / (kms * 1e-3) / 1e9 / peak, "algorithmic_bytes": nbytes}
-        ctx.set_matvec_form("runs")
         # FP32 against FP64 on the same input: relative L2 difference
         x64 = torch.rand(V, dtype=torch.float64, device=f"cuda:{local}") * 2 - 1
         y64, y32 = torch.empty_like(x64), torch.empty(V, dtype=torch.float32, device=f"cuda:{local}")
@@ -721,8 +717,8 @@ def run_poisson(args, dg, ctx, local):
            "fine_nodes": mg.sizes[0][1], "build_balance_ms": 1e3 * t_build, "mg_setup_ms": 1e3 * t_setup,
            "mg_setup_kernels_ms": setup_kernels}
     xs = {}
-    # fp32_vcycle: FP32 V-cycle, double-single CG operator (the default);
-    # fp32_vcycle_fp64op: FP32 V-cycle, FP64 CG operator; fp32_vcycle_fp32op:
+    # fp32_vcycle: FP32 V-cycle, fixed-point CG operator on FP64 vectors (the default);
+    # fp32_vcycle_fp64op: the same loop, asked for as FP64; fp32_vcycle_fp32op:
     # FP32 V-cycle and FP32 CG operator with FP64 residual replacement;
     # fp64_vcycle: all FP64
     for name, prec, op in (("fp32_vcycle", 32, 48), ("fp32_vcycle_fp64op", 32, 64), ("fp32_vcycle_fp32op", 32, 32),
@@ -948,11 +944,11 @@ def run_ours(args):
             "higher_is_better": True,
             "scaling": "weak",
             "vs_baseline": None,
-            "dtype": "int keys (octree, mesh); FP32 V-cycle, FP64 CG vectors with a double-single operator (solve)",
+            "dtype": "int keys (octree, mesh); FP32 V-cycle, FP64 CG vectors with a 64-bit fixed-point operator (solve)",
             "data": "synthetic",
             "config": {"workload": "serving stream", "requests": serve["requests"], "points": serve["points"],
                        "rate_req_s": SERVE_RATE, "sizes": list(SERVE_SIZES), "seed": SERVE_SEED,
-                       "max_depth": 30, "max_pts_per_octant": 1, "solve": f"FP32 V(2,2) CG (double-single operator, FP64 vectors) to 1e-8, <= {SOLVE_MAXIT} it",
+                       "max_depth": 30, "max_pts_per_octant": 1, "solve": f"FP32 V(2,2) CG (64-bit fixed-point operator, FP64 vectors) to 1e-8, <= {SOLVE_MAXIT} it",
                        "parallelism": f"replicas x{ws}",
                        "l2": f"inputs larger than L2 ({24 * serve['points'] / 1e9:.2f} GB of points per step)"},
             "autotune": serve["autotune"],

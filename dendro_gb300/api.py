@@ -676,8 +676,8 @@ class MultiGrid:
         return out
 
     def matvec(self, level: int, x, precision: int = 64):
-        """DirichletJacobianMatMult on a level: FP64 (64), FP32 (32), or FP64
-        vectors in 64-bit fixed point (48)."""
+        """DirichletJacobianMatMult on a level: FP64 (64; 48 is the same loop)
+        or FP32 (32)."""
         n = self.sizes[level][1]
         return self._op(self.ctx._L.dg_mg_matvec, level, x, n, n, precision)
 
@@ -695,9 +695,9 @@ class MultiGrid:
         check(self.ctx.handle, self.ctx._L.dg_mg_set_smoother(self.handle, omega, nu_pre, nu_post), "set_smoother")
 
     def set_cg_operator(self, precision: int = 48, reliable_delta: float = 1e-3):
-        """The CG's operator q = A p with an FP32 V-cycle: 64-bit fixed
-        point on FP64 vectors (48, the default), FP64 (64), or FP32
-        with FP64 residual replacement (32)."""
+        """The CG's operator q = A p with an FP32 V-cycle: on FP64 vectors
+        (48, the default, or 64: the same loop), or FP32 with FP64 residual
+        replacement (32)."""
         check(self.ctx.handle, self.ctx._L.dg_mg_set_cg_operator(self.handle, precision, reliable_delta),
               "set_cg_operator")
 

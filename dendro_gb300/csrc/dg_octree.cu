@@ -48,7 +48,7 @@ namespace dg {
 // operations only move the exponent, so the value is x * 2^(D - e), truncated
 // from the bits of x by integer shifts: GB300's narrow FP64 pipe, which the
 // multiplications, comparisons and conversions of three coordinates kept busy,
-// does nothing (16e6 points: 0.45 -> 0.14 ms).  Where x * 2^D would leave the
+// does nothing (16e6 points: 0.45 -> 0.37 ms).  Where x * 2^D would leave the
 // normal range the value is 0 or out of the domain either way.
 __device__ __forceinline__ bool quantize_pow2(double x, int shift, unsigned D, uint32_t &q) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
