@@ -196,7 +196,7 @@ void assemble_csr(Context &ctx, const Mesh &m, const uint8_t *bdy, double lap_fa
     k_incidence<<<grid_for(np, 256), 256, 0, s>>>(conn, E, ka.get());
     DG_LAUNCH_CHECK();
   }
-  uint64_t *key = radix_sort<uint64_t>(ctx, ka.get(), kb.get(), np, 32 + (int)bits_of(V));
+  uint64_t *key = radix_sort<uint64_t>(ctx, ka.get(), kb.get(), np, 32 + (int)bits_of(V), 0, true);
   check_device_flags(ctx, "radix sort");
   DBuf<uint64_t> start(V + 1, s);
   DBuf<uint32_t> len(V, s);

@@ -1579,7 +1579,7 @@ static void octree_to_xyzl_hilbert(Context &ctx, const Octree &o, uint32_t *d_xy
     ProfScope _prof(ctx, "hilbert_order", (double)n * 16 * 36);
     k_hilbert_keys<<<grid_for(n, 256), 256, 0, s>>>(o.keys + off[g], n, D, o.nseg > 1, tab, a.get() + off[g]);
     DG_LAUNCH_CHECK();
-    Key128 *srt = radix_sort<Key128>(ctx, a.get() + off[g], b.get() + off[g], n, 3 * (int)D + 5 + 32);
+    Key128 *srt = radix_sort<Key128>(ctx, a.get() + off[g], b.get() + off[g], n, 3 * (int)D + 5 + 32, 0, true);
     check_device_flags(ctx, "Hilbert order");
     k_gather_xyzl<<<grid_for(n, 256), 256, 0, s>>>(o.keys + off[g], srt, n, D, o.nseg > 1,
                                                    reinterpret_cast<uint4 *>(d_xyzl) + off[g]);
@@ -1617,7 +1617,7 @@ void octree_from_xyzl(Context &ctx, const uint32_t *d_xyzl, size_t n, unsigned D
       DBuf<Key128> a(n, ctx.stream), b(n, ctx.stream);
       k_to_sortform<<<grid_for(n, 256), 256, 0, ctx.stream>>>(k.get(), n, a.get());
       DG_LAUNCH_CHECK();
-      Key128 *srt = radix_sort<Key128>(ctx, a.get(), b.get(), n, 3 * (int)D + 5);
+      Key128 *srt = radix_sort<Key128>(ctx, a.get(), b.get(), n, 3 * (int)D + 5, 0, true);
       check_device_flags(ctx, "Hilbert order");
       k_from_sortform<<<grid_for(n, 256), 256, 0, ctx.stream>>>(srt, n, k.get());
       DG_LAUNCH_CHECK();
@@ -1654,7 +1654,7 @@ void complete_octree(Context &ctx, const uint32_t *d_xyzl, size_t n, unsigned D,
   Key128 *sorted = a.get();
   size_t m = n;
   if (!is_unique) m = sort_unique<Key128>(ctx, a.get(), b.get(), n, bits, &sorted);
-  else if (!is_sorted) sorted = radix_sort<Key128>(ctx, a.get(), b.get(), n, bits);
+  else if (!is_sorted) sorted = radix_sort<Key128>(ctx, a.get(), b.get(), n, bits, 0, true);
   Key128 *other = (sorted == a.get()) ? b.get() : a.get();
   DBuf<uint32_t> keep(m, s);
   {
@@ -1715,7 +1715,7 @@ void sort_octants(Context &ctx, const uint32_t *d_xyzl, size_t n, unsigned D, in
   size_t m = n;
   if (unique) m = sort_unique<Key128>(ctx, a.get(), b.get(), n, bits, &srt);
   else {
-    srt = radix_sort<Key128>(ctx, a.get(), b.get(), n, bits);
+    srt = radix_sort<Key128>(ctx, a.get(), b.get(), n, bits, 0, true);
     check_device_flags(ctx, "sortOctants");
   }
   if (mode == 2) {
