@@ -30,8 +30,9 @@ struct MGLevel {
 
 struct MG {
   std::vector<MGLevel> lv;  // 0 = finest
-  size_t nc = 0;            // nodes of the coarsest level
-  double *ca64 = nullptr;    // the coarsest level's assembled operator (dense, FP64)
+  size_t nc = 0;             // interior nodes of the coarsest level
+  uint32_t *clist = nullptr;  // its nodes, the interior ones first
+  double *ca64 = nullptr;    // the coarsest level's assembled operator on its interior nodes (dense, FP64)
   float *cinv32 = nullptr;   // its inverse in FP32 (refined in FP64 when the FP64 V-cycle applies it)
   double omega = 0.667;  // Jacobi damping (bin/options:190)
   int nu_pre = 2, nu_post = 2;
