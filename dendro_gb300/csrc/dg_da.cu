@@ -166,14 +166,19 @@ __global__ void k_node_table(const K *__restrict__ nodes, size_t nn, unsigned Lm
   if (i >= nn) return;
   const auto key = node_wide(nodes[i]);
   uint64_t h = node_hash(key, Lm) & mask;
-  for (int probe = 0; probe < BAL_PROBES; probe++) {
-    if (slot_cas(tab + h, key) == node_empty(key)) {
+  for (int probe = 0; probe < NODE_PROBES; probe++) {
+    const auto cur = slot_cas(tab + h, key);
+    if (cur == node_empty(key)) {
       val[h] = (uint32_t)i;
       return;
     }
-    h = (h + 8) & mask;
+    if (cur == key) {  // twice in the list
+      set_flag(flags, DGF_INTERNAL);
+      return;
+    }
+    h = (h + NODE_STEP) & mask;
   }
-  set_flag(flags, DGF_INTERNAL);
+  set_flag(flags, DGF_CAPACITY);
 }
 
 // Per node and child: x the nodes before the child in preorder (its own index
@@ -1052,22 +1057,12 @@ static void build_from_nodes(Context &ctx, const Octree &bal, const Octree &tree
   const size_t n = bal.n, n_int = tree.n_node;
   const unsigned D = bal.max_depth, Lm = tree.top - 1;
   const K *nodes = static_cast<const K *>(tree.nodes);
-  size_t slots = 1024;
-  while (slots < 2 * n_int) slots <<= 1;
-  DBuf<K> tab(slots, s);
-  DBuf<uint32_t> val(slots, s), rank(n_int, s), block(8 * n_int, s), state(n_int, s), list(n_int, s);
+  DBuf<K> tab;
+  DBuf<uint32_t> val, rank(n_int, s), block(8 * n_int, s), state(n_int, s), list(n_int, s);
   DBuf<uint2> kids(8 * n_int, s);
   DBuf<uint8_t> leafs(n_int, s);
   DBuf<uint32_t> meta(n, s), base(n, s);
   uint32_t *d_total = reinterpret_cast<uint32_t *>(ctx.d_scratch);  // {families with a leaf, mesh nodes}
-  DG_CUDA(cudaMemsetAsync(tab.get(), 0xff, slots * sizeof(K), s));
-  DG_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), s));
-  {
-    ProfScope _prof(ctx, "da_node_table", (double)n_int * (2 * sizeof(K) + 4));
-    k_node_table<K><<<grid_for(n_int, 256), 256, 0, s>>>(nodes, n_int, Lm, tab.get(), val.get(), slots - 1,
-                                                         ctx.d_flags);
-    DG_LAUNCH_CHECK();
-  }
   {
     ProfScope _prof(ctx, "da_node_children", (double)n_int * (sizeof(K) + 69));
     k_node_children<K><<<grid_for(8 * n_int, 256), 256, 0, s>>>(nodes, n_int, Lm, kids.get(), leafs.get(),
@@ -1075,16 +1070,33 @@ static void build_from_nodes(Context &ctx, const Octree &bal, const Octree &tree
     DG_LAUNCH_CHECK();
   }
   exclusive_scan<uint32_t, uint32_t>(rank.get(), rank.get(), n_int, d_total, s);
-  {
-    ProfScope _prof(ctx, "da_elems", (double)n_int * (sizeof(K) + 77) + (double)n * 8);
-    k_family_elems<K><<<grid_for(8 * n_int, 256), 256, 0, s>>>(
-        nodes, n_int, Lm, tab.get(), val.get(), slots - 1, kids.get(), leafs.get(), rank.get(), ctx.d_etype_of,
-        block.get(), state.get(), list.get(), meta.get(), base.get(), ctx.d_flags);
-    DG_LAUNCH_CHECK();
+  size_t slots = 1024;
+  while (slots < 2 * n_int) slots <<= 1;
+  for (;; slots *= 2) {  // again where a node found no slot
+    tab.alloc(slots, s);
+    val.alloc(slots, s);
+    DG_CUDA(cudaMemsetAsync(tab.get(), 0xff, slots * sizeof(K), s));
+    DG_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(uint32_t), s));
+    {
+      ProfScope _prof(ctx, "da_node_table", (double)n_int * (2 * sizeof(K) + 4));
+      k_node_table<K><<<grid_for(n_int, 256), 256, 0, s>>>(nodes, n_int, Lm, tab.get(), val.get(), slots - 1,
+                                                           ctx.d_flags);
+      DG_LAUNCH_CHECK();
+    }
+    {
+      ProfScope _prof(ctx, "da_elems", (double)n_int * (sizeof(K) + 77) + (double)n * 8);
+      k_family_elems<K><<<grid_for(8 * n_int, 256), 256, 0, s>>>(
+          nodes, n_int, Lm, tab.get(), val.get(), slots - 1, kids.get(), leafs.get(), rank.get(), ctx.d_etype_of,
+          block.get(), state.get(), list.get(), meta.get(), base.get(), ctx.d_flags);
+      DG_LAUNCH_CHECK();
+    }
+    exclusive_scan<uint32_t, uint32_t>(base.get(), base.get(), n, d_total + 1, s);
+    DG_CUDA(cudaMemcpyAsync(ctx.h_scratch + 4, d_total, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    const uint32_t f = read_scalar(ctx, ctx.d_flags);
+    if (f & DGF_CAPACITY) continue;
+    if (f) check_device_flags(ctx, "DA");
+    break;
   }
-  exclusive_scan<uint32_t, uint32_t>(base.get(), base.get(), n, d_total + 1, s);
-  DG_CUDA(cudaMemcpyAsync(ctx.h_scratch + 4, d_total, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  check_device_flags(ctx, "DA");
   uint32_t total[2];
   std::memcpy(total, ctx.h_scratch + 4, sizeof(total));
   const size_t nf = total[0], nn = total[1], np = (nf + FAM - 1) / FAM;
