@@ -68,6 +68,19 @@ __device__ __forceinline__ K node_of(Key128 anchor, unsigned l, unsigned Lm, uns
   return N::narrow(idx << (3 * (Lm - l)) << 5 | (typename N::W)l);
 }
 
+// Whether `next` may stand behind `prev` in the preorder list of an octree's
+// nodes (or, with none, at its head): later, and a child of `prev` or of an
+// ancestor of it, or the root of another cloud.  A list of which this holds all
+// along has no node twice and every node's parent.
+template <typename W>
+__host__ __device__ __forceinline__ bool node_follows(bool any, W prev, W next, unsigned Lm) {
+  const unsigned d = (unsigned)next & 31u;
+  if (d > Lm || (any && next <= prev)) return false;
+  if (d == 0) return ((next >> 5) & (((W)1 << (3 * Lm)) - 1)) == 0;
+  const unsigned sh = 5 + 3 * (Lm - d + 1);  // to the parent's path
+  return any && ((unsigned)prev & 31u) + 1 >= d && prev >> sh == next >> sh;
+}
+
 // sum of the octal digits of v
 __device__ __forceinline__ unsigned digit_sum(uint64_t v) {
   const uint64_t m = 0x1249249249249249ull;  // bits 0, 3, ..., 60

@@ -887,7 +887,7 @@ __global__ void k_bal_node_levels(const K *__restrict__ nodes, size_t nn, unsign
 template <typename K, bool LEAVES>
 __global__ void __launch_bounds__(256) k_bal_start(const void *__restrict__ in, size_t n, unsigned D, unsigned Lm,
                                                    K *__restrict__ tab, uint64_t mask, K *__restrict__ list,
-                                                   BalCounts *__restrict__ cnt, uint32_t *flags) {
+                                                   size_t room, BalCounts *__restrict__ cnt, uint32_t *flags) {
   __shared__ unsigned num[32];
   __shared__ unsigned long long base[32];
   if (threadIdx.x < 32) num[threadIdx.x] = 0;
@@ -919,7 +919,9 @@ __global__ void __launch_bounds__(256) k_bal_start(const void *__restrict__ in, 
     base[threadIdx.x] =
         bal_off(cnt, threadIdx.x) + atomicAdd(&cnt->start[threadIdx.x], (unsigned long long)num[threadIdx.x]);
   __syncthreads();
-  if (won) list[base[l] + rank] = key;
+  if (!won) return;
+  if (base[l] + rank < room) list[base[l] + rank] = key;
+  else set_flag(flags, DGF_INTERNAL);
 }
 
 // One level of the recursion: for every node q of level l the 8 parents (level
@@ -941,11 +943,13 @@ struct BalSmem {
   unsigned long long at;
 };
 
-// appends v of the lanes that say so to a list in shared memory; all lanes of
-// the warp take part, which also brings them together again after the
-// diverging probes (with each lane adding to the counter where it left its
-// probes, entries were at times read across the next barrier before they were
-// written, with 128-bit keys)
+// appends v of the lanes that say so to a list in shared memory.  All lanes of
+// the warp take part, which brings them together after the diverging probes and
+// before the block's next barrier.  With each lane adding to the counter where
+// it left its probes, balances of 1.4e8 nodes with 128-bit keys at times lost or
+// repeated a few; why is not established (the barrier alone orders the writes
+// before the reads).  So entries are checked before they are used as indices,
+// and the sorted list of all nodes by k_bal_check.
 __device__ __forceinline__ void warp_append(bool mine, uint16_t v, unsigned *n, uint16_t *list) {
   const unsigned m = __ballot_sync(0xffffffffu, mine);
   if (!m) return;
@@ -1024,8 +1028,10 @@ __global__ void __launch_bounds__(BAL_TILE) k_bal_level(unsigned l, unsigned Lm,
     __syncthreads();
     const unsigned nc = S.n_cand;
     for (unsigned r = 0; r < nc; r += BAL_TILE) {
-      const unsigned q = r + t, me = q < nc ? S.list[q] & (BAL_CAND - 1) : 0u;
-      const bool won = q < nc && node_insert<K>(tab, mask, node_wide(S.cand[me]), Lm, flags);
+      const unsigned q = r + t, me = q < nc ? S.list[q] : 0u;
+      const bool ok = q < nc && me < 8 * here;
+      if (q < nc && !ok) set_flag(flags, DGF_INTERNAL);
+      const bool won = ok && node_insert<K>(tab, mask, node_wide(S.cand[me]), Lm, flags);
       warp_append(won, (uint16_t)me, &S.n_won, S.won);
     }
     __syncthreads();
@@ -1033,7 +1039,9 @@ __global__ void __launch_bounds__(BAL_TILE) k_bal_level(unsigned l, unsigned Lm,
     if (t == 0 && nw) S.at = next + atomicAdd(&cnt->grown[l - 1], (unsigned long long)nw);
     __syncthreads();
     for (unsigned q = t; q < nw; q += BAL_TILE) {
-      if (S.at + q < grown_cap) grown[S.at + q] = S.cand[S.won[q] & (BAL_CAND - 1)];
+      const unsigned me = S.won[q];
+      if (me >= 8 * here) set_flag(flags, DGF_INTERNAL);
+      else if (S.at + q < grown_cap) grown[S.at + q] = S.cand[me];
       else set_flag(flags, DGF_CAPACITY);
     }
     __syncthreads();
@@ -1053,6 +1061,32 @@ __global__ void k_bal_gather(const K *__restrict__ start, BalGather g, size_t n_
   while (l < 31 && i >= g.off[l + 1]) l++;
   const size_t r = i - g.off[l];
   if (r < g.num[l]) out[g.to[l] + r] = start[i];
+}
+
+// the sorted nodes as an octree's: neighbours that do not follow one another
+// raise DGF_INTERNAL.  Four per thread, loaded together (1.25e7 nodes: 27 us, 43
+// with one).
+constexpr int CHECK_PER = 4;
+template <typename K>
+__global__ void __launch_bounds__(256) k_bal_check(const K *__restrict__ nodes, size_t nn, unsigned Lm,
+                                                   uint32_t *flags) {
+  const size_t i0 = (size_t)blockIdx.x * (256 * CHECK_PER) + threadIdx.x;
+  K k[CHECK_PER], prev[CHECK_PER];
+#pragma unroll
+  for (int j = 0; j < CHECK_PER; j++) {
+    const size_t i = i0 + 256 * j;
+    if (i < nn) {
+      k[j] = nodes[i];
+      prev[j] = nodes[i > 0 ? i - 1 : 0];
+    }
+  }
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < CHECK_PER; j++) {
+    const size_t i = i0 + 256 * j;
+    if (i < nn) ok = ok && node_follows(i > 0, node_wide(prev[j]), node_wide(k[j]), Lm);
+  }
+  if (!ok) set_flag(flags, DGF_INTERNAL);
 }
 
 // the sorted nodes of the balanced refinement; d_hist: per level the nodes (an
@@ -1085,10 +1119,10 @@ static size_t balance_nodes(Context &ctx, const Octree &in, unsigned top, const 
                                                  : (double)in.n * 16 + (double)room * 2 * sizeof(K));
       if (in.nodes)
         k_bal_start<K, false><<<grid_for(in.n_node, 256), 256, 0, s>>>(in.nodes, in.n_node, D, Lm, tab.get(),
-                                                                       slots - 1, start.get(), cnt, ctx.d_flags);
+                                                                       slots - 1, start.get(), room, cnt, ctx.d_flags);
       else
         k_bal_start<K, true><<<grid_for(in.n, 256), 256, 0, s>>>(in.keys, in.n, D, Lm, tab.get(), slots - 1,
-                                                                 start.get(), cnt, ctx.d_flags);
+                                                                 start.get(), room, cnt, ctx.d_flags);
       DG_LAUNCH_CHECK();
     }
     const unsigned grid =
@@ -1128,6 +1162,11 @@ static size_t balance_nodes(Context &ctx, const Octree &in, unsigned top, const 
   }
   if (n1) DG_CUDA(cudaMemcpyAsync(a.get() + n0, grown.get(), n1 * sizeof(K), cudaMemcpyDeviceToDevice, s));
   *sorted = radix_sort<K>(ctx, a.get(), b.get(), nn, 3 * (int)Lm + 5 + (int)in.seg_bits);
+  {
+    ProfScope _prof(ctx, "bal_check", (double)nn * sizeof(K));
+    k_bal_check<K><<<grid_for(nn, 256 * CHECK_PER), 256, 0, s>>>(*sorted, nn, Lm, ctx.d_flags);
+    DG_LAUNCH_CHECK();
+  }
   return nn;
 }
 
