@@ -174,7 +174,7 @@ int dg_ctx_destroy(dg_ctx ctx) {
   if (ctx->c.h_scratch) cudaFreeHost(ctx->c.h_scratch);
   if (ctx->c.d_sten64) cudaFree(ctx->c.d_sten64);
   if (ctx->c.d_sten32) cudaFree(ctx->c.d_sten32);
-  for (dg::Context::DiagTable *t : {&ctx->c.dtab64, &ctx->c.dtab32})
+  for (dg::Context::CubeTable *t : {&ctx->c.cubes64, &ctx->c.cubes32})
     if (t->p) cudaFree(t->p);
   if (ctx->c.d_etype_of) cudaFree(ctx->c.d_etype_of);
   if (ctx->c.d_etype_mask) cudaFree(ctx->c.d_etype_mask);

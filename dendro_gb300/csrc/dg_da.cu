@@ -1209,27 +1209,28 @@ void mesh_free(Context &ctx, Mesh &m) {
 // ------------------------------------------------------------------------
 // element loop
 // ------------------------------------------------------------------------
-// the diagonal table of the element loop for these factors (kept on the
-// context until a call with others)
-// (FP64: the fixed-point table follows it)
+// the element loop's tables for these factors (kept on the context until a call
+// with others): the elements' operators per level, and for FP64 vectors the
+// fixed-point modes behind them
 template <typename T>
-static const T *diag_table(Context &ctx, double lap_fac, double mass_fac) {
+static const Cube<T> *cube_table(Context &ctx, double lap_fac, double mass_fac) {
   constexpr bool dbl = std::is_same<T, double>::value;
-  Context::DiagTable &t = dbl ? ctx.dtab64 : ctx.dtab32;
-  if (!t.p) DG_CUDA(cudaMalloc(&t.p, DTAB_ENTRIES * (dbl ? sizeof(T) + sizeof(int2) : sizeof(T))));
+  Context::CubeTable &t = dbl ? ctx.cubes64 : ctx.cubes32;
+  if (!t.p) DG_CUDA(cudaMalloc(&t.p, DTAB_LEVELS * sizeof(Cube<T>) + (dbl ? DTAB_ENTRIES * sizeof(int2) : 0)));
+  Cube<T> *p = static_cast<Cube<T> *>(t.p);
   if (!t.ok || t.lap != lap_fac || t.mass != mass_fac) {
-    k_dtab<T><<<(DTAB_ENTRIES + 127) / 128, 128, 0, ctx.stream>>>(static_cast<T *>(t.p), lap_fac, mass_fac);
+    k_cube_table<T><<<1, 32, 0, ctx.stream>>>(p, lap_fac, mass_fac);
     DG_LAUNCH_CHECK();
     if (dbl) {
-      k_fix_table<<<(DTAB_ENTRIES + 127) / 128, 128, 0, ctx.stream>>>(
-          reinterpret_cast<int2 *>(static_cast<T *>(t.p) + DTAB_ENTRIES), lap_fac, mass_fac);
+      k_fix_table<<<(DTAB_ENTRIES + 127) / 128, 128, 0, ctx.stream>>>(reinterpret_cast<int2 *>(p + DTAB_LEVELS),
+                                                                      lap_fac, mass_fac);
       DG_LAUNCH_CHECK();
     }
     t.lap = lap_fac;
     t.mass = mass_fac;
     t.ok = true;
   }
-  return static_cast<const T *>(t.p);
+  return p;
 }
 
 // blocks of a grid-strided patch kernel
@@ -1258,9 +1259,9 @@ void launch_matvec(Context &ctx, const Mesh &m, const uint8_t *bdy, const float 
   if (elem_matvec<float, DIR>(ctx, m, bdy, x, y, lap_fac, mass_fac, name, bytes)) return;
   const size_t smem = family_smem(m.max_run);
   const unsigned grid = patch_grid(ctx, k_family_matvec<DIR>, smem, m.n_patch);
-  const float *dtab = diag_table<float>(ctx, lap_fac, mass_fac);
+  const Cube<float> *tab = cube_table<float>(ctx, lap_fac, mass_fac);
   ProfScope _prof(ctx, name, bytes);
-  k_family_matvec<DIR><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch, m.max_run, dtab,
+  k_family_matvec<DIR><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch, m.max_run, tab,
                                                         x, y);
   DG_LAUNCH_CHECK();
 }
@@ -1271,10 +1272,10 @@ void launch_matvec(Context &ctx, const Mesh &m, const uint8_t *bdy, const double
   if (elem_matvec<double, DIR>(ctx, m, bdy, x, y, lap_fac, mass_fac, name, bytes)) return;
   const size_t smem = family_fix_smem(m.max_run);
   const unsigned grid = patch_grid(ctx, k_family_matvec_fix<DIR>, smem, m.n_patch);
-  const double *dtab = diag_table<double>(ctx, lap_fac, mass_fac);
+  const Cube<double> *tab = cube_table<double>(ctx, lap_fac, mass_fac);
   ProfScope _prof(ctx, name, bytes);
   k_family_matvec_fix<DIR><<<grid, FAM, smem, ctx.stream>>>(m.fam, m.prun, m.pinfo, m.n_fam, m.n_patch, m.max_run,
-                                                            reinterpret_cast<const int2 *>(dtab + DTAB_ENTRIES), dtab,
+                                                            reinterpret_cast<const int2 *>(tab + DTAB_LEVELS), tab,
                                                             x, y);
   DG_LAUNCH_CHECK();
 }

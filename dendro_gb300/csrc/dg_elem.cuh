@@ -17,18 +17,26 @@
 // the reference's 18 element types, so the elements themselves are all the
 // plain trilinear one, and no stencil table is read.
 //
-// Elements: K and M are tensor products, diagonal in a basis of sums and
-// differences.  For the assembled 2x2x2 family, per axis
+// Elements in floating point: of the 8 x 8 entries of the trilinear K and M only
+// those of a vertex itself, of its opposite and of its class (the vertices an
+// even number of steps away) and the other class differ from one another, so a
+// row is one multiply-add for each of the first two and the classes' sums,
+// formed once per element (lat_cubes): 36 operations per element where a dense
+// stencil takes 64 multiply-adds.  Every row is a sum of its own entries times
+// x, as with the stencil, so a row among small values keeps its accuracy beside
+// large ones.
+//
+// Elements in fixed point: K and M are tensor products, diagonal in a basis of
+// sums and differences.  For the assembled 2x2x2 family, per axis
 //   M = 1/4 s s^T + 1/3 o o^T + 1/12 q q^T,  A = 1/4 o o^T + 1/4 q q^T
 // with s = (1,2,1), o = (1,0,-1), q = (1,-2,1); for one element
 //   M = 1/2 s s^T + 1/6 d d^T,  A = 1/2 d d^T,  s = (1,1), d = (1,-1).
 // So a complete family (3 of 4) costs 27 lines each way (4 and 5 operations a
-// line, all coefficients 1 or 2) and 27 multiplications: 262 operations for 8
-// elements, where 8 dense 8x8 stencils cost 512 multiply-adds.  A family with
-// subdivided children is applied element by element: 397 operations.
+// line, all coefficients 1 or 2) and 27 multiplications, which are what counts
+// there; one with subdivided children is applied element by element.
 //
-// On 1.1e7 elements of a Gaussian cloud (GB300) FP32 takes 109 us and FP64
-// vectors 350 us; what bounds them stands at the kernels.  An element-wise loop
+// On 1.1e7 elements of a Gaussian cloud (GB300) FP32 takes 96 us and FP64
+// vectors 341 us; what bounds them stands at the kernels.  An element-wise loop
 // over dense stencils, 8 gathers and 8 atomics per element, took 348 and 1,820
 // us.  128 families per patch: 64 and 256 measured 152 / 150 us where 128 took
 // 143 (FP32); a patch of 256 leaves too few blocks on small meshes.
@@ -97,9 +105,31 @@ __device__ __forceinline__ bool is_finite(double v) {
   return ((uint32_t)__double2hiint(v) & 0x7ff00000u) != 0x7ff00000u;
 }
 
-// entry i of the table: lap and mass already scaled by h / 2 and h^3 / 8
+// The trilinear element's operator lap K + mass M (scaled by h / 2 and h^3 / 8):
+// row i is own x_i + opp x_opposite + cls (sum of i's class) / 4 + other (sum of
+// the other class) / 4.  Quarters, so that a sum stays within the range of its
+// terms.
 template <typename T>
-__device__ __forceinline__ T dtab_entry(int i, T lap, T mass) {
+struct __align__(16) Cube {
+  T own, opp, cls, other;
+};
+template <typename T>
+__device__ __forceinline__ Cube<T> cube_of(T lap, T mass) {
+  return Cube<T>{lap * (T)(5.0 / 6.0) + mass * (T)(2.0 / 9.0), -lap * (T)(1.0 / 6.0) - mass * (T)(1.0 / 9.0),
+                 -lap * (T)(2.0 / 3.0) + mass * (T)(8.0 / 27.0), mass * (T)(16.0 / 27.0)};
+}
+// ... per level
+template <typename T>
+__global__ void k_cube_table(Cube<T> *__restrict__ out, double lapf, double massf) {
+  const int l = threadIdx.x;
+  if (l >= DTAB_LEVELS) return;
+  const double h = ldexp(1.0, -l);
+  const Cube<double> c = cube_of<double>(lapf * h * 0.5, massf * h * h * h * 0.125);
+  out[l] = Cube<T>{(T)c.own, (T)c.opp, (T)c.cls, (T)c.other};
+}
+
+// entry i of the table of modes, lap and mass scaled likewise
+__device__ __forceinline__ double dtab_entry(int i, double lap, double mass) {
   double m[3], a[3];  // mode weights of the three axes
   if (i < DTAB_CHILD) {
     const int o = i < 4 ? 0 : i < 7 ? 1 : i < 9 ? 2 : 3;
@@ -114,19 +144,10 @@ __device__ __forceinline__ T dtab_entry(int i, T lap, T mass) {
       a[k] = k < i - DTAB_CHILD ? 0.5 : 0.0;
     }
   }
-  return lap * (T)(a[0] * m[1] * m[2] + m[0] * a[1] * m[2] + m[0] * m[1] * a[2]) + mass * (T)(m[0] * m[1] * m[2]);
+  return lap * (a[0] * m[1] * m[2] + m[0] * a[1] * m[2] + m[0] * m[1] * a[2]) + mass * (m[0] * m[1] * m[2]);
 }
 
-template <typename T>
-__global__ void k_dtab(T *__restrict__ out, double lapf, double massf) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= DTAB_ENTRIES) return;
-  const double h = ldexp(1.0, -(i / DTAB_STRIDE));
-  const int q = i % DTAB_STRIDE;
-  out[i] = q < DTAB_CHILD + 4 ? (T)dtab_entry<double>(q, lapf * h * 0.5, massf * h * h * h * 0.125) : (T)0;
-}
-
-// The same table for 64-bit fixed point, a row per level: entry i times
+// The table of modes for 64-bit fixed point, a row per level: entry i times
 // 2^(63 - k), split into its upper bits and its 30 lowest, with 2^k the power
 // of two not below the level's |lap| + |mass| (so that |entry| <= 2^(k - 3));
 // k in the row's last place, FIX_NONE where it leaves the range that the element
@@ -145,7 +166,7 @@ static __global__ void k_fix_table(int2 *__restrict__ out, double lapf, double m
   int2 e = make_int2(0, 0);
   if (q == FIX_K) e.x = ok ? k : FIX_NONE;
   else if (ok) {
-    const long long f = __double2ll_rn(ldexp(dtab_entry<double>(q, lap, mass), 63 - k));
+    const long long f = __double2ll_rn(ldexp(dtab_entry(q, lap, mass), 63 - k));
     e = make_int2((int)(f & ((1 << 30) - 1)), (int)(f >> 30));
   }
   out[i] = e;
@@ -154,15 +175,11 @@ static __global__ void k_fix_table(int2 *__restrict__ out, double lapf, double m
 // arithmetic of one lattice value: FP32, FP64 or 64-bit fixed point
 template <typename V>
 struct LatOps {
-  static __device__ __forceinline__ V add_twice(V a, V b) { return a + (V)2 * b; }
-  static __device__ __forceinline__ V sub_twice(V a, V b) { return a - (V)2 * b; }
   static __device__ __forceinline__ V half_add(V v, V half_of) { return v + (V)0.5 * half_of; }
-  static __device__ __forceinline__ V mean(V a, V b) { return (V)0.5 * (a + b); }
+  static __device__ __forceinline__ V mean(V a, V b) { return (V)0.5 * a + (V)0.5 * b; }  // no overflow
 };
 template <>
 struct LatOps<long long> {
-  static __device__ __forceinline__ long long add_twice(long long a, long long b) { return a + 2 * b; }
-  static __device__ __forceinline__ long long sub_twice(long long a, long long b) { return a - 2 * b; }
   static __device__ __forceinline__ long long half_add(long long v, long long half_of) { return v + (half_of >> 1); }
   static __device__ __forceinline__ long long mean(long long a, long long b) { return (a + b) >> 1; }
 };
@@ -185,31 +202,52 @@ __device__ __forceinline__ void lat_distribute(V (&v)[27], uint32_t hang) {
     }
 }
 
+// any family in floating point, v = sum over its elements of S u; coef(c): child
+// c's operator.  A child that is not there gets no value, and a value that is not
+// finite reaches the rows of its elements only.
+__host__ __device__ constexpr bool odd_vertex(int k) { return ((k ^ k >> 1 ^ k >> 2) & 1) != 0; }
+template <typename T, typename Coef>
+__device__ __forceinline__ void lat_cubes(const T (&u)[27], T (&v)[27], uint32_t mask, Coef &&coef) {
+#pragma unroll
+  for (int i = 0; i < 27; i++) v[i] = (T)0;
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    if (!(mask >> c & 1u)) continue;
+    const Cube<T> s = coef(c);
+    T sum[2] = {(T)0, (T)0};
+#pragma unroll
+    for (int k = 0; k < 8; k++) sum[odd_vertex(k)] += (T)0.25 * u[lat_vertex(c, k)];
+    const T cls[2] = {s.cls * sum[0] + s.other * sum[1], s.cls * sum[1] + s.other * sum[0]};
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      v[lat_vertex(c, k)] +=
+          s.own * u[lat_vertex(c, k)] + (s.opp * u[lat_vertex(c, k ^ 7)] + cls[odd_vertex(k)]);
+  }
+}
+
 // a complete family: to the sum / difference basis and back, in place
-template <typename V>
-__device__ __forceinline__ void lat_forward(V (&u)[27]) {
+__device__ __forceinline__ void lat_forward(long long (&u)[27]) {
 #pragma unroll
   for (int ax = 0; ax < 3; ax++) {
     const int st = ax == 0 ? 1 : ax == 1 ? 3 : 9;
 #pragma unroll
     for (int n = 0; n < 9; n++) {
       const int i = ax == 0 ? 3 * n : ax == 1 ? n % 3 + 9 * (n / 3) : n;
-      const V e = u[i] + u[i + 2 * st], o = u[i] - u[i + 2 * st], b = u[i + st];
-      u[i] = LatOps<V>::add_twice(e, b);
+      const long long e = u[i] + u[i + 2 * st], o = u[i] - u[i + 2 * st], b = u[i + st];
+      u[i] = e + 2 * b;
       u[i + st] = o;
-      u[i + 2 * st] = LatOps<V>::sub_twice(e, b);
+      u[i + 2 * st] = e - 2 * b;
     }
   }
 }
-template <typename V>
-__device__ __forceinline__ void lat_backward(V (&u)[27]) {
+__device__ __forceinline__ void lat_backward(long long (&u)[27]) {
 #pragma unroll
   for (int ax = 0; ax < 3; ax++) {
     const int st = ax == 0 ? 1 : ax == 1 ? 3 : 9;
 #pragma unroll
     for (int n = 0; n < 9; n++) {
       const int i = ax == 0 ? 3 * n : ax == 1 ? n % 3 + 9 * (n / 3) : n;
-      const V t = u[i] + u[i + 2 * st], r = u[i] - u[i + 2 * st], o = u[i + st];
+      const long long t = u[i] + u[i + 2 * st], r = u[i] - u[i + 2 * st], o = u[i + st];
       u[i] = t + o;
       u[i + st] = r + r;
       u[i + 2 * st] = t - o;
@@ -217,8 +255,8 @@ __device__ __forceinline__ void lat_backward(V (&u)[27]) {
   }
 }
 // the modes times their table entries; mul(t, i): t times entry i
-template <typename V, typename Mul>
-__device__ __forceinline__ void lat_scale(V (&u)[27], Mul &&mul) {
+template <typename Mul>
+__device__ __forceinline__ void lat_scale(long long (&u)[27], Mul &&mul) {
 #pragma unroll
   for (int i = 0; i < 27; i++) {
     const int x = i % 3, y = i / 3 % 3, z = i / 9;
@@ -229,10 +267,11 @@ __device__ __forceinline__ void lat_scale(V (&u)[27], Mul &&mul) {
 // any family, v = sum over its elements of S u, element by element in the
 // basis of one element, the sums and differences of shared edges and faces
 // formed once: 148 operations in, 64 multiplications, 185 out for 8 elements
-// (333 for each on its own: 512).  begin(c) before child c; mul(t, p): t times
-// its entry for p factors d.  A child that is not there gets no value.
-template <typename V, typename Begin, typename Mul>
-__device__ __forceinline__ void lat_elements(const V (&u)[27], V (&v)[27], uint32_t mask, Begin &&begin, Mul &&mul) {
+// (333 for each on its own: 512).  mul(t, p): t times the entry for p factors d.
+// A child that is not there gets no value.
+template <typename Mul>
+__device__ __forceinline__ void lat_elements(const long long (&u)[27], long long (&v)[27], uint32_t mask, Mul &&mul) {
+  typedef long long V;
 #pragma unroll
   for (int cx = 0; cx < 2; cx++) {
     V a[2][9], sum_x[2][9];  // [factor along x][y + 3 z]
@@ -255,7 +294,6 @@ __device__ __forceinline__ void lat_elements(const V (&u)[27], V (&v)[27], uint3
       for (int cz = 0; cz < 2; cz++) {
         const int c = cx + 2 * cy + 4 * cz;
         const bool there = mask >> c & 1u;
-        begin(c);
 #pragma unroll
         for (int m = 0; m < 4; m++) {
           const int p = (m & 1) + (m >> 1);
@@ -299,60 +337,31 @@ __device__ __forceinline__ uint32_t fam_hang(const uint4 (&w)[4]) {
 // Family f in floating point: its lattice from xs, its elements in registers,
 // its lattice added into ys with shared-memory atomics.  COEF: element e's
 // factors are coef[2e] (Laplacian) and coef[2e + 1] (mass) instead of the
-// table's; fchild[8 f + c] gives e.  A family whose values are not all finite
-// takes the element path, so that a non-finite x reaches exactly the rows of
-// the elements that hold it.
+// table's; fchild[8 f + c] gives e.
 template <typename T, bool COEF>
-__device__ __forceinline__ void family_floating(const uint4 (&w)[4], size_t f, const T *xs, T *ys, const T *dt,
+__device__ __forceinline__ void family_floating(const uint4 (&w)[4], size_t f, const T *xs, T *ys, const Cube<T> *tab,
                                                 const double *__restrict__ coef,
                                                 const uint32_t *__restrict__ fchild) {
-  const uint32_t mask = fam_mask(w), hang = fam_hang(w);
-  T u[27];
-  auto gather = [&]() {
+  const uint32_t hang = fam_hang(w);
+  T u[27], v[27];
 #pragma unroll
-    for (int i = 0; i < 27; i++) u[i] = xs[fam_u16(w, i)];
-    lat_interpolate(u, hang);
-  };
-  gather();
-  bool regather = false;
-  // a warp takes one path: both cost more than the dearer one
-  bool whole = !COEF && __all_sync(__activemask(), mask == 255u);
-  if (whole) {
-    lat_forward(u);
-    regather = !is_finite(u[0]);  // the weighted sum of all 27
-    whole = !regather;
-  }
-  if (whole) {
-    const T *d = dt + fam_level(w) * DTAB_STRIDE;
-    lat_scale(u, [&](T t, int i) { return t * d[i]; });
-    lat_backward(u);
-  } else {
-    if (regather) gather();
-    T v[27], d[4];
-    if constexpr (!COEF) {
-#pragma unroll
-      for (int k = 0; k < 4; k++) d[k] = dt[fam_level(w) * DTAB_STRIDE + DTAB_CHILD + k];
+  for (int i = 0; i < 27; i++) u[i] = xs[fam_u16(w, i)];
+  lat_interpolate(u, hang);
+  Cube<T> s;
+  if constexpr (!COEF) s = tab[fam_level(w)];
+  lat_cubes(u, v, fam_mask(w), [&](int c) {
+    if constexpr (COEF) {
+      const size_t e = fchild[8 * f + c];
+      const T h = exp2_neg((T)0, fam_level(w));
+      s = cube_of<T>((T)coef[2 * e] * h * (T)0.5, (T)coef[2 * e + 1] * h * h * h * (T)0.125);
     }
-    lat_elements(
-        u, v, mask,
-        [&](int c) {
-          if constexpr (COEF) {
-            const size_t e = fchild[8 * f + c];  // 0 where there is none
-            const T h = exp2_neg((T)0, fam_level(w));
-            const T lf = (T)coef[2 * e] * h * (T)0.5, mf = (T)coef[2 * e + 1] * h * h * h * (T)0.125;
-#pragma unroll
-            for (int k = 0; k < 4; k++) d[k] = dtab_entry(DTAB_CHILD + k, lf, mf);
-          }
-        },
-        [&](T t, int q) { return t * d[q]; });
-#pragma unroll
-    for (int i = 0; i < 27; i++) u[i] = v[i];
-  }
-  lat_distribute(u, hang);
+    return s;
+  });
+  lat_distribute(v, hang);
 #pragma unroll
   for (int i = 0; i < 27; i++) {
     const uint32_t n = fam_u16(w, i);
-    if (n) atomicAdd(&ys[n], u[i]);
+    if (n) atomicAdd(&ys[n], v[i]);
   }
 }
 
@@ -368,9 +377,10 @@ __device__ __forceinline__ void family_floating(const uint4 (&w)[4], size_t f, c
 // DIR, the Dirichlet form: boundary rows are the identity (y = x), boundary
 // columns are dropped.
 //
-// 1.1e7 elements: 109 us.  With x gathered after each barrier 142 us (warps
-// waited 6.6 of 15.2 cycles per instruction for it), with the copies but the
-// words of step 3 loaded in step 3 118 us.  The shared-memory and load/store
+// 1.1e7 elements: 96 us; with the elements in the basis of sums and differences,
+// which spilled registers, 109 us, and in that form with x gathered after each
+// barrier 142 us (warps waited 6.6 of 15.2 cycles per instruction for it), with
+// the copies but the words of step 3 loaded in step 3 118 us.  The shared-memory and load/store
 // pipe is two thirds busy; DRAM traffic alone would take 34.  Blocks per SM
 // (registers, shared memory): 3, 4, 5, 6 took 165, 135, 121, 118 us; 12 words
 // ahead 112, 4 words 115.
@@ -385,16 +395,16 @@ __device__ __forceinline__ size_t run_base(uint4 info) { return (size_t)info.x |
 template <bool DIR>
 __global__ void __launch_bounds__(FAM, 6)
     k_family_matvec(const uint4 *__restrict__ fam, const uint32_t *__restrict__ prun, const uint4 *__restrict__ pinfo,
-                    size_t n_fam, size_t n_patch, int max_run, const float *__restrict__ dtab,
+                    size_t n_fam, size_t n_patch, int max_run, const Cube<float> *__restrict__ tab,
                     const float *__restrict__ x, float *__restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float *xs = reinterpret_cast<float *>(smem_raw);  // two buffers
   float *ys = xs + 2 * (max_run + 1);
   uint32_t *ids = reinterpret_cast<uint32_t *>(ys + (max_run + 1));  // words of the next patch (a thread reads its own)
-  float *dt = reinterpret_cast<float *>(ids + (max_run + 1));
+  Cube<float> *st = reinterpret_cast<Cube<float> *>(ids + (max_run + 1));
   const int tid = threadIdx.x;
   const uint4 none = make_uint4(0, 0, 0, 0);
-  for (int i = tid; i < DTAB_ENTRIES; i += FAM) dt[i] = dtab[i];
+  if (tid < DTAB_LEVELS) st[tid] = tab[tid];
   for (int i = tid; i <= max_run; i += FAM) ys[i] = 0.f;
   if (tid == 0) xs[0] = xs[max_run + 1] = 0.f;
   auto copy_ids = [&](uint4 info) {
@@ -428,7 +438,7 @@ __global__ void __launch_bounds__(FAM, 6)
     copy_x(next, par ^ 1);
     copy_ids(after);
     if (p * FAM + tid < n_fam)
-      family_floating<float, false>(w, p * FAM + tid, xs + par * (max_run + 1), ys, dt, nullptr, nullptr);
+      family_floating<float, false>(w, p * FAM + tid, xs + par * (max_run + 1), ys, st, nullptr, nullptr);
     const uint32_t *run = prun + run_base(info);
     const int nr = (int)info.z;
     constexpr int AHEAD = 8;
@@ -455,7 +465,7 @@ __global__ void __launch_bounds__(FAM, 6)
   }
 }
 
-inline size_t family_smem(int max_run) { return (4 * (size_t)(max_run + 1) + DTAB_ENTRIES) * 4; }
+inline size_t family_smem(int max_run) { return 16 * (size_t)(max_run + 1) + DTAB_LEVELS * sizeof(Cube<float>); }
 
 // Elements with factors of their own (FP32 and FP64): as above without the
 // copies ahead.
@@ -591,11 +601,11 @@ __device__ __forceinline__ double fix_to_double(long long f, int s) {
 
 // a family of a patch that takes floating point (out of line, it is rare)
 __device__ __noinline__ void family_fp64(const uint4 *__restrict__ fw, const double *xs, double *ys,
-                                         const double *__restrict__ dtab) {
+                                         const Cube<double> *__restrict__ tab) {
   uint4 w[4];
 #pragma unroll
   for (int q = 0; q < 4; q++) w[q] = fw[q * FAM];
-  family_floating<double, false>(w, 0, xs, ys, dtab, nullptr, nullptr);
+  family_floating<double, false>(w, 0, xs, ys, tab, nullptr, nullptr);
 }
 
 // a child whose values, not all zero, lie below 2^-8 of the family's largest
@@ -627,7 +637,7 @@ template <bool DIR>
 __global__ void __launch_bounds__(FAM, 4)
     k_family_matvec_fix(const uint4 *__restrict__ fam, const uint32_t *__restrict__ prun,
                         const uint4 *__restrict__ pinfo, size_t n_fam, size_t n_patch, int max_run,
-                        const int2 *__restrict__ ftab, const double *__restrict__ dtab,
+                        const int2 *__restrict__ ftab, const Cube<double> *__restrict__ tab,
                         const double *__restrict__ x, double *__restrict__ y) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   long long *xs = reinterpret_cast<long long *>(smem_raw);
@@ -690,7 +700,7 @@ __global__ void __launch_bounds__(FAM, 4)
       } else {
         long long v[27];
         plain = plain || fix_uneven(u, mask);
-        lat_elements(u, v, mask, [](int) {}, [&](long long t, int i) { return fix_mul(t, d[DTAB_CHILD + i]); });
+        lat_elements(u, v, mask, [&](long long t, int i) { return fix_mul(t, d[DTAB_CHILD + i]); });
 #pragma unroll
         for (int i = 0; i < 27; i++) u[i] = v[i];
       }
@@ -722,7 +732,7 @@ __global__ void __launch_bounds__(FAM, 4)
         xd[u + 1] = (DIR && (r & PRUN_BDY)) ? 0.0 : x[r & PRUN_NODE];
       }
       __syncthreads();
-      if (have) family_fp64(fam + p * 4 * FAM + tid, xd, reinterpret_cast<double *>(ys), dtab);
+      if (have) family_fp64(fam + p * 4 * FAM + tid, xd, reinterpret_cast<double *>(ys), tab);
     }
     __syncthreads();
 #pragma unroll 1
@@ -744,12 +754,12 @@ inline size_t family_fix_smem(int max_run) { return ((size_t)max_run + 1) * 20 +
 // children are alike: hanging vertices are r = 1, 2, 4 (mean of 0 and r) and 3,
 // 5, 6 (mean of 0, r and its two edges).
 //
-// The rule: a patch takes 12 us in FP32 and 16 us in FP64 from its first load to
+// The rule: a patch takes 10 us in FP32 and 16 us in FP64 from its first load to
 // its last store, however few there are; this chain (node numbers, values, some
-// 120 operations, global atomic adds) is shorter until the atomics, and in FP64
-// the operations, fill the chip.  Patches / elements in us: FP32 12.2 / 6.5 at
-// 4e3 elements, 12.3 / 8.4 at 3.0e4, 12.2 / 10.6 at 8.6e4, 12.0 / 12.6 at 1.35e5;
-// FP64 16.3 / 10.6, 16.4 / 14.5, 17.0 / 18.7 at 4.7e4, 17.9 / 26.3.
+// 60 operations, global atomic adds) is shorter until the atomics, and in FP64
+// the operations, fill the chip.  Patches / elements in us: FP32 10.1 / 7.1 at
+// 7.1e3 elements, 10.4 / 8.5 at 3.7e4, 10.1 / 9.0 at 5.4e4; FP64 15.4 / 8.9 at
+// 7.1e3, 16 / 12.7 at 2.0e4.
 template <typename T>
 constexpr size_t elem_wise_max = sizeof(T) == 4 ? 90000 : 32000;
 
@@ -779,37 +789,26 @@ __global__ void __launch_bounds__(128)
   uint32_t hang = 0;
 #pragma unroll
   for (int r = 1; r < 7; r++) hang |= (hm >> (r ^ c) & 1u) << r;
-  T v[8];
+  T v[8], sum[2] = {(T)0, (T)0};
 #pragma unroll
   for (int r = 0; r < 8; r++) {
     v[r] = u[r];
     const int a = r == 3 || r == 5 ? 1 : 2, b = r ^ a;
     if (hang >> r & 1u) {
-      if (r == 1 || r == 2 || r == 4) v[r] = (T)0.5 * (u[0] + u[r]);
-      else v[r] = (T)0.25 * ((u[0] + u[r]) + (u[a] + u[b]));
+      if (r == 1 || r == 2 || r == 4) v[r] = (T)0.5 * u[0] + (T)0.5 * u[r];
+      else v[r] = ((T)0.25 * u[0] + (T)0.25 * u[r]) + ((T)0.25 * u[a] + (T)0.25 * u[b]);
     }
+    sum[odd_vertex(r)] += (T)0.25 * v[r];
   }
+  const T h = exp2_neg((T)0, me & 31u);
+  const Cube<T> s = cube_of<T>(lapf * h * (T)0.5, massf * h * h * h * (T)0.125);
+  const T cls[2] = {s.cls * sum[0] + s.other * sum[1], s.cls * sum[1] + s.other * sum[0]};
 #pragma unroll
-  for (int s = 1; s < 8; s <<= 1)
-#pragma unroll
-    for (int r = 0; r < 8; r++)
-      if (!(r & s)) {
-        const T p = v[r] + v[r | s], m = v[r] - v[r | s];
-        v[r] = p;
-        v[r | s] = m;
-      }
-  const T h = exp2_neg((T)0, me & 31u), lap = lapf * h * (T)0.5, mass = massf * h * h * h * (T)0.125;
-#pragma unroll
-  for (int r = 0; r < 8; r++) v[r] *= dtab_entry(DTAB_CHILD + (r & 1) + (r >> 1 & 1) + (r >> 2), lap, mass);
-#pragma unroll
-  for (int s = 1; s < 8; s <<= 1)
-#pragma unroll
-    for (int r = 0; r < 8; r++)
-      if (!(r & s)) {
-        const T p = v[r] + v[r | s], m = v[r] - v[r | s];
-        v[r] = p;
-        v[r | s] = m;
-      }
+  for (int r = 0; r < 4; r++) {
+    const T p = v[r], m = v[r ^ 7];
+    v[r] = s.own * p + (s.opp * m + cls[odd_vertex(r)]);
+    v[r ^ 7] = s.own * m + (s.opp * p + cls[odd_vertex(r ^ 7)]);
+  }
   T w[8];
 #pragma unroll
   for (int r = 0; r < 8; r++) w[r] = v[r];

@@ -52,13 +52,12 @@ struct Context {
   float *d_sten32 = nullptr;
   uint8_t *d_etype_of = nullptr;   // [8][256] -> element type or 255
   uint8_t *d_etype_mask = nullptr; // [8][18] -> hanging mask
-  // diagonal tables of the element loop (dg_elem.cuh) for the factors of its
-  // last call
-  struct DiagTable {
+  // tables of the element loop (dg_elem.cuh) for the factors of its last call
+  struct CubeTable {
     void *p = nullptr;
     double lap = 0, mass = 0;
     bool ok = false;
-  } dtab64, dtab32;
+  } cubes64, cubes32;
   bool prof = false;
   std::map<std::string, ProfStat> prof_stats;
   std::vector<ProfPending> prof_pending;
