@@ -36,7 +36,7 @@
 // there; one with subdivided children is applied element by element.
 //
 // On 1.1e7 elements of a Gaussian cloud (GB300) FP32 takes 96 us and FP64
-// vectors 341 us; what bounds them stands at the kernels.  An element-wise loop
+// vectors 344 us; what bounds them stands at the kernels.  An element-wise loop
 // over dense stencils, 8 gathers and 8 atomics per element, took 348 and 1,820
 // us.  128 families per patch: 64 and 256 measured 152 / 150 us where 128 took
 // 143 (FP32); a patch of 256 leaves too few blocks on small meshes.
@@ -522,35 +522,42 @@ inline size_t family_coef_smem(int max_run) {
 //     in units of 2^(k - 3) u.  A child's row sums |entries| to at most
 //     4/3 (|lap| + |mass|), a family's lattice point to 8 of them, so |v| <
 //     2^(55 + 3.42 + 3): sums in between may wrap, the results do not;
-//   - a node's sum is kept in half the finest unit of the families that touch
-//     it: at most 43 times 2^(55 + 2) < 2^63 (4 of 8 octants around it
-//     refined, all their edges and faces hanging).  The unit is the coarsest of
-//     those families', found by one more round of shared-memory atomics where
-//     the patch's families differ by more than FIX_EVEN binary places (without
-//     the rule 394 -> 357 us); the sum becomes FP64 once per node.
+//   - a node's sum is kept in half the unit of the coarsest of the families that
+//     touch it: at most 43 times 2^(55 + 2) < 2^63 (4 of 8 octants around it
+//     refined, all their edges and faces hanging).  That unit is found by one
+//     more round of shared-memory atomics where the patch's families differ by
+//     more than FIX_EVEN binary places (without the rule 394 -> 357 us); the sum
+//     becomes FP64 once per node.
 // Errors in a family's result are a few units, 2^-57 of its largest value
-// times the level's |lap| + |mass|; those of the FP64 form in the same basis
-// are 2^-53 of that.  Measured against extended precision (norm; 1.6e5
-// elements): uniform random x 8.9e-17 (FP64 1.2e-16, dense stencils 1.4e-16),
-// products of sines 3.9e-16 (1.9e-15, 3.0e-15), a Gaussian 1.4e-15 (3.9e-15,
-// 7.0e-15), one node 7.9e-17 (5.1e-17, 2.2e-17).
-// Patches outside that range take floating point, all of it: values that are
-// not finite or not within 2^-511 .. 2^511, factors beyond 2^+-400, and
-// families with subdivided children where a child's values, not all zero, lie
-// below 2^-8 of the family's: FP64 applies those child by child, and the rows
-// that only such a child touches would be less exact here (a bound of 2^-4
-// sent some patches at the domain's corners there in every solve: FP64 solve of
-// 5e5 points 9.37 -> 10.3 ms).
-// What bounds it: 350 us on 1.1e7 elements (DRAM traffic alone 50): 3,500
+// times the level's |lap| + |mass|.  Measured against extended precision (norm;
+// 1.6e5 elements; dense FP64 stencils in brackets): uniform random x 8.9e-17
+// (1.4e-16), products of sines 3.9e-16 (3.0e-15), a Gaussian 8.3e-16 (7.0e-15),
+// one node 1.4e-17 (2.2e-17).
+// Values far below their family's largest do not keep their own last places, so
+// families in which that would show leave the fixed form: each row of a child has
+// a part of the size of its class (the vertices an even number of steps away,
+// itself among them), so where the largest value of every class of every child
+// lies within 2^-4 of the family's, a row is off by at most 2^-44 of the sum of
+// its terms' magnitudes, and mostly by less than FP64 is.  A family with a class
+// below that (1 in 1e4 where x is random) is applied in FP64 and added to y
+// directly (families_alone).  Classes that hold boundary nodes of the Dirichlet
+// form alone have no rows; they occur at the domain's corners in every solve.
+// The limit: at 2^-4, 2^-3, 2^-2 344, 360, 446 us on 1.1e7 elements, 9.2, 9.9, 11.9
+// ms for an FP64 solve of 5e5 points (9.2 without a limit).
+// Patches with values that are not finite or not within 2^-509 .. 2^511, or
+// factors beyond 2^+-400, take floating point, all of them.
+// What bounds it: 344 us on 1.1e7 elements (DRAM traffic alone 50): 3,600
 // instructions per 32 families at 1.5 per clock per SM; warps wait for the
 // gathers (3.0 of 10.5 cycles per instruction), barriers (1.6) and
 // instructions (1.5: the code is long, so loops over nodes unroll no further
-// than they must: by 4 and 1 350 us, 4 and 4 359, 8 and 8 405).  Copying the next
+// than they must: by 4 and 1 350 us, 4 and 4 359, 8 and 8 405, before the limit was looked at).  Copying the next
 // patch's x ahead gains 3% here and loses as much on half as many elements.  Blocks per
 // SM: at 3, 4, 5, 6 451, 387, 411, 480 us.  Small meshes are bound by latency
 // (2e4 elements 16 us).
-// x as one word: its 53-bit mantissa, signed, above a 10-bit exponent (0: zero)
+// x as one word: its 53-bit mantissa, signed, above a 10-bit exponent (0: zero; 1:
+// no value's)
 constexpr int FIX_EXP = 10, FIX_BIAS = 511;
+constexpr long long FIX_EDGE = 1;  // a boundary column of the Dirichlet form
 constexpr uint32_t FIX_EVEN = 2;
 constexpr uint32_t FIX_EMASK = (1u << FIX_EXP) - 1;
 
@@ -558,7 +565,7 @@ __device__ __forceinline__ long long fix_pack(double v, bool &outside) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
   if (!(b << 1)) return 0;
   const int e = ((int)(b >> 52) & 0x7ff) - FIX_BIAS;
-  outside = outside || e < 1 || e > (int)FIX_EMASK;
+  outside = outside || e < 2 || e > (int)FIX_EMASK;
   const long long m = (long long)((b & 0xfffffffffffffull) | 1ull << 52);
   return (long long)((unsigned long long)((long long)b < 0 ? -m : m) << FIX_EXP) | (e & (int)FIX_EMASK);
 }
@@ -608,29 +615,88 @@ __device__ __noinline__ void family_fp64(const uint4 *__restrict__ fw, const dou
   family_floating<double, false>(w, 0, xs, ys, tab, nullptr, nullptr);
 }
 
-// a child whose values, not all zero, lie below 2^-8 of the family's largest
-// (which is 2^54 or more)
-__device__ __forceinline__ bool fix_uneven(const long long (&u)[27], uint32_t mask) {
-  uint32_t m[27];  // upper words' magnitudes, then their unions over an element
+// The families of a patch that go alone (a bit each), in FP64 from x and onto y, a
+// pair of warps for each: thread = child and vertex.  One thread per family took
+// 17 us: a warp issues an FP64 operation every 64 clocks, however few lanes.  A
+// vertex hangs where the family has no node at its lattice point.
+template <bool DIR>
+__device__ __noinline__ void families_alone(const uint4 *__restrict__ fam, const uint32_t *alone,
+                                            const uint32_t *__restrict__ run, const double *x, double *y,
+                                            const Cube<double> *__restrict__ tab) {
+  const int k = threadIdx.x & 7, c = threadIdx.x >> 3 & 7, d = k ^ c, low = d & -d;
+  int turn = 0;
+  for (int w = 0; w < FAM / 32; w++)
+    for (uint32_t m = alone[w]; m; m &= m - 1, turn++) {
+      if ((turn & 1) != (int)(threadIdx.x >> 6)) continue;
+      const uint4 *fw = fam + 32 * w + __ffs((int)m) - 1;
+      auto u16 = [&](int i) -> uint32_t { return reinterpret_cast<const uint16_t *>(fw + (i >> 3) * FAM)[i & 7]; };
+      const bool there = u16(28) >> c & 1u;
+      const uint32_t own = u16(lat_vertex(c, k));
+      const int cnt = own ? 1 : __popc(d) == 1 ? 2 : 4;  // nodes that the vertex takes the mean of
+      const double share = cnt == 1 ? 1.0 : cnt == 2 ? 0.5 : 0.25;
+      uint32_t r[4];
+      double u = 0.0;
 #pragma unroll
-  for (int i = 0; i < 27; i++) {
-    const int h = (int)(u[i] >> 32);
-    m[i] = (uint32_t)(h ^ h >> 31);
-  }
-  bool any = false;
+      for (int j = 0; j < 4; j++) {
+        const int s = j == 0 ? 0 : j == 1 ? low : j == 2 ? d ^ low : d;
+        const uint32_t n = !there || j >= cnt ? 0u : own ? own : u16(lat_corner(c ^ s));
+        r[j] = n ? run[n - 1] : PRUN_NODE;  // PRUN_NODE: no row
+        if (n && !(DIR && (r[j] & PRUN_BDY))) u += x[r[j] & PRUN_NODE] * share;
+        else r[j] = PRUN_NODE;
+      }
+      const Cube<double> s = tab[u16(27) & 31u];
+      const double opp = __shfl_xor_sync(0xffffffffu, u, 7);
+      const double sum = 0.25 * u + 0.25 * __shfl_xor_sync(0xffffffffu, u, 3) +
+                         0.25 * __shfl_xor_sync(0xffffffffu, u, 5) + 0.25 * __shfl_xor_sync(0xffffffffu, u, 6);
+      const double other = __shfl_xor_sync(0xffffffffu, sum, 7);
+      const double v = (s.own * u + (s.opp * opp + (s.cls * sum + s.other * other))) * share;
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (r[j] != PRUN_NODE) atomicAdd(&y[r[j] & PRUN_NODE], v);
+    }
+}
+
+// the upper words' magnitudes of the family's values, united over each class of
+// each child: the least of them (children that are not there left out) ...
+constexpr uint32_t FIX_SMALL = 1u << 18;  // 2^-4 of a family's largest, which is 2^54 or more
+__device__ __forceinline__ uint32_t fix_least(const long long (&u)[27], uint32_t mask) {
+  uint32_t m[27], least = 0xffffffffu;
+#pragma unroll
+  for (int i = 0; i < 27; i++) m[i] = (uint32_t)abs((int)(u[i] >> 32));
 #pragma unroll
   for (int c = 0; c < 8; c++) {
-    uint32_t o = 0;
+    uint32_t o[2];
+    o[0] = o[1] = (mask >> c & 1u) ? 0u : 0xffffffffu;
 #pragma unroll
-    for (int k = 0; k < 8; k++) o |= m[lat_vertex(c, k)];
-    if ((mask >> c & 1u) && o < 1u << 14) {
-      long long nz = 0;
+    for (int k = 0; k < 8; k++) o[odd_vertex(k)] |= m[lat_vertex(c, k)];
+    least = min(least, min(o[0], o[1]));
+  }
+  return least;
+}
+// ... and whether one below the limit has a node that is not a boundary column
+// (fw: the family's words, xs: the patch's packed values)
+__device__ __forceinline__ bool fix_rows(const long long (&u)[27], uint32_t mask, const uint4 *__restrict__ fw,
+                                         const long long *xs) {
+  uint32_t small = 0;  // bit 2 c the even class of child c, 2 c + 1 the odd one
 #pragma unroll
-      for (int k = 0; k < 8; k++) nz |= u[lat_vertex(c, k)];
-      any = any || nz != 0;
+  for (int c = 0; c < 8; c++) {
+    uint32_t o[2] = {0, 0};
+#pragma unroll
+    for (int k = 0; k < 8; k++) o[odd_vertex(k)] |= (uint32_t)abs((int)(u[lat_vertex(c, k)] >> 32));
+    if (mask >> c & 1u) small |= (o[0] < FIX_SMALL ? 1u << (2 * c) : 0u) | (o[1] < FIX_SMALL ? 2u << (2 * c) : 0u);
+  }
+#pragma unroll 1
+  for (; small; small &= small - 1) {
+    const int b = __ffs((int)small) - 1;
+#pragma unroll 1
+    for (int k = 0; k < 8; k++) {
+      if (odd_vertex(k) != (b & 1)) continue;
+      const int i = lat_vertex(b >> 1, k);
+      const uint32_t n = reinterpret_cast<const uint16_t *>(fw + (i >> 3) * FAM)[i & 7];
+      if (!n || xs[n] != FIX_EDGE) return true;
     }
   }
-  return any;
+  return false;
 }
 
 template <bool DIR>
@@ -644,7 +710,8 @@ __global__ void __launch_bounds__(FAM, 4)
   long long *ys = xs + (max_run + 1);
   int2 *ft = reinterpret_cast<int2 *>(ys + (max_run + 1));
   uint32_t *unit = reinterpret_cast<uint32_t *>(ft + DTAB_ENTRIES);
-  __shared__ uint32_t s_q[2];  // most and least unit of the patch's families
+  __shared__ uint32_t s_q[2];           // most and least unit of the patch's families
+  __shared__ uint32_t s_alone[FAM / 32];  // families that go alone
   const int tid = threadIdx.x;
   for (int i = tid; i < DTAB_ENTRIES; i += FAM) ft[i] = ftab[i];
   if (tid == 0) xs[0] = 0;
@@ -662,7 +729,7 @@ __global__ void __launch_bounds__(FAM, 4)
 #pragma unroll 4
     for (int u = tid; u < nr; u += FAM) {
       const uint32_t r = prun[base + u];
-      xs[u + 1] = (DIR && (r & PRUN_BDY)) ? 0ll : fix_pack(x[r & PRUN_NODE], plain);
+      xs[u + 1] = (DIR && (r & PRUN_BDY)) ? FIX_EDGE : fix_pack(x[r & PRUN_NODE], plain);
       ys[u + 1] = 0;
       unit[u + 1] = 0;
     }
@@ -679,19 +746,26 @@ __global__ void __launch_bounds__(FAM, 4)
       }
       plain = plain || k == FIX_NONE;
     }
-    const uint32_t q = emax ? emax + (uint32_t)k + 1024u : 0u;
-    const uint32_t hi = __reduce_max_sync(0xffffffffu, q), lo = __reduce_min_sync(0xffffffffu, q ? q : 0xffffffffu);
-    if ((tid & 31) == 0) {
-      atomicMax(&s_q[0], hi);
-      atomicMin(&s_q[1], lo);
-    }
-    if (emax) {
+    bool alone = false;
+    if (emax > 1) {
 #pragma unroll
       for (int i = 0; i < 27; i++) {
         const uint32_t e = (uint32_t)u[i] & FIX_EMASK;
         u[i] = fix_shr(u[i] & ~(long long)FIX_EMASK, FIX_EXP - 2 + emax - e);
       }
       lat_interpolate(u, hang);
+      if (fix_least(u, mask) < FIX_SMALL) alone = !DIR || fix_rows(u, mask, fam + p * 4 * FAM + tid, xs);
+    }
+    const bool fixed = emax > 1 && !alone;
+    const uint32_t q = fixed ? emax + (uint32_t)k + 1024u : 0u;
+    const uint32_t hi = __reduce_max_sync(0xffffffffu, q), lo = __reduce_min_sync(0xffffffffu, q ? q : 0xffffffffu);
+    const uint32_t apart = __ballot_sync(0xffffffffu, alone);
+    if ((tid & 31) == 0) {
+      atomicMax(&s_q[0], hi);
+      atomicMin(&s_q[1], lo);
+      s_alone[tid >> 5] = apart;
+    }
+    if (fixed) {
       const int2 *d = ft + level * DTAB_STRIDE;
       if (__all_sync(__activemask(), mask == 255u)) {
         lat_forward(u);
@@ -699,7 +773,6 @@ __global__ void __launch_bounds__(FAM, 4)
         lat_backward(u);
       } else {
         long long v[27];
-        plain = plain || fix_uneven(u, mask);
         lat_elements(u, v, mask, [&](long long t, int i) { return fix_mul(t, d[DTAB_CHILD + i]); });
 #pragma unroll
         for (int i = 0; i < 27; i++) u[i] = v[i];
@@ -711,7 +784,7 @@ __global__ void __launch_bounds__(FAM, 4)
     const bool even = qmax - qmin <= FIX_EVEN;
     if (!plain) {
       if (!even) {
-        if (emax)
+        if (fixed)
 #pragma unroll
           for (int i = 0; i < 27; i++) {
             const uint32_t n = fam_u16(w, i);
@@ -719,7 +792,7 @@ __global__ void __launch_bounds__(FAM, 4)
           }
         __syncthreads();
       }
-      if (emax)
+      if (fixed)
 #pragma unroll
         for (int i = 0; i < 27; i++) {
           const uint32_t n = fam_u16(w, i);
@@ -735,15 +808,18 @@ __global__ void __launch_bounds__(FAM, 4)
       if (have) family_fp64(fam + p * 4 * FAM + tid, xd, reinterpret_cast<double *>(ys), tab);
     }
     __syncthreads();
+    static_assert(FAM == 128, "four words of families");
+    const bool store = plain || !(s_alone[0] | s_alone[1] | s_alone[2] | s_alone[3]);
 #pragma unroll 1
     for (int u = tid; u < nr; u += FAM) {
       const uint32_t r = prun[base + u], g = r & PRUN_NODE;
       const double v = plain ? __longlong_as_double(ys[u + 1])
                              : fix_to_double(ys[u + 1], 1024 + 1079 - FIX_BIAS - (int)(even ? qmax : unit[u + 1]));
       if (DIR && (r & PRUN_BDY)) y[g] = x[g];
-      else if (r & PRUN_COMPLETE) y[g] = v;
+      else if ((r & PRUN_COMPLETE) && store) y[g] = v;
       else atomicAdd(&y[g], v);
     }
+    if (!store) families_alone<DIR>(fam + p * 4 * FAM, s_alone, prun + base, x, y, tab);
   }
 }
 

@@ -12,6 +12,11 @@ transpose 6, sums of a class 5, its two products 3, a row 4, the 8 elements of a
 family 8, the families of a node 8, factors 4: 38, and as many in the FP64
 reference: 64 in FP32, 96 in FP64.
 
+FP64 by families runs in fixed point: the values are cut at U = 2^-54 of the
+family's largest, which a row's terms (2 (lap + mass) U with the roundings) feel by
+at most 2^5 (classes of vertices reach 2^-5 of the largest) times 6 / 2: 96 u of
+the bound, and 256 with both.
+
 The reference is the dense form in FP64 with the matrices' zeros as zeros (the
 oracle's stencil tables hold 1e-17 in their place where the compiler contracts
 multiplications and additions)."""
@@ -162,3 +167,15 @@ def test_double_precision_element_by_element(mesh, field):
     for lap, mass in ((1.0, 1.0), (1.0, 0.0), (0.0, 1.0), (-3.0, 40.0)):
         _check(da.matvec(_put(x, p), lapFac=lap, massFac=mass)[p], dense.apply(x, lap, mass), dense.bound(x, lap, mass), 96, 2.0**-53)
     _check(MultiGrid(bal).matvec(0, _put(x, p))[p], *dense.dirichlet(x), 96, 2.0**-53)
+
+
+@pytest.mark.parametrize("field", FIELDS)
+def test_double_precision_by_families(mesh, field):
+    bal, da, oda, p, dense = mesh
+    if not da.compressLut and da.n_elem < 32_000:
+        pytest.skip("goes element by element")
+    x = _field(field, oda)
+    for lap, mass in ((1.0, 1.0), (1.0, 0.0), (0.0, 1.0), (-3.0, 40.0)):
+        _check(da.matvec(_put(x, p), lapFac=lap, massFac=mass)[p], dense.apply(x, lap, mass), dense.bound(x, lap, mass), 256, 2.0**-53)
+    if not da.compressLut:
+        _check(MultiGrid(bal).matvec(0, _put(x, p))[p], *dense.dirichlet(x), 256, 2.0**-53)
