@@ -173,11 +173,9 @@ int dg_ctx_destroy(dg_ctx ctx) {
   if (ctx->c.d_scratch) cudaFree(ctx->c.d_scratch);
   if (ctx->c.h_scratch) cudaFreeHost(ctx->c.h_scratch);
   if (ctx->c.d_sten64) cudaFree(ctx->c.d_sten64);
-  if (ctx->c.d_sten32) cudaFree(ctx->c.d_sten32);
   for (dg::Context::CubeTable *t : {&ctx->c.cubes64, &ctx->c.cubes32})
     if (t->p) cudaFree(t->p);
   if (ctx->c.d_etype_of) cudaFree(ctx->c.d_etype_of);
-  if (ctx->c.d_etype_mask) cudaFree(ctx->c.d_etype_mask);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->c.side_ev[0]) cudaEventDestroy(ctx->c.side_ev[0]);
@@ -710,11 +708,10 @@ int dg_mg_level_octree(dg_ctx ctx, dg_mg mg, size_t level, uint32_t *xyzl, int d
 int dg_mg_matvec(dg_ctx ctx, dg_mg mg, size_t level, const void *in, void *out, int precision, int on_device) {
   if (!mg || level >= mg->mg.lv.size()) return DG_ERR_INVALID_ARG;
   const dg::MGLevel &L = mg->mg.lv[level];
-  const bool ds = precision == 48;  // FP64 vectors, fixed-point arithmetic
-  return level_op(ctx, mg, L.mesh.n_node, L.mesh.n_node, in, out, ds ? 64 : precision, on_device,
+  if (precision == 48) precision = 64;  // one loop on FP64 vectors
+  return level_op(ctx, mg, L.mesh.n_node, L.mesh.n_node, in, out, precision, on_device,
                   [&](dg::Context &c, const void *x, void *y) {
-                    if (ds) dg::dirichlet_matvec_ds(c, L, (const double *)x, (double *)y);
-                    else if (precision == 64) dg::dirichlet_matvec<double>(c, L, (const double *)x, (double *)y);
+                    if (precision == 64) dg::dirichlet_matvec<double>(c, L, (const double *)x, (double *)y);
                     else dg::dirichlet_matvec<float>(c, L, (const float *)x, (float *)y);
                   });
 }

@@ -114,33 +114,24 @@ void ensure_stencils(Context &ctx) {
   std::vector<double> lap(8 * 18 * 64), mass(8 * 18 * 64);
   gen_stencils(lap.data(), mass.data());
   std::vector<double> s64(STEN_ENTRIES);
-  std::vector<float> s32(STEN_ENTRIES);
   for (int ct = 0; ct < 8 * 18; ct++)
     for (int q = 0; q < 64; q++) {
       s64[ct * 128 + q] = lap[ct * 64 + q];
       s64[ct * 128 + 64 + q] = mass[ct * 64 + q];
     }
-  for (int i = 0; i < STEN_ENTRIES; i++) s32[i] = (float)s64[i];
   uint8_t masks[8 * 18], etype_of[8 * 256];
   gen_etype_masks(masks);
   std::memset(etype_of, 0xff, sizeof(etype_of));
   for (int c = 0; c < 8; c++)
     for (int t = 0; t < 18; t++) etype_of[c * 256 + masks[c * 18 + t]] = (uint8_t)t;
   double *d64 = nullptr;
-  float *d32 = nullptr;
-  uint8_t *det = nullptr, *dem = nullptr;
+  uint8_t *det = nullptr;
   DG_CUDA(cudaMalloc((void **)&d64, STEN_ENTRIES * sizeof(double)));
-  DG_CUDA(cudaMalloc((void **)&d32, STEN_ENTRIES * sizeof(float)));
   DG_CUDA(cudaMalloc((void **)&det, sizeof(etype_of)));
-  DG_CUDA(cudaMalloc((void **)&dem, sizeof(masks)));
   DG_CUDA(cudaMemcpy(d64, s64.data(), STEN_ENTRIES * sizeof(double), cudaMemcpyHostToDevice));
-  DG_CUDA(cudaMemcpy(d32, s32.data(), STEN_ENTRIES * sizeof(float), cudaMemcpyHostToDevice));
   DG_CUDA(cudaMemcpy(det, etype_of, sizeof(etype_of), cudaMemcpyHostToDevice));
-  DG_CUDA(cudaMemcpy(dem, masks, sizeof(masks), cudaMemcpyHostToDevice));
   ctx.d_sten64 = d64;
-  ctx.d_sten32 = d32;
   ctx.d_etype_of = det;
-  ctx.d_etype_mask = dem;
 }
 
 // ------------------------------------------------------------------------
@@ -849,7 +840,6 @@ struct PatchFamSmem {
   uint32_t node[FAM_MAX_RUN];    // node of each number
   uint16_t num[PF_HT];           // number of each hash slot
   uint8_t order[FAM];            // family at each place
-  uint32_t minlev;
   int counter;
   unsigned long long base;
 };
@@ -865,10 +855,7 @@ __global__ void __launch_bounds__(FAM)
   const int t = threadIdx.x, lane = t & 31;
   const size_t p = blockIdx.x;
   for (int i = t; i < PF_HT; i += FAM) S.hkey[i] = NO_NODE;
-  if (t == 0) {
-    S.counter = 0;
-    S.minlev = 31;
-  }
+  if (t == 0) S.counter = 0;
   __syncthreads();
   // 1. complete families first
   {
@@ -889,7 +876,6 @@ __global__ void __launch_bounds__(FAM)
     mask = state[f] >> 24;
     hang = state[f] & 0x3ffffu;
     lev = state[f] >> STATE_LEVEL & 31u;
-    atomicMin(&S.minlev, lev);
     uint4 *fc = reinterpret_cast<uint4 *>(fchild + 8 * (p * FAM + t));
     uint4 el[4];
 #pragma unroll
@@ -931,7 +917,7 @@ __global__ void __launch_bounds__(FAM)
   if (t == 0) {
     S.base = atomicAdd(n_run, (unsigned long long)nr);
     atomicMax(max_run, (uint32_t)nr);
-    pinfo[p] = make_uint4((uint32_t)S.base, (uint32_t)(S.base >> 32), (uint32_t)nr, S.minlev);
+    pinfo[p] = make_uint4((uint32_t)S.base, (uint32_t)(S.base >> 32), (uint32_t)nr, 0u);
   }
   uint32_t w[16];
 #pragma unroll

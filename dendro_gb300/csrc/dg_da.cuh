@@ -25,7 +25,7 @@ struct Mesh {
   size_t n_fam = 0, n_patch = 0, n_run = 0;
   int max_run = 0;             // most nodes of a patch
   uint4 *fam = nullptr;        // 4 x FAM words per patch
-  uint4 *pinfo = nullptr;      // per patch: offset in prun (64 bits), nodes, coarsest level
+  uint4 *pinfo = nullptr;      // per patch: offset in prun (64 bits), nodes
   uint32_t *prun = nullptr;    // nodes of each patch with two flags
   uint32_t *fchild = nullptr;  // 8 per family: the element of each child that is a leaf
   // compressed mode (the reference's compressLut): conn is released once the

@@ -47,8 +47,8 @@
 // lattice point (0: no node there), then 16 bits level and 8 bits mask of the
 // children that are leaves, then 18 bits of hanging points.  Complete families
 // come first, so that most warps hold one kind.  pinfo[p] = {offset of the
-// patch's nodes in prun (64 bits), their number, the level of its coarsest
-// element}; prun holds the nodes, number 1 first, with two flags.
+// patch's nodes in prun (64 bits), their number, unused}; prun holds the nodes,
+// number 1 first, with two flags.
 #pragma once
 
 #include "dg_prims.cuh"

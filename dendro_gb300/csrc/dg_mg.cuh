@@ -36,8 +36,8 @@ struct MG {
   float *cinv32 = nullptr;   // its inverse in FP32 (refined in FP64 when the FP64 V-cycle applies it)
   double omega = 0.667;  // Jacobi damping (bin/options:190)
   int nu_pre = 2, nu_post = 2;
-  // CG operator with an FP32 V-cycle: 48 (the default) applies A p in
-  // 64-bit fixed point on FP64 vectors (dg_elem.cuh); 64 in FP64; 32 in FP32, with the recurrence residual
+  // CG operator with an FP32 V-cycle: 48 (the default) and 64 apply A p to the
+  // FP64 vectors (dg_elem.cuh); 32 in FP32, with the recurrence residual
   // replaced by the FP64 residual b - A x whenever it has fallen by
   // reliable_delta since the last replacement (and before stopping)
   int cg_operator = 48;
@@ -65,8 +65,6 @@ void mg_solve(Context &ctx, MG &mg, const double *b, double *x, int precision, d
 // building blocks (level operators), exposed for tests and callers
 template <typename T>
 void dirichlet_matvec(Context &ctx, const MGLevel &L, const T *x, T *y);  // DirichletJacobianMatMult
-// the same operator on FP64 vectors in 64-bit fixed point (dg_elem.cuh)
-void dirichlet_matvec_ds(Context &ctx, const MGLevel &L, const double *x, double *y);
 // DirichletJacobianMatGetDiagonal (omgJac.C:1111): 1 on boundary nodes
 void dirichlet_diagonal(Context &ctx, const MGLevel &L, double *diag);
 template <typename T>

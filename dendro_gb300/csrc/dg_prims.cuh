@@ -25,8 +25,6 @@ struct KeyOps<uint64_t> {
   static constexpr int BITS = 64;
   __device__ __forceinline__ static unsigned digit(uint64_t k, int shift) { return (unsigned)(k >> shift) & 0xffu; }
   __device__ __forceinline__ static bool eq(uint64_t a, uint64_t b) { return a == b; }
-  __device__ __forceinline__ static uint64_t bor(uint64_t a, uint64_t b) { return a | b; }
-  __device__ __forceinline__ static uint64_t band(uint64_t a, uint64_t b) { return a & b; }
 };
 
 template <>
@@ -38,8 +36,6 @@ struct KeyOps<Key128> {
     return (unsigned)((k.lo >> shift) | (k.hi << (64 - shift))) & 0xffu;
   }
   __device__ __forceinline__ static bool eq(Key128 a, Key128 b) { return a.lo == b.lo && a.hi == b.hi; }
-  __device__ __forceinline__ static Key128 bor(Key128 a, Key128 b) { return Key128{a.lo | b.lo, a.hi | b.hi}; }
-  __device__ __forceinline__ static Key128 band(Key128 a, Key128 b) { return Key128{a.lo & b.lo, a.hi & b.hi}; }
 };
 
 // ------------------------------------------------------------------------
@@ -572,9 +568,9 @@ __global__ void k_flag_unique(const K *__restrict__ keys, size_t n, uint32_t *__
 // memory (bitonic network, padded with the largest key), repeated keys are
 // dropped and the rest written in order with their count.  Keys agree on
 // every bit above the sorted ones, so whole-key order is the radix order.
-// Used by sort_unique below the size where the radix sort's passes, each a
-// launch, and its histogram read-back cost more than the keys themselves
-// (the deep and coarse levels of a balance, most multigrid levels).
+// Used by sort_unique (completeOctree, the sorts of records) below the size where
+// the radix sort's passes, each a launch, and its read-back cost more than the
+// keys themselves.
 constexpr int SMALL_SORT_MAX = 4096;
 constexpr int SMALL_SORT_BLOCK = 1024;
 

@@ -47,11 +47,9 @@ struct Context {
   unsigned long long *h_scratch = nullptr;  // pinned mirror of d_scratch
   int num_sms = 0;
   std::string last_error;
-  // stencil tables (FP64 and FP32) on the device, created on first use
+  // stencil tables on the device, created on first use
   double *d_sten64 = nullptr;
-  float *d_sten32 = nullptr;
   uint8_t *d_etype_of = nullptr;   // [8][256] -> element type or 255
-  uint8_t *d_etype_mask = nullptr; // [8][18] -> hanging mask
   // tables of the element loop (dg_elem.cuh) for the factors of its last call
   struct CubeTable {
     void *p = nullptr;
