@@ -17,14 +17,14 @@
 // the reference's 18 element types, so the elements themselves are all the
 // plain trilinear one, and no stencil table is read.
 //
-// Elements in floating point: of the 8 x 8 entries of the trilinear K and M only
-// those of a vertex itself, of its opposite and of its class (the vertices an
-// even number of steps away) and the other class differ from one another, so a
-// row is one multiply-add for each of the first two and the classes' sums,
-// formed once per element (lat_cubes): 36 operations per element where a dense
-// stencil takes 64 multiply-adds.  Every row is a sum of its own entries times
-// x, as with the stencil, so a row among small values keeps its accuracy beside
-// large ones.
+// Elements in floating point (cube_rows): the entries of the trilinear K are 0
+// for vertices an odd number of steps apart but for the opposite one, and its rows
+// sum to 0, so K x needs the differences within a vertex's class (the vertices an
+// even number of steps away) and to its opposite only; M adds the classes' sums.
+// 44 operations per element where a dense stencil takes 64 multiply-adds.  Every
+// row is made of its own entries times x, as with the stencil, so a row among
+// small values keeps its accuracy beside large ones; and of differences, so that
+// smooth fields, on which the stencil's terms cancel, keep theirs.
 //
 // Elements in fixed point: K and M are tensor products, diagonal in a basis of
 // sums and differences.  For the assembled 2x2x2 family, per axis
@@ -35,7 +35,7 @@
 // line, all coefficients 1 or 2) and 27 multiplications, which are what counts
 // there; one with subdivided children is applied element by element.
 //
-// On 1.1e7 elements of a Gaussian cloud (GB300) FP32 takes 96 us and FP64
+// On 1.1e7 elements of a Gaussian cloud (GB300) FP32 takes 105 us and FP64
 // vectors 344 us; what bounds them stands at the kernels.  An element-wise loop
 // over dense stencils, 8 gathers and 8 atomics per element, took 348 and 1,820
 // us.  128 families per patch: 64 and 256 measured 152 / 150 us where 128 took
@@ -105,18 +105,44 @@ __device__ __forceinline__ bool is_finite(double v) {
   return ((uint32_t)__double2hiint(v) & 0x7ff00000u) != 0x7ff00000u;
 }
 
-// The trilinear element's operator lap K + mass M (scaled by h / 2 and h^3 / 8):
-// row i is own x_i + opp x_opposite + cls (sum of i's class) / 4 + other (sum of
-// the other class) / 4.  Quarters, so that a sum stays within the range of its
-// terms.
+// The trilinear element's operator lap K + mass M (scaled by h / 2 and h^3 / 8).
+// With r one vertex of i's class, e = x - r within it, E the sum of those, D = x of
+// i's opposite - x_i, and T the sum over the other class: row i is
+//   within e_i + across D_i + cls E + other (T + 11/4 r).
 template <typename T>
 struct __align__(16) Cube {
-  T own, opp, cls, other;
+  T within, across, cls, other;
 };
 template <typename T>
 __device__ __forceinline__ Cube<T> cube_of(T lap, T mass) {
-  return Cube<T>{lap * (T)(5.0 / 6.0) + mass * (T)(2.0 / 9.0), -lap * (T)(1.0 / 6.0) - mass * (T)(1.0 / 9.0),
-                 -lap * (T)(2.0 / 3.0) + mass * (T)(8.0 / 27.0), mass * (T)(16.0 / 27.0)};
+  return Cube<T>{lap * (T)(2.0 / 3.0) + mass * (T)(1.0 / 9.0), -lap * (T)(1.0 / 6.0) - mass * (T)(1.0 / 9.0),
+                 -lap * (T)(1.0 / 6.0) + mass * (T)(2.0 / 27.0), mass * (T)(4.0 / 27.0)};
+}
+// the rows of one element, add(k, row) for vertex k; classes {0, 3, 5, 6} and
+// their opposites {7, 4, 2, 1}
+template <typename T, typename X, typename Add>
+__device__ __forceinline__ void cube_rows(const Cube<T> &s, X &&x, Add &&add) {
+  T e[2][4], c[2], sum[2];
+#pragma unroll
+  for (int p = 0; p < 2; p++) {
+    const int o = 7 * p;
+    const T r = x(o);
+    e[p][1] = x(3 ^ o) - r;
+    e[p][2] = x(5 ^ o) - r;
+    e[p][3] = x(6 ^ o) - r;
+    const T all = e[p][1] + e[p][2] + e[p][3];
+    sum[p] = (T)4 * r + all;
+    c[p] = s.cls * all + s.other * (T)2.75 * r;
+  }
+  c[0] += s.other * sum[1];
+  c[1] += s.other * sum[0];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    const int k = j == 0 ? 0 : j == 1 ? 3 : j == 2 ? 5 : 6;
+    const T d = s.across * (x(k ^ 7) - x(k));
+    add(k, j == 0 ? d + c[0] : s.within * e[0][j] + (d + c[0]));
+    add(k ^ 7, j == 0 ? c[1] - d : s.within * e[1][j] + (c[1] - d));
+  }
 }
 // ... per level
 template <typename T>
@@ -125,7 +151,7 @@ __global__ void k_cube_table(Cube<T> *__restrict__ out, double lapf, double mass
   if (l >= DTAB_LEVELS) return;
   const double h = ldexp(1.0, -l);
   const Cube<double> c = cube_of<double>(lapf * h * 0.5, massf * h * h * h * 0.125);
-  out[l] = Cube<T>{(T)c.own, (T)c.opp, (T)c.cls, (T)c.other};
+  out[l] = Cube<T>{(T)c.within, (T)c.across, (T)c.cls, (T)c.other};
 }
 
 // entry i of the table of modes, lap and mass scaled likewise
@@ -211,18 +237,9 @@ __device__ __forceinline__ void lat_cubes(const T (&u)[27], T (&v)[27], uint32_t
 #pragma unroll
   for (int i = 0; i < 27; i++) v[i] = (T)0;
 #pragma unroll
-  for (int c = 0; c < 8; c++) {
-    if (!(mask >> c & 1u)) continue;
-    const Cube<T> s = coef(c);
-    T sum[2] = {(T)0, (T)0};
-#pragma unroll
-    for (int k = 0; k < 8; k++) sum[odd_vertex(k)] += (T)0.25 * u[lat_vertex(c, k)];
-    const T cls[2] = {s.cls * sum[0] + s.other * sum[1], s.cls * sum[1] + s.other * sum[0]};
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-      v[lat_vertex(c, k)] +=
-          s.own * u[lat_vertex(c, k)] + (s.opp * u[lat_vertex(c, k ^ 7)] + cls[odd_vertex(k)]);
-  }
+  for (int c = 0; c < 8; c++)
+    if (mask >> c & 1u)
+      cube_rows<T>(coef(c), [&](int k) { return u[lat_vertex(c, k)]; }, [&](int k, T row) { v[lat_vertex(c, k)] += row; });
 }
 
 // a complete family: to the sum / difference basis and back, in place
@@ -337,15 +354,18 @@ __device__ __forceinline__ uint32_t fam_hang(const uint4 (&w)[4]) {
 // Family f in floating point: its lattice from xs, its elements in registers,
 // its lattice added into ys with shared-memory atomics.  COEF: element e's
 // factors are coef[2e] (Laplacian) and coef[2e + 1] (mass) instead of the
-// table's; fchild[8 f + c] gives e.
+// table's; fchild[8 f + c] gives e.  Differences and sums of the values may pass
+// the end of the range where the rows do not: where the results are not all
+// finite, nothing is added and the caller tries again with values scaled down (by a
+// power of two below 1).
 template <typename T, bool COEF>
-__device__ __forceinline__ void family_floating(const uint4 (&w)[4], size_t f, const T *xs, T *ys, const Cube<T> *tab,
+__device__ __forceinline__ bool family_floating(const uint4 (&w)[4], size_t f, const T *xs, T *ys, const Cube<T> *tab,
                                                 const double *__restrict__ coef,
-                                                const uint32_t *__restrict__ fchild) {
+                                                const uint32_t *__restrict__ fchild, T scale = (T)1) {
   const uint32_t hang = fam_hang(w);
   T u[27], v[27];
 #pragma unroll
-  for (int i = 0; i < 27; i++) u[i] = xs[fam_u16(w, i)];
+  for (int i = 0; i < 27; i++) u[i] = xs[fam_u16(w, i)] * scale;
   lat_interpolate(u, hang);
   Cube<T> s;
   if constexpr (!COEF) s = tab[fam_level(w)];
@@ -358,11 +378,29 @@ __device__ __forceinline__ void family_floating(const uint4 (&w)[4], size_t f, c
     return s;
   });
   lat_distribute(v, hang);
+  if (scale == (T)1) {
+    T all = (T)0;
+#pragma unroll
+    for (int i = 0; i < 27; i++) all += v[i];
+    if (!is_finite(all)) return false;
+  }
+  const T back = (T)1 / scale;
 #pragma unroll
   for (int i = 0; i < 27; i++) {
     const uint32_t n = fam_u16(w, i);
-    if (n) atomicAdd(&ys[n], v[i]);
+    if (n) atomicAdd(&ys[n], v[i] * back);
   }
+  return true;
+}
+// ... out of line, fw: the family's words
+template <typename T, bool COEF>
+__device__ __noinline__ void family_scaled(const uint4 *__restrict__ fw, size_t f, const T *xs, T *ys,
+                                           const Cube<T> *tab, const double *__restrict__ coef,
+                                           const uint32_t *__restrict__ fchild) {
+  uint4 w[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) w[q] = fw[q * FAM];
+  family_floating<T, COEF>(w, f, xs, ys, tab, coef, fchild, (T)0.0625);
 }
 
 // FP32: one block per patch, grid-strided, the next patch's x on its way while
@@ -377,10 +415,12 @@ __device__ __forceinline__ void family_floating(const uint4 (&w)[4], size_t f, c
 // DIR, the Dirichlet form: boundary rows are the identity (y = x), boundary
 // columns are dropped.
 //
-// 1.1e7 elements: 96 us; with the elements in the basis of sums and differences,
-// which spilled registers, 109 us, and in that form with x gathered after each
-// barrier 142 us (warps waited 6.6 of 15.2 cycles per instruction for it), with
-// the copies but the words of step 3 loaded in step 3 118 us.  The shared-memory and load/store
+// 1.1e7 elements: 105 us; with the elements in the basis of sums and differences
+// 109 us, and in that form with x gathered after each barrier 142 us (warps waited
+// 6.6 of 15.2 cycles per instruction for it), with the copies but the words of step
+// 3 loaded in step 3 118 us.  With sums of the classes in place of differences 96
+// us, but on 9e7 elements a CG with this operator, which takes 7 iterations to
+// 1e-8, then stops gaining at 1e-5.  The shared-memory and load/store
 // pipe is two thirds busy; DRAM traffic alone would take 34.  Blocks per SM
 // (registers, shared memory): 3, 4, 5, 6 took 165, 135, 121, 118 us; 12 words
 // ahead 112, 4 words 115.
@@ -437,8 +477,9 @@ __global__ void __launch_bounds__(FAM, 6)
     __syncthreads();  // x of this patch is there, ys is zero, the other buffer is free
     copy_x(next, par ^ 1);
     copy_ids(after);
-    if (p * FAM + tid < n_fam)
-      family_floating<float, false>(w, p * FAM + tid, xs + par * (max_run + 1), ys, st, nullptr, nullptr);
+    if (p * FAM + tid < n_fam &&
+        !family_floating<float, false>(w, 0, xs + par * (max_run + 1), ys, st, nullptr, nullptr))
+      family_scaled<float, false>(fam + p * 4 * FAM + tid, 0, xs + par * (max_run + 1), ys, st, nullptr, nullptr);
     const uint32_t *run = prun + run_base(info);
     const int nr = (int)info.z;
     constexpr int AHEAD = 8;
@@ -494,7 +535,8 @@ __global__ void __launch_bounds__(FAM, sizeof(T) == 4 ? 6 : 3)
       ys[u + 1] = (T)0;
     }
     __syncthreads();
-    if (have) family_floating<T, true>(w, p * FAM + tid, xs, ys, nullptr, coef, fchild);
+    if (have && !family_floating<T, true>(w, p * FAM + tid, xs, ys, nullptr, coef, fchild))
+      family_scaled<T, true>(fam + p * 4 * FAM + tid, p * FAM + tid, xs, ys, nullptr, coef, fchild);
     __syncthreads();
 #pragma unroll 4
     for (int u = tid; u < nr; u += FAM) {
@@ -607,12 +649,12 @@ __device__ __forceinline__ double fix_to_double(long long f, int s) {
 }
 
 // a family of a patch that takes floating point (out of line, it is rare)
-__device__ __noinline__ void family_fp64(const uint4 *__restrict__ fw, const double *xs, double *ys,
-                                         const Cube<double> *__restrict__ tab) {
+__device__ __noinline__ bool family_fp64(const uint4 *__restrict__ fw, const double *xs, double *ys,
+                                         const Cube<double> *__restrict__ tab, double scale) {
   uint4 w[4];
 #pragma unroll
   for (int q = 0; q < 4; q++) w[q] = fw[q * FAM];
-  family_floating<double, false>(w, 0, xs, ys, tab, nullptr, nullptr);
+  return family_floating<double, false>(w, 0, xs, ys, tab, nullptr, nullptr, scale);
 }
 
 // The families of a patch that go alone (a bit each), in FP64 from x and onto y, a
@@ -645,11 +687,12 @@ __device__ __noinline__ void families_alone(const uint4 *__restrict__ fam, const
         else r[j] = PRUN_NODE;
       }
       const Cube<double> s = tab[u16(27) & 31u];
-      const double opp = __shfl_xor_sync(0xffffffffu, u, 7);
-      const double sum = 0.25 * u + 0.25 * __shfl_xor_sync(0xffffffffu, u, 3) +
-                         0.25 * __shfl_xor_sync(0xffffffffu, u, 5) + 0.25 * __shfl_xor_sync(0xffffffffu, u, 6);
-      const double other = __shfl_xor_sync(0xffffffffu, sum, 7);
-      const double v = (s.own * u + (s.opp * opp + (s.cls * sum + s.other * other))) * share;
+      // cube_rows with r = x_i: e_i = 0
+      const double e = __shfl_xor_sync(0xffffffffu, u, 3) - u + (__shfl_xor_sync(0xffffffffu, u, 5) - u) +
+                       (__shfl_xor_sync(0xffffffffu, u, 6) - u);
+      const double across = __shfl_xor_sync(0xffffffffu, u, 7) - u;
+      const double sum = __shfl_xor_sync(0xffffffffu, 4.0 * u + e, 7);
+      const double v = (s.across * across + (s.cls * e + s.other * (sum + 2.75 * u))) * share;
 #pragma unroll
       for (int j = 0; j < 4; j++)
         if (r[j] != PRUN_NODE) atomicAdd(&y[r[j] & PRUN_NODE], v);
@@ -805,7 +848,9 @@ __global__ void __launch_bounds__(FAM, 4)
         xd[u + 1] = (DIR && (r & PRUN_BDY)) ? 0.0 : x[r & PRUN_NODE];
       }
       __syncthreads();
-      if (have) family_fp64(fam + p * 4 * FAM + tid, xd, reinterpret_cast<double *>(ys), tab);
+      double *yd = reinterpret_cast<double *>(ys);
+      if (have && !family_fp64(fam + p * 4 * FAM + tid, xd, yd, tab, 1.0))
+        family_fp64(fam + p * 4 * FAM + tid, xd, yd, tab, 0.0625);
     }
     __syncthreads();
     static_assert(FAM == 128, "four words of families");
@@ -832,10 +877,10 @@ inline size_t family_fix_smem(int max_run) { return ((size_t)max_run + 1) * 20 +
 //
 // The rule: a patch takes 10 us in FP32 and 16 us in FP64 from its first load to
 // its last store, however few there are; this chain (node numbers, values, some
-// 60 operations, global atomic adds) is shorter until the atomics, and in FP64
-// the operations, fill the chip.  Patches / elements in us: FP32 10.1 / 7.1 at
-// 7.1e3 elements, 10.4 / 8.5 at 3.7e4, 10.1 / 9.0 at 5.4e4; FP64 15.4 / 8.9 at
-// 7.1e3, 16 / 12.7 at 2.0e4.
+// 70 operations, global atomic adds) is shorter until the atomics, and in FP64
+// the operations, fill the chip.  Patches / elements in us: FP32 10.1 / 6.5 at
+// 7.1e3 elements, 10.4 / 8.6 at 3.7e4, 10.1 / 9.5 at 5.4e4; FP64 15.3 / 10.8 at
+// 7.1e3, 16 / 12.4 at 2.0e4.
 template <typename T>
 constexpr size_t elem_wise_max = sizeof(T) == 4 ? 90000 : 32000;
 
@@ -865,7 +910,7 @@ __global__ void __launch_bounds__(128)
   uint32_t hang = 0;
 #pragma unroll
   for (int r = 1; r < 7; r++) hang |= (hm >> (r ^ c) & 1u) << r;
-  T v[8], sum[2] = {(T)0, (T)0};
+  T v[8];
 #pragma unroll
   for (int r = 0; r < 8; r++) {
     v[r] = u[r];
@@ -874,20 +919,18 @@ __global__ void __launch_bounds__(128)
       if (r == 1 || r == 2 || r == 4) v[r] = (T)0.5 * u[0] + (T)0.5 * u[r];
       else v[r] = ((T)0.25 * u[0] + (T)0.25 * u[r]) + ((T)0.25 * u[a] + (T)0.25 * u[b]);
     }
-    sum[odd_vertex(r)] += (T)0.25 * v[r];
   }
   const T h = exp2_neg((T)0, me & 31u);
   const Cube<T> s = cube_of<T>(lapf * h * (T)0.5, massf * h * h * h * (T)0.125);
-  const T cls[2] = {s.cls * sum[0] + s.other * sum[1], s.cls * sum[1] + s.other * sum[0]};
+  T w[8], all = (T)0;
+  cube_rows<T>(s, [&](int r) { return v[r]; }, [&](int r, T row) {
+    w[r] = row;
+    all += row;
+  });
+  if (!is_finite(all))  // as family_floating
+    cube_rows<T>(s, [&](int r) { return (T)0.0625 * v[r]; }, [&](int r, T row) { w[r] = (T)16 * row; });
 #pragma unroll
-  for (int r = 0; r < 4; r++) {
-    const T p = v[r], m = v[r ^ 7];
-    v[r] = s.own * p + (s.opp * m + cls[odd_vertex(r)]);
-    v[r ^ 7] = s.own * m + (s.opp * p + cls[odd_vertex(r ^ 7)]);
-  }
-  T w[8];
-#pragma unroll
-  for (int r = 0; r < 8; r++) w[r] = v[r];
+  for (int r = 0; r < 8; r++) v[r] = w[r];
 #pragma unroll
   for (int r = 1; r < 7; r++) {
     const int a = r == 3 || r == 5 ? 1 : 2, b = r ^ a;

@@ -5,12 +5,16 @@ element and on meshes (and packed ones) that go by families.
 
 Bound of row i: u B_i times a count of roundings, with u the unit roundoff and
 B = sum over the elements of |P^T| (2 |lap| |K| + 7 |mass| M) |P| |x|, P the
-hanging vertices' interpolation; the factors cover how the loop splits an entry
-between a vertex, its opposite and the classes (own 5/6 + 1/6 where K has 2/3,
-opposite 3/27 + 4/27 where M has 1/27).  Roundings: interpolation and its
-transpose 6, sums of a class 5, its two products 3, a row 4, the 8 elements of a
-family 8, the families of a node 8, factors 4: 38, and as many in the FP64
-reference: 64 in FP32, 96 in FP64.
+hanging vertices' interpolation; the factors cover how a loop splits an entry
+into sums and differences within a vertex's class and to its opposite (opposite
+3/27 + 4/27 where M has 1/27).  Roundings: interpolation and its transpose 6, sums
+and differences of a class 5, its products 3, a row 4, the 8 elements of a family 8,
+the families of a node 8, factors 4: 38, and as many in the FP64 reference: 64 in
+FP32, 96 in FP64.
+
+Smooth fields: the rows of K sum to 0, and a row is as exact as the differences
+between its vertices allow, B = sum of |P^T| (2 |lap| |K_ij| |x_j - x_i| + 7 |mass|
+M |x|), to which hanging vertices, whose values are rounded, add themselves.
 
 FP64 by families runs in fixed point: the values are cut at U = 2^-54 of the
 family's largest, which a row's terms (2 (lap + mass) U with the roundings) feel by
@@ -65,8 +69,32 @@ class Dense:
     def apply(self, x, lap=1.0, mass=1.0):
         return self._sum(x, _K, _M, lap, mass)
 
+    def exact(self, x):
+        """K x + M x in extended precision"""
+        d, ld = self.oda, np.longdouble
+        k = np.array([ld(2) / 3, ld(0), -ld(1) / 6, -ld(1) / 6])[_STEPS]
+        m = np.array([8, 4, 2, 1], ld)[_STEPS] / ld(27)
+        h = (2.0 ** -d.level.astype(float)).astype(ld)
+        y = np.zeros(d.n_node, ld)
+        for e, p in self.groups:
+            a = x.astype(ld)[d.nodes[e]] @ p.T.astype(ld)
+            r = (a @ k) * (h[e] / 2)[:, None] + (a @ m) * (h[e] ** 3 / 8)[:, None]
+            np.add.at(y, d.nodes[e].ravel(), (r @ p.astype(ld)).ravel())
+        return y
+
     def bound(self, x, lap=1.0, mass=1.0):
         return self._sum(np.abs(x), 2 * np.abs(_K), 7 * _M, np.abs(lap), np.abs(mass))
+
+    def smooth_bound(self, x, lap=1.0, mass=1.0):
+        d = self.oda
+        y = self._sum(np.abs(x), 0 * _K, 7 * _M, 0.0, abs(mass))
+        for e, p in self.groups:
+            a = x[d.nodes[e]] @ p.T
+            held = np.abs(a) * ((p != 0).sum(1) > 1)  # hanging
+            diff = np.abs(a[:, None, :] - a[:, :, None]) + held[:, None, :] + held[:, :, None]
+            r = np.einsum("ij,eij->ei", 2 * np.abs(_K), diff) * (abs(lap) * 2.0 ** -d.level[e].astype(float) / 2)[:, None]
+            np.add.at(y, d.nodes[e].ravel(), (r @ np.abs(p)).ravel())
+        return y
 
     def dirichlet(self, x):
         """... with boundary rows the identity and boundary columns dropped"""
@@ -179,3 +207,23 @@ def test_double_precision_by_families(mesh, field):
         _check(da.matvec(_put(x, p), lapFac=lap, massFac=mass)[p], dense.apply(x, lap, mass), dense.bound(x, lap, mass), 256, 2.0**-53)
     if not da.compressLut:
         _check(MultiGrid(bal).matvec(0, _put(x, p))[p], *dense.dirichlet(x), 256, 2.0**-53)
+
+
+@pytest.mark.parametrize("field", ["constant", "linear", "sines"])
+def test_smooth_fields(mesh, field):
+    _, da, oda, p, dense = mesh
+    at = oda.node_xyz / 2.0**DEPTH
+    x = {"constant": np.full(oda.n_node, 0.7), "linear": 1.0 + at @ np.array([0.5, -0.25, 2.0]),
+         "sines": 1.5 + np.sin(np.pi * at).prod(1)}[field]
+    one = np.ones((da.n_elem, 2))
+    for t, roundings, unit in ((np.float32, 64, 2.0**-24), (np.float64, 96, 2.0**-53)):
+        xt = x.astype(t)
+        x64, prec = xt.astype(np.float64), 32 if t is np.float32 else 64
+        if prec == 64 and da.n_elem > 32_000:
+            continue  # by families in fixed point; extended precision takes long
+        want, bound = dense.apply(x64) if prec == 32 else dense.exact(x64), dense.smooth_bound(x64)
+        loops = [da.matvec_coef(one, _put(xt, p), precision=prec)[p]]
+        if prec == 32 or not da.compressLut:
+            loops.append(da.matvec(_put(xt, p), precision=prec)[p])
+        for got in loops:
+            assert (np.abs(got - want) <= roundings * unit * bound).all()
