@@ -331,8 +331,10 @@ int dg_mg_set_smoother(dg_mg mg, double omega, int nu_pre, int nu_post);
 /* The CG's own operator application q = A p when the V-cycle runs in FP32
  * (precision 32 of dg_mg_solve).  48 (the default) and 64: A p on the FP64
  * vectors, as dg_mg_matvec with 64 (meshes of 32,000 elements and more in
- * 64-bit fixed point with an exponent per family of siblings, its results as
- * exact as FP64's; GB300's FP64 pipe issues 2 multiply-adds per clock per SM).
+ * 64-bit fixed point with an exponent per family of siblings, families of
+ * uneven values in FP64: each row to 2^-44 of the sum of its terms' magnitudes
+ * or better, in norm closer than dense FP64 stencils; GB300's FP64 pipe issues 2
+ * multiply-adds per clock per SM).
  * 32: A p in FP32 (the FP32 element loop), and the recurrence residual
  * replaced by the FP64 residual b - A x whenever it has fallen by
  * reliable_delta since the last replacement, and before the stopping test

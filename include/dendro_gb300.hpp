@@ -566,8 +566,9 @@ class MultiGrid {
   }
   // load vector of a nodal field on level 0
   void rhs(const double *f, double *b) const { cxx::check(c_, dg_mg_rhs(c_, mg_, f, b, 0), "dg_mg_rhs"); }
-  // the CG's operator with an FP32 V-cycle: 48 fixed point (the default),
-  // 64 FP64, 32 FP32 with FP64 residual replacement (dg_mg_set_cg_operator)
+  // the CG's operator with an FP32 V-cycle: on the FP64 vectors (48, the
+  // default, or 64: one loop), 32 FP32 with FP64 residual replacement
+  // (dg_mg_set_cg_operator)
   void setCgOperator(int precision, double reliableDelta = 1e-3) {
     cxx::check(c_, dg_mg_set_cg_operator(mg_, precision, reliableDelta), "dg_mg_set_cg_operator");
   }
