@@ -586,8 +586,11 @@ inline size_t family_coef_smem(int max_run) {
 // form alone have no rows; they occur at the domain's corners in every solve.
 // The limit: at 2^-4, 2^-3, 2^-2 344, 360, 446 us on 1.1e7 elements, 9.2, 9.9, 11.9
 // ms for an FP64 solve of 5e5 points (9.2 without a limit).
-// Patches with values that are not finite or not within 2^-509 .. 2^511, or
-// factors beyond 2^+-400, take floating point, all of them.
+// Patches with more than FIX_ALONE such families, values that are not finite or not
+// within 2^-509 .. 2^511, or factors beyond 2^+-400, take floating point, all of
+// them.  1.1e7 elements in us with at most 8, 16, 32, 128 alone: x over 16 decades
+// 1,585, 1,580, 1,583, 2,992; 1 in 100 nodes 1e12 times larger 1,580, 1,377, 841, 783;
+// 1 in 1,000 546, 494, 491, 489; zero on one side 462, 396, 372, 372.
 // What bounds it: 344 us on 1.1e7 elements (DRAM traffic alone 50): 3,600
 // instructions per 32 families at 1.5 per clock per SM; warps wait for the
 // gathers (3.0 of 10.5 cycles per instruction), barriers (1.6) and
@@ -601,6 +604,7 @@ inline size_t family_coef_smem(int max_run) {
 constexpr int FIX_EXP = 10, FIX_BIAS = 511;
 constexpr long long FIX_EDGE = 1;  // a boundary column of the Dirichlet form
 constexpr uint32_t FIX_EVEN = 2;
+constexpr int FIX_ALONE = 32;  // most families of a patch that go alone
 constexpr uint32_t FIX_EMASK = (1u << FIX_EXP) - 1;
 
 __device__ __forceinline__ long long fix_pack(double v, bool &outside) {
@@ -802,11 +806,11 @@ __global__ void __launch_bounds__(FAM, 4)
     const bool fixed = emax > 1 && !alone;
     const uint32_t q = fixed ? emax + (uint32_t)k + 1024u : 0u;
     const uint32_t hi = __reduce_max_sync(0xffffffffu, q), lo = __reduce_min_sync(0xffffffffu, q ? q : 0xffffffffu);
-    const uint32_t apart = __ballot_sync(0xffffffffu, alone);
+    const uint32_t uneven = __ballot_sync(0xffffffffu, alone);
     if ((tid & 31) == 0) {
       atomicMax(&s_q[0], hi);
       atomicMin(&s_q[1], lo);
-      s_alone[tid >> 5] = apart;
+      s_alone[tid >> 5] = uneven;
     }
     if (fixed) {
       const int2 *d = ft + level * DTAB_STRIDE;
@@ -823,6 +827,9 @@ __global__ void __launch_bounds__(FAM, 4)
       lat_distribute(u, hang);
     }
     plain = __syncthreads_or(plain);
+    static_assert(FAM == 128, "four words of families");
+    const int apart = __popc(s_alone[0]) + __popc(s_alone[1]) + __popc(s_alone[2]) + __popc(s_alone[3]);
+    plain = plain || apart > FIX_ALONE;
     const uint32_t qmax = s_q[0], qmin = s_q[1];
     const bool even = qmax - qmin <= FIX_EVEN;
     if (!plain) {
@@ -853,8 +860,7 @@ __global__ void __launch_bounds__(FAM, 4)
         family_fp64(fam + p * 4 * FAM + tid, xd, yd, tab, 0.0625);
     }
     __syncthreads();
-    static_assert(FAM == 128, "four words of families");
-    const bool store = plain || !(s_alone[0] | s_alone[1] | s_alone[2] | s_alone[3]);
+    const bool store = plain || apart == 0;
 #pragma unroll 1
     for (int u = tid; u < nr; u += FAM) {
       const uint32_t r = prun[base + u], g = r & PRUN_NODE;
